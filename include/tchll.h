@@ -180,10 +180,10 @@ int tchll_get_count_hub(int32_t* out4 /* host */);
  * and a hybrid count's HLL pass on a second stream beside the exact pairs;
  * overlap 2 also moves an exact count's short-list pair kernel there, after
  * the core pass, beside the hub kernel; 0 runs everything on the caller's
- * stream (the second stream is joined before the call returns).  bank_sort != 0 orders each packed
- * list's keys by the shared-memory bank of their bitmap word (fewer bank
- * conflicts in the hub kernel, a slower core pass).  out4 receives the four
- * values.  Results are identical for every setting.  These kernels read
+ * stream (the second stream is joined before the call returns).  Packed
+ * lists hold their dense part, the core's most popular vertices, as bitmaps.
+ * bank_sort is kept and returned but has no effect (the lists once had a
+ * bank-ordered form).  out4 receives the four values.  Results are identical for every setting.  These kernels read
  * col_idx values as vertex indices: a value outside [0, n_nodes) is
  * reported as TCHLL_STATUS_BAD_KEY. */
 int tchll_set_count_core(int32_t bitmap_log2, int32_t overlap, int32_t packed, int32_t bank_sort);

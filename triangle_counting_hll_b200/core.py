@@ -307,9 +307,9 @@ def set_count_tuning(chunk: int = 256, slots_log2: int = 10, tiny: int = 16, blo
     of the 32-bit hub bitmap buffer (0: off); overlap: 0 one stream, 1 the
     hub core pass (and a hybrid's HLL pass) on a second stream beside the
     exact pairs, 2 also the short-list pair kernel there, beside the hub
-    kernel; packed: 16-bit hub probe lists when
-    the core has at most 131,070 vertices; bank_sort: packed lists ordered by
-    bitmap bank.  hll_row_cache_p / hll_lanes:
+    kernel; packed: 16-bit hub probe lists with
+    their dense part as bitmaps, when the core has at most 131,070 vertices;
+    bank_sort: kept, no effect.  hll_row_cache_p / hll_lanes:
     the HLL pass's one-pass threshold on p and lanes per edge (0: by p)."""
     L = load()
     cur = get_count_tuning()

@@ -726,8 +726,9 @@ struct HubParams {
     const int32_t* hy;  // y of each hub pair, grouped by x
     const int32_t* pcol;  // padded lists in core coordinates (core_pad_kernel) or null: raw lists
     const int32_t* cidx;  // core index of each vertex, -1 outside the core (with pcol)
-    const int32_t* n_core;  // device: core size C, vertex of core index kPlane (with pcol)
-    const int4* pl;         // packed lists per row: {first 16-byte unit, plane-0 units, all units, 0}
+    const int32_t* n_core;  // device: core size C (with pcol)
+    const int4* pl;         // packed lists per row (core_lists_kernel)
+    const uint4* pool;      // their bitmap units
     int packed;             // packed 16-bit lists when C <= kCore16Max
     const HubSeg* segs;
     const unsigned long long* n_segs;
@@ -744,7 +745,8 @@ struct HubParams {
 // lists the core (R-MAT scale 22: 108 K of 2.4 M vertices, because
 // orientation by (degree, id) puts every long list's members among the
 // highest-degree vertices).  The hub kernels work in core coordinates:
-//   * cidx[w] = rank of w among the core vertices (ascending id), else -1;
+//   * cidx[w] = rank of w among the core vertices, the most popular first
+//     (core_index_kernel), else -1;
 //   * each probe list is rewritten in core indices, a member outside the
 //     core becoming the sentinel C (the core size), which can never hit;
 //   * a table side's list becomes a C-bit bitmap in shared memory (13.5 KB
@@ -762,17 +764,29 @@ __device__ __forceinline__ int64_t pad_start(int32_t rs, int32_t y) {
     return (((int64_t)rs + 3) & ~(int64_t)3) + 8 * (int64_t)y;
 }
 
-// flag[w] = 1 for every w in N+(x) of every x with hub pairs: one warp per
-// hub segment (a segment names its x; the segments of one x are consecutive,
-// and only the first marks x's list).  Going by segments rather than by
-// vertex id keeps the warps balanced: hub vertices cluster at low ids in
-// R-MAT graphs.  Each lane has four list members in flight (the loop is
-// bound by the latency of the dependent flag reads, not by bandwidth).
-// Values outside [0, n_nodes) are reported, not stored.
+// The core, the w in N+(x) of the x with hub pairs, and how popular its
+// members are: a counted hub adds to cnt[w], the others set bit w of `bits`;
+// w is in the core when it has either.  Few hubs are all counted, of many
+// every kMarkStep-th (by id): the counts only order the core, where a sample
+// will do, and setting bits is cheaper than counting, except that with few
+// hubs all warps would queue to set the same words first.  One warp per hub
+// segment (a segment names its x; the segments of one x are
+// consecutive, and only the first marks x's list); going by segments rather
+// than by vertex id keeps the warps balanced, because hub vertices cluster at
+// low ids in R-MAT graphs.  Each lane has four list members in flight.  The
+// bits are read first, through L1 (they fit it, and the core's members
+// recur; a stale 0 just repeats the atomic), and each warp starts at another
+// place of its list: hub lists begin with the same few popular members, and
+// warps that all start there queue on the same L2 lines.  With an int flag
+// per vertex and every list walked from its start: 316 us on R-MAT 18
+// (edge factor 24), 367 us on R-MAT 22.  Values outside [0, n_nodes) are
+// reported, not stored.
+constexpr int64_t kMarkAll = 8192;
+constexpr int kMarkStep = 8;
 __global__ void core_mark_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int64_t nnz,
                                  const int32_t* __restrict__ col, const HubSeg* __restrict__ segs,
-                                 const unsigned long long* __restrict__ n_segs, int64_t max_segs, int32_t* flag,
-                                 tchll_count_result* result) {
+                                 const unsigned long long* __restrict__ n_segs, int64_t max_segs, uint32_t* bits,
+                                 int32_t* cnt, tchll_count_result* result) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -790,195 +804,329 @@ __global__ void core_mark_kernel(const int32_t* __restrict__ row_ptr, int64_t n_
             status |= ST_BAD_ROW;
             continue;
         }
-        for (int32_t i0 = s; i0 < e; i0 += 128) {
+        const bool counted = nseg <= kMarkAll || (uint32_t)x % kMarkStep == 0;
+        const uint32_t parts = ((uint32_t)(e - s) + 127u) >> 7;
+        uint32_t part = parts ? (uint32_t)sg % parts : 0;
+        for (uint32_t q = 0; q < parts; ++q) {
+            const int64_t i0 = (int64_t)s + 128 * (int64_t)part;
+            part = part + 1 < parts ? part + 1 : 0;
             int32_t w[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int32_t i = i0 + 32 * k + lane;
+                const int64_t i = i0 + 32 * k + lane;
                 w[k] = i < e ? __ldg(col + i) : -1;
                 if (i < e && (uint64_t)(uint32_t)w[k] >= (uint64_t)n_nodes) {
                     status |= ST_BAD_KEY;
                     w[k] = -1;
                 }
             }
-            // the core's members recur in many hub lists: read first, and
-            // store only a flag not yet seen set (a stale 0 read just
-            // repeats an idempotent store)
-            int32_t f[4];
+            if (counted) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) f[k] = w[k] >= 0 ? flag[w[k]] : 1;
+                for (int k = 0; k < 4; ++k)
+                    if (w[k] >= 0) atomicAdd(cnt + w[k], 1);
+                continue;
+            }
+            uint32_t f[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] = w[k] >= 0 ? bits[w[k] >> 5] : ~0u;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (f[k] == 0) flag[w[k]] = 1;
+                if (!((f[k] >> (w[k] & 31)) & 1u)) atomicOr(bits + (w[k] >> 5), 1u << (w[k] & 31));
         }
     }
     status = __reduce_or_sync(FULL, status);
     if (lane == 0 && status) atomicOr(&result->status, status);
 }
 
-// Packed probe lists hold a core index in 16 bits plus a plane: plane 0 the
-// indices below kPlane, plane 1 the others minus kPlane, each plane padded
-// with 0xFFFF.  In the bitmap, core index c sits at bit c (plane 0) or c + 1
-// (plane 1), so bit 65535 (plane 0's padding) and bit 131071 (plane 1's) are
-// never set; that works while C <= kCore16Max.
-constexpr int32_t kPlane = 65535;
-constexpr int32_t kCore16Max = 131070;
+// Core indices by falling popularity: a counting sort of the core vertices
+// by their count's leading four bits (256 buckets, most popular first; the
+// order inside a bucket is arbitrary, and no result depends on it).  Popular
+// members come first so that the low core indices, where the lists are
+// dense, can be held as bitmaps (core_lists_kernel).
+__device__ __forceinline__ int pop_bucket(const uint32_t* __restrict__ bits, const int32_t* cnt, int64_t w) {
+    int32_t c = cnt[w];
+    if (c == 0) {
+        if (!((__ldg(bits + (w >> 5)) >> (w & 31)) & 1u)) return -1;  // not in the core
+        c = 1;
+    }
+    const int e = 31 - __clz(c);
+    return 255 - (8 * e + (int)((((int64_t)c << 3) >> e) & 7));
+}
 
-// n_core[1] (set to -1 before) receives the vertex of core index kPlane.
-__global__ void core_index_kernel(int32_t* flag_cidx, const int32_t* __restrict__ pos, int64_t n_nodes,
-                                  int32_t* n_core) {
-    for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w <= n_nodes;
-         w += (int64_t)gridDim.x * blockDim.x) {
-        if (w == n_nodes) {
-            n_core[0] = __ldg(pos + n_nodes);
-        } else {
-            const bool f = flag_cidx[w] != 0;
-            const int32_t c = __ldg(pos + w);
-            flag_cidx[w] = f ? c : -1;
-            if (f && c == kPlane) n_core[1] = (int32_t)w;
-        }
+__global__ void __launch_bounds__(256) core_bucket_kernel(const uint32_t* __restrict__ bits,
+                                                          const int32_t* __restrict__ cnt, int64_t n_nodes,
+                                                          int32_t* hist) {
+    __shared__ int h[256];
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    for (int64_t w = blockIdx.x * 256ll + threadIdx.x; w < n_nodes; w += gridDim.x * 256ll) {
+        const int b = pop_bucket(bits, cnt, w);
+        if (b >= 0) atomicAdd(h + b, 1);
+    }
+    __syncthreads();
+    if (h[threadIdx.x]) atomicAdd(hist + threadIdx.x, h[threadIdx.x]);
+}
+
+// cnt_cidx[w]: count -> core index (-1 outside the core); n_core[0] = C.
+// A CTA takes a contiguous range of vertices and claims its share of every
+// bucket with one atomic (cursor: 256 zeroed words).
+__global__ void __launch_bounds__(256) core_index_kernel(const uint32_t* __restrict__ bits, int32_t* cnt_cidx,
+                                                         int64_t n_nodes,
+                                                         const int32_t* __restrict__ hist, int32_t* cursor,
+                                                         int32_t* n_core) {
+    __shared__ int h[256], part[8];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t per = (n_nodes + gridDim.x - 1) / gridDim.x;
+    const int64_t lo = blockIdx.x * per, hi = min(n_nodes, lo + per);
+    h[tid] = 0;
+    __syncthreads();
+    for (int64_t w = lo + tid; w < hi; w += 256) {
+        const int b = pop_bucket(bits, cnt_cidx, w);
+        if (b >= 0) atomicAdd(h + b, 1);
+    }
+    // exclusive scan of the 256 bucket sizes
+    const int mine = __ldg(hist + tid);
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) part[tid >> 5] = incl;
+    __syncthreads();
+    int before = 0;
+    for (int i = 0; i < (tid >> 5); ++i) before += part[i];
+    const int n_here = h[tid];
+    const int base = before + incl - mine + (n_here ? atomicAdd(cursor + tid, n_here) : 0);
+    if (blockIdx.x == 0 && tid == 255) n_core[0] = before + incl;
+    __syncthreads();
+    h[tid] = base;
+    __syncthreads();
+    for (int64_t w = lo + tid; w < hi; w += 256) {
+        const int b = pop_bucket(bits, cnt_cidx, w);
+        cnt_cidx[w] = b >= 0 ? atomicAdd(h + b, 1) : -1;
     }
 }
 
 // Packed probe lists (used when C <= kCore16Max; core_pad_kernel writes the
-// 32-bit ones otherwise): row y starts at uint16 index pad16_start(y), a
-// multiple of 8 (16 bytes); plane 0 (members below the vertex of core index
-// kPlane) takes lo_units 16-byte units, plane 1 the next ones; pl[y] =
-// {pad16_start(y) / 8, lo_units, all units, 0}, one 16-byte record so that
-// the hub kernel finds a pair's list with one load.  roundup8(row_ptr[y]) +
-// 24 y leaves room for both planes' padding (at most 7 each) of every row
-// before y.  Rows are sorted (as every CSR of the reference is), so the
-// planes split the row at one position P, found by an 8-way search down to
-// 64 members and a count of those; a member on the wrong side of P (an
-// unsorted row) or outside the core becomes padding and cannot match.
+// 32-bit ones otherwise).  A row is held as
+//   * a bitmap of the core indices below 128 B: B 16-byte units, unit b the
+//     indices [128 b, 128 b + 128) (from a pool, units claimed with one atomic
+//     per row; B = 0 when the pool is used up);
+//   * its other core indices as 16-bit keys in two planes, plane 0 the
+//     indices below kPlane, plane 1 the others minus kPlane, each plane padded
+//     to 16-byte units of 8 keys with 0xFFFF.  In the hub kernel's bitmap,
+//     core index c sits at bit c (plane 0) or c + 1 (plane 1), so bit 65535
+//     (plane 0's padding) and bit 131071 (plane 1's) are never set; that
+//     works while C <= kCore16Max.
+// Members outside the core are dropped: they cannot match.  Row y's keys
+// start at uint16 index pad16_start(y) = roundup8(row_ptr[y]) + 24 y, which
+// leaves room for both planes' padding (at most 7 each) of every row before
+// y; pl[y] = {pad16_start(y) / 8, plane-0 units, first bitmap unit,
+// B | plane-1 units << 8}, one 16-byte record, so that the hub kernel finds a
+// pair's list with one load.
+//
+// Why bitmaps: a key costs a random 4-byte shared load (3.8 wavefronts per
+// 32), a bitmap unit one conflict-free 16-byte one for 128 columns; ordered
+// by popularity, the low columns are dense enough for that on every skewed
+// graph (R-MAT 22: 58 M hub pairs probe 11.5 G keys = 1.47 G key units;
+// with bitmaps about 0.4 G bitmap + 0.7 G key units).  B is one of a few
+// sizes up to 32, chosen per row by kUnitCost per bitmap unit against kKeyCost per
+// unit of 8 keys.  The L1 pipe alone would put the ratio at 0.35, but the
+// list loads weigh in: hub kernel on R-MAT 22 with 8, 11, 14, 18, 24, 30 to 34:
+// 6.57, 6.31, 5.65, 5.36, 5.46, 5.47 ms (keys only: 7.29 ms).
+constexpr int32_t kPlane = 65535;
+constexpr int32_t kCore16Max = 131070;
+constexpr int kBmSteps = 8;
+constexpr int kBmMax = 32;  // units of the longest bitmap
+__device__ __forceinline__ constexpr int bm_units(int k) {  // the B a row chooses from (and 0)
+    return k < 4 ? 1 << k : (k & 1 ? 1 << (k / 2 + 2) : 3 << (k / 2));
+}
+static_assert(bm_units(3) == 8 && bm_units(4) == 12 && bm_units(5) == 16 && bm_units(6) == 24 && bm_units(7) == kBmMax);
+constexpr int kUnitCost = 18;   // hub kernel cost of a bitmap unit : of a key unit
+constexpr int kKeyCost = 34;
+constexpr int kStage = 512;     // core indices of a row staged in shared memory (longer rows gather twice)
+
 __device__ __forceinline__ int64_t pad16_start(int32_t rs, int32_t y) {
     return (((int64_t)rs + 7) & ~(int64_t)7) + 24 * (int64_t)y;
 }
 
-__device__ __forceinline__ uint32_t plane_key(const int32_t* __restrict__ col, const int32_t* __restrict__ cidx,
-                                              int64_t n_nodes, int32_t i, int plane, uint32_t& status) {
+// Core index of row member i, or -1 (outside the core, or not a vertex).
+__device__ __forceinline__ int32_t core_of(const int32_t* __restrict__ col, const int32_t* __restrict__ cidx,
+                                           int64_t n_nodes, int64_t i, uint32_t& status) {
     const int32_t w = __ldg(col + i);
     if ((uint64_t)(uint32_t)w >= (uint64_t)n_nodes) {
         status |= ST_BAD_KEY;
-        return 0xFFFFu;
+        return -1;
     }
-    const int32_t c = __ldg(cidx + w);
-    if (plane == 0) return (c >= 0 && c < kPlane) ? (uint32_t)c : 0xFFFFu;
-    return c >= kPlane ? (uint32_t)(c - kPlane) : 0xFFFFu;
+    return __ldg(cidx + w);
 }
 
-// By default the keys keep the row's order.  With bank_sort, within each
-// plane the keys are ordered by the shared-memory bank of their bitmap word
-// ((key >> 5) & 31; a list is a set, so order is free): the hub kernel deals
-// consecutive 8-key units to consecutive lanes, so one load instruction then
-// mostly touches distinct banks (R-MAT 21: 3.3 instead of 3.8 shared-memory
-// wavefronts per load, but the sort costs this pass more than the hub
-// kernel saves).  A counting sort per row and plane: 8 lanes count the 32
-// banks in shared memory, scan them and scatter the keys; the order inside a
-// bank is arbitrary; a plane of at most 8 keys is one unit and is not sorted.
-__global__ void __launch_bounds__(256) core_pad16_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes,
+// One row by a whole warp; stage and bits are the warp's shared memory.
+__device__ __forceinline__ void core_list_warp(const int32_t* __restrict__ col, const int32_t* __restrict__ cidx,
+                                               int64_t n_nodes, int32_t rs, int32_t d, int32_t y,
+                                               uint16_t* __restrict__ pcol16, int4* __restrict__ pl,
+                                               uint4* __restrict__ pool, int32_t pool_cap, int32_t* pool_used,
+                                               int32_t* stage, uint32_t* bits, uint32_t& status) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    int lt[kBmSteps], n_all = 0, n_hi = 0;
+#pragma unroll
+    for (int k = 0; k < kBmSteps; ++k) lt[k] = 0;
+    for (int32_t i0 = 0; i0 < d; i0 += 128) {
+        int32_t c[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int32_t i = i0 + 32 * t + lane;
+            c[t] = i < d ? core_of(col, cidx, n_nodes, (int64_t)rs + i, status) : -1;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int32_t i = i0 + 32 * t + lane;
+            if (i < kStage) stage[i] = c[t];
+            n_all += __popc(__ballot_sync(FULL, c[t] >= 0));
+            n_hi += __popc(__ballot_sync(FULL, c[t] >= kPlane));
+#pragma unroll
+            for (int k = 0; k < kBmSteps; ++k) lt[k] += __popc(__ballot_sync(FULL, (uint32_t)c[t] < 128u * bm_units(k)));
+        }
+    }
+    const int n_lo = n_all - n_hi, u_hi = (n_hi + 7) >> 3;
+    int B = 0, in_bits = 0, best = kKeyCost * ((n_lo + 7) >> 3);
+#pragma unroll
+    for (int k = 0; k < kBmSteps; ++k) {
+        const int cost = kUnitCost * bm_units(k) + kKeyCost * ((n_lo - lt[k] + 7) >> 3);
+        if (cost < best) {
+            best = cost;
+            B = bm_units(k);
+            in_bits = lt[k];
+        }
+    }
+    int32_t first = 0;
+    if (B) {
+        if (lane == 0) first = atomicAdd(pool_used, B);
+        first = __shfl_sync(FULL, first, 0);
+        if (first < 0 || first > pool_cap - B) B = 0;
+    }
+    uint16_t* out = pcol16 + pad16_start(rs, y);
+    while (true) {
+        if (B == 0) in_bits = 0;
+        const int keys_lo = n_lo - in_bits, u_lo = (keys_lo + 7) >> 3;
+        __syncwarp();
+        for (int i = lane; i < 4 * B; i += 32) bits[i] = 0u;
+        __syncwarp();
+        int p0 = 0, p1 = 8 * u_lo;
+        for (int32_t i0 = 0; i0 < d; i0 += 32) {
+            const int32_t i = i0 + lane;
+            int32_t c = -1;
+            if (i < d) c = i < kStage ? stage[i] : core_of(col, cidx, n_nodes, (int64_t)rs + i, status);
+            const bool in = (uint32_t)c < 128u * (uint32_t)B;
+            if (in) atomicOr(bits + (c >> 5), 1u << (c & 31));
+            const bool lo = c >= 0 && c < kPlane && !in, hi = c >= kPlane;
+            const unsigned mlo = __ballot_sync(FULL, lo), mhi = __ballot_sync(FULL, hi);
+            if (lo) out[p0 + __popc(mlo & lt_mask)] = (uint16_t)c;
+            if (hi) out[p1 + __popc(mhi & lt_mask)] = (uint16_t)(c - kPlane);
+            p0 += __popc(mlo);
+            p1 += __popc(mhi);
+        }
+        if (p0 + lane < 8 * u_lo) out[p0 + lane] = 0xFFFFu;
+        if (p1 + lane < 8 * (u_lo + u_hi)) out[p1 + lane] = 0xFFFFu;
+        __syncwarp();
+        int set = 0;
+        for (int i = lane; i < B; i += 32) {
+            const uint4 q = reinterpret_cast<const uint4*>(bits)[i];
+            pool[first + i] = q;
+            set += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
+        }
+        // a row that lists a member twice keeps both as keys
+        if (B && (int)__reduce_add_sync(FULL, (unsigned)set) != in_bits) {
+            B = 0;
+            continue;
+        }
+        if (u_hi >= (1 << 23)) {  // a row of over 2^26 repeated members
+            status |= ST_BAD_ROW;
+            if (lane == 0) pl[y] = make_int4(0, 0, 0, 0);
+        } else if (lane == 0) {
+            pl[y] = make_int4((int32_t)(pad16_start(rs, y) >> 3), u_lo, first, B | (u_hi << 8));
+        }
+        return;
+    }
+}
+
+// A warp claims eight rows at a time: rows of at least 32 members one by one
+// (core_list_warp), the others four at a time, eight lanes each, as keys only.
+__global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes,
                                                          int64_t nnz, const int32_t* __restrict__ col,
                                                          const int32_t* __restrict__ cidx,
                                                          const int32_t* __restrict__ n_core, int packed,
-                                                         int bank_sort, uint16_t* __restrict__ pcol16,
-                                                         int4* __restrict__ pl, tchll_count_result* result) {
-    __shared__ int s_cnt[32][32];  // per 8-lane group: bank counters, then cursors
-    const int32_t C = n_core[0];
-    if (!packed || C > kCore16Max) return;  // grid-uniform: the 32-bit lists apply
-    const int32_t wsplit = n_core[1];       // -1: no plane 1
-    const int lane = threadIdx.x & 31;
-    const int sub = threadIdx.x & 7;        // 8 lanes per row
-    const unsigned gmask = 0xFFu << (lane & 24);
-    int* cnt = s_cnt[threadIdx.x >> 3];
-    const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
-    const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 3;
+                                                         uint16_t* __restrict__ pcol16, int4* __restrict__ pl,
+                                                         uint4* __restrict__ pool, int32_t pool_cap,
+                                                         int32_t* pool_used, unsigned long long* row_ctr,
+                                                         const unsigned long long* __restrict__ n_segs,
+                                                         tchll_count_result* result) {
+    __shared__ int32_t s_stage[8][kStage];
+    __shared__ __align__(16) uint32_t s_bits[8][4 * kBmMax];
+    // grid-uniform: the 32-bit lists apply, or no hub pair will read a list
+    if (!packed || n_core[0] > kCore16Max || *n_segs == 0) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int sub = lane & 7, grp = lane >> 3;
     uint32_t status = 0;
-    for (int64_t y = g; y < n_nodes; y += ng) {
-        const int32_t rs = __ldg(row_ptr + y), re = __ldg(row_ptr + y + 1);
-        if (rs < 0 || re < rs || (int64_t)re > nnz) {
-            status |= ST_BAD_ROW;
-            if (sub == 0) pl[y] = make_int4(0, 0, 0, 0);
-            continue;
+    while (true) {
+        unsigned long long y0 = 0;
+        if (lane == 0) y0 = atomicAdd(row_ctr, 8ull);
+        y0 = __shfl_sync(FULL, y0, 0);
+        if (y0 >= (unsigned long long)n_nodes) break;
+        int32_t rs = 0, d = 0;
+        if (lane < 8 && (int64_t)y0 + lane < n_nodes) {
+            const int64_t y = (int64_t)y0 + lane;
+            const int32_t a = __ldg(row_ptr + y), b = __ldg(row_ptr + y + 1);
+            if (a < 0 || b < a || (int64_t)b > nnz) status |= ST_BAD_ROW;  // an empty list
+            else rs = a, d = b - a;
         }
-        const int32_t d = re - rs;
-        int32_t P = d;
-        if (wsplit >= 0) {  // P = first member >= wsplit, in [lo, hi]
-            int32_t lo = 0, hi = d;
-            while (hi - lo > 64) {  // group-uniform: 8 probes cut [lo, hi) into 9 parts
-                const int64_t len = hi - lo;
-                const bool lt = __ldg(col + rs + lo + (int32_t)(((sub + 1) * len) / 9)) < wsplit;
-                const int t = __popc((__ballot_sync(gmask, lt) >> (lane & 24)) & 0xFFu);
-                const int32_t nlo = t > 0 ? lo + (int32_t)((t * len) / 9) + 1 : lo;
-                hi = t < 8 ? lo + (int32_t)(((t + 1) * len) / 9) : hi;
-                lo = nlo;
-            }
-            int c = 0;  // hi - lo <= 64: eight independent loads per lane
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                const int32_t m = lo + sub + 8 * t;
-                if (m < hi) c += __ldg(col + rs + m) < wsplit;
-            }
-            c += __shfl_xor_sync(gmask, c, 1);
-            c += __shfl_xor_sync(gmask, c, 2);
-            c += __shfl_xor_sync(gmask, c, 4);
-            P = lo + c;
-        }
-        const int32_t lo_units = (P + 7) >> 3, units = lo_units + ((d - P + 7) >> 3);
-        const int64_t ps = pad16_start(rs, (int32_t)y);
-        const int4 rec = make_int4((int32_t)(ps >> 3), lo_units, units, 0);
-        if (!bank_sort) {  // list order: one 16-byte unit per lane
-            for (int32_t u = sub; u < units; u += 8) {
-                const int plane = u < lo_units ? 0 : 1;
-                const int32_t m0 = plane == 0 ? 8 * u : P + 8 * (u - lo_units);
-                const int32_t end = plane == 0 ? P : d;
-                uint32_t k[8];
+        for (int h = 0; h < 8; h += 4) {
+            const int32_t grs = __shfl_sync(FULL, rs, h + grp), gd = __shfl_sync(FULL, d, h + grp);
+            const int64_t y = (int64_t)y0 + h + grp;
+            const bool mine = gd < 32 && y < n_nodes;
+            int32_t c[4];
+            int n_lo = 0, n_hi = 0;
 #pragma unroll
-                for (int t = 0; t < 8; ++t)
-                    k[t] = (m0 + t < end) ? plane_key(col, cidx, n_nodes, rs + m0 + t, plane, status) : 0xFFFFu;
-                *reinterpret_cast<uint4*>(pcol16 + ps + 8 * u) =
-                    make_uint4(k[0] | (k[1] << 16), k[2] | (k[3] << 16), k[4] | (k[5] << 16), k[6] | (k[7] << 16));
+            for (int t = 0; t < 4; ++t) {
+                const int32_t i = 8 * t + sub;
+                c[t] = mine && i < gd ? core_of(col, cidx, n_nodes, (int64_t)grs + i, status) : -1;
             }
-            if (sub == 0) pl[y] = rec;
-            continue;
-        }
-        for (int plane = 0; plane < 2; ++plane) {
-            const int32_t m0 = plane ? P : 0, m1 = plane ? d : P;
-            if (m1 <= m0) continue;  // group-uniform
-            uint16_t* out = pcol16 + ps + (plane ? 8 * (int64_t)lo_units : 0);
-            if (m1 - m0 <= 8) {  // one unit: one lane probes all its keys, order is moot
-                out[sub] = m0 + sub < m1 ? (uint16_t)plane_key(col, cidx, n_nodes, rs + m0 + sub, plane, status)
-                                         : (uint16_t)0xFFFFu;
-                continue;
-            }
-            for (int b = sub; b < 32; b += 8) cnt[b] = 0;
-            __syncwarp(gmask);
-            for (int32_t m = m0 + sub; m < m1; m += 8)
-                atomicAdd(cnt + ((plane_key(col, cidx, n_nodes, rs + m, plane, status) >> 5) & 31u), 1);
-            __syncwarp(gmask);
-            // exclusive scan of the 32 counters, 4 per lane
-            const int c0 = cnt[4 * sub], c1 = cnt[4 * sub + 1], c2 = cnt[4 * sub + 2], c3 = cnt[4 * sub + 3];
-            int incl = c0 + c1 + c2 + c3;
+            unsigned mlo[4], mhi[4];
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                const int t = __shfl_up_sync(gmask, incl, o, 8);
-                if (sub >= o) incl += t;
+            for (int t = 0; t < 4; ++t) {
+                mlo[t] = (__ballot_sync(FULL, c[t] >= 0 && c[t] < kPlane) >> (8 * grp)) & 0xFFu;
+                mhi[t] = (__ballot_sync(FULL, c[t] >= kPlane) >> (8 * grp)) & 0xFFu;
+                n_lo += __popc(mlo[t]);
+                n_hi += __popc(mhi[t]);
             }
-            const int ex = incl - (c0 + c1 + c2 + c3);
-            __syncwarp(gmask);
-            cnt[4 * sub] = ex;
-            cnt[4 * sub + 1] = ex + c0;
-            cnt[4 * sub + 2] = ex + c0 + c1;
-            cnt[4 * sub + 3] = ex + c0 + c1 + c2;
-            __syncwarp(gmask);
-            for (int32_t m = m0 + sub; m < m1; m += 8) {
-                const uint32_t k = plane_key(col, cidx, n_nodes, rs + m, plane, status);
-                out[atomicAdd(cnt + ((k >> 5) & 31u), 1)] = (uint16_t)k;
+            if (!mine) continue;
+            const int u_lo = (n_lo + 7) >> 3, u_hi = (n_hi + 7) >> 3;
+            const int64_t ps = pad16_start(grs, (int32_t)y);
+            uint16_t* out = pcol16 + ps;
+            const unsigned below = (1u << sub) - 1u;
+            int p0 = 0, p1 = 8 * u_lo;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if ((mlo[t] >> sub) & 1u) out[p0 + __popc(mlo[t] & below)] = (uint16_t)c[t];
+                if ((mhi[t] >> sub) & 1u) out[p1 + __popc(mhi[t] & below)] = (uint16_t)(c[t] - kPlane);
+                p0 += __popc(mlo[t]);
+                p1 += __popc(mhi[t]);
             }
-            const int32_t nk = m1 - m0;
-            for (int32_t t = nk + sub; t < ((nk + 7) & ~7); t += 8) out[t] = 0xFFFFu;
-            __syncwarp(gmask);  // the counters are reused by the next plane / row
+            if (p0 + sub < 8 * u_lo) out[p0 + sub] = 0xFFFFu;
+            if (p1 + sub < 8 * (u_lo + u_hi)) out[p1 + sub] = 0xFFFFu;
+            if (sub == 0) pl[y] = make_int4((int32_t)(ps >> 3), u_lo, 0, u_hi << 8);
         }
-        if (sub == 0) pl[y] = rec;
+        unsigned big = __ballot_sync(FULL, d >= 32);
+        while (big) {
+            const int j = __ffs(big) - 1;
+            big &= big - 1;
+            core_list_warp(col, cidx, n_nodes, __shfl_sync(FULL, rs, j), __shfl_sync(FULL, d, j),
+                           (int32_t)(y0 + j), pcol16, pl, pool, pool_cap, pool_used, s_stage[wid], s_bits[wid],
+                           status);
+        }
     }
     status = __reduce_or_sync(FULL, status);
     if (lane == 0 && status) atomicOr(&result->status, status);
@@ -995,7 +1143,8 @@ __global__ void core_pad_kernel(const int32_t* __restrict__ row_ptr, int64_t n_n
                                 const int32_t* __restrict__ n_core, int packed, int32_t* __restrict__ pcol,
                                 tchll_count_result* result) {
     const int32_t C = n_core[0];
-    if (packed && C <= kCore16Max) return;  // grid-uniform: core_pad16_kernel writes the lists
+    // grid-uniform: core_lists_kernel writes the lists, or no pair reads one
+    if ((packed && C <= kCore16Max) || C == 0) return;
     const int sub = threadIdx.x & 7;
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
     const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 3;
@@ -1399,24 +1548,38 @@ __global__ void __launch_bounds__(256, 6) hub_bitmap_kernel(const HubParams H) {
     }
 }
 
-// hub_bitmap_kernel over packed probe lists (C <= kCore16Max): 8 keys per
-// 16-byte unit, so the probe lists, which all pairs read from L2 or HBM, take
-// half the bytes.  The bitmap has 65,536 bits (C <= 65535) or 131,072 bits
-// (16 KB of shared memory); a unit's plane (the bitmap's half) follows from
-// its position in the list: units at or past the list's plane-0 units are
-// plane 1.  The bitmap is built from x's own packed list (16-byte loads of 8
-// keys; x's members are the core's by construction, so no member can miss
-// and there is no binary-search fallback).  Otherwise as hub_bitmap_kernel.
+// hub_bitmap_kernel over packed lists (core_lists_kernel; C <= kCore16Max):
+// a list is B bitmap units of 128 columns and units of 8 16-bit keys.  The
+// CTA's bitmap of N+(x) has 65,536 bits (C <= 65535) or 131,072 bits (16 KB of
+// shared memory) and is set from x's own list (16-byte loads; x's members
+// are the core's by construction, so no member can miss and there is no
+// binary-search fallback).  A round's lists are walked as two flattened
+// streams, so that no warp mixes the two kinds: the bitmap units (one
+// 16-byte list load, one 16-byte shared load of the same columns, four
+// AND + popc; consecutive lanes read consecutive units, so the shared load is
+// conflict-free), then the key units (eight random 4-byte shared loads; a
+// unit's plane, the bitmap's half, follows from its position in the list).
+// A lane finds its unit's list as in hub_bitmap_kernel; the lists' bases sit
+// in a shared-memory slot per warp.  Bound by the L1 data pipe (81% busy on
+// R-MAT 21, issue 65%): R-MAT 18 / 20 / 22 249 / 1189 / 7291 us with key lists
+// alone, 140 / 720 / 5270 us here.
+constexpr int kHub16Threads = 128;
 template <int UNR>
-__global__ void __launch_bounds__(256, 8) hub_bitmap16_kernel(const HubParams H) {
+__global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitmap16_kernel(const HubParams H) {
     extern __shared__ __align__(16) uint32_t bm[];  // 4096 words
     __shared__ HubSeg s_seg;
     __shared__ int s_round;
+    __shared__ int2 s_list[kHub16Threads / 32][32];
     const int C = H.n_core[0];
     if (!H.packed || C > kCore16Max) return;  // grid-uniform: a 32-bit kernel counts
     const int tid = threadIdx.x, lane = tid & 31;
     const unsigned lane_le = (2u << lane) - 1u;
-    const int nw4 = C > kPlane ? 1024 : 512;  // uint4 words: 131,072 or 65,536 bits
+    int2* lst = s_list[tid >> 5];
+    uint4* bm4 = reinterpret_cast<uint4*>(bm);
+    // uint4 words that can hold a set bit (core index c: bit c or c + 1); the
+    // padding's words stay clear
+    const int nw4 = (C >> 7) + 1;
+    if (tid < 2) bm4[512 * tid + 511] = make_uint4(0u, 0u, 0u, 0u);
     const uint4* __restrict__ pq = reinterpret_cast<const uint4*>(H.pcol);
     const int64_t nseg = min((int64_t)*H.n_segs, H.max_segs);
     uint64_t acc = 0;
@@ -1433,17 +1596,18 @@ __global__ void __launch_bounds__(256, 8) hub_bitmap16_kernel(const HubParams H)
             }
             s_round = 0;
         }
-        for (int i = tid; i < nw4; i += blockDim.x) reinterpret_cast<uint4*>(bm)[i] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = tid; i < nw4; i += blockDim.x) bm4[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
         const HubSeg sg = s_seg;
         if (sg.x < 0) break;
         if (tid == 0) n_pairs += sg.len;
         {
-            // N+(x) from x's own packed list (x's members are the core's by
-            // construction): 8 keys per 16-byte load, padding skipped;
-            // plane-1 key k is core index k + kPlane, bit k + kPlane + 1
-            const int4 xr = H.pl[sg.x];
-            for (int i = tid; i < xr.z; i += blockDim.x) {
+            // bitmap units are whole words of their own; plane-1 key k is
+            // core index k + kPlane, bit k + kPlane + 1
+            const int4 xr = __ldg(H.pl + sg.x);
+            const int xb = xr.w & 0xFF, xk = xr.y + (xr.w >> 8);
+            for (int i = tid; i < xb; i += blockDim.x) bm4[i] = __ldg(H.pool + xr.z + i);
+            for (int i = tid; i < xk; i += blockDim.x) {
                 const uint4 q = __ldg(pq + xr.x + i);
                 const uint32_t hb = i >= xr.y ? 65536u : 0u;
                 const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
@@ -1455,80 +1619,82 @@ __global__ void __launch_bounds__(256, 8) hub_bitmap16_kernel(const HubParams H)
             }
         }
         __syncthreads();
-        int rsz = (sg.len + 15) >> 4;
+        constexpr int kShare = kHub16Threads / 16;  // two rounds per warp
+        int rsz = (sg.len + kShare - 1) / kShare;
         rsz = rsz < 4 ? 4 : (rsz > 32 ? 32 : rsz);
         while (true) {
             int r = 0;
             if (lane == 0) r = atomicAdd(&s_round, rsz);
             r = __shfl_sync(FULL, r, 0);
             if (r >= sg.len) break;
-            const int np = min(rsz, sg.len - r);
-            int32_t q0 = 0, nq = 0, lo = 0;
-            if (lane < np) {
-                const int4 u = H.pl[__ldg(H.hy + sg.start + r + lane)];
-                q0 = u.x;
-                lo = u.y;
-                nq = u.z;
-            }
-            const unsigned ne = __ballot_sync(FULL, nq > 0);
-            const int k = __popc(ne);
-            const int src = lane < k ? (int)__fns(ne, 0, lane + 1) : lane;
-            const int c_q0 = __shfl_sync(FULL, q0, src);
-            int c_nq = __shfl_sync(FULL, nq, src);
-            const int c_lo = __shfl_sync(FULL, lo, src);
-            if (lane >= k) c_nq = 0;
-            int incl = c_nq;
+            int4 rec = make_int4(0, 0, 0, 0);
+            if (lane < min(rsz, sg.len - r)) rec = __ldg(H.pl + __ldg(H.hy + sg.start + r + lane));
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int excl = incl - c_nq;
-            const int W = __shfl_sync(FULL, incl, 31);
-            const int qb = c_q0 - excl;   // unit of stream position t in list j: qb[j] + t
-            const int thr = excl + c_lo;  // stream positions >= thr[j] are list j's plane 1
-            const bool starts = lane < k;
-            int S = 0;
-            for (int T0 = 0; T0 < W; T0 += 32 * UNR) {
-                int qd[UNR], hw[UNR];
+            for (int kind = 0; kind < 2; ++kind) {  // 0: bitmap units, 1: key units
+                const int nu = kind == 0 ? (rec.w & 0xFF) : rec.y + (rec.w >> 8);
+                int incl = nu;
 #pragma unroll
-                for (int i = 0; i < UNR; ++i) {
-                    const int Ti = T0 + 32 * i;
-                    qd[i] = -1;
-                    hw[i] = 0;
-                    if (Ti < W) {  // warp-uniform
-                        const unsigned d = (unsigned)(excl - Ti);
-                        const unsigned B = __reduce_or_sync(FULL, (starts && d < 32u) ? (1u << d) : 0u);
-                        const int j = (S + __popc(B & lane_le) - 1) & 31;
-                        S += __popc(B);
-                        const int my_qb = __shfl_sync(FULL, qb, j);
-                        const int my_thr = __shfl_sync(FULL, thr, j);
-                        const int t = Ti + lane;
-                        if (t < W) {
-                            qd[i] = my_qb + t;
-                            hw[i] = t >= my_thr ? 2048 : 0;  // plane 1: the bitmap's upper half
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= o) incl += t;
+                }
+                const int W = __shfl_sync(FULL, incl, 31);
+                if (W == 0) continue;
+                const int excl = incl - nu;
+                // non-empty lists, in order: {unit of stream position 0, the
+                // position of its first unit / of its first plane-1 unit}
+                const unsigned ne = __ballot_sync(FULL, nu > 0);
+                __syncwarp();
+                if (nu > 0)
+                    lst[__popc(ne & (lane_le >> 1))] = make_int2((kind == 0 ? rec.z : rec.x) - excl,
+                                                                 kind == 0 ? excl : excl + rec.y);
+                __syncwarp();
+                int S = -1;
+                for (int T0 = 0; T0 < W; T0 += 32 * UNR) {
+                    uint4 q[UNR];
+                    int at[UNR];
+#pragma unroll
+                    for (int i = 0; i < UNR; ++i) {
+                        const int Ti = T0 + 32 * i, t = Ti + lane;
+                        // padding keys (bit 65535, never set) / empty bitmap units
+                        q[i] = kind == 0 ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(~0u, ~0u, ~0u, ~0u);
+                        at[i] = 0;
+                        if (Ti < W) {  // warp-uniform
+                            const unsigned d = (unsigned)(excl - Ti);
+                            const unsigned B = __reduce_or_sync(FULL, (nu > 0 && d < 32u) ? (1u << d) : 0u);
+                            const int2 l = lst[(S + __popc(B & lane_le)) & 31];
+                            S += __popc(B);
+                            if (t < W) {
+                                q[i] = __ldcg((kind == 0 ? H.pool : pq) + (l.x + t));  // no reuse in L1
+                                // the unit's columns / plane 1: the bitmap's upper half
+                                at[i] = kind == 0 ? t - l.y : (t >= l.y ? 8192 : 0);
+                            }
                         }
                     }
-                }
-                uint4 q[UNR];
+                    uint32_t c = 0;
 #pragma unroll
-                for (int i = 0; i < UNR; ++i) {
-                    q[i] = make_uint4(~0u, ~0u, ~0u, ~0u);  // padding keys: bit 65535, never set
-                    if (qd[i] >= 0) q[i] = __ldg(pq + qd[i]);
-                }
-                uint32_t c = 0;
+                    for (int i = 0; i < UNR; ++i) {
+                        if (i > 0 && T0 + 32 * i >= W) break;  // warp-uniform
+                        if (kind == 0) {
+                            const uint4 b = bm4[at[i]];
+                            c += __popc(q[i].x & b.x) + __popc(q[i].y & b.y) + __popc(q[i].z & b.z) +
+                                 __popc(q[i].w & b.w);
+                        } else {
+                            // byte offset of the key's word: (key >> 5) * 4, plus the plane's 8 KB
+                            const char* b = reinterpret_cast<const char*>(bm);
+                            const uint32_t pl = (uint32_t)at[i];
+                            const uint32_t w4[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
 #pragma unroll
-                for (int i = 0; i < UNR; ++i) {
-                    const uint32_t* b = bm + hw[i];
-                    const uint32_t w4[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        const uint32_t w = w4[t];
-                        c += __funnelshift_r(b[(w >> 5) & 0x7FFu], 0u, w) & 1u;
-                        c += __funnelshift_r(b[w >> 21], 0u, w >> 16) & 1u;
+                            for (int t = 0; t < 4; ++t) {
+                                const uint32_t w = w4[t];
+                                const uint32_t lo = *reinterpret_cast<const uint32_t*>(b + (((w >> 3) & 0x1FFCu) | pl));
+                                const uint32_t hi = *reinterpret_cast<const uint32_t*>(b + (((w >> 19) & 0x1FFCu) | pl));
+                                c += (__funnelshift_r(lo, 0u, w) & 1u) + (__funnelshift_r(hi, 0u, w >> 16) & 1u);
+                            }
+                        }
                     }
+                    acc += c;
                 }
-                acc += c;
             }
         }
         if (H.batched) {  // this segment's totals belong to its graph
@@ -1990,7 +2156,7 @@ struct Tuning {
     int bitmap_lg = 15;     // hub bitmap buffer: 2^15 bytes = 262,144 core vertices (0: hash tables only)
     int overlap = 1;        // side stream: 1 the hub core pass (+ the hybrid HLL pass); 2 also the short-list pairs
     int packed = 1;         // hub probe lists as 16-bit core indices when the core allows
-    int bank_sort = 0;      // packed lists ordered by bitmap bank within each plane
+    int bank_sort = 0;      // kept for its setter and getter: no effect
     int hll_row_cache_p = 0;   // HLL pass: keep u's register row in registers for p <= this (0: never)
     int hll_lanes = 0;      // HLL pass: lanes per edge (0: chosen by p)
 };
@@ -2110,10 +2276,12 @@ struct CountWs {
     int64_t max_segs;
     int32_t* pcol;            // padded lists in core coordinates for the hub kernels, pcap entries (null: not carved)
     int64_t pcap;
-    int32_t* cflag;           // n_nodes + 1: core flags, then core indices (with pcol)
-    int32_t* cpos;            // n_nodes + 1: scan of the flags (with pcol)
-    int32_t* ncore;           // core size, vertex of core index kPlane (with pcol)
-    int4* pl;                 // n_nodes: packed lists' {first unit, plane-0 units, all units, 0} (with pcol)
+    int32_t* cflag;           // n_nodes + 1: popularity counts, then core indices (with pcol)
+    uint32_t* cbits;          // (n_nodes + 31) / 32 + 1: core membership (with pcol)
+    int32_t* ncore;           // kCoreWords words: see launch_core_pass (with pcol)
+    int4* pl;                 // n_nodes: packed lists' records (with pcol)
+    uint4* pool;              // pool_cap bitmap units (with pcol)
+    int64_t pool_cap;
     void* tmp;
     size_t tmp_bytes;
 };
@@ -2127,6 +2295,11 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
     const int64_t w16 = (nnz + 24 * (n_nodes + 1) + 24 + 1) / 2 + 4;
     return w32 > w16 ? w32 : w16;
 }
+
+// The hub core pass's small arrays: [0] core size, [1] pool units claimed,
+// [2..3] the list kernel's row counter (64 bits), [4 ..) popularity buckets'
+// sizes and cursors (256 each).  Cleared together.
+constexpr int kCoreWords = 4 + 2 * 256;
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
@@ -2148,9 +2321,11 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     W.pcap = pad ? pad_capacity(n_nodes, (int64_t)E) : 0;
     W.pcol = pad ? cv.take<int32_t>((size_t)W.pcap) : nullptr;
     W.cflag = pad ? cv.take<int32_t>(N) : nullptr;
-    W.cpos = pad ? cv.take<int32_t>(N) : nullptr;
-    W.ncore = pad ? cv.take<int32_t>(4) : nullptr;
+    W.cbits = pad ? cv.take<uint32_t>(N / 32 + 1) : nullptr;
+    W.ncore = pad ? cv.take<int32_t>(kCoreWords) : nullptr;
     W.pl = pad ? cv.take<int4>(N) : nullptr;
+    W.pool_cap = pad ? (int64_t)(E / 16) + 1024 : 0;
+    W.pool = pad ? cv.take<uint4>((size_t)W.pool_cap) : nullptr;
     W.tmp_bytes = tb;
     W.tmp = cv.take<char>(tb);
     if (need) *need = cv.off;
@@ -2359,19 +2534,24 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
     }
     const int64_t N = P.n_nodes + 1;
     TCHLL_CUDA(cudaMemsetAsync(W.cflag, 0, sizeof(int32_t) * N, st));
+    TCHLL_CUDA(cudaMemsetAsync(W.cbits, 0, sizeof(uint32_t) * (N / 32 + 1), st));
+    TCHLL_CUDA(cudaMemsetAsync(W.ncore, 0, sizeof(int32_t) * kCoreWords, st));
     core_mark_kernel<<<sm_count() * 8, 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.segs, W.ctr + 2,
-                                                      W.max_segs, W.cflag, P.result);
+                                                      W.max_segs, W.cbits, W.cflag, P.result);
     TCHLL_CHECK_LAUNCH("core_mark_kernel");
-    size_t tb = W.tmp_bytes;
-    TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(W.tmp, tb, W.cflag, W.cpos, (int)N, st));
-    count_launch();
-    TCHLL_CUDA(cudaMemsetAsync(W.ncore + 1, 0xFF, sizeof(int32_t), st));
-    core_index_kernel<<<grid_rows(N, 256), 256, 0, st>>>(W.cflag, W.cpos, P.n_nodes, W.ncore);
+    int64_t gv = (P.n_nodes + 1023) / 1024;
+    gv = gv < 1 ? 1 : (gv > 4 * (int64_t)sm_count() ? 4 * (int64_t)sm_count() : gv);
+    core_bucket_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4);
+    TCHLL_CHECK_LAUNCH("core_bucket_kernel");
+    core_index_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4, W.ncore + 4 + 256, W.ncore);
     TCHLL_CHECK_LAUNCH("core_index_kernel");
-    core_pad16_kernel<<<grid_rows(P.n_nodes, 32), 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag,
-                                                                W.ncore, T.packed, T.bank_sort,
-                                                                reinterpret_cast<uint16_t*>(W.pcol), W.pl, P.result);
-    TCHLL_CHECK_LAUNCH("core_pad16_kernel");
+    int64_t gl = (P.n_nodes + 63) / 64;
+    gl = gl < 1 ? 1 : (gl > 6 * (int64_t)sm_count() ? 6 * (int64_t)sm_count() : gl);
+    core_lists_kernel<<<(int)gl, 256, 0, st>>>(
+        P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag, W.ncore, T.packed, reinterpret_cast<uint16_t*>(W.pcol), W.pl,
+        W.pool, (int32_t)(W.pool_cap < INT32_MAX / 2 ? W.pool_cap : INT32_MAX / 2), W.ncore + 1,
+        reinterpret_cast<unsigned long long*>(W.ncore + 2), W.ctr + 2, P.result);
+    TCHLL_CHECK_LAUNCH("core_lists_kernel");
     core_pad_kernel<<<grid_rows(P.n_nodes, 32), 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag,
                                                               W.ncore, T.packed, W.pcol, P.result);
     TCHLL_CHECK_LAUNCH("core_pad_kernel");
@@ -2405,6 +2585,7 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
         H.cidx = W.cflag;
         H.n_core = W.ncore;
         H.pl = W.pl;
+        H.pool = W.pool;
         H.packed = T.packed;
     }
     if (ps.active()) cudaEventRecord(g_phase.hub_ev[2], st);
@@ -2416,10 +2597,10 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
                              "cudaFuncSetAttribute(hub_bitmap16_kernel)", true);
         if (rc) return rc;
         int bps = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, 256, smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kHub16Threads, smem);
         if (e != cudaSuccess) return cuda_status(e, "occupancy(hub_bitmap16_kernel)");
         if (bps < 1) bps = 1;
-        kern<<<sm_count() * bps, 256, smem, st>>>(H);
+        kern<<<sm_count() * bps, kHub16Threads, smem, st>>>(H);
         TCHLL_CHECK_LAUNCH("hub_bitmap16_kernel");
     }
     if (pad && T.bitmap_lg > 0) {
