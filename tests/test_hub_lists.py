@@ -25,10 +25,18 @@ def _csr(rng, n, lens, skew):
     return row_ptr, np.concatenate(rows).astype(np.int32)
 
 
-def _gpu(row_ptr, col, eu, ev):
+def _gpu(row_ptr, col, eu, ev, **tuning):
+    """The count with the edges regrouped, which small graphs do not choose
+    by themselves (pairs=2)."""
     import torch
+    from triangle_counting_hll_b200 import core
     from triangle_counting_hll_b200.gpu_hybrid import gpu_exact_triangle_count
-    return gpu_exact_triangle_count(*(torch.from_numpy(a).cuda() for a in (row_ptr, col, eu, ev)))[0]
+    base = core.get_count_tuning()
+    try:
+        core.set_count_tuning(**dict(base, pairs=2, **tuning))
+        return gpu_exact_triangle_count(*(torch.from_numpy(a).cuda() for a in (row_ptr, col, eu, ev)))[0]
+    finally:
+        core.set_count_tuning(**base)
 
 
 # core sizes: one bitmap word, one plane, two planes, beyond the packed lists
@@ -41,7 +49,9 @@ def test_list_forms(tchll, oracle, n, hubs, skew):
     lens = edge * 3 + [int(x) for x in rng.integers(129, min(n // 2, 900), hubs)] + long
     row_ptr, col = _csr(rng, n, lens, skew)
     eu, ev = (rng.integers(0, len(lens), 60000).astype(np.int32) for _ in range(2))
-    assert _gpu(row_ptr, col, eu, ev) == oracle.exact_count(row_ptr, col, eu, ev)
+    ref = oracle.exact_count(row_ptr, col, eu, ev)
+    for tuning in ({}, {"packed": False}, {"packed": False, "bitmap_lg": 0}, {"overlap": 0}, {"overlap": 2}):
+        assert _gpu(row_ptr, col, eu, ev, **tuning) == ref, tuning
 
 
 def test_repeated_members_stay_keys(tchll):

@@ -294,13 +294,15 @@ def hybrid_count_compact_tensors(row_ptr, col_idx, edge_u, edge_v, degrees, rows
 
 
 def set_count_tuning(chunk: int = 256, slots_log2: int = 10, tiny: int = 16, blocks_per_sm: int = 0,
-                     warps: Optional[int] = None, pairs: Optional[bool] = None,
+                     warps: Optional[int] = None, pairs: Optional[int] = None,
                      sparse: Optional[bool] = None, hub: Optional[int] = None, hub_seg: Optional[int] = None,
                      hub_lg: Optional[int] = None, hub_unroll: Optional[int] = None,
                      bitmap_lg: Optional[int] = None, overlap: Optional[int] = None,
                      packed: Optional[bool] = None, bank_sort: Optional[bool] = None,
                      hll_row_cache_p: Optional[int] = None, hll_lanes: Optional[int] = None) -> None:
     """Launch shape of the counting kernels (results do not depend on it).
+    pairs: 0 edges as given, 1 regrouped by the longer list when the graph is
+    large enough for it to pay, 2 regrouped whatever its size.
     hub / hub_seg / hub_lg / hub_unroll: threshold on d+(x) above which a pair
     goes to the CTA-shared table kernels (0: off), pairs per work unit, log2
     hash-table slots, probe loads in flight per lane.  bitmap_lg: log2 bytes
@@ -325,7 +327,7 @@ def set_count_tuning(chunk: int = 256, slots_log2: int = 10, tiny: int = 16, blo
                                 int(cur["hub_unroll"] if hub_unroll is None else hub_unroll)))
     check(L.tchll_set_count_table(int(cur["sparse"] if sparse is None else bool(sparse))))
     w = cur["warps"] if warps is None else int(warps)
-    pr = cur["pairs"] if pairs is None else int(bool(pairs))
+    pr = cur["pairs"] if pairs is None else int(pairs)
     # one warp fits every table size, so go through it to reach any valid shape
     check(L.tchll_set_count_shape(1, pr))
     check(L.tchll_set_count_tuning(int(chunk), int(slots_log2), int(tiny), int(blocks_per_sm)))

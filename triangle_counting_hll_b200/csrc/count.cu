@@ -81,7 +81,8 @@ struct CountParams {
     double* pe_s_cl;      // per-edge HLL clamped support (details)
     uint8_t* pe_method;   // per-edge 0 exact / 1 hll (details)
     tchll_count_result* result;
-    unsigned long long* work;
+    unsigned long long* work;  // chunks are claimed here (null: dealt to the warps in turn)
+    int check_ids;  // validate every row first
     int chunk;
     int slots_log2;  // per-warp table capacity (log2 slots)
     int tiny;        // lane-local merge when |N+x| + |N+y| <= tiny
@@ -179,6 +180,30 @@ __device__ __forceinline__ bool load_edge(const CountParams& P, int64_t e, int32
     return true;
 }
 
+// Every row's extent and every listed neighbour id, by the whole grid: what
+// the hub core's passes check as they read the rows, for the calls that do
+// not need them.  Well-formed rows cover col[row_ptr[0] .. row_ptr[n_nodes]).
+__device__ __forceinline__ void validate_rows(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int64_t nnz,
+                                              const int32_t* __restrict__ col, uint32_t& status) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = t0; r < n_nodes; r += step) {
+        const int32_t a = __ldg(row_ptr + r), b = __ldg(row_ptr + r + 1);
+        if (a < 0 || b < a || (int64_t)b > nnz) status |= ST_BAD_ROW;
+    }
+    const int64_t lo = __ldg(row_ptr), hi = __ldg(row_ptr + n_nodes);
+    if (lo < 0 || hi > nnz) return;
+    const int64_t l4 = min((lo + 3) & ~(int64_t)3, hi), h4 = max(hi & ~(int64_t)3, l4);
+    const uint32_t n = (uint32_t)n_nodes;
+    bool bad = false;
+    for (int64_t q = (l4 >> 2) + t0; q < h4 >> 2; q += step) {  // col is 16-byte aligned
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(col) + q);
+        bad |= v.x >= n || v.y >= n || v.z >= n || v.w >= n;
+    }
+    if (lo + t0 < l4) bad |= (uint32_t)__ldg(col + lo + t0) >= n;
+    if (h4 + t0 < hi) bad |= (uint32_t)__ldg(col + h4 + t0) >= n;
+    if (bad) status |= ST_BAD_KEY;
+}
+
 // Hybrid routing (src/hybrid.py:107-115): wants = min(deg) >= gamma,
 // both = both endpoints have a sketch.  Returns false on a bad slot.
 __device__ __forceinline__ bool route(const CountParams& P, int32_t u, int32_t v, int32_t& du, int32_t& dv,
@@ -247,6 +272,21 @@ __device__ __forceinline__ void lane_runs(int32_t key, int lane, int& head_lane,
     run_len = (after ? __ffs(after) - 1 : 32) - head_lane;
 }
 
+// Appends the lanes' HLL-routed edges to the list, one atomic per warp.
+__device__ __forceinline__ void append_hll(const CountParams& P, bool hll, int32_t u, int32_t v, int lane) {
+    const unsigned bal = __ballot_sync(FULL, hll);
+    if (bal) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(P.hll_n, (unsigned long long)__popc(bal));
+        base = __shfl_sync(FULL, base, 0);
+        if (hll) {
+            const unsigned long long pos = base + __popc(bal & ((1u << lane) - 1u));
+            P.hll_u[pos] = u;
+            P.hll_v[pos] = v;
+        }
+    }
+}
+
 // Grid-stride loop that whole warps enter and leave together: e may reach
 // past n in the last pass; the body tests it.
 #define WARP_EDGE_LOOP(e, n)                                                                   \
@@ -284,20 +324,7 @@ __global__ void pair_hist_kernel(const CountParams P, int32_t* cnt) {
             lane_runs(x, lane, head, len);
             if (counted && lane == head) atomicAdd(cnt + x, len);
         }
-        if (HYB && P.hll_u) {
-            // warp-aggregated append of the HLL-routed edges
-            const unsigned bal = __ballot_sync(FULL, hll);
-            if (bal) {
-                unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(P.hll_n, (unsigned long long)__popc(bal));
-                base = __shfl_sync(FULL, base, 0);
-                if (hll) {
-                    const unsigned long long pos = base + __popc(bal & ((1u << lane) - 1u));
-                    P.hll_u[pos] = u;
-                    P.hll_v[pos] = v;
-                }
-            }
-        }
+        if (HYB && P.hll_u) append_hll(P, hll, u, v, lane);
     }
     if (status) atomicOr(&P.result->status, status);
     if (HYB && P.hll_u && fallback) atomicAdd((unsigned long long*)&P.result->n_fallback, fallback);
@@ -414,6 +441,9 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     int cur_lg = 5;  // log2 slots of the current table
     const int m = 1 << P.p;
 
+    if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col_idx, status);
+    const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+    unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + wid;
     while (true) {
         unsigned long long e0 = 0;
         int64_t e1;
@@ -427,8 +457,13 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
             e1 = (int64_t)e0 + __ldg(P.chunk_len + ci);
             gcur = __ldg(P.chunk_graph + ci);
         } else {
-            if (lane == 0) e0 = atomicAdd(P.work, (unsigned long long)P.chunk);
-            e0 = __shfl_sync(FULL, e0, 0);
+            if (P.work) {
+                if (lane == 0) e0 = atomicAdd(P.work, (unsigned long long)P.chunk);
+                e0 = __shfl_sync(FULL, e0, 0);
+            } else {
+                e0 = turn * (unsigned long long)P.chunk;
+                turn += n_warps;
+            }
             if (e0 >= (unsigned long long)n_edges) break;
             e1 = min((int64_t)e0 + P.chunk, n_edges);
         }
@@ -453,8 +488,10 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
                 is_hll = valid && wants && both;
                 // n_fallback: counted by the fused launch and, in split mode,
                 // by the HLL launch (which sees every edge in both variants)
-                if (MODE != MODE_HYB_EXACT && valid && wants && !both) ++n_fallback;
+                // or, when the HLL edges are listed here, by this one
+                if ((MODE != MODE_HYB_EXACT || P.hll_u) && valid && wants && !both) ++n_fallback;
             }
+            if (MODE == MODE_HYB_EXACT && P.hll_u) append_hll(P, is_hll, u, v, lane);
             const bool do_exact = valid && !is_hll && MODE != MODE_HYB_HLL;
             const bool do_hll = valid && is_hll && MODE != MODE_HYB_EXACT;
             n_exact += do_exact;
@@ -1065,12 +1102,13 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
                                                          tchll_count_result* result) {
     __shared__ int32_t s_stage[8][kStage];
     __shared__ __align__(16) uint32_t s_bits[8][4 * kBmMax];
-    // grid-uniform: the 32-bit lists apply, or no hub pair will read a list
-    if (!packed || n_core[0] > kCore16Max || *n_segs == 0) return;
+    if (!packed || n_core[0] > kCore16Max) return;  // grid-uniform: the 32-bit lists apply
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int sub = lane & 7, grp = lane >> 3;
     uint32_t status = 0;
-    while (true) {
+    const bool lists = *n_segs > 0;  // grid-uniform; else no hub pair will read one
+    if (!lists) validate_rows(row_ptr, n_nodes, nnz, col, status);
+    while (lists) {
         unsigned long long y0 = 0;
         if (lane == 0) y0 = atomicAdd(row_ctr, 8ull);
         y0 = __shfl_sync(FULL, y0, 0);
@@ -1143,13 +1181,13 @@ __global__ void core_pad_kernel(const int32_t* __restrict__ row_ptr, int64_t n_n
                                 const int32_t* __restrict__ n_core, int packed, int32_t* __restrict__ pcol,
                                 tchll_count_result* result) {
     const int32_t C = n_core[0];
-    // grid-uniform: core_lists_kernel writes the lists, or no pair reads one
-    if ((packed && C <= kCore16Max) || C == 0) return;
+    if (packed && C <= kCore16Max) return;  // grid-uniform: core_lists_kernel writes the lists
     const int sub = threadIdx.x & 7;
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
     const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 3;
     uint32_t status = 0;
-    for (int64_t y = g; y < n_nodes; y += ng) {
+    if (C == 0) validate_rows(row_ptr, n_nodes, nnz, col, status);  // no hub pair will read a list
+    for (int64_t y = C ? g : n_nodes; y < n_nodes; y += ng) {
         const int32_t rs = __ldg(row_ptr + y), re = __ldg(row_ptr + y + 1);
         if (rs < 0 || re < rs || (int64_t)re > nnz) {
             status |= ST_BAD_ROW;
@@ -2147,7 +2185,7 @@ struct Tuning {
     int tiny = 16;
     int blocks_per_sm = 0;  // 0: occupancy maximum
     int warps = 8;          // warps per CTA
-    int pairs = 1;          // table-side / probe-side reorientation
+    int pairs = 1;          // table-side / probe-side reorientation (2: for small graphs too)
     int sparse = 0;         // table load <= 1/4 where it fits
     int hub = 128;          // pairs with d+(x) > hub go to the CTA-table kernels (0: off)
     int hub_seg = 2048;     // hub pairs per CTA work unit
@@ -2160,6 +2198,15 @@ struct Tuning {
     int hll_row_cache_p = 0;   // HLL pass: keep u's register row in registers for p <= this (0: never)
     int hll_lanes = 0;      // HLL pass: lanes per edge (0: chosen by p)
 };
+// Up to this many edges the regrouping's dozen launches cost more than it
+// saves, and the edges are counted as given, with one launch (R-MAT edge
+// factor 16, device time as given / regrouped: 48 K edges 26 / 155 us, 441 K
+// 104 / 238 us, 909 K 211 / 284 us, 1.9 M 464 / 385 us).  Dense graphs are
+// regrouped all the same: lists beyond a warp's table (512 members) are
+// searched one by one (cliques of 300, 600, 1000 vertices: 25 / 122, 260 /
+// 152, 1734 / 211 us).
+constexpr int64_t kDirectEdges = 1 << 19;
+constexpr int64_t kDirectDegree = 128;  // mean forward degree
 constexpr int HUB_MIN = 64;       // smallest hub threshold (bounds the segment count)
 constexpr int HUB_SEG_MIN = 256;  // smallest segment
 
@@ -2262,6 +2309,15 @@ static int launch_count(const CountParams& P, const Tuning& T, bool details, cud
     const bool vec = ((uintptr_t)P.col_idx % 16 == 0) && (P.regs == nullptr || (uintptr_t)P.regs % 16 == 0);
     if (details) return vec ? launch_mode<MODE, true, true>(P, T, st) : launch_mode<MODE, false, true>(P, T, st);
     return vec ? launch_mode<MODE, true, false>(P, T, st) : launch_mode<MODE, false, false>(P, T, st);
+}
+
+// Edges as given (no regrouping): small chunks, so that a small graph reaches
+// every warp (48 K edges, R-MAT 12: 26 us with 8 edges a warp, 40 with 32, 59
+// with 64).
+static int given_chunk(int64_t n_edges, int chunk) {
+    int c = 8;
+    while (c < 32 && n_edges >= 6144 * (int64_t)(2 * c)) c *= 2;
+    return n_edges <= kDirectEdges && c < chunk ? c : chunk;
 }
 
 struct CountWs {
@@ -2747,7 +2803,9 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
         set_error("workspace too small: need %zu bytes, have %zu", need, ws_bytes);
         return TCHLL_EWORKSPACE;
     }
-    TCHLL_CUDA(cudaMemsetAsync(W.ctr, 0, 4 * sizeof(unsigned long long), st));
+    const bool direct = P.n_edges <= kDirectEdges && P.n_edges <= kDirectDegree * P.n_nodes && T.pairs != 2;
+    if (!direct || mode != MODE_EXACT)  // a direct exact count claims nothing
+        TCHLL_CUDA(cudaMemsetAsync(W.ctr, 0, 4 * sizeof(unsigned long long), st));
     TCHLL_CUDA(cudaMemsetAsync(P.result, 0, sizeof(tchll_count_result), st));
     if (details && P.pe_support) TCHLL_CUDA(cudaMemsetAsync(P.pe_support, 0, sizeof(int64_t) * P.n_edges, st));
     if (details && P.pe_method) TCHLL_CUDA(cudaMemsetAsync(P.pe_method, 0, P.n_edges, st));
@@ -2760,7 +2818,11 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
     P.hll_v = nullptr;
     P.hll_n = nullptr;
     if (P.n_edges == 0) return TCHLL_OK;
-    const bool pairs = T.pairs && !details;
+    // small graphs refuse what the hub core's passes refuse in large ones
+    P.check_ids = direct && T.pairs && !details && hub_threshold(P, T) > 0 && hub_pad_usable(P, W) &&
+                  (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));
+    const bool pairs = T.pairs && !details && !direct;
+    if (!pairs) P.chunk = given_chunk(P.n_edges, T.chunk);
     if (col_ready && !(mode == MODE_EXACT && pairs)) {
         TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
         col_ready = nullptr;
@@ -2815,6 +2877,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 phase_used(ps, 0, 1);
                 return rc ? rc : rj;
             }
+            if (direct) P.work = nullptr;
             phase_mark(ps, 1, st);
             rc = launch_count<MODE_EXACT>(P, T, details, st);
             phase_mark(ps, 2, st);
@@ -2880,6 +2943,21 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 rc = fork.end();
                 phase_used(ps, 0, 1, 2);
                 if (ps.active()) g_phase.hll_split = true;
+                return rc;
+            }
+            if (direct && T.pairs && !details && ((uintptr_t)P.regs % 16 == 0)) {
+                // the exact launch lists the HLL edges for hll_edges_kernel
+                P.hll_u = HW.hll_u;
+                P.hll_v = HW.hll_v;
+                P.hll_n = HW.hll_n;
+                TCHLL_CUDA(cudaMemsetAsync(HW.hll_n, 0, sizeof(unsigned long long), st));
+                phase_mark(ps, 1, st);
+                rc = launch_count<MODE_HYB_EXACT>(P, T, false, st);
+                if (rc) return rc;
+                phase_mark(ps, 2, st);
+                rc = launch_hll_edges(P, HW, T, st);
+                phase_mark(ps, 3, st);
+                phase_used(ps, 1, 2);
                 return rc;
             }
             P.work = W.ctr;
@@ -3053,7 +3131,7 @@ TCHLL_EXPORT int tchll_set_count_shape(int32_t warps_per_cta, int32_t pairs) {
     TCHLL_ARG((size_t)warps_per_cta * ((size_t)4 << g_tuning.slots_log2) <= 227 * 1024,
               "warps x 2^slots_log2 x 4 bytes must fit 227 KB of shared memory");
     g_tuning.warps = warps_per_cta;
-    g_tuning.pairs = pairs ? 1 : 0;
+    g_tuning.pairs = pairs == 2 ? 2 : (pairs ? 1 : 0);
     return TCHLL_OK;
 }
 
