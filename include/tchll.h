@@ -248,6 +248,10 @@ int tchll_phase_hub_ms(float* ms2 /* host */);
 int tchll_build_sketches_dense(const int32_t* row_ptr, int64_t n_nodes, const int32_t* col_idx, int64_t nnz,
                                int64_t theta, int32_t p, uint8_t* sketch_regs, uint8_t* has_sketch, void* stream);
 
+/* Clears n bytes of device memory: the zeroed dense rows of
+ * alloc_sketch_arrays (src/gpu_hll.py:128-133), which can be gigabytes. */
+int tchll_zero_bytes(void* ptr, int64_t n, void* stream);
+
 /*
  * Compact sketches (src/hybrid.py:15-41): tchll_sketch_slots (workspace from
  * tchll_sketch_workspace_bytes) writes

@@ -83,6 +83,7 @@ SIGNATURES = {
     "tchll_phase_hub_ms": (C.c_int, [_P]),
     "tchll_sketch_workspace_bytes": (C.c_int, [_I64, C.POINTER(_SZ)]),
     "tchll_build_sketches_dense": (C.c_int, [_P, _I64, _P, _I64, _I64, _I32, _P, _P, _P]),
+    "tchll_zero_bytes": (C.c_int, [_P, _I64, _P]),
     "tchll_sketch_slots": (C.c_int, [_P, _I64, _I64, _P, _P, _P, _SZ, _P]),
     "tchll_build_sketches_compact": (C.c_int, [_P, _I64, _P, _P, _I64, _P, _I64, _I32, _P, _P]),
     "tchll_hll_add": (C.c_int, [_P, _I32, _P, _I64, _P]),

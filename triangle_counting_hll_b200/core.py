@@ -377,6 +377,14 @@ def build_sketches_dense_tensors(row_ptr, col_idx, n_nodes: int, theta: int, p: 
                                             stream_handle(dev)), "build sketches")
 
 
+def zeros_u8(n: int, device) -> torch.Tensor:
+    """Zeroed uint8 device tensor (one pass of 16-byte stores)."""
+    t = torch.empty(n, dtype=torch.uint8, device=device)
+    with torch.cuda.device(t.device):
+        check(load().tchll_zero_bytes(ptr(t), n, stream_handle(t.device)), "zero")
+    return t
+
+
 def sketch_slots(row_ptr: torch.Tensor, theta: int) -> Tuple[torch.Tensor, int]:
     """slot[u] = rank among rows of length >= theta, else -1; returns (slot, n)."""
     dev = row_ptr.device

@@ -7,12 +7,10 @@
 //              src/gpu_hll.py:47-81 (dense n x 2^p layout + has_sketch)
 //   estimate   src/hll.py:37-54,98-100,112-120
 //
-// Sketch build: one CTA per sketched vertex.  The CTA stages the 2^p-byte row
-// in shared memory (words of four registers, byte max by compare-and-swap),
-// hashes the vertex's neighbour list with coalesced loads, then writes the row
-// out with 16-byte stores.  CTAs walk the vertex range in tiles of 256 ids,
-// compacting the tile's sketched vertices with warp ballots, so vertices below
-// the threshold cost one coalesced read.
+// Sketch build: the 2^p-byte row of a sketched vertex is staged in shared
+// memory (words of four registers, byte max by compare-and-swap), its
+// neighbour list hashed with coalesced loads, and the row written out with
+// 16-byte stores.  A warp takes a vertex up to p = kWarpRowP, a CTA above.
 #include <cub/cub.cuh>
 
 #include "common.cuh"
@@ -21,76 +19,113 @@
 namespace tchll {
 
 constexpr int kSketchThreads = 256;
+constexpr int kSketchWarps = kSketchThreads / 32;
+constexpr int kWarpRowP = 12;  // 8 rows of 4 KB per CTA
 
+// Merges the hashes of N+(w) into the staged row; `tid` of `nt` threads.
 template <bool DENSE>
+__device__ __forceinline__ void sketch_list(uint32_t* words, const int32_t* __restrict__ col_idx,
+                                            const int64_t* __restrict__ keys, int64_t n_nodes, int32_t rs, int32_t re,
+                                            int p, int tid, int nt) {
+    for (int64_t k0 = rs; k0 < re; k0 += 4 * nt) {
+        int32_t c[4];
+        bool in[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const int64_t k = k0 + t * nt + tid;
+            in[t] = k < re;
+            c[t] = in[t] ? __ldg(col_idx + k) : 0;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            if (!in[t]) continue;
+            uint64_t x = (uint64_t)(int64_t)c[t];
+            if (!DENSE && keys) {
+                if (c[t] < 0 || (int64_t)c[t] >= n_nodes) continue;  // malformed column: skipped
+                x = (uint64_t)__ldg(keys + c[t]);
+            }
+            uint32_t j, rho;
+            hll_index_rank(x, p, j, rho);
+            smem_byte_max(words, j, rho);
+        }
+    }
+}
+
+// A CTA's tile is 32 groups of 8 consecutive vertices, the groups spread
+// evenly over the vertex range: sketched vertices cluster (at low ids in
+// R-MAT graphs), and 256 consecutive ones could all be sketched while most
+// tiles had none.  Bound by the latency of its short list reads; R-MAT 22,
+// p = 10, theta = 256 (35 K sketches): 616 us with consecutive tiles and a
+// CTA per vertex, 100 us so; R-MAT 17, p = 16 (a CTA per vertex) 1302, 406.  The tile's sketched vertices are compacted
+// with warp ballots and taken by its warps (WARP) or by the CTA one by one.
+template <bool DENSE, bool WARP>
 __global__ void __launch_bounds__(kSketchThreads)
     sketch_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, const int32_t* __restrict__ col_idx,
                   const int64_t* __restrict__ keys, int64_t nnz, int64_t theta, int p, uint8_t* has,
                   const int64_t* __restrict__ slot, int64_t n_rows, uint8_t* rows) {
     extern __shared__ __align__(16) uint32_t words[];
-    __shared__ int list[kSketchThreads];
-    __shared__ int warp_cnt[kSketchThreads / 32];
-    __shared__ int total;
+    __shared__ int4 list[kSketchThreads];  // vertex (two words), row start, row end
+    __shared__ int warp_cnt[kSketchWarps];
+    __shared__ int total, next;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int m = 1 << p;
-    const int nwords = m >> 2;
-    for (int64_t base = (int64_t)blockIdx.x * kSketchThreads; base < n_nodes;
-         base += (int64_t)gridDim.x * kSketchThreads) {
-        const int64_t u = base + tid;
+    if (DENSE) {  // the flags, in order
+        for (int64_t u = blockIdx.x * (int64_t)kSketchThreads + tid; u < n_nodes; u += (int64_t)gridDim.x * kSketchThreads)
+            has[u] = (int64_t)(__ldg(row_ptr + u + 1) - __ldg(row_ptr + u)) >= theta ? 1 : 0;
+    }
+    const int64_t tiles = (n_nodes + kSketchThreads - 1) / kSketchThreads;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t u = 8 * (tile + (tid >> 3) * tiles) + (tid & 7);
         bool flag = false;
+        int32_t rs = 0, re = 0;
         if (u < n_nodes) {
             // Rows with a malformed extent or an out-of-range slot are skipped
             // (the counting kernels report such input through their status).
-            const int32_t rs = row_ptr[u], re = row_ptr[u + 1];
-            const bool row_ok = rs >= 0 && re >= rs && (int64_t)re <= nnz;
+            rs = __ldg(row_ptr + u);
+            re = __ldg(row_ptr + u + 1);
             if (DENSE) {
                 flag = (int64_t)(re - rs) >= theta;
-                has[u] = flag ? 1 : 0;
             } else {
                 const int64_t s = slot[u];
                 flag = s >= 0 && s < n_rows;
             }
-            flag = flag && row_ok;
+            flag = flag && rs >= 0 && re >= rs && (int64_t)re <= nnz;
         }
         const unsigned bal = __ballot_sync(FULL, flag);
         if (lane == 0) warp_cnt[wid] = __popc(bal);
         __syncthreads();
         if (tid == 0) {
             int s = 0;
-            for (int w = 0; w < kSketchThreads / 32; ++w) { int c = warp_cnt[w]; warp_cnt[w] = s; s += c; }
+            for (int w = 0; w < kSketchWarps; ++w) { int c = warp_cnt[w]; warp_cnt[w] = s; s += c; }
             total = s;
+            next = 0;
         }
         __syncthreads();
-        if (flag) list[warp_cnt[wid] + __popc(bal & ((1u << lane) - 1u))] = (int)(u - base);
+        if (flag)
+            list[warp_cnt[wid] + __popc(bal & ((1u << lane) - 1u))] =
+                make_int4((int32_t)(uint32_t)u, (int32_t)(u >> 32), rs, re);
         __syncthreads();
         const int cnt = total;
-        for (int t = 0; t < cnt; ++t) {
-            const int64_t w = base + list[t];
-            const int32_t rs = row_ptr[w], re = row_ptr[w + 1];
-            uint8_t* row = DENSE ? rows + w * (int64_t)m : rows + slot[w] * (int64_t)m;
-            uint4* row4 = reinterpret_cast<uint4*>(row);
-            uint4* w4 = reinterpret_cast<uint4*>(words);
-            if (DENSE) {
-                for (int i = tid; i < (m >> 4); i += kSketchThreads) w4[i] = row4[i];
-            } else {
-                for (int i = tid; i < nwords; i += kSketchThreads) words[i] = 0u;
+        uint32_t* mine = WARP ? words + (size_t)wid * (m >> 2) : words;
+        uint4* w4 = reinterpret_cast<uint4*>(mine);
+        const int t0 = WARP ? lane : tid, nt = WARP ? 32 : kSketchThreads;
+        for (int t = 0; WARP || t < cnt; ++t) {
+            if (WARP) {
+                if (lane == 0) t = atomicAdd(&next, 1);
+                t = __shfl_sync(FULL, t, 0);
+                if (t >= cnt) break;
             }
-            __syncthreads();
-            for (int32_t k = rs + tid; k < re; k += kSketchThreads) {
-                const int32_t c = col_idx[k];
-                uint64_t x = (uint64_t)(int64_t)c;
-                if (keys) {
-                    if (c < 0 || (int64_t)c >= n_nodes) continue;  // malformed column: skipped
-                    x = (uint64_t)keys[c];
-                }
-                uint32_t j, rho;
-                hll_index_rank(x, p, j, rho);
-                smem_byte_max(words, j, rho);
-            }
-            __syncthreads();
-            for (int i = tid; i < (m >> 4); i += kSketchThreads) row4[i] = w4[i];
-            __syncthreads();
+            const int4 it = list[t];
+            const int64_t w = (int64_t)(((uint64_t)(uint32_t)it.y << 32) | (uint32_t)it.x);
+            uint4* row4 = reinterpret_cast<uint4*>(rows + (DENSE ? w : slot[w]) * (int64_t)m);
+            for (int i = t0; i < (m >> 4); i += nt) w4[i] = DENSE ? row4[i] : make_uint4(0u, 0u, 0u, 0u);
+            if (WARP) __syncwarp(); else __syncthreads();
+            sketch_list<DENSE>(mine, col_idx, keys, n_nodes, it.z, it.w, p, t0, nt);
+            if (WARP) __syncwarp(); else __syncthreads();
+            for (int i = t0; i < (m >> 4); i += nt) row4[i] = w4[i];
+            if (WARP) __syncwarp(); else __syncthreads();
         }
+        __syncthreads();
     }
 }
 
@@ -109,6 +144,25 @@ __global__ void slot_fix_kernel(const int32_t* __restrict__ row_ptr, int64_t n, 
 }
 
 __global__ void zero_i64_kernel(int64_t* p) { *p = 0; }
+
+// n bytes at p: `head` to the first 16-byte boundary, n16 16-byte words, the
+// rest; a grid that stays resident, four stores in flight per thread (2.45 GB:
+// 416 us, 5.9 TB/s; a fill of one 16-byte store per thread takes 623 us).
+__global__ void __launch_bounds__(512) zero_kernel(uint8_t* p, int64_t head, int64_t n16, int64_t n) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    uint4* q = reinterpret_cast<uint4*>(p + head);
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    int64_t i = t0;
+    for (; i + 3 * step < n16; i += 4 * step) {
+        q[i] = z;
+        q[i + step] = z;
+        q[i + 2 * step] = z;
+        q[i + 3 * step] = z;
+    }
+    for (; i < n16; i += step) q[i] = z;
+    if (t0 < head) p[t0] = 0;
+    if (head + 16 * n16 + t0 < n) p[head + 16 * n16 + t0] = 0;
+}
 
 __device__ __forceinline__ void global_byte_max(uint32_t* words, uint32_t j, uint32_t rho) {
     uint32_t* w = words + (j >> 2);
@@ -167,14 +221,15 @@ static int launch_sketch(const int32_t* row_ptr, int64_t n, const int32_t* col_i
                          int64_t nnz, int64_t theta, int p, uint8_t* has, const int64_t* slot, int64_t n_rows,
                          uint8_t* rows, cudaStream_t st) {
     if (n == 0) return TCHLL_OK;
-    auto kern = sketch_kernel<DENSE>;
-    const size_t smem = (size_t)1 << p;
-    static size_t smem_set[kMaxDevices] = {};  // per device: the attribute is per device
+    const bool warp = p <= kWarpRowP;
+    auto kern = warp ? sketch_kernel<DENSE, true> : sketch_kernel<DENSE, false>;
+    const size_t smem = ((size_t)1 << p) * (warp ? kSketchWarps : 1);
+    static size_t smem_set[2][kMaxDevices] = {};  // per device: the attribute is per device
     const int dev = current_device();
     if (dev < 0) return cuda_status(cudaErrorInvalidDevice, "cudaGetDevice");
-    if (smem > smem_set[dev]) {
+    if (smem > smem_set[warp][dev]) {
         TCHLL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        smem_set[dev] = smem;
+        smem_set[warp][dev] = smem;
     }
     int bps = 1;
     TCHLL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, kSketchThreads, smem));
@@ -190,6 +245,21 @@ static int launch_sketch(const int32_t* row_ptr, int64_t n, const int32_t* col_i
 }  // namespace tchll
 
 using namespace tchll;
+
+TCHLL_EXPORT int tchll_zero_bytes(void* ptr, int64_t n, void* stream) {
+    TCHLL_ARG(n >= 0 && (n == 0 || ptr), "bad arguments");
+    if (n == 0) return TCHLL_OK;
+    uint8_t* p = (uint8_t*)ptr;
+    int64_t head = (int64_t)((16 - ((uintptr_t)p & 15)) & 15);
+    if (head > n) head = n;
+    const int64_t n16 = (n - head) >> 4;
+    int64_t g = (n16 + 4 * 512 - 1) / (4 * 512);
+    const int64_t cap = (int64_t)sm_count() * 4;
+    g = g < 1 ? 1 : (g > cap ? cap : g);
+    zero_kernel<<<(int)g, 512, 0, (cudaStream_t)stream>>>(p, head, n16, n);
+    TCHLL_CHECK_LAUNCH("zero_kernel");
+    return TCHLL_OK;
+}
 
 TCHLL_EXPORT int tchll_sketch_workspace_bytes(int64_t n_nodes, size_t* bytes) {
     TCHLL_ARG(bytes != nullptr && n_nodes >= 0, "bad arguments");

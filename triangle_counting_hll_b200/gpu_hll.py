@@ -102,9 +102,7 @@ def alloc_sketch_arrays_device(n_nodes: int, p: int, device=None):
     (no host zeros to copy, unlike alloc_sketch_arrays + to_device)."""
     _lib.require_cuda()
     dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
-    m = 1 << p
-    return (torch.zeros(n_nodes * m, dtype=torch.uint8, device=dev),
-            torch.zeros(n_nodes, dtype=torch.uint8, device=dev))
+    return core.zeros_u8(int(n_nodes) * (1 << p), dev), core.zeros_u8(int(n_nodes), dev)
 
 
 def union_estimate_rows(sketch_regs, u, v, p: int) -> float:
