@@ -209,21 +209,18 @@ def hub_kernel_name(tuning: dict, core_vertices: int) -> str:
 
 
 def phase_report(pair_ms, count_ms, hub_ms, core_ms, tuning: dict) -> dict:
-    """Phase times of one exact count.  With the overlap on, the hub core pass
-    runs on the second stream beside the pair scatter and the short-list
-    pair kernel, so it is reported apart from the serial phases."""
+    """Phase times of one exact count.  pair_regroup is the first pass over the
+    edges (which also counts the short-list pairs) and the scatter of the hub
+    pairs.  With the overlap on, the hub core pass runs on the second stream
+    beside the scatter, so it is reported apart from the serial phases."""
     out = {"pair_regroup": pair_ms, "count": count_ms, "hub_kernels": hub_ms}
     if not hub_ms:
         out["pair_kernel"] = count_ms
-    elif tuning.get("overlap", 0) >= 2:  # the short-list pairs run on the second stream too
-        out["hub_core_pass_beside"] = core_ms
-        out["core_wait"] = count_ms - hub_ms
     elif tuning.get("overlap"):
         out["hub_core_pass_beside"] = core_ms
-        out["pair_kernel_and_core_wait"] = count_ms - hub_ms
+        out["core_wait"] = count_ms - hub_ms
     else:
         out["hub_core_pass"] = core_ms
-        out["pair_kernel"] = count_ms - hub_ms - (core_ms or 0.0)
     return out
 
 

@@ -72,10 +72,10 @@ uint64_t tchll_launch_count(void);
 
 /* --------------------------------------------- exact / hybrid counting --- */
 /* Workspace for tchll_exact_count / tchll_hybrid_count_* on a CSR of n_nodes
- * rows and n_edges edges: the regrouped pair lists, per-vertex histograms and
- * offsets, the long-list work units, 16-byte-aligned copies of the probe
- * lists and, for hybrid counts, the HLL edge list -- about 20 bytes per edge
- * + 110 per vertex.  The aligned copies are optional: a workspace too small
+ * rows and n_edges edges: the hub pairs, a table of row extents, per-vertex
+ * histograms and offsets, the long-list work units, the packed lists of the
+ * hub kernels and, for hybrid counts, the HLL edge list -- about 17 bytes per
+ * edge + 110 per vertex.  The packed lists are optional: a workspace too small
  * for them but large enough otherwise runs without them (same results). */
 int tchll_count_workspace_bytes(int64_t n_nodes, int64_t n_edges, size_t* bytes);
 
@@ -146,10 +146,12 @@ int tchll_hybrid_count_compact(const int32_t* row_ptr, int64_t n_nodes, const in
  * counterpart in the reference, whose block size is fixed at 256,
  * src/gpu_hybrid.py:13).  chunk: edges claimed per warp (multiple of 32);
  * slots_log2: per-warp hash table capacity; tiny: lane-local merge threshold
- * on |N+u|+|N+v|; blocks_per_sm: 0 = occupancy maximum; warps_per_cta: 1-8;
+ * on |N+u|+|N+v| (both: small dense graphs, per-edge outputs and fused hybrid
+ * counts, which count edges as given with tables); blocks_per_sm: 0 = occupancy maximum; warps_per_cta: 1-8;
  * pairs: 1 = probe the shorter list into a table of the longer one (edges
- * regrouped by a device counting sort) when the graph has more than 2^19
- * edges or 128 per vertex, 2 = whatever its size, 0 = edges as given; sparse: 1 = hash
+ * with a long list regrouped by a device counting sort) when the graph has
+ * more than 2^19 edges and 3 per vertex, or 128 per vertex, 2 = whatever its
+ * size, 0 = edges as given; sparse: 1 = hash
  * tables at load <= 1/4 where they fit (else <= 1/2).  out8 receives chunk,
  * slots_log2, tiny, blocks_per_sm, warps_per_cta, pairs, sparse and a
  * reserved 0.  Results are identical for every setting. */
@@ -158,11 +160,14 @@ int tchll_set_count_shape(int32_t warps_per_cta, int32_t pairs);
 int tchll_set_count_table(int32_t sparse);
 int tchll_get_count_tuning(int32_t* out8 /* host */);
 
-/* Hub pairs (pairs layout only, col_idx 16-byte aligned): pairs whose table
- * side x has d+(x) > threshold are counted by a kernel in which a whole CTA
- * shares one hash table of N+(x) (load <= 1/16 where 2^table_log2 slots of
- * shared memory allow), seg_pairs of x's pairs per work unit, unroll 16-byte
- * probe loads in flight per lane.  threshold 0 turns it off; otherwise
+/* Hub pairs (pairs layout only): pairs whose table side x has d+(x) >
+ * threshold are counted by a kernel in which a whole CTA shares one bitmap or
+ * hash table of N+(x) (hash: load <= 1/16 where 2^table_log2 slots of shared
+ * memory allow), at most seg_pairs of x's pairs per work unit, unroll 16-byte
+ * probe loads in flight per lane; all other pairs are counted by binary search
+ * of the longer list in the first pass over the edges.  threshold 128, the
+ * default, is taken as 64 where that is faster (up to 28 M edges; batches: a
+ * mean forward degree of at least 12).  threshold 0 turns it off; otherwise
  * threshold >= 64, seg_pairs in [256, 2^20], table_log2 in [10, 15], unroll 2
  * or 4.  out4 receives the four values.  Results are identical for every
  * setting. */
@@ -177,11 +182,9 @@ int tchll_get_count_hub(int32_t* out4 /* host */);
  * hold 16-bit core indices (two planes) and the bitmap takes 16 KB; else,
  * when the core fits 8 * 2^bitmap_log2 bits (minus 32), 32-bit lists and a
  * bitmap of that size; else hash tables.  bitmap_log2 0 turns the 32-bit
- * bitmap off; otherwise in [10, 17].  overlap 1 runs the hub core pass
- * and a hybrid count's HLL pass on a second stream beside the exact pairs;
- * overlap 2 also moves an exact count's short-list pair kernel there, after
- * the core pass, beside the hub kernel; 0 runs everything on the caller's
- * stream (the second stream is joined before the call returns).  Packed
+ * bitmap off; otherwise in [10, 17].  overlap 1 (or 2, the same) runs the hub
+ * core pass and a hybrid count's HLL pass on a second stream beside the exact
+ * pairs; 0 runs everything on the caller's stream (the second stream is joined before the call returns).  Packed
  * lists hold their dense part, the core's most popular vertices, as bitmaps.
  * bank_sort is kept and returned but has no effect (the lists once had a
  * bank-ordered form).  out4 receives the four values.  Results are identical for every setting.  These kernels read
@@ -206,9 +209,10 @@ int tchll_get_hll_pass(int32_t* out2 /* host */);
  * result as tchll_exact_count without per-edge output, but the scratch comes
  * from a fixed array of TCHLL_NOALLOC_SCRATCH_BYTES inside the library that
  * every GPU loading the library reserves until the process exits; graphs
- * needing more scratch (about 8 bytes per edge + 32 per vertex: the pair
- * lists, four per-vertex histograms / offsets and the work-unit list, so for
- * example 3 M edges on 200 K vertices fit) are rejected with TCHLL_EINVAL.
+ * needing more scratch (about 4 bytes per edge + 32 per vertex: the hub
+ * pairs, per-vertex histograms / offsets and row extents and the work-unit
+ * list, so for example 6 M edges on 200 K vertices fit) are rejected with
+ * TCHLL_EINVAL.
  * The first
  * call in each CUDA context looks up the array's device address (cached per
  * context id, so a context made current by the caller, or one re-created

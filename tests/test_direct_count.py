@@ -60,3 +60,63 @@ def test_neighbour_ids_are_checked_without_long_lists(tchll, pairs, at):
             core.exact_from_result(res)
     finally:
         core.set_count_tuning(**base)
+
+
+def _random_csr(rng, lens, n):
+    row_ptr = np.zeros(n + 1, dtype=np.int32)
+    row_ptr[1:] = np.cumsum(lens)
+    col = np.concatenate([np.sort(rng.permutation(n)[:d]) for d in lens] or [[]]).astype(np.int32)
+    return row_ptr, col
+
+
+# list lengths around 16-byte quads and the short / hub line, starts at every
+# alignment, an array that does or does not end in a whole quad
+@pytest.mark.parametrize("pairs,offset", [(1, 0), (2, 0), (1, 1), (2, 1)])
+@pytest.mark.parametrize("tail", [0, 1, 2, 3])
+def test_searched_lists(tchll, oracle, pairs, offset, tail):
+    import torch
+    from triangle_counting_hll_b200 import core
+    rng = np.random.default_rng(11 + tail)
+    n = 900
+    lens = rng.choice([0, 1, 2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 33, 63, 64, 65, 127, 128, 129], n)
+    lens[-1] = 6
+    lens[-1] += (tail - lens.sum()) % 4
+    row_ptr, col = _random_csr(rng, lens, n)
+    assert len(col) % 4 == tail
+    eu, ev = (rng.integers(0, n, 40001).astype(np.int32) for _ in range(2))
+    eu[:7], ev[:7] = n - 1, rng.integers(0, n, 7)
+    ref = oracle.exact_count(row_ptr, col, eu, ev)
+    buf = torch.zeros(len(col) + offset, dtype=torch.int32, device="cuda")  # offset: not 16-byte aligned
+    buf[offset:] = torch.from_numpy(col).cuda()
+    base = core.get_count_tuning()
+    try:
+        core.set_count_tuning(**dict(base, pairs=pairs))
+        res, _ = core.exact_count_tensors(torch.from_numpy(row_ptr).cuda(), buf[offset:], torch.from_numpy(eu).cuda(),
+                                          torch.from_numpy(ev).cuda())
+        assert core.exact_from_result(res) == ref
+    finally:
+        core.set_count_tuning(**base)
+
+
+def test_batch_mixes_graphs_with_and_without_long_lists(tchll, oracle):
+    """Only the graphs with hub pairs get lists and their own core numbering;
+    counts and totals equal one graph at a time."""
+    import torch
+    from triangle_counting_hll_b200 import batch, core
+    graphs = []
+    for i in range(60):
+        if i % 5 == 2:  # a clique inside an R-MAT graph: lists past the hub line
+            u, v = core.gen_rmat(10, 8, seed=i)
+            iu, iv = np.triu_indices(150 + i, 1)
+            u = torch.cat([u, torch.from_numpy(iu.astype(np.int32)).cuda()])
+            v = torch.cat([v, torch.from_numpy(iv.astype(np.int32)).cuda()])
+            graphs.append((u, v, 1 << 10))
+        else:
+            graphs.append((*core.gen_er(37 + 11 * i, 200 + 30 * i, seed=i), 37 + 11 * i))
+    b = batch.GraphBatch.from_edge_lists(graphs)
+    csrs = [core.csr_from_edges(u, v) for u, v, _ in graphs]
+    assert np.array_equal(b.exact_counts(), batch.plain_exact_counts(csrs))
+    totals, stats = b.hybrid_counts(64, 64, 10)
+    want, wstats = batch.plain_hybrid_counts(csrs, batch.plain_sketches(csrs, 64, 10), 64, 10)
+    assert np.array_equal(totals, want)
+    assert all(np.array_equal(stats[k], wstats[k]) for k in stats)

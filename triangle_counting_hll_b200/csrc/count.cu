@@ -12,27 +12,25 @@
 //
 // Design
 //   * Table side / probe side.  |N+(u) cap N+(v)| is symmetric, so each exact
-//     edge becomes a pair (x, y) with x the endpoint of the LONGER list: a
-//     device counting sort (histogram, scan, scatter) groups the pairs by x.
-//     A warp then keeps N+(x) in a private shared-memory hash table while it
-//     streams the shorter N+(y) lists through it: the probe count drops from
-//     sum d+(v) to sum min(d+u, d+v) (43.4 G list elements -> 11.8 G probes on
-//     R-MAT scale 22).  Per-edge outputs (details) use the edges as given.
-//   * One persistent launch, work stealing: a warp claims CHUNK consecutive
-//     pairs with one atomicAdd and walks them 32 at a time; pairs sharing x
-//     form a group and reuse the warp's table (built once per group per chunk).
-//   * The table keeps one 4-byte word per slot at load <= 1/8: a key sits in
-//     its home slot or, flagged there, on a second-hash walk, so a lookup is
-//     one 4-byte shared load with a rare walk (the warp seldom diverges).
-//   * Pairs whose x has a long list (d+(x) > hub threshold; 90% of the probes
-//     on R-MAT scale 22) are counted by a CTA-wide kernel: all warps of a CTA
-//     share one table of N+(x) of up to 32 KB, so long lists also get the
-//     low load factor.
-//   * The group's probe lists are flattened into one stream of 16-byte quads
-//     dealt to the 32 lanes by a warp scan, so short and long lists keep
-//     every lane busy.
-//   * Tiny pairs are merged lane-locally; tables too large for a warp fall
-//     back to a warp binary search.
+//     edge becomes a pair (x, y) with x the endpoint of the LONGER list: the
+//     members of the shorter list are looked up in the longer one, which drops
+//     the look-ups from sum d+(v) to sum min(d+u, d+v) (43.4 G list elements ->
+//     11.8 G on R-MAT scale 22).
+//   * A first pass over the edges (pair_pass_kernel) counts every pair of
+//     short lists on the spot by binary search and counts the others, the hub
+//     pairs (d+(x) > hub threshold; 98% of the look-ups on R-MAT scale 22),
+//     per table side; a counting sort then groups those by x.
+//   * Hub pairs are counted by a CTA per group of x's pairs, all its warps
+//     sharing one bitmap of N+(x) in shared memory (hub_bitmap16_kernel), in
+//     the coordinates of the core, the vertices of the hub lists.
+//   * Small dense graphs, per-edge outputs and fused hybrid counts take the
+//     edges as given: a warp keeps N+(u) in a private hash table (count_kernel:
+//     one 4-byte word per slot at load <= 1/8, a lookup is one shared load
+//     with a rare walk) while it streams the N+(v) lists through it; tiny
+//     pairs are merged lane-locally, lists too long for the table searched.
+//   * Lists of a group are flattened into one stream of 16-byte units dealt to
+//     the 32 lanes by a warp scan, so short and long lists keep every lane
+//     busy.
 //   * HLL edges: the warp reads both 2^p-byte register rows with 16-byte
 //     loads, merges them with __vmaxu4 and accumulates sum 2^-r EXACTLY as a
 //     128-bit fixed-point integer; one lane applies the FP64 corrections,
@@ -61,13 +59,13 @@ enum : uint32_t {
 
 struct CountParams {
     const int32_t* row_ptr;
+    const int2* rows;  // {row_ptr[v], row_ptr[v + 1]} per vertex, or null
     int64_t n_nodes;
     const int32_t* col_idx;
     int64_t nnz;
     const int32_t* edge_u;
     const int32_t* edge_v;
     int64_t n_edges;
-    const int32_t* n_edges_dev;  // when set, the edge count is read here (pairs)
     const int32_t* degrees;      // forward degree for routing (hybrid modes)
     const uint8_t* regs;         // register rows
     int64_t n_rows;              // rows available in regs
@@ -96,6 +94,9 @@ struct CountParams {
     const int64_t* n_chunks_dev;
     const int32_t* graph_vbase;  // vertex range of graph g: [vbase[g], vbase[g+1])
     int64_t n_graphs;            // batched calls: graphs in graph_vbase (else 0)
+    int32_t* graph_hub;          // batched calls: 1 for a graph with hub pairs (first pass)
+    int32_t* live_flag;          // batched calls: 1 for 64 rows that touch such a graph
+    int32_t* live_list;          // and those blocks of 64 rows, listed
     // Hybrid with pairs: the routing pass appends HLL edges here
     int32_t* hll_u;
     int32_t* hll_v;
@@ -165,15 +166,25 @@ __device__ __forceinline__ bool load_edge(const CountParams& P, int64_t e, int32
     // L1 for the row_ptr entries of the high-degree endpoints, which recur
     u = __ldcs(P.edge_u + e);
     v = __ldcs(P.edge_v + e);
-    if (u < 0 || v < 0 || (int64_t)u >= P.n_nodes || (int64_t)v >= P.n_nodes) {
+    const uint32_t n = (uint32_t)P.n_nodes, nnz = (uint32_t)P.nnz;  // both below 2^31
+    if ((uint32_t)u >= n || (uint32_t)v >= n) {
         status |= ST_BAD_EDGE;
         return false;
     }
-    us = __ldg(P.row_ptr + u);
-    ue = __ldg(P.row_ptr + u + 1);
-    vs = __ldg(P.row_ptr + v);
-    ve = __ldg(P.row_ptr + v + 1);
-    if (us < 0 || ue < us || (int64_t)ue > P.nnz || vs < 0 || ve < vs || (int64_t)ve > P.nnz) {
+    if (P.rows) {  // the same, one load per endpoint
+        const int2 ru = __ldg(P.rows + u), rv = __ldg(P.rows + v);
+        us = ru.x;
+        ue = ru.y;
+        vs = rv.x;
+        ve = rv.y;
+    } else {
+        us = __ldg(P.row_ptr + u);
+        ue = __ldg(P.row_ptr + u + 1);
+        vs = __ldg(P.row_ptr + v);
+        ve = __ldg(P.row_ptr + v + 1);
+    }
+    // 0 <= start <= end <= nnz
+    if ((uint32_t)us > (uint32_t)ue || (uint32_t)ue > nnz || (uint32_t)vs > (uint32_t)ve || (uint32_t)ve > nnz) {
         status |= ST_BAD_ROW;
         return false;
     }
@@ -228,26 +239,26 @@ __device__ __forceinline__ bool route(const CountParams& P, int32_t u, int32_t v
 }
 
 // ------------------------------------------------------------ pair build ----
-// Exact edges (all edges, or in hybrid mode the exact-routed ones) become
-// pairs (x, y), x the endpoint with the longer forward list (ties: u).
-template <bool HYB>
-__device__ __forceinline__ bool pair_of(const CountParams& P, int64_t e, int32_t& x, int32_t& y, int32_t& xl,
-                                        uint32_t& status) {
-    int32_t u, v, us, ue, vs, ve;
-    if (!load_edge(P, e, u, v, us, ue, vs, ve, status)) return false;
-    if (HYB) {
-        int32_t du, dv;
-        int64_t su, sv;
-        bool wants, both;
-        if (!route(P, u, v, du, dv, su, sv, wants, both, status)) return false;
-        if (wants && both) return false;  // HLL-routed
-    }
-    const bool ux = (ue - us) >= (ve - vs);
-    x = ux ? u : v;
-    y = ux ? v : u;
-    xl = ux ? (ue - us) : (ve - vs);
-    return true;
+// An exact edge is a pair of lists: the longer is its table side, the shorter
+// its probe side (ties: u is the table side).
+struct PairSides {
+    int32_t x, y;            // table side, probe side
+    int32_t xs, xl, ys, yl;  // their lists: start, length
+};
+__device__ __forceinline__ PairSides sides_of(int32_t u, int32_t v, int32_t us, int32_t ue, int32_t vs, int32_t ve) {
+    const int32_t lu = ue - us, lv = ve - vs;
+    const bool ux = lu >= lv;
+    PairSides S;
+    S.x = ux ? u : v;
+    S.y = ux ? v : u;
+    S.xs = ux ? us : vs;
+    S.xl = ux ? lu : lv;
+    S.ys = ux ? vs : us;
+    S.yl = ux ? lv : lu;
+    return S;
 }
+// Hub pairs: a long table side and something to probe it with.
+__device__ __forceinline__ bool is_hub_pair(const PairSides& S, int hub) { return hub > 0 && S.xl > hub && S.yl > 0; }
 
 // Batched calls: the graph of vertex v, the last g with vbase[g] <= v.
 __device__ __forceinline__ int64_t graph_of(const int32_t* vbase, int64_t n_graphs, int32_t v) {
@@ -294,72 +305,57 @@ __device__ __forceinline__ void append_hll(const CountParams& P, bool hll, int32
                  e = _wb + (threadIdx.x & 31u);                                                \
          _wb < (n); _wb += (int64_t)gridDim.x * blockDim.x, e = _wb + (threadIdx.x & 31u))
 
+// Hub pairs' probe sides, grouped by table side: py[cursor[x] ...).
 template <bool HYB>
-__global__ void pair_hist_kernel(const CountParams P, int32_t* cnt) {
-    uint32_t status = 0;
-    unsigned long long fallback = 0;
-    const int lane = threadIdx.x & 31;
-    WARP_EDGE_LOOP(e, P.n_edges) {
-        int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
-        bool ok = e < P.n_edges && load_edge(P, e, u, v, us, ue, vs, ve, status);
-        bool hll = false;
-        if (HYB && ok) {
-            int32_t du, dv;
-            int64_t su, sv;
-            bool wants, both;
-            ok = route(P, u, v, du, dv, su, sv, wants, both, status);
-            hll = ok && wants && both;
-            if (ok && wants && !both) {
-                if (P.graph_vbase && P.hll_u)  // batched: this edge's graph
-                    atomicAdd((unsigned long long*)&P.result[graph_of(P.graph_vbase, P.n_graphs, u)].n_fallback, 1ull);
-                else
-                    ++fallback;
-            }
-        }
-        {
-            // a run of lanes with the same table side adds with one atomic
-            const bool counted = ok && !hll;
-            const int32_t x = counted ? (((ue - us) >= (ve - vs)) ? u : v) : -1 - lane;
-            int head, len;
-            lane_runs(x, lane, head, len);
-            if (counted && lane == head) atomicAdd(cnt + x, len);
-        }
-        if (HYB && P.hll_u) append_hll(P, hll, u, v, lane);
+__device__ __forceinline__ void scatter_step(const CountParams& P, int64_t e, bool in, int32_t* cursor, int hub,
+                                             int32_t* py, int lane) {
+    uint32_t status = 0;  // reported by the first pass
+    int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
+    bool ok = in && load_edge(P, e, u, v, us, ue, vs, ve, status);
+    const PairSides S = sides_of(u, v, us, ue, vs, ve);
+    ok = ok && is_hub_pair(S, hub);
+    if (HYB && ok) {
+        int32_t du, dv;
+        int64_t su, sv;
+        bool wants, both;
+        ok = route(P, u, v, du, dv, su, sv, wants, both, status) && !(wants && both);  // not HLL-routed
     }
-    if (status) atomicOr(&P.result->status, status);
-    if (HYB && P.hll_u && fallback) atomicAdd((unsigned long long*)&P.result->n_fallback, fallback);
+    // a run of lanes with the same x claims its positions with one atomic
+    int head, len;
+    lane_runs(ok ? S.x : -1 - lane, lane, head, len);
+    int32_t base = 0;
+    if (ok && lane == head) base = atomicAdd(cursor + S.x, len);
+    base = __shfl_sync(FULL, base, head);
+    if (ok) py[base + (lane - head)] = S.y;
 }
 
-// Small pairs go to [cursor[x]...) of px / py; with hub > 0, pairs whose x
-// has d+(x) > hub go to the hub list, py[*n_small + cursorh[x]...] (y only).
 template <bool HYB>
-__global__ void pair_scatter_kernel(const CountParams P, int32_t* cursor, int32_t* cursorh, int hub,
-                                    const int32_t* n_small, int32_t* px, int32_t* py) {
-    uint32_t status = 0;
+__global__ void pair_scatter_kernel(const CountParams P, int32_t* cursor, const unsigned long long* n_pairs, int hub,
+                                    int32_t* py) {
+    if (*n_pairs == 0) return;  // grid-uniform
     const int lane = threadIdx.x & 31;
-    const int64_t hbase = hub > 0 ? (int64_t)*n_small : 0;
-    WARP_EDGE_LOOP(e, P.n_edges) {
-        int32_t x = 0, y = 0, xl = 0;
-        const bool ok = e < P.n_edges && pair_of<HYB>(P, e, x, y, xl, status);
-        // a run of lanes with the same x claims its positions with one
-        // atomic (x's list length, hence its list, is the same for all)
-        int head, len;
-        lane_runs(ok ? x : -1 - lane, lane, head, len);
-        const bool to_hub = hub > 0 && xl > hub;
-        int32_t base = 0;
-        if (ok && lane == head) base = atomicAdd((to_hub ? cursorh : cursor) + x, len);
-        base = __shfl_sync(FULL, base, head);
-        if (ok) {
-            const int32_t pos = base + (lane - head);
-            if (to_hub) {
-                py[hbase + pos] = y;
-            } else {
-                px[pos] = x;
-                py[pos] = y;
+    if (P.chunk_start) {  // batched: the chunks of the graphs with hub pairs
+        const int64_t n = *P.n_chunks_dev;
+        const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+        for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < n; c += warps) {
+            const int32_t g = __ldg(P.chunk_graph + c);
+            if (!P.graph_hub[g]) continue;
+            const int32_t lo_v = __ldg(P.graph_vbase + g), hi_v = __ldg(P.graph_vbase + g + 1);
+            const int64_t e0 = __ldg(P.chunk_start + c);
+            const int32_t len = __ldg(P.chunk_len + c);
+            for (int32_t i = 0; i < len; i += 32) {
+                const int64_t e = e0 + i + lane;
+                bool in = i + lane < len;
+                if (in) {  // not an edge of another graph (the first pass skipped and reported it)
+                    const int32_t u = __ldg(P.edge_u + e), v = __ldg(P.edge_v + e);
+                    in = u >= lo_v && u < hi_v && v >= lo_v && v < hi_v;
+                }
+                scatter_step<HYB>(P, e, in, cursor, hub, py, lane);
             }
         }
+        return;
     }
-    (void)status;
+    WARP_EDGE_LOOP(e, P.n_edges) scatter_step<HYB>(P, e, e < P.n_edges, cursor, hub, py, lane);
 }
 
 // Warp-cooperative binary-search intersection count of two sorted lists in
@@ -421,6 +417,222 @@ __device__ __forceinline__ void publish(tchll_count_result* R, uint64_t acc, U12
     }
 }
 
+// What the first pass needs beforehand, in one launch: {row_ptr[v], row_ptr[v
+// + 1]} side by side (the passes over all edges look both up at random v, and
+// that is one load instead of two), and everything that starts at zero.
+struct Prepare {
+    const int32_t* row_ptr;
+    int64_t n_nodes;
+    int2* rows;
+    int32_t* zero_n[2];   // n_nodes + 1 words each (or null)
+    uint32_t* zero[3];    // words[i] words
+    int64_t words[3];
+};
+__global__ void prepare_kernel(const Prepare Q) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t v = t0; v <= Q.n_nodes; v += step) {
+        if (v < Q.n_nodes) Q.rows[v] = make_int2(__ldg(Q.row_ptr + v), __ldg(Q.row_ptr + v + 1));
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            if (Q.zero_n[i]) Q.zero_n[i][v] = 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        for (int64_t w = t0; w < Q.words[i]; w += step) Q.zero[i][w] = 0;
+}
+
+// The first pass over the edges.  Pairs with a long table side (hub pairs)
+// are counted per table side in cnth, for the hub kernels; every other pair
+// is counted here and now, by looking each member of its shorter list up in
+// the longer one by binary search.  A warp takes 32 edges at a time and deals
+// their probe members to its lanes as one stream (two windows of 32 in
+// flight), so lists of any length keep the lanes busy; a search touches the
+// few lines of one short list, mostly in L1.  No table has to be built, so
+// short-list pairs need no regrouping.  Against a per-warp hash table and
+// a lane-local merge over regrouped pairs, which these replaced:
+// 2,048 graphs of 88 M edges 6.1 -> 2.9 ms (exact, all launches), 49 M
+// Erdos-Renyi edges 3.1 -> 1.2 ms, R-MAT 22 with its 6 M short-list pairs 1.6
+// -> 1.3 ms.  Bound by instruction issue (76%, ALU 68%): no wide load or
+// higher occupancy changes it.
+// Edges come in chunks of P.chunk, claimed from P.work or dealt to the warps
+// in turn (null), or, batched, from the chunk list (a chunk is one graph's,
+// and so are its totals).
+enum : int { PASS_HIST = 1, PASS_SHORT = 2 };
+// Adds warp-uniform totals to *R.
+__device__ __forceinline__ void pass_publish(tchll_count_result* R, uint64_t acc, int64_t n_exact, int64_t n_fallback,
+                                             uint32_t status, int lane) {
+    status = __reduce_or_sync(FULL, status);
+    if (lane == 0) {
+        if (acc) atomicAdd((unsigned long long*)&R->exact, (unsigned long long)acc);
+        if (n_exact) atomicAdd((unsigned long long*)&R->n_exact, (unsigned long long)n_exact);
+        if (n_fallback) atomicAdd((unsigned long long*)&R->n_fallback, (unsigned long long)n_fallback);
+        if (status) atomicOr(&R->status, status);
+    }
+}
+
+template <bool HYB, bool VEC, int UNR = 2>
+__global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, int what, int hub,
+                                                           int32_t* __restrict__ cnth) {
+    __shared__ int4 s_list[8][32];
+    __shared__ int32_t s_len[8][32];
+    const int lane = threadIdx.x & 31;
+    int4* lst = s_list[threadIdx.x >> 5];
+    int32_t* len = s_len[threadIdx.x >> 5];
+    const unsigned lane_le = (2u << lane) - 1u;
+    const int32_t* __restrict__ col = P.col_idx;
+    uint64_t acc = 0;
+    int64_t n_exact = 0, n_fallback = 0;  // warp-uniform, as acc
+    uint32_t status = 0;
+    if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col, status);
+    const int32_t full_quads = (int32_t)(P.nnz >> 2);
+    const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
+    unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    while (true) {
+        int32_t e0, e1;  // below 2^31
+        int32_t g = -1;
+        uint32_t lo_v = 0, in_v = (uint32_t)P.n_nodes;
+        {
+            unsigned long long c = turn;
+            if (P.work) {
+                if (lane == 0) c = atomicAdd(P.work, 1ull);
+                c = __shfl_sync(FULL, c, 0);
+            }
+            turn += n_warps;
+            if (P.chunk_start) {
+                if ((int64_t)c >= *P.n_chunks_dev) break;
+                e0 = (int32_t)__ldg(P.chunk_start + c);
+                e1 = e0 + __ldg(P.chunk_len + c);
+                g = __ldg(P.chunk_graph + c);
+                lo_v = (uint32_t)__ldg(P.graph_vbase + g);
+                in_v = (uint32_t)__ldg(P.graph_vbase + g + 1) - lo_v;
+            } else {
+                if ((int64_t)c * P.chunk >= P.n_edges) break;
+                e0 = (int32_t)c * P.chunk;
+                e1 = (int32_t)min((int64_t)e0 + P.chunk, P.n_edges);
+            }
+        }
+        bool any_hub = false;
+        for (int32_t eb = e0; eb < e1; eb += 32) {
+            const int32_t e = eb + lane;
+            int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
+            bool ok = e < e1 && load_edge(P, e, u, v, us, ue, vs, ve, status);
+            if (ok && ((uint32_t)u - lo_v >= in_v || (uint32_t)v - lo_v >= in_v)) {
+                status |= ST_BAD_EDGE;  // an edge of another graph inside this graph's chunk
+                ok = false;
+            }
+            if (HYB) {
+                bool hll = false, fall = false;
+                if (ok) {
+                    int32_t du, dv;
+                    int64_t su, sv;
+                    bool wants, both;
+                    ok = route(P, u, v, du, dv, su, sv, wants, both, status);
+                    hll = ok && wants && both;
+                    fall = ok && wants && !both;
+                }
+                n_fallback += __popc(__ballot_sync(FULL, fall));
+                append_hll(P, hll, u, v, lane);
+                ok = ok && !hll;
+            }
+            const PairSides S = sides_of(u, v, us, ue, vs, ve);
+            const bool to_hub = ok && is_hub_pair(S, hub);
+            if (hub > 0 && (what & PASS_HIST) && __any_sync(FULL, to_hub)) {
+                // a run of lanes with the same table side adds with one atomic
+                int head, run;
+                lane_runs(to_hub ? S.x : -1 - lane, lane, head, run);
+                if (to_hub && lane == head) atomicAdd(cnth + S.x, run);
+                any_hub = true;
+            }
+            if (!(what & PASS_SHORT)) continue;
+            const bool mine = ok && !to_hub;
+            n_exact += __popc(__ballot_sync(FULL, mine));
+            const int np = mine ? S.yl : 0;
+            int incl = np;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(FULL, incl, o);
+                if (lane >= o) incl += t;
+            }
+            const int W = __shfl_sync(FULL, incl, 31);
+            if (W == 0) continue;
+            const int excl = incl - np;
+            const unsigned ne = __ballot_sync(FULL, np > 0);
+            __syncwarp();
+            // {probe member of stream position 0, the table list's first unit
+            // (VEC: 16-byte quad) and units, its start}, its length
+            if (np > 0) {
+                const int k = __popc(ne & (lane_le >> 1));
+                const int q0 = VEC ? S.xs >> 2 : S.xs;
+                lst[k] = make_int4(S.ys - excl, q0, VEC ? ((S.xs + S.xl - 1) >> 2) - q0 + 1 : S.xl, S.xs);
+                len[k] = S.xl;
+            }
+            __syncwarp();
+            int B = -1;  // lists that start before the window, less one
+            uint32_t hits = 0;
+            for (int T0 = 0; T0 < W; T0 += 32 * UNR) {
+                int32_t key[UNR], at[UNR], j[UNR];
+                int n[UNR], most = 0;
+#pragma unroll
+                for (int i = 0; i < UNR; ++i) {
+                    const int Ti = T0 + 32 * i, t = Ti + lane;
+                    const unsigned d = (unsigned)(excl - Ti);
+                    const unsigned st = __reduce_or_sync(FULL, (np > 0 && d < 32u) ? (1u << d) : 0u);
+                    j[i] = (B + __popc(st & lane_le)) & 31;
+                    B += __popc(st);
+                    const int4 l = lst[j[i]];
+                    // lanes past the end search for their list's last member
+                    key[i] = __ldg(col + l.x + min(t, W - 1));
+                    at[i] = l.y;
+                    n[i] = l.z;
+                    most = max(most, l.z);
+                }
+                // at = the last unit whose first member is <= key, or the
+                // first unit (a later unit's first member lies in the list)
+                for (; __any_sync(FULL, most > 1); most -= most >> 1) {
+#pragma unroll
+                    for (int i = 0; i < UNR; ++i) {
+                        const int half = n[i] >> 1, m = at[i] + half;
+                        if (__ldg(VEC ? col + 4 * (int64_t)m : col + m) <= key[i]) at[i] = m;
+                        n[i] -= half;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < UNR; ++i) {
+                    bool hit;
+                    if (!VEC) {
+                        hit = __ldg(col + at[i]) == key[i];
+                    } else {
+                        // the unit's members inside [xs, xs + length)
+                        int4 q;
+                        if (at[i] < full_quads) {
+                            q = __ldg(reinterpret_cast<const int4*>(col) + at[i]);
+                        } else {  // the array's last, partial quad
+                            const int64_t m = 4 * (int64_t)at[i];
+                            q.x = __ldg(col + m);
+                            q.y = m + 1 < P.nnz ? __ldg(col + m + 1) : 0;
+                            q.z = m + 2 < P.nnz ? __ldg(col + m + 2) : 0;
+                            q.w = 0;
+                        }
+                        const uint32_t o = 4u * (uint32_t)at[i] - (uint32_t)lst[j[i]].w, l = (uint32_t)len[j[i]];
+                        hit = (q.x == key[i] && o < l) || (q.y == key[i] && o + 1u < l) ||
+                              (q.z == key[i] && o + 2u < l) || (q.w == key[i] && o + 3u < l);
+                    }
+                    hits += hit && T0 + 32 * i + lane < W;
+                }
+            }
+            acc += __reduce_add_sync(FULL, hits);
+        }
+        if (g >= 0) {  // batched: this chunk's totals belong to its graph
+            if (any_hub && lane == 0 && __ldcg(P.graph_hub + g) == 0) P.graph_hub[g] = 1;
+            pass_publish(P.result + g, acc, n_exact, n_fallback, status, lane);
+            acc = 0;
+            n_exact = n_fallback = 0;
+            status = 0;
+        }
+    }
+    if (!P.chunk_start || status) pass_publish(P.result, acc, n_exact, n_fallback, status, lane);
+}
+
 template <int MODE, bool VEC, bool DETAILS>
 __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     extern __shared__ __align__(16) int32_t smem[];
@@ -431,7 +643,7 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     uint32_t* table = reinterpret_cast<uint32_t*>(smem) + ((size_t)wid << cap_lg);
 
     const int32_t* __restrict__ col_idx = P.col_idx;
-    const int64_t n_edges = P.n_edges_dev ? (int64_t)*P.n_edges_dev : P.n_edges;
+    const int64_t n_edges = P.n_edges;
 
     uint64_t acc = 0;
     U128 hacc;
@@ -945,6 +1157,51 @@ __global__ void __launch_bounds__(256) core_index_kernel(const uint32_t* __restr
     }
 }
 
+// Batched counts: a CTA per graph numbers that graph's core on its own (two
+// lists of a pair are the same graph's), so a batch's many small cores fit
+// the packed lists whatever their sum; C is the largest graph's.
+__global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* __restrict__ bits, int32_t* cnt_cidx,
+                                                                int64_t n_nodes, const int32_t* __restrict__ vbase,
+                                                                const int32_t* __restrict__ graph_hub,
+                                                                int32_t* live_flag, int32_t* live_list,
+                                                                int32_t* n_live, int32_t* n_core) {
+    __shared__ int h[256], part[8];
+    if (graph_hub[blockIdx.x] == 0) return;  // no core
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int32_t lo = __ldg(vbase + blockIdx.x), hi = __ldg(vbase + blockIdx.x + 1);
+    if (lo < 0 || hi < lo || (int64_t)hi > n_nodes) return;  // flagged by check_vbase_kernel
+    if (tid < 256) h[tid] = 0;
+    __syncthreads();
+    for (int32_t w = lo + tid; w < hi; w += 1024) {
+        const int b = pop_bucket(bits, cnt_cidx, w);
+        if (b >= 0) atomicAdd(h + b, 1);
+        if (((w & 63) == 0 || w == lo) && atomicExch(live_flag + (w >> 6), 1) == 0)
+            live_list[atomicAdd(n_live, 1)] = w >> 6;
+    }
+    __syncthreads();
+    int mine = 0, incl = 0;
+    if (tid < 256) {
+        incl = mine = h[tid];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) part[tid >> 5] = incl;
+    }
+    __syncthreads();
+    if (tid < 256) {
+        for (int i = 0; i < (tid >> 5); ++i) incl += part[i];
+        h[tid] = incl - mine;
+        if (tid == 255 && incl) atomicMax(n_core, incl);
+    }
+    __syncthreads();
+    for (int32_t w = lo + tid; w < hi; w += 1024) {
+        const int b = pop_bucket(bits, cnt_cidx, w);
+        cnt_cidx[w] = b >= 0 ? atomicAdd(h + b, 1) : -1;
+    }
+}
+
 // Packed probe lists (used when C <= kCore16Max; core_pad_kernel writes the
 // 32-bit ones otherwise).  A row is held as
 //   * a bitmap of the core indices below 128 B: B 16-byte units, unit b the
@@ -1099,6 +1356,8 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
                                                          uint4* __restrict__ pool, int32_t pool_cap,
                                                          int32_t* pool_used, unsigned long long* row_ctr,
                                                          const unsigned long long* __restrict__ n_segs,
+                                                         const int32_t* __restrict__ live,
+                                                         const int32_t* __restrict__ n_live,
                                                          tchll_count_result* result) {
     __shared__ int32_t s_stage[8][kStage];
     __shared__ __align__(16) uint32_t s_bits[8][4 * kBmMax];
@@ -1108,11 +1367,16 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
     uint32_t status = 0;
     const bool lists = *n_segs > 0;  // grid-uniform; else no hub pair will read one
     if (!lists) validate_rows(row_ptr, n_nodes, nnz, col, status);
+    // batched: only the listed blocks of 64 rows, those near a graph with hub
+    // pairs, are ever read as lists; the other rows are only checked
+    if (lists && live) validate_rows(row_ptr, n_nodes, nnz, col, status);
+    const unsigned long long n_claim = live ? 64ull * (unsigned)*n_live : (unsigned long long)n_nodes;
     while (lists) {
         unsigned long long y0 = 0;
         if (lane == 0) y0 = atomicAdd(row_ctr, 8ull);
         y0 = __shfl_sync(FULL, y0, 0);
-        if (y0 >= (unsigned long long)n_nodes) break;
+        if (y0 >= n_claim) break;
+        if (live) y0 = 64ull * (unsigned)__ldg(live + (y0 >> 6)) + (y0 & 63);
         int32_t rs = 0, d = 0;
         if (lane < 8 && (int64_t)y0 + lane < n_nodes) {
             const int64_t y = (int64_t)y0 + lane;
@@ -1753,53 +2017,70 @@ __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitma
     }
 }
 
-// Hub segments: x's hub pairs [offh[x], offh[x] + cnth[x]) (shifted by the
-// small-pair total *n_small) cut into pieces of at most seg pairs.
-// Batched counts (vbase != null) record the graph of x, found by binary
-// search in the ascending vertex offsets vbase[0..n_graphs].
-__global__ void hub_segments_kernel(const int32_t* __restrict__ cnth, const int32_t* __restrict__ offh,
-                                    const int32_t* __restrict__ n_small, int64_t n_nodes, int seg, HubSeg* segs,
-                                    unsigned long long* n_segs, int64_t max_segs, const int32_t* __restrict__ vbase,
-                                    int64_t n_graphs) {
-    const int32_t base_pairs = *n_small;
-    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n_nodes;
-         x += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t c = __ldg(cnth + x);
-        if (c <= 0) continue;
-        int32_t g = 0;
-        if (vbase) {  // last g with vbase[g] <= x
-            int64_t lo = 0, hi = n_graphs - 1;
-            while (lo < hi) {
-                const int64_t mid = (lo + hi + 1) >> 1;
-                if (__ldg(vbase + mid) <= x) lo = mid; else hi = mid - 1;
-            }
-            g = (int32_t)lo;
+// Places of the hub pairs and the hub segments: x's cnth[x] hub pairs get the
+// range [offh[x], + cnth[x]) of the list and are cut into segments of at most
+// seg pairs, x's next to each other.  The order of the ranges does not matter,
+// so a CTA of 1024 vertices scans its own and claims room with one atomic
+// each for pairs and segments (a scan over all vertices and one atomic per x
+// took 94 us on R-MAT 22).  Batched counts (vbase != null)
+// record the graph of x, found by binary search in the ascending vertex
+// offsets vbase[0..n_graphs].
+__global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restrict__ cnth, int64_t n_nodes, int seg,
+                                                        int32_t* __restrict__ offh, unsigned long long* n_pairs,
+                                                        HubSeg* segs, unsigned long long* n_segs, int64_t max_segs,
+                                                        const int32_t* __restrict__ vbase, int64_t n_graphs) {
+    __shared__ unsigned long long warp_sum[8], base[2];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t x0 = blockIdx.x * 1024ll + tid;
+    int32_t c[4];
+    unsigned long long mine = 0;  // pairs << 32 | segments
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int64_t x = x0 + 256 * i;
+        c[i] = x < n_nodes ? __ldg(cnth + x) : 0;
+        mine += ((unsigned long long)c[i] << 32) + (unsigned)((c[i] + seg - 1) / seg);
+    }
+    unsigned long long incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) warp_sum[tid >> 5] = incl;
+    __syncthreads();
+    if (tid == 0) {
+        unsigned long long sum = 0;
+        for (int w = 0; w < 8; ++w) {
+            const unsigned long long t = warp_sum[w];
+            warp_sum[w] = sum;
+            sum += t;
         }
-        const int k = (c + seg - 1) / seg;
-        const unsigned long long b = atomicAdd(n_segs, (unsigned long long)k);
-        for (int j = 0; j < k; ++j) {
-            if ((int64_t)(b + j) >= max_segs) break;  // cannot happen: sized for the worst case
-            HubSeg s;
-            s.start = base_pairs + __ldg(offh + x) + j * seg;
-            s.x = (int32_t)x;
-            s.len = min(seg, c - j * seg);
-            s.graph = g;
-            segs[b + j] = s;
+        if (sum) {
+            base[0] = atomicAdd(n_pairs, sum >> 32);
+            base[1] = atomicAdd(n_segs, sum & 0xFFFFFFFFull);
         }
     }
-}
-
-// Splits the pair histogram: cnt[x] keeps x's small pairs, cnth[x] gets its
-// hub pairs (all of x's pairs go one way: hub-ness depends on d+(x) only).
-__global__ void hub_split_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int hub, int32_t* cnt,
-                                 int32_t* cnth) {
-    for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x <= n_nodes;
-         x += (int64_t)gridDim.x * blockDim.x) {
-        int32_t c = cnt[x];
-        bool is_hub = false;
-        if (x < n_nodes && c > 0) is_hub = (__ldg(row_ptr + x + 1) - __ldg(row_ptr + x)) > hub;
-        cnth[x] = is_hub ? c : 0;
-        if (is_hub) cnt[x] = 0;
+    __syncthreads();
+    if (mine == 0) return;
+    const unsigned long long excl = warp_sum[tid >> 5] + incl - mine;
+    int32_t at = (int32_t)(base[0] + (excl >> 32));
+    int64_t sg = (int64_t)(base[1] + (excl & 0xFFFFFFFFull));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (c[i] <= 0) continue;
+        const int64_t x = x0 + 256 * i;
+        const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, (int32_t)x) : 0;
+        offh[x] = at;
+        for (int32_t j = 0; j < c[i]; j += seg, ++sg) {
+            if (sg >= max_segs) break;  // cannot happen: sized for the worst case
+            HubSeg s;
+            s.start = at + j;
+            s.x = (int32_t)x;
+            s.len = min(seg, c[i] - j);
+            s.graph = g;
+            segs[sg] = s;
+        }
+        at += c[i];
     }
 }
 
@@ -2179,6 +2460,9 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (CACHE ? 3 : 4)) hll_edges_ker
 }
 
 // ---------------------------------------------------------------- host ------
+constexpr int kHubDefault = 128;
+constexpr int64_t kHub64Edges = 28000000;
+constexpr int64_t kHub64Degree = 12;
 struct Tuning {
     int chunk = 256;
     int slots_log2 = 10;    // 1024 slots = 4 KB per warp: a table side of up to 128 keys at load <= 1/8
@@ -2187,12 +2471,12 @@ struct Tuning {
     int warps = 8;          // warps per CTA
     int pairs = 1;          // table-side / probe-side reorientation (2: for small graphs too)
     int sparse = 0;         // table load <= 1/4 where it fits
-    int hub = 128;          // pairs with d+(x) > hub go to the CTA-table kernels (0: off)
+    int hub = kHubDefault;  // pairs with d+(x) > hub go to the CTA-table kernels (0: off)
     int hub_seg = 2048;     // hub pairs per CTA work unit
     int hub_lg = 13;        // largest CTA hash table: 2^13 slots = 32 KB
     int hub_unroll = 2;     // quads per lane in flight (2 or 4)
     int bitmap_lg = 15;     // hub bitmap buffer: 2^15 bytes = 262,144 core vertices (0: hash tables only)
-    int overlap = 1;        // side stream: 1 the hub core pass (+ the hybrid HLL pass); 2 also the short-list pairs
+    int overlap = 1;        // side stream: the hub core pass (+ the hybrid HLL pass); 2 does the same as 1
     int packed = 1;         // hub probe lists as 16-bit core indices when the core allows
     int bank_sort = 0;      // kept for its setter and getter: no effect
     int hll_row_cache_p = 0;   // HLL pass: keep u's register row in registers for p <= this (0: never)
@@ -2200,13 +2484,21 @@ struct Tuning {
 };
 // Up to this many edges the regrouping's dozen launches cost more than it
 // saves, and the edges are counted as given, with one launch (R-MAT edge
-// factor 16, device time as given / regrouped: 48 K edges 26 / 155 us, 441 K
-// 104 / 238 us, 909 K 211 / 284 us, 1.9 M 464 / 385 us).  Dense graphs are
+// factor 16 to 32, device time as given / regrouped: 85 K edges 33 / 89 us,
+// 388 K 101 / 123 us, 441 K 119 / 123 us).  Dense graphs are
 // regrouped all the same: lists beyond a warp's table (512 members) are
-// searched one by one (cliques of 300, 600, 1000 vertices: 25 / 122, 260 /
-// 152, 1734 / 211 us).
+// searched one by one (cliques of 600 and 1000 vertices: 260 / 139, 1734 / 208
+// us).
 constexpr int64_t kDirectEdges = 1 << 19;
 constexpr int64_t kDirectDegree = 128;  // mean forward degree
+// Of those, graphs of at most this mean forward degree are counted by
+// binary search, the others with a hash table per u: ER 100 K edges 12 / 16 us,
+// R-MAT 14 (edge factor 32, mean 28) 224 / 103 us.
+constexpr int64_t kSparseDegree = 8;
+// Up to this mean forward degree graphs of any size are counted as given:
+// road networks have no long lists at all (a million-vertex lattice, mean
+// 2.2: 120 us of device time regrouped, 45 as given).
+constexpr int64_t kRoadDegree = 3;
 constexpr int HUB_MIN = 64;       // smallest hub threshold (bounds the segment count)
 constexpr int HUB_SEG_MIN = 256;  // smallest segment
 
@@ -2321,13 +2613,15 @@ static int given_chunk(int64_t n_edges, int chunk) {
 }
 
 struct CountWs {
-    unsigned long long* ctr;  // work counters: [0] [1] chunks, [2] hub segments made, [3] hub segments claimed
-    int32_t* cnt;             // n_nodes + 1 (histogram of small pairs)
-    int32_t* off;             // n_nodes + 1 (scan, then scatter cursor)
+    // counters: [0] [1] chunks, [2] hub segments made, [3] hub segments
+    // claimed, [4] HLL edges, [5] hub pairs; with ncore and cbits one run of
+    // zero_words words
+    unsigned long long* ctr;
+    int64_t zero_words;
     int32_t* cnth;            // n_nodes + 1 (histogram of hub pairs)
-    int32_t* offh;            // n_nodes + 1
-    int32_t* px;              // n_edges
-    int32_t* py;              // n_edges (small pairs, then the hub list)
+    int32_t* offh;            // n_nodes + 1 (scan, then scatter cursor)
+    int32_t* py;              // n_edges (probe sides of the hub pairs, by table side)
+    int2* rows;               // n_nodes (rows_kernel)
     HubSeg* segs;             // max_segs
     int64_t max_segs;
     int32_t* pcol;            // padded lists in core coordinates for the hub kernels, pcap entries (null: not carved)
@@ -2338,8 +2632,6 @@ struct CountWs {
     int4* pl;                 // n_nodes: packed lists' records (with pcol)
     uint4* pool;              // pool_cap bitmap units (with pcol)
     int64_t pool_cap;
-    void* tmp;
-    size_t tmp_bytes;
 };
 
 // Padded lists need nnz + 8 (n_nodes + 1) entries; the workspace holds them
@@ -2354,36 +2646,35 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
 
 // The hub core pass's small arrays: [0] core size, [1] pool units claimed,
 // [2..3] the list kernel's row counter (64 bits), [4 ..) popularity buckets'
-// sizes and cursors (256 each).  Cleared together.
-constexpr int kCoreWords = 4 + 2 * 256;
+// sizes and cursors (256 each), last the number of live row blocks.  Cleared
+// together.
+constexpr int kCoreWords = 4 + 2 * 256 + 1;
+constexpr int kCounters = 6;
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
     const size_t N = (size_t)(n_nodes > 0 ? n_nodes : 0) + 1;
     const size_t E = (size_t)(n_edges > 0 ? n_edges : 1);
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, (int32_t*)nullptr, (int32_t*)nullptr, (int)N);
     Carve cv(ws, bytes);
-    W.ctr = cv.take<unsigned long long>(4);
-    W.cnt = cv.take<int32_t>(N);
-    W.off = cv.take<int32_t>(N);
+    // [counters][ncore][cbits]
+    const size_t cb = pad ? N / 32 + 1 : 0, nc = pad ? kCoreWords : 0;
+    W.zero_words = (int64_t)(2 * kCounters + nc + cb);
+    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words));
+    W.ncore = pad ? reinterpret_cast<int32_t*>(W.ctr + kCounters) : nullptr;
+    W.cbits = pad ? reinterpret_cast<uint32_t*>(W.ncore + kCoreWords) : nullptr;
     W.cnth = cv.take<int32_t>(N);
     W.offh = cv.take<int32_t>(N);
-    W.px = cv.take<int32_t>(E);
     W.py = cv.take<int32_t>(E);
+    W.rows = cv.take<int2>(N);
     // every hub x with pairs opens one segment, every HUB_SEG_MIN pairs at most one more
     W.max_segs = (int64_t)(N < E ? N : E) + (int64_t)(E / HUB_SEG_MIN) + 1;
     W.segs = cv.take<HubSeg>((size_t)W.max_segs);
     W.pcap = pad ? pad_capacity(n_nodes, (int64_t)E) : 0;
     W.pcol = pad ? cv.take<int32_t>((size_t)W.pcap) : nullptr;
     W.cflag = pad ? cv.take<int32_t>(N) : nullptr;
-    W.cbits = pad ? cv.take<uint32_t>(N / 32 + 1) : nullptr;
-    W.ncore = pad ? cv.take<int32_t>(kCoreWords) : nullptr;
     W.pl = pad ? cv.take<int4>(N) : nullptr;
     W.pool_cap = pad ? (int64_t)(E / 16) + 1024 : 0;
     W.pool = pad ? cv.take<uint4>((size_t)W.pool_cap) : nullptr;
-    W.tmp_bytes = tb;
-    W.tmp = cv.take<char>(tb);
     if (need) *need = cv.off;
     return cv.ok();
 }
@@ -2413,7 +2704,6 @@ static bool carve_count_hybrid(void* ws, size_t bytes, int64_t n_nodes, int64_t 
     char* b = cv.take<char>(base);
     H.hll_u = cv.take<int32_t>(E);
     H.hll_v = cv.take<int32_t>(E);
-    H.hll_n = cv.take<unsigned long long>(1);
     H.zm = nullptr;
     H.zst = 0;
     if (zm_rows > 0) {
@@ -2423,6 +2713,7 @@ static bool carve_count_hybrid(void* ws, size_t bytes, int64_t n_nodes, int64_t 
     if (need) *need = cv.off;
     if (!cv.ok()) return false;
     if (!cv.dry) carve_count(b, base, n_nodes, n_edges, W, nullptr, pad);
+    H.hll_n = W.ctr + 4;
     return true;
 }
 
@@ -2519,47 +2810,80 @@ static int grid_edges(int64_t n) {
     return g < 1 ? 1 : (int)g;
 }
 
-// Pair regrouping, part 1: histogram of table sides and its exclusive scan
-// (W.off[x] = first pair of x, W.off[n_nodes] = number of pairs).
-// With hub > 0 the histogram is split into small and hub pairs, both are
-// scanned, and the hub segments are listed (before the scatter moves offh).
-template <bool HYB>
-static int pairs_hist_scan(const CountParams& P, const CountWs& W, int hub, int hub_seg, cudaStream_t st,
-                           const int32_t* vbase = nullptr, int64_t n_graphs = 0) {
-    const int64_t N = P.n_nodes + 1;
-    TCHLL_CUDA(cudaMemsetAsync(W.cnt, 0, sizeof(int32_t) * N, st));
-    pair_hist_kernel<HYB><<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.cnt);
-    TCHLL_CHECK_LAUNCH("pair_hist_kernel");
-    if (hub > 0) {
-        hub_split_kernel<<<grid_edges(N), 256, 0, st>>>(P.row_ptr, P.n_nodes, hub, W.cnt, W.cnth);
-        TCHLL_CHECK_LAUNCH("hub_split_kernel");
-    }
-    size_t tb = W.tmp_bytes;
-    TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(W.tmp, tb, W.cnt, W.off, (int)N, st));
-    count_launch();
-    if (hub > 0) {
-        tb = W.tmp_bytes;
-        TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(W.tmp, tb, W.cnth, W.offh, (int)N, st));
-        count_launch();
-        hub_segments_kernel<<<grid_edges(P.n_nodes), 256, 0, st>>>(W.cnth, W.offh, W.off + P.n_nodes, P.n_nodes,
-                                                                   hub_seg, W.segs, W.ctr + 2,
-                                                                   W.max_segs, vbase, n_graphs);
-        TCHLL_CHECK_LAUNCH("hub_segments_kernel");
-    }
+// Before the first pass: the row table, and all counters, flags and results
+// cleared (more: words of the caller's own).
+static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_results, uint32_t* more,
+                        int64_t more_words, cudaStream_t st) {
+    Prepare Q{};
+    Q.row_ptr = P.row_ptr;
+    Q.n_nodes = P.n_nodes;
+    Q.rows = W.rows;
+    Q.zero_n[0] = hub > 0 ? W.cnth : nullptr;
+    Q.zero_n[1] = hub > 0 ? W.cflag : nullptr;
+    Q.zero[0] = reinterpret_cast<uint32_t*>(W.ctr);
+    Q.words[0] = W.zero_words;
+    Q.zero[1] = reinterpret_cast<uint32_t*>(P.result);
+    Q.words[1] = n_results * (int64_t)(sizeof(tchll_count_result) / 4);
+    Q.zero[2] = more;
+    Q.words[2] = more_words;
+    prepare_kernel<<<grid_edges(P.n_nodes + 1), 256, 0, st>>>(Q);
+    TCHLL_CHECK_LAUNCH("prepare_kernel");
+    P.rows = W.rows;
     return TCHLL_OK;
 }
 
-// Part 2: scatter the pairs (advances W.off[x] / W.offh[x] for x < n_nodes
-// only, so the totals in [n_nodes] survive) and point Q at the small-pair list.
+// Edges per claim: a few claims per warp at least, so that the last ones
+// even out.
+static int pass_chunk(int64_t n_edges, int chunk) {
+    while (chunk > 32 && n_edges < (int64_t)chunk * 48 * 8 * sm_count()) chunk >>= 1;
+    return chunk < 32 ? 32 : chunk & ~31;
+}
+
+// The first pass: `what` of PASS_HIST (hub pairs counted per table side) and
+// PASS_SHORT (all others counted for good).
 template <bool HYB>
-static int pairs_scatter(const CountParams& P, const CountWs& W, int hub, CountParams& Q, cudaStream_t st) {
-    pair_scatter_kernel<HYB><<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.off, W.offh, hub, W.off + P.n_nodes,
-                                                                   W.px, W.py);
+static int pair_pass(CountParams P, const CountWs& W, int what, int hub, unsigned long long* work, cudaStream_t st) {
+    const bool vec = (uintptr_t)P.col_idx % 16 == 0;
+    auto kern = vec ? pair_pass_kernel<HYB, true> : pair_pass_kernel<HYB, false>;
+    static int bps[kMaxDevices] = {};
+    const int dev = current_device();
+    if (dev < 0) return cuda_status(cudaErrorInvalidDevice, "cudaGetDevice");
+    if (bps[dev] == 0) {
+        int b = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 256, 0);
+        if (e != cudaSuccess) return cuda_status(e, "occupancy(pair_pass_kernel)");
+        bps[dev] = b < 1 ? 1 : b;
+    }
+    P.work = work;
+    int64_t grid = (int64_t)sm_count() * bps[dev];
+    if (!P.chunk_start) {  // no more warps than chunks
+        const int64_t need = (P.n_edges + 8 * (int64_t)P.chunk - 1) / (8 * (int64_t)P.chunk);
+        const int64_t ids = P.check_ids ? (P.n_nodes > P.nnz / 4 ? P.n_nodes : P.nnz / 4) / 1024 + 1 : 1;
+        const int64_t most = need > ids ? need : ids;
+        if (grid > most) grid = most;
+    }
+    kern<<<(int)grid, 256, 0, st>>>(P, what, hub, W.cnth);
+    TCHLL_CHECK_LAUNCH("pair_pass_kernel");
+    return TCHLL_OK;
+}
+
+// After PASS_HIST: room for the hub pairs, and the hub segments (smaller ones
+// in small graphs, so that every CTA gets a few).
+static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaStream_t st,
+                     const int32_t* vbase = nullptr, int64_t n_graphs = 0) {
+    while (hub_seg > HUB_SEG_MIN && P.n_edges < (int64_t)hub_seg * 24 * sm_count()) hub_seg >>= 1;
+    if (hub_seg < HUB_SEG_MIN) hub_seg = HUB_SEG_MIN;
+    const int grid = (int)(P.n_nodes > 0 ? (P.n_nodes + 1023) / 1024 : 1);
+    hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, P.n_nodes, hub_seg, W.offh, W.ctr + 5, W.segs, W.ctr + 2,
+                                           W.max_segs, vbase, n_graphs);
+    TCHLL_CHECK_LAUNCH("hub_alloc_kernel");
+    return TCHLL_OK;
+}
+
+template <bool HYB>
+static int pairs_scatter(const CountParams& P, const CountWs& W, int hub, cudaStream_t st) {
+    pair_scatter_kernel<HYB><<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.offh, W.ctr + 5, hub, W.py);
     TCHLL_CHECK_LAUNCH("pair_scatter_kernel");
-    Q = P;
-    Q.edge_u = W.px;
-    Q.edge_v = W.py;
-    Q.n_edges_dev = W.off + P.n_nodes;
     return TCHLL_OK;
 }
 
@@ -2588,29 +2912,34 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
         cudaEventRecord(g_phase.hub_ev[0], st);
         g_phase.core_used = true;
     }
-    const int64_t N = P.n_nodes + 1;
-    TCHLL_CUDA(cudaMemsetAsync(W.cflag, 0, sizeof(int32_t) * N, st));
-    TCHLL_CUDA(cudaMemsetAsync(W.cbits, 0, sizeof(uint32_t) * (N / 32 + 1), st));
-    TCHLL_CUDA(cudaMemsetAsync(W.ncore, 0, sizeof(int32_t) * kCoreWords, st));
     core_mark_kernel<<<sm_count() * 8, 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.segs, W.ctr + 2,
                                                       W.max_segs, W.cbits, W.cflag, P.result);
     TCHLL_CHECK_LAUNCH("core_mark_kernel");
-    int64_t gv = (P.n_nodes + 1023) / 1024;
-    gv = gv < 1 ? 1 : (gv > 4 * (int64_t)sm_count() ? 4 * (int64_t)sm_count() : gv);
-    core_bucket_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4);
-    TCHLL_CHECK_LAUNCH("core_bucket_kernel");
-    core_index_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4, W.ncore + 4 + 256, W.ncore);
-    TCHLL_CHECK_LAUNCH("core_index_kernel");
+    if (P.graph_vbase) {
+        core_index_batch_kernel<<<(int)P.n_graphs, 1024, 0, st>>>(W.cbits, W.cflag, P.n_nodes, P.graph_vbase,
+                                                                 P.graph_hub, P.live_flag, P.live_list,
+                                                                 W.ncore + kCoreWords - 1, W.ncore);
+        TCHLL_CHECK_LAUNCH("core_index_batch_kernel");
+    } else {
+        int64_t gv = (P.n_nodes + 1023) / 1024;
+        gv = gv < 1 ? 1 : (gv > 4 * (int64_t)sm_count() ? 4 * (int64_t)sm_count() : gv);
+        core_bucket_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4);
+        TCHLL_CHECK_LAUNCH("core_bucket_kernel");
+        core_index_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4, W.ncore + 4 + 256, W.ncore);
+        TCHLL_CHECK_LAUNCH("core_index_kernel");
+    }
     int64_t gl = (P.n_nodes + 63) / 64;
     gl = gl < 1 ? 1 : (gl > 6 * (int64_t)sm_count() ? 6 * (int64_t)sm_count() : gl);
     core_lists_kernel<<<(int)gl, 256, 0, st>>>(
         P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag, W.ncore, T.packed, reinterpret_cast<uint16_t*>(W.pcol), W.pl,
         W.pool, (int32_t)(W.pool_cap < INT32_MAX / 2 ? W.pool_cap : INT32_MAX / 2), W.ncore + 1,
-        reinterpret_cast<unsigned long long*>(W.ncore + 2), W.ctr + 2, P.result);
+        reinterpret_cast<unsigned long long*>(W.ncore + 2), W.ctr + 2, P.live_list, W.ncore + kCoreWords - 1, P.result);
     TCHLL_CHECK_LAUNCH("core_lists_kernel");
-    core_pad_kernel<<<grid_rows(P.n_nodes, 32), 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag,
-                                                              W.ncore, T.packed, W.pcol, P.result);
-    TCHLL_CHECK_LAUNCH("core_pad_kernel");
+    if (!T.packed || P.n_nodes > kCore16Max) {  // else the packed lists always apply
+        core_pad_kernel<<<grid_rows(P.n_nodes, 32), 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag,
+                                                                  W.ncore, T.packed, W.pcol, P.result);
+        TCHLL_CHECK_LAUNCH("core_pad_kernel");
+    }
     if (ps.active()) cudaEventRecord(g_phase.hub_ev[1], st);
     return TCHLL_OK;
 }
@@ -2659,7 +2988,8 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
         kern<<<sm_count() * bps, kHub16Threads, smem, st>>>(H);
         TCHLL_CHECK_LAUNCH("hub_bitmap16_kernel");
     }
-    if (pad && T.bitmap_lg > 0) {
+    const bool sure = pad && T.packed && P.n_nodes <= kCore16Max;  // the packed lists apply: C <= n_nodes
+    if (pad && T.bitmap_lg > 0 && !sure) {
         const size_t smem = (size_t)1 << T.bitmap_lg;
         H.cap_bits = (int)(8 * smem);
         auto kern = T.hub_unroll == 4 ? hub_bitmap_kernel<4> : hub_bitmap_kernel<2>;
@@ -2673,6 +3003,13 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
         if (bps < 1) bps = 1;
         kern<<<sm_count() * bps, 256, smem, st>>>(H);
         TCHLL_CHECK_LAUNCH("hub_bitmap_kernel");
+    }
+    if (sure) {
+        if (ps.active()) {
+            cudaEventRecord(g_phase.hub_ev[3], st);
+            g_phase.hub_used = true;
+        }
+        return TCHLL_OK;
     }
     const int vi = (T.hub_unroll == 4 ? 2 : 0) + (pad ? 1 : 0);
     auto kern = vi == 3 ? hub_count_kernel<4, true>
@@ -2694,9 +3031,22 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
     return TCHLL_OK;
 }
 
-// Hub path in use: pairs on, and 16-byte aligned col_idx (quad loads).
-static int hub_threshold(const CountParams& P, const Tuning& T) {
-    return (T.hub > 0 && (uintptr_t)P.col_idx % 16 == 0) ? T.hub : 0;
+// Hub path in use: with the packed or padded lists, or (quad loads of the
+// raw ones) a 16-byte aligned col_idx.
+// The default threshold, 128, is taken as 64 up to kHub64Edges edges: bitmap
+// lists are the faster way for pairs of 64 to 128 members too, as long as the
+// core that they bring in fits the packed lists (R-MAT 17 / 18 / 20, edge
+// factor 16 to 21: 630 / 789 / 2006 us at 128, 480 / 569 / 1719 at 64; R-MAT 22
+// with edge factor 2: 1325, 897; R-MAT 22 has a core of 108 K vertices at 128,
+// 262 K at 64).  Batches number each graph's core on its own, so the size does
+// not matter there, but they need many such pairs to a table side for the
+// core pass, which nothing overlaps, to pay: a mean forward degree of 12 (256
+// R-MAT 12, mean 19: 2.56 ms at 128, 1.85 at 64; 40 R-MAT 13, mean 10.5: 367,
+// 443 us).
+static int hub_threshold(const CountParams& P, const CountWs& W, const Tuning& T) {
+    if (T.hub <= 0 || (!hub_pad_usable(P, W) && (uintptr_t)P.col_idx % 16 != 0)) return 0;
+    const bool half = P.graph_vbase ? P.n_edges >= kHub64Degree * P.n_nodes : P.n_edges <= kHub64Edges;
+    return T.hub == kHubDefault && half ? kHubDefault / 2 : T.hub;
 }
 
 // A second stream per device for work that overlaps the caller's stream: the
@@ -2710,7 +3060,7 @@ static int hub_threshold(const CountParams& P, const Tuning& T) {
 // capture: the first call of a process is never captured by this package).
 struct SideStream {
     cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr, back = nullptr;
+    cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr;
     std::mutex mu;
 };
 static SideStream g_side[kMaxDevices];
@@ -2731,7 +3081,6 @@ class SideFork {
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming));
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.mid, cudaEventDisableTiming));
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming));
-                TCHLL_CUDA(cudaEventCreateWithFlags(&S.back, cudaEventDisableTiming));
             }
         }
         lock_ = std::unique_lock<std::mutex>(S.mu);
@@ -2750,12 +3099,6 @@ class SideFork {
     }
     int wait_mark() {
         TCHLL_CUDA(cudaStreamWaitEvent(caller_, side_->mid, 0));
-        return TCHLL_OK;
-    }
-    // The side stream waits for the caller's work so far (once per fork).
-    int side_waits_caller() {
-        TCHLL_CUDA(cudaEventRecord(side_->back, caller_));
-        TCHLL_CUDA(cudaStreamWaitEvent(side_->s, side_->back, 0));
         return TCHLL_OK;
     }
     // Joins: the caller's stream waits for everything enqueued on the side
@@ -2803,44 +3146,63 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
         set_error("workspace too small: need %zu bytes, have %zu", need, ws_bytes);
         return TCHLL_EWORKSPACE;
     }
-    const bool direct = P.n_edges <= kDirectEdges && P.n_edges <= kDirectDegree * P.n_nodes && T.pairs != 2;
-    if (!direct || mode != MODE_EXACT)  // a direct exact count claims nothing
-        TCHLL_CUDA(cudaMemsetAsync(W.ctr, 0, 4 * sizeof(unsigned long long), st));
-    TCHLL_CUDA(cudaMemsetAsync(P.result, 0, sizeof(tchll_count_result), st));
+    const bool direct = T.pairs != 2 && (P.n_edges <= kDirectEdges ? P.n_edges <= kDirectDegree * P.n_nodes
+                                                                   : P.n_edges <= kRoadDegree * P.n_nodes);
+    const bool direct_pass = direct && T.pairs && !details;
+    const bool sparse = P.n_edges <= kSparseDegree * P.n_nodes;
+    const bool pairs = T.pairs && !details && !direct;
+    const bool prepared = pairs && P.n_edges > 0 &&
+                          (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));  // by pass_prepare
+    if (!prepared) {
+        if (!direct_pass || mode != MODE_EXACT)  // a direct exact count claims nothing
+            TCHLL_CUDA(cudaMemsetAsync(W.ctr, 0, kCounters * sizeof(unsigned long long), st));
+        TCHLL_CUDA(cudaMemsetAsync(P.result, 0, sizeof(tchll_count_result), st));
+    }
     if (details && P.pe_support) TCHLL_CUDA(cudaMemsetAsync(P.pe_support, 0, sizeof(int64_t) * P.n_edges, st));
     if (details && P.pe_method) TCHLL_CUDA(cudaMemsetAsync(P.pe_method, 0, P.n_edges, st));
     P.chunk = T.chunk;
     P.slots_log2 = T.slots_log2;
     P.tiny = T.tiny;
     P.sparse = T.sparse;
-    P.n_edges_dev = nullptr;
     P.hll_u = nullptr;
     P.hll_v = nullptr;
     P.hll_n = nullptr;
     if (P.n_edges == 0) return TCHLL_OK;
     // small graphs refuse what the hub core's passes refuse in large ones
-    P.check_ids = direct && T.pairs && !details && hub_threshold(P, T) > 0 && hub_pad_usable(P, W) &&
+    P.check_ids = direct_pass && T.hub > 0 && (uintptr_t)P.col_idx % 16 == 0 && hub_pad_usable(P, W) &&
                   (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));
-    const bool pairs = T.pairs && !details && !direct;
-    if (!pairs) P.chunk = given_chunk(P.n_edges, T.chunk);
+    if (direct_pass) P.chunk = P.n_edges <= kDirectEdges ? given_chunk(P.n_edges, T.chunk) : pass_chunk(P.n_edges, T.chunk);
     if (col_ready && !(mode == MODE_EXACT && pairs)) {
         TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
         col_ready = nullptr;
     }
     int rc;
-    CountParams Q;
+    const int hub = hub_threshold(P, W, T);
     PhaseScope ps;
     phase_reset(ps);
     switch (mode) {
         case MODE_EXACT:
-            P.work = W.ctr;
+            if (direct_pass) {
+                P.work = nullptr;
+                phase_mark(ps, 1, st);
+                rc = sparse ? pair_pass<false>(P, W, PASS_SHORT, 0, nullptr, st) : launch_count<MODE_EXACT>(P, T, false, st);
+                phase_mark(ps, 2, st);
+                phase_used(ps, 1);
+                return rc;
+            }
             if (pairs) {
-                // after the histogram, the hub core pass runs on the side
-                // stream beside the pair scatter and the short-list pairs;
-                // the hub kernels wait for it
-                const int hub = hub_threshold(P, T);
+                // after the first pass, the hub core pass runs on the side
+                // stream beside the pair scatter; the hub kernels wait for
+                // both.  While col_idx is still being copied, the short-list
+                // pairs, which read it, come after the scatter instead.
                 phase_mark(ps, 0, st);
-                rc = pairs_hist_scan<false>(P, W, hub, T.hub_seg, st);
+                P.chunk = pass_chunk(P.n_edges, T.chunk);
+                rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
+                if (rc) return rc;
+                const bool split = col_ready && hub > 0;
+                if (col_ready && !split) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
+                rc = pair_pass<false>(P, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc) return rc;
                 SideFork fork;
                 const bool side = hub > 0 && T.overlap && hub_pad_usable(P, W);
@@ -2854,30 +3216,24 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
-                rc = pairs_scatter<false>(P, W, hub, Q, st);
+                if (hub > 0) rc = pairs_scatter<false>(P, W, hub, st);
                 if (rc) return rc;
-                if (col_ready) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
+                if (split) {
+                    TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
+                    rc = pair_pass<false>(P, W, PASS_SHORT, hub, W.ctr + 1, st);
+                    if (rc) return rc;
+                }
                 phase_mark(ps, 1, st);
-                if (side && T.overlap >= 2) {
-                    // the short-list pairs follow the core pass on the side
-                    // stream (once scattered) and run beside the hub kernel
-                    rc = fork.side_waits_caller();
-                    if (rc == TCHLL_OK) rc = launch_count<MODE_EXACT>(Q, T, false, fork.stream());
-                    if (rc == TCHLL_OK) rc = fork.wait_mark();
+                if (hub > 0) {
+                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
-                } else {
-                    rc = launch_count<MODE_EXACT>(Q, T, false, st);
-                    if (rc == TCHLL_OK && hub > 0) {
-                        rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, ps, st);
-                        if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
-                    }
                 }
                 phase_mark(ps, 2, st);
                 const int rj = fork.end();
                 phase_used(ps, 0, 1);
                 return rc ? rc : rj;
             }
-            if (direct) P.work = nullptr;
+            P.work = W.ctr;
             phase_mark(ps, 1, st);
             rc = launch_count<MODE_EXACT>(P, T, details, st);
             phase_mark(ps, 2, st);
@@ -2892,22 +3248,23 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
             return rc;
         case 2:  // split: exact-routed edges, then HLL-routed edges
             if (pairs && ((uintptr_t)P.regs % 16 == 0)) {
-                // One routing pass builds both work lists: the exact pairs
-                // (counted by the pair launches, which also count n_exact)
-                // and the HLL edge list (estimated by hll_edges_kernel, which
-                // counts n_approx / n_clamped); the routing pass counts
-                // n_fallback.  The HLL pass needs only the routing pass, so
-                // it forks onto the side stream there and overlaps the
-                // scatter and the pair launches (all add integers into the
-                // same result block).
+                // One first pass routes: it counts the short-list exact pairs
+                // (and n_fallback), lists the hub pairs' table sides and the
+                // HLL edges (estimated by hll_edges_kernel, which counts
+                // n_approx / n_clamped).  The HLL pass needs only that pass,
+                // so it forks onto the side stream there and overlaps the
+                // scatter and the hub kernels (all add integers into the same
+                // result block).
                 P.work = W.ctr;
                 P.hll_u = HW.hll_u;
                 P.hll_v = HW.hll_v;
                 P.hll_n = HW.hll_n;
-                TCHLL_CUDA(cudaMemsetAsync(HW.hll_n, 0, sizeof(unsigned long long), st));
-                const int hub = hub_threshold(P, T);
                 phase_mark(ps, 0, st);
-                rc = pairs_hist_scan<true>(P, W, hub, T.hub_seg, st);
+                P.chunk = pass_chunk(P.n_edges, T.chunk);
+                rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
+                if (rc) return rc;
+                rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc) return rc;
                 // side stream: the hub core pass first (the hub kernels wait
                 // for it), then the HLL pass
@@ -2928,12 +3285,9 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 rc = launch_hll_edges(P, HW, T, hst);
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[1], hst);
                 if (rc) return rc;
-                rc = pairs_scatter<true>(P, W, hub, Q, st);
+                if (hub > 0) rc = pairs_scatter<true>(P, W, hub, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
-                Q.hll_u = nullptr;
-                rc = launch_count<MODE_EXACT>(Q, T, false, st);
-                if (rc) return rc;
                 if (hub > 0) {
                     rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
@@ -2945,14 +3299,15 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 if (ps.active()) g_phase.hll_split = true;
                 return rc;
             }
-            if (direct && T.pairs && !details && ((uintptr_t)P.regs % 16 == 0)) {
-                // the exact launch lists the HLL edges for hll_edges_kernel
+            if (direct_pass && ((uintptr_t)P.regs % 16 == 0)) {
+                // the pass lists the HLL edges for hll_edges_kernel
                 P.hll_u = HW.hll_u;
                 P.hll_v = HW.hll_v;
                 P.hll_n = HW.hll_n;
-                TCHLL_CUDA(cudaMemsetAsync(HW.hll_n, 0, sizeof(unsigned long long), st));
                 phase_mark(ps, 1, st);
-                rc = launch_count<MODE_HYB_EXACT>(P, T, false, st);
+                P.work = nullptr;
+                rc = sparse ? pair_pass<true>(P, W, PASS_SHORT, 0, nullptr, st)
+                            : launch_count<MODE_HYB_EXACT>(P, T, false, st);
                 if (rc) return rc;
                 phase_mark(ps, 2, st);
                 rc = launch_hll_edges(P, HW, T, st);
@@ -3348,7 +3703,7 @@ TCHLL_EXPORT int tchll_exact_count_noalloc(const int32_t* row_ptr, int64_t n_nod
     size_t need = 0;
     carve_count(nullptr, 0, n_nodes, n_edges, W, &need, false);  // padded lists only when they fit too
     if (need > (size_t)TCHLL_NOALLOC_SCRATCH_BYTES) {
-        set_error("graph too large for tchll_exact_count_noalloc: needs %zu bytes of scratch (about 8 per edge + "
+        set_error("graph too large for tchll_exact_count_noalloc: needs %zu bytes of scratch (about 4 per edge + "
                   "32 per vertex), the fixed limit is %u bytes; use tchll_exact_count with a workspace",
                   need, (unsigned)TCHLL_NOALLOC_SCRATCH_BYTES);
         return TCHLL_EINVAL;
@@ -3440,6 +3795,10 @@ struct BatchWs {
     int64_t* cstart;  // max chunks
     int32_t* clen;
     int32_t* cgraph;
+    int32_t* ghub;    // n_graphs: the graph has hub pairs
+    int32_t* rflag;   // n_nodes / 64 + 1: 64 rows touch such a graph
+    int32_t* rlist;   // those blocks
+    size_t flag_bytes;  // of ghub and rflag, which are next to each other
     void* tmp;
     size_t tmp_bytes;
 };
@@ -3463,17 +3822,22 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     B.cstart = cv.take<int64_t>(MC);
     B.clen = cv.take<int32_t>(MC);
     B.cgraph = cv.take<int32_t>(MC);
+    const size_t RL = (size_t)(n_nodes > 0 ? n_nodes : 0) / 64 + 1;
+    B.flag_bytes = (G + RL) * sizeof(int32_t);
+    B.ghub = cv.take<int32_t>(G + 2 * RL);
+    B.rflag = B.ghub + G;
+    B.rlist = B.rflag + RL;
     B.tmp_bytes = tb;
     B.tmp = cv.take<char>(tb);
     const size_t E = (size_t)(n_edges > 0 ? n_edges : 1);
     B.hw.hll_u = cv.take<int32_t>(E);
     B.hw.hll_v = cv.take<int32_t>(E);
-    B.hw.hll_n = cv.take<unsigned long long>(1);
     B.hw.zm = nullptr;
     B.hw.zst = 0;
     if (need) *need = cv.off;
     if (!cv.ok() || cv.dry) return cv.ok();
     carve_count(cbase, cneed, n_nodes, n_edges, B.cw, nullptr);
+    B.hw.hll_n = B.cw.ctr + 4;
     return true;
 }
 
@@ -3496,6 +3860,15 @@ static int build_chunks(const int32_t* base, const int32_t* vbase, int64_t n_gra
     return TCHLL_OK;
 }
 
+static int check_vbase(const int32_t* vbase, int64_t n_graphs, int64_t n_nodes, tchll_count_result* results,
+                       cudaStream_t st) {
+    int64_t g = (n_graphs + 255) / 256;
+    if (g > 1024) g = 1024;
+    check_vbase_kernel<<<(int)g, 256, 0, st>>>(vbase, n_graphs, n_nodes, results);
+    TCHLL_CHECK_LAUNCH("check_vbase_kernel");
+    return TCHLL_OK;
+}
+
 static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n_graphs, void* ws, size_t wsb,
                      cudaStream_t st) {
     const Tuning T = tuning_snapshot();
@@ -3505,32 +3878,25 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
         set_error("workspace too small: need %zu bytes, have %zu", need, wsb);
         return TCHLL_EWORKSPACE;
     }
-    TCHLL_CUDA(cudaMemsetAsync(P.result, 0, sizeof(tchll_count_result) * n_graphs, st));
-    TCHLL_CUDA(cudaMemsetAsync(B.cw.ctr, 0, 4 * sizeof(unsigned long long), st));
+    if (n_graphs == 0 || P.n_edges == 0) TCHLL_CUDA(cudaMemsetAsync(P.result, 0, sizeof(tchll_count_result) * n_graphs, st));
     if (n_graphs == 0) return TCHLL_OK;
-    {
-        int64_t g = (n_graphs + 255) / 256;
-        if (g > 1024) g = 1024;
-        check_vbase_kernel<<<(int)g, 256, 0, st>>>(vbase, n_graphs, P.n_nodes, P.result);
-        TCHLL_CHECK_LAUNCH("check_vbase_kernel");
-    }
     P.chunk = T.chunk;
     P.slots_log2 = T.slots_log2;
     P.tiny = T.tiny;
     P.sparse = T.sparse;
-    P.n_edges_dev = nullptr;
     P.graph_vbase = vbase;
     P.n_graphs = n_graphs;
     P.n_chunks_dev = B.coff + n_graphs;
     P.chunk_start = B.cstart;
     P.chunk_len = B.clen;
     P.chunk_graph = B.cgraph;
-    if (P.n_edges == 0) return TCHLL_OK;
+    P.graph_hub = B.ghub;
+    P.live_flag = B.rflag;
+    P.live_list = B.rlist;
     int rc;
-    CountParams Q;
+    if (P.n_edges == 0) return check_vbase(vbase, n_graphs, P.n_nodes, P.result, st);
     PhaseScope ps;
     phase_reset(ps);
-    P.work = B.cw.ctr;
     // Hybrid: the routing pass also appends the HLL-routed edges to a list
     // (16-byte aligned register rows; else the HLL edges take a second pass
     // over each graph's edges below).
@@ -3538,25 +3904,31 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     P.hll_u = hll_list ? B.hw.hll_u : nullptr;
     P.hll_v = hll_list ? B.hw.hll_v : nullptr;
     P.hll_n = hll_list ? B.hw.hll_n : nullptr;
-    if (hll_list) TCHLL_CUDA(cudaMemsetAsync(B.hw.hll_n, 0, sizeof(unsigned long long), st));
     phase_mark(ps, 0, st);
-    // pairs with a long table side go to the hub kernels, which publish per
-    // segment into the graph of x
-    const int hub = hub_threshold(P, T);
-    if (hybrid) rc = pairs_hist_scan<true>(P, B.cw, hub, T.hub_seg, st, vbase, n_graphs);
-    else rc = pairs_hist_scan<false>(P, B.cw, hub, T.hub_seg, st, vbase, n_graphs);
+    // one pass over each graph's edges as given; pairs with a long table side
+    // go to the hub kernels, which publish per segment into the graph of x
+    const int hub = hub_threshold(P, B.cw, T);
+    rc = pass_prepare(P, B.cw, hub, n_graphs, reinterpret_cast<uint32_t*>(B.ghub), (int64_t)(B.flag_bytes / 4), st);
+    if (rc == TCHLL_OK) rc = check_vbase(vbase, n_graphs, P.n_nodes, P.result, st);
+    if (rc == TCHLL_OK) rc = build_chunks(P.row_ptr, vbase, n_graphs, P.n_nodes, B, T.chunk, st);
     if (rc) return rc;
-    rc = build_chunks(B.cw.off, vbase, n_graphs, P.n_nodes, B, T.chunk, st);  // pair ranges (before the scatter)
-    if (rc) return rc;
-    if (hybrid) rc = pairs_scatter<true>(P, B.cw, hub, Q, st);
-    else rc = pairs_scatter<false>(P, B.cw, hub, Q, st);
-    if (rc) return rc;
+    if (hll_list || !hybrid) {
+        if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, hub, B.cw.ctr, st);
+        else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, hub, B.cw.ctr, st);
+        if (rc) return rc;
+    } else {
+        P.work = B.cw.ctr;
+        rc = launch_count<MODE_HYB_EXACT>(P, T, false, st);
+        if (rc) return rc;
+    }
+    const bool hubs = hub > 0 && (hll_list || !hybrid);
+    if (hubs) {
+        rc = hub_alloc(P, B.cw, T.hub_seg, st, vbase, n_graphs);
+        if (rc == TCHLL_OK) rc = hybrid ? pairs_scatter<true>(P, B.cw, hub, st) : pairs_scatter<false>(P, B.cw, hub, st);
+        if (rc) return rc;
+    }
     phase_mark(ps, 1, st);
-    Q.n_edges_dev = nullptr;
-    Q.hll_u = nullptr;
-    rc = launch_count<MODE_EXACT>(Q, T, false, st);
-    if (rc) return rc;
-    if (hub > 0) {
+    if (hubs) {
         rc = launch_core_pass(P, B.cw, T, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
@@ -3571,9 +3943,6 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
         return rc;
     }
     // HLL-routed edges: chunks over each graph's CSR edge range
-    TCHLL_CUDA(cudaMemsetAsync(B.cw.ctr + 1, 0, sizeof(unsigned long long), st));
-    rc = build_chunks(P.row_ptr, vbase, n_graphs, P.n_nodes, B, T.chunk, st);
-    if (rc) return rc;
     P.work = B.cw.ctr + 1;
     rc = launch_count<MODE_HYB_HLL>(P, T, false, st);
     phase_mark(ps, 3, st);
