@@ -54,7 +54,11 @@ struct CsrWs {
     size_t tmp_bytes;
 };
 
+// (the same call asks three times per build: the last answer of the thread is kept)
 static size_t csr_cub_tmp(int64_t n_raw) {
+    static thread_local int64_t last_n = -1;
+    static thread_local size_t last_bytes = 0;
+    if (n_raw == last_n) return last_bytes;
     const int R = (int)(n_raw > 0 ? n_raw : 1);
     size_t a = 0, b = 0, c = 0, d = 0, e = 0, f = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, a, (uint64_t*)nullptr, (uint64_t*)nullptr, R, 0, 63);
@@ -70,6 +74,8 @@ static size_t csr_cub_tmp(int64_t n_raw) {
     if (d > m) m = d;
     if (e > m) m = e;
     if (f > m) m = f;
+    last_n = n_raw;
+    last_bytes = m;
     return m;
 }
 
@@ -314,6 +320,263 @@ static int bits_for(int64_t maxv) {
     return b;
 }
 
+// ------------------------------------------------------- small builds ------
+// Up to kSmallRaw raw edges the dozen sort passes cost their launches and
+// little else, so the build takes another way: the canonical pairs go into a
+// hash table (2 n_raw slots, in the sort's key buffers), which drops
+// duplicates and counts the degrees as it goes (ids too large for direct
+// tables are first replaced by their rank among the sorted endpoints); the
+// oriented pairs are scattered from the table into their rows, in
+// no order, and a warp sorts each row in registers or shared memory.  A
+// forward list has at most sqrt(2 n_edges) members (each of the d members of
+// u's list has a degree of at least u's, which is at least d), 2048 here.
+// Whole builds, sorted / so: R-MAT 10, 13, 15, 16, 17 (16 K, 90 K, 524 K, 1 M, 2 M
+// raw edges) 197 / 119, 236 / 138, 281 / 208, 343 / 289, 507 / 437 us; bound by
+// launches and the two read-backs, then by the atomics on the popular ids.
+constexpr int64_t kSmallRaw = 1 << 21;
+constexpr int kSmallRow = 2048;
+constexpr uint64_t kEmptySlot = ~0ull;
+
+__device__ __forceinline__ uint32_t pair_slot(uint64_t key, uint32_t slots) {
+    return (uint32_t)__umul64hi(splitmix64_fin(key), (uint64_t)slots);
+}
+
+// Endpoints of the raw edges; self-loops become kEndSentinel.
+__global__ void small_ends_kernel(const int32_t* __restrict__ ru, const int32_t* __restrict__ rv, int64_t n,
+                                  uint32_t* ends) {
+    GRID_STRIDE(i, n) {
+        const bool loop = ru[i] == rv[i];
+        ends[2 * i] = loop ? kEndSentinel : (uint32_t)ru[i];
+        ends[2 * i + 1] = loop ? kEndSentinel : (uint32_t)rv[i];
+    }
+}
+
+// cnt[0] += unique pairs; deg[id]: undirected degrees.  With nodes (sorted,
+// cnt[1] of them) an id stands for its place there.
+__global__ void small_insert_kernel(const int32_t* __restrict__ ru, const int32_t* __restrict__ rv, int64_t n,
+                                    const uint32_t* __restrict__ nodes, unsigned long long* table, uint32_t slots,
+                                    int32_t* deg, int64_t* cnt) {
+    uint32_t fresh = 0;
+    const int64_t nn = nodes ? n_real_nodes(nodes, cnt) : 0;
+    GRID_STRIDE(i, n) {
+        int32_t u = ru[i], v = rv[i];
+        if (u == v) continue;  // negative ids never get here
+        if (nodes) {
+            u = (int32_t)lower_bound_u32(nodes, nn, (uint32_t)u);
+            v = (int32_t)lower_bound_u32(nodes, nn, (uint32_t)v);
+        }
+        const uint64_t key = ((uint64_t)(uint32_t)min(u, v) << 32) | (uint32_t)max(u, v);
+        uint32_t s = pair_slot(key, slots);
+        bool mine = false;
+        for (uint32_t k = 0; k < slots; ++k) {  // at most half the slots ever fill
+            const unsigned long long old = atomicCAS(table + s, kEmptySlot, key);
+            mine = old == kEmptySlot;
+            if (mine || old == key) break;
+            s = s + 1 < slots ? s + 1 : 0;
+        }
+        if (mine) {
+            ++fresh;
+            atomicAdd(deg + u, 1);
+            atomicAdd(deg + v, 1);
+        }
+    }
+    fresh = __reduce_add_sync(0xFFFFFFFFu, fresh);
+    if ((threadIdx.x & 31) == 0 && fresh) atomicAdd((unsigned long long*)cnt, (unsigned long long)fresh);
+}
+
+// Tiles of 1024 entries, 256 threads: how many entries count (FLAG: 1 per
+// non-zero entry, else the entry itself).
+template <bool FLAG>
+__global__ void __launch_bounds__(256) tile_sum_kernel(const int32_t* __restrict__ in, int64_t n, int32_t* sums) {
+    __shared__ int32_t w[8];
+    int32_t c = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int64_t k = blockIdx.x * 1024ll + 256 * i + threadIdx.x;
+        const int32_t x = k < n ? in[k] : 0;
+        c += FLAG ? (x != 0) : x;
+    }
+    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int32_t t = 0;
+        for (int i = 0; i < 8; ++i) t += w[i];
+        sums[blockIdx.x] = t;
+    }
+}
+
+// Exclusive prefix of this thread's 4 consecutive entries x[] of the tile, by
+// adding up the tiles before (no tile waits for another).
+__device__ __forceinline__ int32_t tile_prefix(const int32_t* __restrict__ sums, int32_t mine, int32_t* w) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    int32_t before = 0;
+    for (int64_t k = tid; k < (int64_t)blockIdx.x; k += 256) before += __ldg(sums + k);
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    int32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) w[tid >> 5] = incl;
+    if (lane == 0) w[8 + (tid >> 5)] = before;
+    __syncthreads();
+    int32_t base = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        base += w[8 + i];
+        if (i < (tid >> 5)) base += w[i];
+    }
+    return base + incl - mine;
+}
+
+// rank[id] among the ids that occur, nodes[rank] = id (or, when the ids stand
+// for places in nodes already, left alone); the last tile writes the sizes.
+__global__ void __launch_bounds__(256) small_rank_kernel(const int32_t* __restrict__ deg, int64_t ids,
+                                                         const int32_t* __restrict__ sums, int32_t* rank,
+                                                         uint32_t* nodes, int places, const int64_t* cnt,
+                                                         int64_t* sizes) {
+    __shared__ int32_t w[16];
+    const int64_t k0 = blockIdx.x * 1024ll + 4 * threadIdx.x;
+    int32_t f[4], c = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c += f[i] = k0 + i < ids && deg[k0 + i] != 0;
+    int32_t at = tile_prefix(sums, c, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (f[i]) {
+            rank[k0 + i] = at;
+            if (!places) nodes[at] = (uint32_t)(k0 + i);
+            ++at;
+        }
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 255) {
+        sizes[0] = at;
+        sizes[1] = cnt[0];
+    }
+}
+
+// The oriented pair of a table slot in ranks; false for an empty slot.
+__device__ __forceinline__ bool small_pair(unsigned long long key, const int32_t* __restrict__ deg,
+                                           const int32_t* __restrict__ rank, int32_t& src, int32_t& dst) {
+    if (key == kEmptySlot) return false;
+    const int32_t a = (int32_t)(key >> 32), b = (int32_t)(key & 0xFFFFFFFFull);  // a < b
+    const int32_t da = __ldg(deg + a), db = __ldg(deg + b), ra = __ldg(rank + a), rb = __ldg(rank + b);
+    const bool first = da <= db;  // ties: the lower id
+    src = first ? ra : rb;
+    dst = first ? rb : ra;
+    return true;
+}
+
+__global__ void small_count_kernel(const unsigned long long* __restrict__ table, int64_t slots,
+                                   const int32_t* __restrict__ deg, const int32_t* __restrict__ rank, int32_t* fdeg) {
+    GRID_STRIDE(i, slots) {
+        int32_t s, d;
+        if (small_pair(table[i], deg, rank, s, d)) atomicAdd(fdeg + s, 1);
+    }
+}
+
+// row_ptr, the node outputs, and fdeg turned into the rows' write cursors.
+__global__ void __launch_bounds__(256) small_rows_kernel(int32_t* fdeg, int64_t n, const int32_t* __restrict__ sums,
+                                                         const uint32_t* __restrict__ nodes, const int64_t* cnt,
+                                                         int64_t direct_ids, const int32_t* __restrict__ deg,
+                                                         int32_t* row_ptr, int32_t* degrees, int32_t* node_ids,
+                                                         int32_t* undirected) {
+    __shared__ int32_t w[16];
+    const bool places = cnt[3] + 1 > direct_ids;  // as phase 1 decided: deg goes by place
+    const int64_t k0 = blockIdx.x * 1024ll + 4 * threadIdx.x;
+    int32_t f[4], c = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c += f[i] = k0 + i < n ? fdeg[k0 + i] : 0;
+    int32_t at = tile_prefix(sums, c, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int64_t k = k0 + i;
+        if (k < n) {
+            const uint32_t id = nodes[k];
+            row_ptr[k] = at;
+            fdeg[k] = at;
+            degrees[k] = f[i];
+            node_ids[k] = (int32_t)id;
+            if (undirected) undirected[k] = deg[places ? k : (int64_t)id];  // id < direct_ids
+            at += f[i];
+            if (k == n - 1) row_ptr[n] = at;
+        }
+    }
+}
+
+__global__ void small_scatter_kernel(const unsigned long long* __restrict__ table, int64_t slots,
+                                     const int32_t* __restrict__ deg, const int32_t* __restrict__ rank,
+                                     int32_t* cursor, int32_t* out) {
+    GRID_STRIDE(i, slots) {
+        int32_t s, d;
+        if (small_pair(table[i], deg, rank, s, d)) out[atomicAdd(cursor + s, 1)] = d;
+    }
+}
+
+// Sorts the rows in[row_ptr[r] .. row_ptr[r + 1]) (distinct values) into
+// col_idx and edge_v and writes edge_u; a warp per row.  Up to 64 members: each
+// lane counts, for its two, the members below them; longer rows: a bitonic
+// sort in the warp's shared memory.
+__global__ void __launch_bounds__(128) small_sort_kernel(const int32_t* __restrict__ row_ptr, int64_t n,
+                                                         const int32_t* __restrict__ in, int32_t* col_idx,
+                                                         int32_t* edge_u, int32_t* edge_v) {
+    __shared__ int32_t buf[4][kSmallRow];
+    const int lane = threadIdx.x & 31;
+    int32_t* b = buf[threadIdx.x >> 5];
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
+        const int32_t s = __ldg(row_ptr + r), d = __ldg(row_ptr + r + 1) - s;
+        if (d <= 64) {
+            const int32_t none = 0x7FFFFFFF;  // above every rank
+            const int32_t x0 = lane < d ? __ldg(in + s + lane) : none;
+            const int32_t x1 = 32 + lane < d ? __ldg(in + s + 32 + lane) : none;
+            int r0 = 0, r1 = 0;
+            for (int i = 0; i < d; ++i) {
+                const int32_t y = i < 32 ? __shfl_sync(0xFFFFFFFFu, x0, i) : __shfl_sync(0xFFFFFFFFu, x1, i - 32);
+                r0 += y < x0;
+                r1 += y < x1;
+            }
+            if (lane < d) {
+                col_idx[s + r0] = x0;
+                edge_v[s + r0] = x0;
+                edge_u[s + lane] = (int32_t)r;
+            }
+            if (32 + lane < d) {
+                col_idx[s + r1] = x1;
+                edge_v[s + r1] = x1;
+                edge_u[s + 32 + lane] = (int32_t)r;
+            }
+            continue;
+        }
+        int m = 128;  // the next power of two
+        while (m < d) m <<= 1;
+        __syncwarp();
+        for (int i = lane; i < m; i += 32) b[i] = i < d ? __ldg(in + s + i) : 0x7FFFFFFF;
+        __syncwarp();
+        for (int k = 2; k <= m; k <<= 1) {
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                for (int t = lane; t < m / 2; t += 32) {
+                    const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
+                    const int32_t x = b[lo], y = b[hi];
+                    if ((x > y) == ((lo & k) == 0)) {
+                        b[lo] = y;
+                        b[hi] = x;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        for (int i = lane; i < d; i += 32) {
+            const int32_t x = b[i];
+            col_idx[s + i] = x;
+            edge_v[s + i] = x;
+            edge_u[s + i] = (int32_t)r;
+        }
+    }
+}
+
 // ------------------------------------------------- forward_adj -> CSR ------
 __global__ void iota_kernel(int64_t* a, int64_t n) {
     GRID_STRIDE(i, n) a[i] = i;
@@ -410,6 +673,33 @@ TCHLL_EXPORT int tchll_csr_build_phase1(const int32_t* raw_u, const int32_t* raw
         return TCHLL_OK;
     }
     const int64_t max_id = hc[1];
+    if (n_raw <= kSmallRaw) {
+        // deg in W.deg (cleared above), rank in W.e1, nodes in W.e0, tile sums
+        // in W.fdeg
+        const bool places = max_id + 1 > 2 * (int64_t)R;
+        const int64_t slots = 2 * (int64_t)R, ids = places ? slots : max_id + 1, tiles = (ids + 1023) / 1024;
+        unsigned long long* table = reinterpret_cast<unsigned long long*>(W.k0);
+        if (places) {
+            small_ends_kernel<<<grid_n(n_raw), 256, 0, st>>>(raw_u, raw_v, n_raw, W.e0);
+            TCHLL_CHECK_LAUNCH("small_ends_kernel");
+            size_t tb = W.tmp_bytes;
+            TCHLL_CUDA(cub::DeviceRadixSort::SortKeys(W.tmp, tb, W.e0, W.e1, 2 * R, 0, 32, st));
+            count_launch();
+            tb = W.tmp_bytes;
+            TCHLL_CUDA(cub::DeviceSelect::Unique(W.tmp, tb, W.e1, W.e0, W.cnt + 1, 2 * R, st));
+            count_launch();
+        }
+        TCHLL_CUDA(cudaMemsetAsync(table, 0xFF, (size_t)slots * sizeof(uint64_t), st));
+        small_insert_kernel<<<grid_n(n_raw), 256, 0, st>>>(raw_u, raw_v, n_raw, places ? W.e0 : nullptr, table,
+                                                           (uint32_t)slots, W.deg, W.cnt);
+        TCHLL_CHECK_LAUNCH("small_insert_kernel");
+        tile_sum_kernel<true><<<(int)tiles, 256, 0, st>>>(W.deg, ids, W.fdeg);
+        TCHLL_CHECK_LAUNCH("tile_sum_kernel");
+        small_rank_kernel<<<(int)tiles, 256, 0, st>>>(W.deg, ids, W.fdeg, reinterpret_cast<int32_t*>(W.e1), W.e0,
+                                                      places ? 1 : 0, W.cnt, sizes);
+        TCHLL_CHECK_LAUNCH("small_rank_kernel");
+        return TCHLL_OK;
+    }
     const int kb = bits_for(max_id);
     canon_kernel<<<grid_n(n_raw), 256, 0, st>>>(raw_u, raw_v, n_raw, kb, W.k0);
     TCHLL_CHECK_LAUNCH("canon_kernel");
@@ -467,6 +757,27 @@ TCHLL_EXPORT int tchll_csr_build_phase2(int64_t n_raw, int64_t n_nodes, int64_t 
         return TCHLL_EWORKSPACE;
     }
     cudaStream_t st = (cudaStream_t)stream;
+    if (n_edges > 0 && n_raw <= kSmallRaw) {
+        TCHLL_ARG(n_nodes > 1, "sizes out of range");
+        const int64_t slots = 2 * n_raw, tiles = (n_nodes + 1023) / 1024;
+        const unsigned long long* table = reinterpret_cast<const unsigned long long*>(W.k0);
+        const int32_t* rank = reinterpret_cast<const int32_t*>(W.e1);
+        TCHLL_CUDA(cudaMemsetAsync(W.fdeg, 0, (size_t)n_nodes * sizeof(int32_t), st));
+        small_count_kernel<<<grid_n(slots), 256, 0, st>>>(table, slots, W.deg, rank, W.fdeg);
+        TCHLL_CHECK_LAUNCH("small_count_kernel");
+        tile_sum_kernel<false><<<(int)tiles, 256, 0, st>>>(W.fdeg, n_nodes, W.ca);
+        TCHLL_CHECK_LAUNCH("tile_sum_kernel");
+        small_rows_kernel<<<(int)tiles, 256, 0, st>>>(W.fdeg, n_nodes, W.ca, W.e0, W.cnt, slots, W.deg, row_ptr, degrees,
+                                                      node_ids, undirected_degrees);
+        TCHLL_CHECK_LAUNCH("small_rows_kernel");
+        small_scatter_kernel<<<grid_n(slots), 256, 0, st>>>(table, slots, W.deg, rank, W.fdeg, W.cb);
+        TCHLL_CHECK_LAUNCH("small_scatter_kernel");
+        int64_t g = (n_nodes + 3) / 4;
+        if (g > (int64_t)sm_count() * 7) g = (int64_t)sm_count() * 7;
+        small_sort_kernel<<<(int)g, 128, 0, st>>>(row_ptr, n_nodes, W.cb, col_idx, edge_u, edge_v);
+        TCHLL_CHECK_LAUNCH("small_sort_kernel");
+        return TCHLL_OK;
+    }
     if (n_edges > 0) {
         // the pairs in the first half of k1's bytes (2 n_raw uint32 >= 2 n_edges);
         // sorted by src straight into edge_u (src) and col_idx (dst)
