@@ -15,9 +15,8 @@
 // table and remap -> degree histogram -> orient -> stable radix sort of the
 // (src, dst) pairs by src alone -> row pointers from the sorted sources.
 // The node table (compacted id = rank of the raw id among the endpoints)
-// comes from a direct table when the id space fits the workspace (flag every
-// endpoint id, scan the flags: rank[id] is the scan, one gather per
-// endpoint), else from sorting and deduplicating all endpoints and a binary
+// comes from a direct table when the id space fits the workspace (degrees by
+// id, a scan of the ids that occur: rank[id]), else from sorting and deduplicating all endpoints and a binary
 // search per endpoint.
 //
 // One sort by src is enough for rows sorted by dst: the pairs reach it in
@@ -29,6 +28,7 @@
 // Sorting, unique and scans use CUB (header templates compiled into this
 // library); the other passes are kernels written here.
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "common.cuh"
 
@@ -40,15 +40,22 @@ namespace tchll {
 __host__ __device__ __forceinline__ uint64_t key_sentinel(int k) { return (k >= 32) ? ~0ull : ((1ull << (2 * k)) - 1ull); }
 constexpr uint32_t kEndSentinel = 0xFFFFFFFFu;
 
+struct Occurs {
+    __host__ __device__ int32_t operator()(int32_t d) const { return d != 0; }
+};
+
 struct CsrWs {
     uint64_t* k0;
     uint64_t* k1;
     uint32_t* e0;
     uint32_t* e1;
     int32_t* deg;
+    // [fdeg 2 n_raw + 2][ca n_raw][cb n_raw], or, in the direct path, info of
+    // up to 2 n_raw ids
     int32_t* fdeg;
     int32_t* ca;
     int32_t* cb;
+    int2* info;
     int64_t* cnt;  // [0] unique keys, [1] unique endpoints, [2] negative-id flag, [3] largest id
     void* tmp;
     size_t tmp_bytes;
@@ -65,7 +72,8 @@ static size_t csr_cub_tmp(int64_t n_raw) {
     cub::DeviceSelect::Unique(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t*)nullptr, R);
     cub::DeviceRadixSort::SortKeys(nullptr, c, (uint32_t*)nullptr, (uint32_t*)nullptr, 2 * R, 0, 32);
     cub::DeviceSelect::Unique(nullptr, d, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t*)nullptr, 2 * R);
-    cub::DeviceScan::ExclusiveSum(nullptr, e, (int32_t*)nullptr, (int32_t*)nullptr, 2 * R + 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, e, thrust::make_transform_iterator((int32_t*)nullptr, Occurs()),
+                                  (int32_t*)nullptr, 2 * R + 1);
     cub::DeviceRadixSort::SortPairs(nullptr, f, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                     (uint32_t*)nullptr, R, 0, 32);
     size_t m = a;
@@ -87,9 +95,10 @@ static bool carve_csr(void* ws, size_t bytes, int64_t n_raw, CsrWs& W, size_t* n
     W.e0 = cv.take<uint32_t>(2 * R);
     W.e1 = cv.take<uint32_t>(2 * R);
     W.deg = cv.take<int32_t>(2 * R + 1);
-    W.fdeg = cv.take<int32_t>(2 * R + 2);
-    W.ca = cv.take<int32_t>(R);
-    W.cb = cv.take<int32_t>(R);
+    W.info = cv.take<int2>(2 * R + 1);
+    W.fdeg = reinterpret_cast<int32_t*>(W.info);
+    W.ca = W.fdeg + 2 * R + 2;
+    W.cb = W.ca + R;
     W.cnt = cv.take<int64_t>(4);
     W.tmp_bytes = csr_cub_tmp(n_raw);
     W.tmp = cv.take<char>(W.tmp_bytes);
@@ -216,56 +225,38 @@ __global__ void remap_kernel(const uint64_t* __restrict__ keys, int64_t cap, con
     }
 }
 
-// Direct path: flag[id] = 1 for both endpoints of every unique edge (flag
-// zeroed over [0, max id + 1] before).  The keys are sorted, so neighbouring
-// lanes mostly share a: only the first lane of each run stores it.
-__global__ void flag_ends_kernel(const uint64_t* __restrict__ keys, int64_t cap, const int64_t* cnt, int kb,
-                                 int32_t* flag) {
+// Direct path: undirected degrees by raw id, of every unique edge (deg zeroed
+// over [0, max id + 1] before).
+__global__ void id_degree_kernel(const uint64_t* __restrict__ keys, int64_t cap, const int64_t* cnt, int kb,
+                                 int32_t* deg) {
     const int64_t ne = n_real_edges(keys, cnt, kb);
     const uint64_t lo = (1ull << kb) - 1ull;
     const int lane = threadIdx.x & 31;
     WARP_GRID_STRIDE(i, cap) {
-        const bool in = i < ne;
-        const uint64_t k = in ? keys[i] : 0;
-        const uint32_t a = (uint32_t)(k >> kb);
-        const uint32_t pa = __shfl_up_sync(0xFFFFFFFFu, a, 1);
-        const bool pin = __shfl_up_sync(0xFFFFFFFFu, (int)in, 1) != 0;
-        if (in) {
-            if (lane == 0 || !pin || pa != a) flag[a] = 1;
-            flag[k & lo] = 1;
-        }
-    }
-}
-
-// Direct path, after rank = exclusive scan of flag over [0, ids] (ids = max
-// id + 2 entries): the node table nodes[rank[id]] = id for flagged ids, and
-// the number of nodes in cnt[1] (its sort-path meaning).
-__global__ void rank_nodes_kernel(const int32_t* __restrict__ flag, const int32_t* __restrict__ rank, int64_t ids,
-                                  uint32_t* nodes, int64_t* cnt) {
-    GRID_STRIDE(i, ids) {
-        if (i == ids - 1) cnt[1] = rank[i];  // flag[ids - 1] = 0: the total
-        else if (flag[i]) nodes[rank[i]] = (uint32_t)i;
-    }
-}
-
-// Direct path: both endpoints of every unique edge through the rank table.
-__global__ void remap_direct_kernel(const uint64_t* __restrict__ keys, int64_t cap, const int32_t* __restrict__ rank,
-                                    const int64_t* cnt, int kb, int32_t* ca, int32_t* cb, int32_t* deg) {
-    const int64_t ne = n_real_edges(keys, cnt, kb);
-    const uint64_t lo = (1ull << kb) - 1ull;
-    const int lane = threadIdx.x & 31;
-    WARP_GRID_STRIDE(i, cap) {
-        const bool in = i < ne;
         int32_t a = -1;
-        if (in) {
+        if (i < ne) {
             const uint64_t k = keys[i];
-            a = __ldg(rank + (k >> kb));
-            const int32_t b = __ldg(rank + (k & lo));
-            ca[i] = a;
-            cb[i] = b;
-            atomicAdd(deg + b, 1);
+            a = (int32_t)(k >> kb);
+            atomicAdd(deg + (k & lo), 1);
         }
         add_runs(deg, a, lane);
+    }
+}
+
+// Direct path, after rank = exclusive scan of "the id occurs" over [0, ids]
+// (ids = max id + 2 entries): the node table nodes[rank[id]] = id, the number
+// of nodes in cnt[1] (its sort-path meaning), and degree and rank of every id
+// side by side for the orientation.
+__global__ void rank_nodes_kernel(const int32_t* __restrict__ deg, const int32_t* __restrict__ rank, int64_t ids,
+                                  uint32_t* nodes, int2* info, int64_t* cnt) {
+    GRID_STRIDE(i, ids) {
+        const int32_t r = rank[i], d = deg[i];
+        if (i == ids - 1) {
+            cnt[1] = r;  // deg[ids - 1] = 0: the total
+        } else {
+            info[i] = make_int2(d, r);
+            if (d) nodes[r] = (uint32_t)i;
+        }
     }
 }
 
@@ -282,11 +273,31 @@ __global__ void sizes_kernel(const uint64_t* keys, const uint32_t* nodes, const 
 
 // Orientation u -> v iff (deg u, u) < (deg v, v): the pair (src, dst) of
 // edge i goes to okey[i] / oval[i] (canonical order kept for the stable sort).
-__global__ void orient_kernel(const int32_t* __restrict__ ca, const int32_t* __restrict__ cb, int64_t ne,
-                              const int32_t* __restrict__ deg, uint32_t* okey, uint32_t* oval) {
+// Direct path (as phase 1 chose it from the largest id, cnt[3]): raw ids from
+// the keys, degree and rank with one 8-byte load per endpoint (a run of keys
+// shares its first).  Ranks rise with the ids, so ids break ties as well.
+// R-MAT 22: flagging the ids, replacing them by ranks while counting degrees
+// and orienting took 0.89 + 0.82 + 0.27 ms; counting by id and this, 0.80 +
+// 0.29 ms.
+__global__ void orient_kernel(const uint64_t* __restrict__ keys, const int2* __restrict__ info,
+                              const int64_t* __restrict__ cnt, int64_t direct_ids, const int32_t* __restrict__ ca,
+                              const int32_t* __restrict__ cb, int64_t ne, const int32_t* __restrict__ deg,
+                              uint32_t* okey, uint32_t* oval) {
+    const int64_t max_id = cnt[3];
+    const bool direct = max_id + 2 <= direct_ids;  // grid-uniform
+    const int kb = max_id > 0 ? 64 - __clzll(max_id) : 1;
+    const uint64_t lo = (1ull << kb) - 1ull;
     GRID_STRIDE(i, ne) {
-        const int32_t a = ca[i], b = cb[i];
-        const int32_t da = deg[a], db = deg[b];
+        int32_t a, b, da, db;
+        if (direct) {
+            const uint64_t k = __ldcs(reinterpret_cast<const unsigned long long*>(keys) + i);
+            const int2 ia = __ldg(info + (k >> kb)), ib = __ldg(info + (k & lo));
+            da = ia.x, a = ia.y;
+            db = ib.x, b = ib.y;
+        } else {
+            a = ca[i], b = cb[i];
+            da = deg[a], db = deg[b];
+        }
         const bool first = (da < db) || (da == db && a < b);
         okey[i] = (uint32_t)(first ? a : b);
         oval[i] = (uint32_t)(first ? b : a);
@@ -305,12 +316,13 @@ __global__ void row_ptr_kernel(const int32_t* __restrict__ src, int64_t ne, int6
 }
 
 __global__ void copy_nodes_kernel(const uint32_t* __restrict__ nodes, int64_t n, const int32_t* __restrict__ row_ptr,
-                                  const int32_t* __restrict__ deg, int32_t* node_ids, int32_t* degrees,
-                                  int32_t* undirected) {
+                                  const int32_t* __restrict__ deg, const int64_t* __restrict__ cnt, int64_t direct_ids,
+                                  int32_t* node_ids, int32_t* degrees, int32_t* undirected) {
+    const bool direct = cnt[3] + 2 <= direct_ids;  // deg goes by id
     GRID_STRIDE(i, n) {
         node_ids[i] = (int32_t)nodes[i];
         degrees[i] = row_ptr[i + 1] - row_ptr[i];
-        if (undirected) undirected[i] = deg[i];
+        if (undirected) undirected[i] = deg[direct ? (int64_t)nodes[i] : i];
     }
 }
 
@@ -714,17 +726,15 @@ TCHLL_EXPORT int tchll_csr_build_phase1(const int32_t* raw_u, const int32_t* raw
     const int64_t ids = max_id + 2;
     const int direct = ids <= 2 * (int64_t)R ? 1 : 0;
     if (direct) {
-        TCHLL_CUDA(cudaMemsetAsync(W.fdeg, 0, (size_t)ids * sizeof(int32_t), st));
-        flag_ends_kernel<<<grid_n(n_raw), 256, 0, st>>>(W.k0, n_raw, W.cnt, kb, W.fdeg);
-        TCHLL_CHECK_LAUNCH("flag_ends_kernel");
+        id_degree_kernel<<<grid_n(n_raw), 256, 0, st>>>(W.k0, n_raw, W.cnt, kb, W.deg);  // cleared above
+        TCHLL_CHECK_LAUNCH("id_degree_kernel");
         int32_t* rank = reinterpret_cast<int32_t*>(W.e1);
         tb = W.tmp_bytes;
-        TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(W.tmp, tb, W.fdeg, rank, (int)ids, st));
+        TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(W.tmp, tb, thrust::make_transform_iterator(W.deg, Occurs()), rank,
+                                                 (int)ids, st));
         count_launch();
-        rank_nodes_kernel<<<grid_n(ids), 256, 0, st>>>(W.fdeg, rank, ids, W.e0, W.cnt);
+        rank_nodes_kernel<<<grid_n(ids), 256, 0, st>>>(W.deg, rank, ids, W.e0, W.info, W.cnt);
         TCHLL_CHECK_LAUNCH("rank_nodes_kernel");
-        remap_direct_kernel<<<grid_n(n_raw), 256, 0, st>>>(W.k0, n_raw, rank, W.cnt, kb, W.ca, W.cb, W.deg);
-        TCHLL_CHECK_LAUNCH("remap_direct_kernel");
     } else {
         ends_kernel<<<grid_n(n_raw), 256, 0, st>>>(W.k0, n_raw, W.cnt, kb, W.e0);
         TCHLL_CHECK_LAUNCH("ends_kernel");
@@ -784,7 +794,8 @@ TCHLL_EXPORT int tchll_csr_build_phase2(int64_t n_raw, int64_t n_nodes, int64_t 
         uint32_t* okey = reinterpret_cast<uint32_t*>(W.k1);
         uint32_t* oval = okey + n_edges;
         const int kn = bits_for(n_nodes > 1 ? n_nodes - 1 : 1);
-        orient_kernel<<<grid_n(n_edges), 256, 0, st>>>(W.ca, W.cb, n_edges, W.deg, okey, oval);
+        orient_kernel<<<grid_n(n_edges), 256, 0, st>>>(W.k0, W.info, W.cnt, 2 * n_raw, W.ca, W.cb, n_edges, W.deg, okey,
+                                                       oval);
         TCHLL_CHECK_LAUNCH("orient_kernel");
         size_t tb = W.tmp_bytes;
         TCHLL_CUDA(cub::DeviceRadixSort::SortPairs(W.tmp, tb, okey, reinterpret_cast<uint32_t*>(edge_u), oval,
@@ -795,8 +806,8 @@ TCHLL_EXPORT int tchll_csr_build_phase2(int64_t n_raw, int64_t n_nodes, int64_t 
     row_ptr_kernel<<<grid_n(n_edges + 1), 256, 0, st>>>(edge_u, n_edges, n_nodes, row_ptr);
     TCHLL_CHECK_LAUNCH("row_ptr_kernel");
     if (n_nodes > 0) {
-        copy_nodes_kernel<<<grid_n(n_nodes), 256, 0, st>>>(W.e0, n_nodes, row_ptr, W.deg, node_ids, degrees,
-                                                            undirected_degrees);
+        copy_nodes_kernel<<<grid_n(n_nodes), 256, 0, st>>>(W.e0, n_nodes, row_ptr, W.deg, W.cnt, 2 * n_raw, node_ids,
+                                                            degrees, undirected_degrees);
         TCHLL_CHECK_LAUNCH("copy_nodes_kernel");
     }
     return TCHLL_OK;
