@@ -59,7 +59,8 @@ enum : uint32_t {
 
 struct CountParams {
     const int32_t* row_ptr;
-    const int2* rows;  // {row_ptr[v], row_ptr[v + 1]} per vertex, or null
+    const int2* rows;  // the row table, or null
+    uint2* codes;      // per 32 edges of the first pass: {hub pairs, of them those with x = u} (with rows)
     int64_t n_nodes;
     const int32_t* col_idx;
     int64_t nnz;
@@ -171,21 +172,45 @@ __device__ __forceinline__ bool load_edge(const CountParams& P, int64_t e, int32
         status |= ST_BAD_EDGE;
         return false;
     }
-    if (P.rows) {  // the same, one load per endpoint
-        const int2 ru = __ldg(P.rows + u), rv = __ldg(P.rows + v);
-        us = ru.x;
-        ue = ru.y;
-        vs = rv.x;
-        ve = rv.y;
-    } else {
-        us = __ldg(P.row_ptr + u);
-        ue = __ldg(P.row_ptr + u + 1);
-        vs = __ldg(P.row_ptr + v);
-        ve = __ldg(P.row_ptr + v + 1);
-    }
+    us = __ldg(P.row_ptr + u);
+    ue = __ldg(P.row_ptr + u + 1);
+    vs = __ldg(P.row_ptr + v);
+    ve = __ldg(P.row_ptr + v + 1);
     // 0 <= start <= end <= nnz
     if ((uint32_t)us > (uint32_t)ue || (uint32_t)ue > nnz || (uint32_t)vs > (uint32_t)ve || (uint32_t)ve > nnz) {
         status |= ST_BAD_ROW;
+        return false;
+    }
+    return true;
+}
+
+// The row table (prepare_kernel): {row start, row end} per vertex, with the
+// vertex's part in the routing in the sign bits: its degree reaches gamma
+// (start), it has a sketch (end).  min(d+u, d+v) >= gamma iff both ends reach
+// it, so one 8-byte load per endpoint replaces up to four.  Malformed entries
+// have start > end.
+constexpr int32_t kRowBad = 0x7FFFFFFF;   // {kRowBad, 0}: a bad extent
+constexpr int32_t kSlotBad = 0x7FFFFFFE;  // {kSlotBad, 0}: a sketch slot outside the rows
+__device__ __forceinline__ bool load_edge_rows(const CountParams& P, int64_t e, int32_t& u, int32_t& v, int32_t& us,
+                                               int32_t& ue, int32_t& vs, int32_t& ve, bool& wants, bool& both,
+                                               uint32_t& status) {
+    u = __ldcs(P.edge_u + e);
+    v = __ldcs(P.edge_v + e);
+    const uint32_t n = (uint32_t)P.n_nodes;
+    if ((uint32_t)u >= n || (uint32_t)v >= n) {
+        status |= ST_BAD_EDGE;
+        return false;
+    }
+    const int2 ru = __ldg(P.rows + u), rv = __ldg(P.rows + v);
+    wants = (ru.x & rv.x) < 0;
+    both = (ru.y & rv.y) < 0;
+    us = ru.x & 0x7FFFFFFF;
+    ue = ru.y & 0x7FFFFFFF;
+    vs = rv.x & 0x7FFFFFFF;
+    ve = rv.y & 0x7FFFFFFF;
+    if (us > ue || vs > ve) {
+        const bool slot = (us <= ue || us == kSlotBad) && (vs <= ve || vs == kSlotBad);
+        status |= slot ? ST_BAD_SLOT : ST_BAD_ROW;
         return false;
     }
     return true;
@@ -298,64 +323,48 @@ __device__ __forceinline__ void append_hll(const CountParams& P, bool hll, int32
     }
 }
 
-// Grid-stride loop that whole warps enter and leave together: e may reach
-// past n in the last pass; the body tests it.
-#define WARP_EDGE_LOOP(e, n)                                                                   \
-    for (int64_t _wb = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u),                \
-                 e = _wb + (threadIdx.x & 31u);                                                \
-         _wb < (n); _wb += (int64_t)gridDim.x * blockDim.x, e = _wb + (threadIdx.x & 31u))
-
-// Hub pairs' probe sides, grouped by table side: py[cursor[x] ...).
-template <bool HYB>
-__device__ __forceinline__ void scatter_step(const CountParams& P, int64_t e, bool in, int32_t* cursor, int hub,
-                                             int32_t* py, int lane) {
-    uint32_t status = 0;  // reported by the first pass
-    int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
-    bool ok = in && load_edge(P, e, u, v, us, ue, vs, ve, status);
-    const PairSides S = sides_of(u, v, us, ue, vs, ve);
-    ok = ok && is_hub_pair(S, hub);
-    if (HYB && ok) {
-        int32_t du, dv;
-        int64_t su, sv;
-        bool wants, both;
-        ok = route(P, u, v, du, dv, su, sv, wants, both, status) && !(wants && both);  // not HLL-routed
+// Hub pairs' probe sides, grouped by table side: py[cursor[x] ...).  Which
+// edges are hub pairs and which end is x comes from the first pass, two bits
+// per edge, so no row is looked up again (R-MAT 22: 1.12 ms with the rows looked up again, 0.81 so).
+__device__ __forceinline__ void scatter_step(const CountParams& P, int64_t e, uint2 code, int32_t* cursor, int32_t* py,
+                                             int lane) {
+    if (code.x == 0) return;  // warp-uniform
+    const bool ok = (code.x >> lane) & 1u, xu = (code.y >> lane) & 1u;
+    int32_t u = 0, v = 0;
+    if (ok) {
+        u = __ldcs(P.edge_u + e);
+        v = __ldcs(P.edge_v + e);
     }
+    const int32_t x = xu ? u : v;
     // a run of lanes with the same x claims its positions with one atomic
     int head, len;
-    lane_runs(ok ? S.x : -1 - lane, lane, head, len);
+    lane_runs(ok ? x : -1 - lane, lane, head, len);
     int32_t base = 0;
-    if (ok && lane == head) base = atomicAdd(cursor + S.x, len);
+    if (ok && lane == head) base = atomicAdd(cursor + x, len);
     base = __shfl_sync(FULL, base, head);
-    if (ok) py[base + (lane - head)] = S.y;
+    if (ok) py[base + (lane - head)] = xu ? v : u;
 }
 
-template <bool HYB>
-__global__ void pair_scatter_kernel(const CountParams P, int32_t* cursor, const unsigned long long* n_pairs, int hub,
+__global__ void pair_scatter_kernel(const CountParams P, int32_t* cursor, const unsigned long long* n_pairs,
                                     int32_t* py) {
     if (*n_pairs == 0) return;  // grid-uniform
     const int lane = threadIdx.x & 31;
+    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     if (P.chunk_start) {  // batched: the chunks of the graphs with hub pairs
         const int64_t n = *P.n_chunks_dev;
-        const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-        for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; c < n; c += warps) {
-            const int32_t g = __ldg(P.chunk_graph + c);
-            if (!P.graph_hub[g]) continue;
-            const int32_t lo_v = __ldg(P.graph_vbase + g), hi_v = __ldg(P.graph_vbase + g + 1);
+        for (int64_t c = warp; c < n; c += warps) {
+            if (!P.graph_hub[__ldg(P.chunk_graph + c)]) continue;
             const int64_t e0 = __ldg(P.chunk_start + c);
             const int32_t len = __ldg(P.chunk_len + c);
-            for (int32_t i = 0; i < len; i += 32) {
-                const int64_t e = e0 + i + lane;
-                bool in = i + lane < len;
-                if (in) {  // not an edge of another graph (the first pass skipped and reported it)
-                    const int32_t u = __ldg(P.edge_u + e), v = __ldg(P.edge_v + e);
-                    in = u >= lo_v && u < hi_v && v >= lo_v && v < hi_v;
-                }
-                scatter_step<HYB>(P, e, in, cursor, hub, py, lane);
-            }
+            for (int32_t i = 0; i < len; i += 32)
+                scatter_step(P, e0 + i + lane, __ldg(P.codes + (e0 >> 5) + c + (i >> 5)), cursor, py, lane);
         }
         return;
     }
-    WARP_EDGE_LOOP(e, P.n_edges) scatter_step<HYB>(P, e, e < P.n_edges, cursor, hub, py, lane);
+    const int64_t steps = (P.n_edges + 31) >> 5;
+    for (int64_t w = warp; w < steps; w += warps)
+        scatter_step(P, 32 * w + lane, __ldg(P.codes + w), cursor, py, lane);
 }
 
 // Warp-cooperative binary-search intersection count of two sorted lists in
@@ -417,12 +426,17 @@ __device__ __forceinline__ void publish(tchll_count_result* R, uint64_t acc, U12
     }
 }
 
-// What the first pass needs beforehand, in one launch: {row_ptr[v], row_ptr[v
-// + 1]} side by side (the passes over all edges look both up at random v, and
-// that is one load instead of two), and everything that starts at zero.
+// What the first pass needs beforehand, in one launch: the row table
+// (load_edge_rows), and everything that starts at zero.
 struct Prepare {
     const int32_t* row_ptr;
     int64_t n_nodes;
+    int64_t nnz;
+    const int32_t* degrees;  // routing (hybrid calls, else null)
+    int64_t gamma;
+    const int64_t* slot;
+    const uint8_t* has;
+    int64_t n_rows;
     int2* rows;
     int32_t* zero_n[2];   // n_nodes + 1 words each (or null)
     uint32_t* zero[3];    // words[i] words
@@ -431,7 +445,19 @@ struct Prepare {
 __global__ void prepare_kernel(const Prepare Q) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t v = t0; v <= Q.n_nodes; v += step) {
-        if (v < Q.n_nodes) Q.rows[v] = make_int2(__ldg(Q.row_ptr + v), __ldg(Q.row_ptr + v + 1));
+        if (v < Q.n_nodes) {
+            const int32_t a = __ldg(Q.row_ptr + v), b = __ldg(Q.row_ptr + v + 1);
+            int2 r = make_int2(a, b);
+            if (a < 0 || b < a || (int64_t)b > Q.nnz) {
+                r = make_int2(kRowBad, 0);
+            } else if (Q.degrees) {
+                const int64_t s = Q.slot ? __ldg(Q.slot + v) : (__ldg(Q.has + v) == 1 ? v : -1);
+                if (s >= Q.n_rows) r = make_int2(kSlotBad, 0);
+                else if (s >= 0) r.y |= (int32_t)0x80000000;
+                if ((int64_t)__ldg(Q.degrees + v) >= Q.gamma) r.x |= (int32_t)0x80000000;
+            }
+            Q.rows[v] = r;
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (Q.zero_n[i]) Q.zero_n[i][v] = 0;
@@ -458,6 +484,20 @@ __global__ void prepare_kernel(const Prepare Q) {
 // in turn (null), or, batched, from the chunk list (a chunk is one graph's,
 // and so are its totals).
 enum : int { PASS_HIST = 1, PASS_SHORT = 2 };
+// The n HLL edges of a warp's buffer go to the list.
+constexpr int kHllBuf = 160;
+__device__ __forceinline__ void flush_hll(const CountParams& P, const int2* buf, int n, int lane) {
+    __syncwarp();
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(P.hll_n, (unsigned long long)n);
+    base = __shfl_sync(FULL, base, 0);
+    for (int i = lane; i < n; i += 32) {
+        P.hll_u[base + i] = buf[i].x;
+        P.hll_v[base + i] = buf[i].y;
+    }
+    __syncwarp();
+}
+
 // Adds warp-uniform totals to *R.
 __device__ __forceinline__ void pass_publish(tchll_count_result* R, uint64_t acc, int64_t n_exact, int64_t n_fallback,
                                              uint32_t status, int lane) {
@@ -475,9 +515,12 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
                                                            int32_t* __restrict__ cnth) {
     __shared__ int4 s_list[8][32];
     __shared__ int32_t s_len[8][32];
+    __shared__ int2 s_hll[HYB ? 8 : 1][HYB ? kHllBuf : 1];
     const int lane = threadIdx.x & 31;
     int4* lst = s_list[threadIdx.x >> 5];
     int32_t* len = s_len[threadIdx.x >> 5];
+    int2* hbuf = s_hll[HYB ? threadIdx.x >> 5 : 0];
+    int n_hll = 0;
     const unsigned lane_le = (2u << lane) - 1u;
     const int32_t* __restrict__ col = P.col_idx;
     uint64_t acc = 0;
@@ -491,6 +534,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
         int32_t e0, e1;  // below 2^31
         int32_t g = -1;
         uint32_t lo_v = 0, in_v = (uint32_t)P.n_nodes;
+        unsigned long long chunk;
         {
             unsigned long long c = turn;
             if (P.work) {
@@ -498,6 +542,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
                 c = __shfl_sync(FULL, c, 0);
             }
             turn += n_warps;
+            chunk = c;
             if (P.chunk_start) {
                 if ((int64_t)c >= *P.n_chunks_dev) break;
                 e0 = (int32_t)__ldg(P.chunk_start + c);
@@ -512,36 +557,50 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             }
         }
         bool any_hub = false;
+        // the chunk's codes: no two chunks of a batch share one
+        const int64_t code0 = (e0 >> 5) + (g >= 0 ? (int64_t)chunk : 0);
         for (int32_t eb = e0; eb < e1; eb += 32) {
             const int32_t e = eb + lane;
             int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
-            bool ok = e < e1 && load_edge(P, e, u, v, us, ue, vs, ve, status);
+            bool ok = e < e1, wants = false, both = false;
+            if (P.rows) {
+                ok = ok && load_edge_rows(P, e, u, v, us, ue, vs, ve, wants, both, status);
+            } else {
+                ok = ok && load_edge(P, e, u, v, us, ue, vs, ve, status);
+                int32_t du, dv;
+                int64_t su, sv;
+                if (HYB && ok) ok = route(P, u, v, du, dv, su, sv, wants, both, status);
+            }
             if (ok && ((uint32_t)u - lo_v >= in_v || (uint32_t)v - lo_v >= in_v)) {
                 status |= ST_BAD_EDGE;  // an edge of another graph inside this graph's chunk
                 ok = false;
             }
             if (HYB) {
-                bool hll = false, fall = false;
-                if (ok) {
-                    int32_t du, dv;
-                    int64_t su, sv;
-                    bool wants, both;
-                    ok = route(P, u, v, du, dv, su, sv, wants, both, status);
-                    hll = ok && wants && both;
-                    fall = ok && wants && !both;
+                const bool hll = ok && wants && both;
+                n_fallback += __popc(__ballot_sync(FULL, ok && wants && !both));
+                // HLL edges wait in the warp's buffer: one atomic on the shared
+                // counter per 128 or so
+                const unsigned m = __ballot_sync(FULL, hll);
+                if (hll) hbuf[n_hll + __popc(m & (lane_le >> 1))] = make_int2(u, v);
+                n_hll += __popc(m);
+                if (n_hll > kHllBuf - 32) {
+                    flush_hll(P, hbuf, n_hll, lane);
+                    n_hll = 0;
                 }
-                n_fallback += __popc(__ballot_sync(FULL, fall));
-                append_hll(P, hll, u, v, lane);
                 ok = ok && !hll;
             }
             const PairSides S = sides_of(u, v, us, ue, vs, ve);
             const bool to_hub = ok && is_hub_pair(S, hub);
-            if (hub > 0 && (what & PASS_HIST) && __any_sync(FULL, to_hub)) {
-                // a run of lanes with the same table side adds with one atomic
-                int head, run;
-                lane_runs(to_hub ? S.x : -1 - lane, lane, head, run);
-                if (to_hub && lane == head) atomicAdd(cnth + S.x, run);
-                any_hub = true;
+            if (hub > 0 && (what & PASS_HIST)) {
+                const unsigned m = __ballot_sync(FULL, to_hub), mu = __ballot_sync(FULL, S.x == u);
+                if (lane == 0) P.codes[code0 + ((eb - e0) >> 5)] = make_uint2(m, mu);
+                if (m) {
+                    // a run of lanes with the same table side adds with one atomic
+                    int head, run;
+                    lane_runs(to_hub ? S.x : -1 - lane, lane, head, run);
+                    if (to_hub && lane == head) atomicAdd(cnth + S.x, run);
+                    any_hub = true;
+                }
             }
             if (!(what & PASS_SHORT)) continue;
             const bool mine = ok && !to_hub;
@@ -630,6 +689,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             status = 0;
         }
     }
+    if (HYB && n_hll) flush_hll(P, hbuf, n_hll, lane);
     if (!P.chunk_start || status) pass_publish(P.result, acc, n_exact, n_fallback, status, lane);
 }
 
@@ -2621,7 +2681,8 @@ struct CountWs {
     int32_t* cnth;            // n_nodes + 1 (histogram of hub pairs)
     int32_t* offh;            // n_nodes + 1 (scan, then scatter cursor)
     int32_t* py;              // n_edges (probe sides of the hub pairs, by table side)
-    int2* rows;               // n_nodes (rows_kernel)
+    int2* rows;               // n_nodes: the row table
+    uint2* codes;             // n_edges / 32 + 1 (batches: their own)
     HubSeg* segs;             // max_segs
     int64_t max_segs;
     int32_t* pcol;            // padded lists in core coordinates for the hub kernels, pcap entries (null: not carved)
@@ -2666,6 +2727,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     W.offh = cv.take<int32_t>(N);
     W.py = cv.take<int32_t>(E);
     W.rows = cv.take<int2>(N);
+    W.codes = cv.take<uint2>(E / 32 + 1);
     // every hub x with pairs opens one segment, every HUB_SEG_MIN pairs at most one more
     W.max_segs = (int64_t)(N < E ? N : E) + (int64_t)(E / HUB_SEG_MIN) + 1;
     W.segs = cv.take<HubSeg>((size_t)W.max_segs);
@@ -2818,6 +2880,12 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     Q.row_ptr = P.row_ptr;
     Q.n_nodes = P.n_nodes;
     Q.rows = W.rows;
+    Q.nnz = P.nnz;
+    Q.degrees = P.regs || P.slot || P.has ? P.degrees : nullptr;
+    Q.gamma = P.gamma;
+    Q.slot = P.slot;
+    Q.has = P.has;
+    Q.n_rows = P.n_rows;
     Q.zero_n[0] = hub > 0 ? W.cnth : nullptr;
     Q.zero_n[1] = hub > 0 ? W.cflag : nullptr;
     Q.zero[0] = reinterpret_cast<uint32_t*>(W.ctr);
@@ -2829,6 +2897,7 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     prepare_kernel<<<grid_edges(P.n_nodes + 1), 256, 0, st>>>(Q);
     TCHLL_CHECK_LAUNCH("prepare_kernel");
     P.rows = W.rows;
+    P.codes = W.codes;
     return TCHLL_OK;
 }
 
@@ -2880,9 +2949,8 @@ static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaSt
     return TCHLL_OK;
 }
 
-template <bool HYB>
-static int pairs_scatter(const CountParams& P, const CountWs& W, int hub, cudaStream_t st) {
-    pair_scatter_kernel<HYB><<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.offh, W.ctr + 5, hub, W.py);
+static int pairs_scatter(const CountParams& P, const CountWs& W, cudaStream_t st) {
+    pair_scatter_kernel<<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.offh, W.ctr + 5, W.py);
     TCHLL_CHECK_LAUNCH("pair_scatter_kernel");
     return TCHLL_OK;
 }
@@ -3216,7 +3284,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
-                if (hub > 0) rc = pairs_scatter<false>(P, W, hub, st);
+                if (hub > 0) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 if (split) {
                     TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
@@ -3285,7 +3353,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 rc = launch_hll_edges(P, HW, T, hst);
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[1], hst);
                 if (rc) return rc;
-                if (hub > 0) rc = pairs_scatter<true>(P, W, hub, st);
+                if (hub > 0) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
@@ -3795,6 +3863,7 @@ struct BatchWs {
     int64_t* cstart;  // max chunks
     int32_t* clen;
     int32_t* cgraph;
+    uint2* codes;     // n_edges / 32 + max chunks + 1
     int32_t* ghub;    // n_graphs: the graph has hub pairs
     int32_t* rflag;   // n_nodes / 64 + 1: 64 rows touch such a graph
     int32_t* rlist;   // those blocks
@@ -3822,6 +3891,7 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     B.cstart = cv.take<int64_t>(MC);
     B.clen = cv.take<int32_t>(MC);
     B.cgraph = cv.take<int32_t>(MC);
+    B.codes = cv.take<uint2>((size_t)(n_edges > 0 ? n_edges : 1) / 32 + MC + 1);
     const size_t RL = (size_t)(n_nodes > 0 ? n_nodes : 0) / 64 + 1;
     B.flag_bytes = (G + RL) * sizeof(int32_t);
     B.ghub = cv.take<int32_t>(G + 2 * RL);
@@ -3838,6 +3908,7 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     if (!cv.ok() || cv.dry) return cv.ok();
     carve_count(cbase, cneed, n_nodes, n_edges, B.cw, nullptr);
     B.hw.hll_n = B.cw.ctr + 4;
+    B.cw.codes = B.codes;
     return true;
 }
 
@@ -3924,7 +3995,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     const bool hubs = hub > 0 && (hll_list || !hybrid);
     if (hubs) {
         rc = hub_alloc(P, B.cw, T.hub_seg, st, vbase, n_graphs);
-        if (rc == TCHLL_OK) rc = hybrid ? pairs_scatter<true>(P, B.cw, hub, st) : pairs_scatter<false>(P, B.cw, hub, st);
+        if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
         if (rc) return rc;
     }
     phase_mark(ps, 1, st);
