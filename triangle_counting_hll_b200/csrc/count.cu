@@ -1073,74 +1073,77 @@ __device__ __forceinline__ int64_t pad_start(int32_t rs, int32_t y) {
     return (((int64_t)rs + 3) & ~(int64_t)3) + 8 * (int64_t)y;
 }
 
-// The core, the w in N+(x) of the x with hub pairs, and how popular its
-// members are: a counted hub adds to cnt[w], the others set bit w of `bits`;
-// w is in the core when it has either.  Few hubs are all counted, of many
-// every kMarkStep-th (by id): the counts only order the core, where a sample
-// will do, and setting bits is cheaper than counting, except that with few
-// hubs all warps would queue to set the same words first.  One warp per hub
-// segment (a segment names its x; the segments of one x are
-// consecutive, and only the first marks x's list); going by segments rather
-// than by vertex id keeps the warps balanced, because hub vertices cluster at
-// low ids in R-MAT graphs.  Each lane has four list members in flight.  The
-// bits are read first, through L1 (they fit it, and the core's members
-// recur; a stale 0 just repeats the atomic), and each warp starts at another
-// place of its list: hub lists begin with the same few popular members, and
-// warps that all start there queue on the same L2 lines.  With an int flag
-// per vertex and every list walked from its start: 316 us on R-MAT 18
-// (edge factor 24), 367 us on R-MAT 22.  Values outside [0, n_nodes) are
-// reported, not stored.
-constexpr int64_t kMarkAll = 8192;
+// The core, the w in N+(x) of the x with long lists (every x with hub pairs
+// among them, and known before the first pass has run), and how popular its
+// members are: a counted list adds to cnt[w], the others set bit w of `bits`;
+// w is in the core when it has either.  In small graphs all are counted, in
+// others every kMarkStep-th (by id): the counts only order the core, where a
+// sample will do, and setting bits is cheaper than counting, except that with
+// few lists all warps would queue to set the same words first.  A warp looks
+// at four groups of 8 vertices from all over the range (long lists cluster at
+// low ids in R-MAT graphs) and takes the long lists one by one, each lane with
+// four members in flight.  The bits are read first, through L1 (they fit it,
+// and the core's members recur; a stale 0 just repeats the atomic), and each
+// list is started at another place: long lists begin with the same few popular
+// members, and warps that all start there queue on the same L2 lines.  With
+// an int flag per vertex and every list walked from its start: 316 us on
+// R-MAT 18 (edge factor 24), 367 us on R-MAT 22; so: 64, 112 us.  Values
+// outside [0, n_nodes) are reported, not stored.
+constexpr int64_t kMarkAllEdges = 8000000;
 constexpr int kMarkStep = 8;
 __global__ void core_mark_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int64_t nnz,
-                                 const int32_t* __restrict__ col, const HubSeg* __restrict__ segs,
-                                 const unsigned long long* __restrict__ n_segs, int64_t max_segs, uint32_t* bits,
-                                 int32_t* cnt, tchll_count_result* result) {
+                                 const int32_t* __restrict__ col, int hub, int count_all,
+                                 const unsigned long long* __restrict__ n_segs, uint32_t* bits, int32_t* cnt,
+                                 tchll_count_result* result) {
+    if (n_segs && *n_segs == 0) return;  // grid-uniform: batched, and no hub pairs
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nseg = min((int64_t)*n_segs, max_segs);
+    const int64_t tiles = (n_nodes + 31) >> 5;
     uint32_t status = 0;
-    for (int64_t sg = warp; sg < nseg; sg += nwarps) {
-        const int32_t x = segs[sg].x;
-        if (sg > 0 && segs[sg - 1].x == x) continue;  // x's first segment marks its list
-        if (x < 0 || (int64_t)x >= n_nodes) {  // warp-uniform; cannot happen
-            status |= ST_BAD_EDGE;
-            continue;
+    for (int64_t tile = warp; tile < tiles; tile += nwarps) {
+        const int64_t x = 8 * (tile + (lane >> 3) * tiles) + (lane & 7);
+        int32_t rs = 0, re = 0;
+        if (x < n_nodes) {
+            rs = __ldg(row_ptr + x);
+            re = __ldg(row_ptr + x + 1);
         }
-        const int32_t s = __ldg(row_ptr + x), e = __ldg(row_ptr + x + 1);
-        if (s < 0 || e < s || (int64_t)e > nnz) {
-            status |= ST_BAD_ROW;
-            continue;
-        }
-        const bool counted = nseg <= kMarkAll || (uint32_t)x % kMarkStep == 0;
-        const uint32_t parts = ((uint32_t)(e - s) + 127u) >> 7;
-        uint32_t part = parts ? (uint32_t)sg % parts : 0;
-        for (uint32_t q = 0; q < parts; ++q) {
-            const int64_t i0 = (int64_t)s + 128 * (int64_t)part;
-            part = part + 1 < parts ? part + 1 : 0;
-            int32_t w[4];
+        // malformed rows are reported with the lists
+        unsigned todo = __ballot_sync(FULL, rs >= 0 && re >= rs && (int64_t)re <= nnz && re - rs > hub);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int32_t s = __shfl_sync(FULL, rs, l), e = __shfl_sync(FULL, re, l);
+            const uint32_t id = (uint32_t)__shfl_sync(FULL, (int32_t)x, l);
+            const bool counted = count_all || id % kMarkStep == 0;
+            const uint32_t parts = ((uint32_t)(e - s) + 127u) >> 7;
+            uint32_t part = (id * 0x9E3779B1u >> 8) % parts;
+            for (uint32_t q = 0; q < parts; ++q) {
+                const int64_t i0 = (int64_t)s + 128 * (int64_t)part;
+                part = part + 1 < parts ? part + 1 : 0;
+                int32_t w[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int64_t i = i0 + 32 * k + lane;
-                w[k] = i < e ? __ldg(col + i) : -1;
-                if (i < e && (uint64_t)(uint32_t)w[k] >= (uint64_t)n_nodes) {
-                    status |= ST_BAD_KEY;
-                    w[k] = -1;
+                for (int k = 0; k < 4; ++k) {
+                    const int64_t i = i0 + 32 * k + lane;
+                    w[k] = i < e ? __ldg(col + i) : -1;
+                    if (i < e && (uint64_t)(uint32_t)w[k] >= (uint64_t)n_nodes) {
+                        status |= ST_BAD_KEY;
+                        w[k] = -1;
+                    }
                 }
-            }
-            if (counted) {
+                if (counted) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (w[k] >= 0) atomicAdd(cnt + w[k], 1);
+                    continue;
+                }
+                uint32_t f[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f[k] = w[k] >= 0 ? bits[w[k] >> 5] : ~0u;
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (w[k] >= 0) atomicAdd(cnt + w[k], 1);
-                continue;
+                    if (!((f[k] >> (w[k] & 31)) & 1u)) atomicOr(bits + (w[k] >> 5), 1u << (w[k] & 31));
             }
-            uint32_t f[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) f[k] = w[k] >= 0 ? bits[w[k] >> 5] : ~0u;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (!((f[k] >> (w[k] & 31)) & 1u)) atomicOr(bits + (w[k] >> 5), 1u << (w[k] & 31));
         }
     }
     status = __reduce_or_sync(FULL, status);
@@ -1425,7 +1428,8 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int sub = lane & 7, grp = lane >> 3;
     uint32_t status = 0;
-    const bool lists = *n_segs > 0;  // grid-uniform; else no hub pair will read one
+    // grid-uniform; else no hub pair will read a list
+    const bool lists = live ? *n_segs > 0 : n_core[0] > 0;
     if (!lists) validate_rows(row_ptr, n_nodes, nnz, col, status);
     // batched: only the listed blocks of 64 rows, those near a graph with hub
     // pairs, are ever read as lists; the other rows are only checked
@@ -2816,6 +2820,17 @@ static int launch_hll_edges_L(HllParams H, bool crow, cudaStream_t st) {
     return TCHLL_OK;
 }
 
+// The zero masks (when the workspace holds them), before launch_hll_edges.
+static int launch_zmask(const CountParams& P, const HybridWs& HW, cudaStream_t st) {
+    if (HW.zm == nullptr) return TCHLL_OK;
+    const int64_t rows = P.slot ? P.n_rows : P.n_nodes;
+    const int64_t wgrid = (rows + 7) / 8;
+    const int grid = (int)(wgrid < 1 ? 1 : (wgrid > (int64_t)sm_count() * 16 ? (int64_t)sm_count() * 16 : wgrid));
+    zmask_kernel<<<grid, 256, 0, st>>>(P.regs, rows, P.slot ? nullptr : P.has, P.p, HW.zst, HW.zm);
+    TCHLL_CHECK_LAUNCH("zmask_kernel");
+    return TCHLL_OK;
+}
+
 static int launch_hll_edges(const CountParams& P, const HybridWs& HW, const Tuning& T, cudaStream_t st) {
     HllParams H;
     H.vbase = P.graph_vbase;
@@ -2848,13 +2863,6 @@ static int launch_hll_edges(const CountParams& P, const HybridWs& HW, const Tuni
     if (crow) width = (1 << P.p) >> 7;
     else if (H.zm) width = P.p <= 10 ? 1 : (P.p <= 12 ? 4 : 8);
     if (T.hll_lanes > 0) width = T.hll_lanes;
-    if (H.zm) {
-        const int64_t rows = P.slot ? P.n_rows : P.n_nodes;
-        const int64_t wgrid = (rows + 7) / 8;
-        const int grid = (int)(wgrid < 1 ? 1 : (wgrid > (int64_t)sm_count() * 16 ? (int64_t)sm_count() * 16 : wgrid));
-        zmask_kernel<<<grid, 256, 0, st>>>(P.regs, rows, P.slot ? nullptr : P.has, P.p, H.zst, HW.zm);
-        TCHLL_CHECK_LAUNCH("zmask_kernel");
-    }
     switch (width >= 32 ? 32 : (width < 1 ? 1 : width)) {
         case 1: return launch_hll_edges_L<1>(H, crow, st);
         case 2: return launch_hll_edges_L<2>(H, crow, st);
@@ -2968,20 +2976,20 @@ static bool hub_pad_usable(const CountParams& P, const CountWs& W) {
     return W.pcol != nullptr && need_pad <= W.pcap && need_pad <= (int64_t)INT32_MAX;
 }
 
-// The hub core pass (needs the hub histogram W.cnth only, so it may run on a
-// second stream beside the pair scatter and the short-list pairs): core
-// flags, their scan, core indices, then the padded lists, packed 16-bit when
-// the core allows it, else 32-bit (each pad kernel checks the core size on
-// the device).
-static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, const PhaseScope& ps,
+// The hub core pass (needs only the CSR and cleared counters, so it may run on
+// a second stream from the start, beside the first pass and the scatter): core
+// members, their numbering, then the lists, packed when the core allows it,
+// else 32-bit (each list kernel checks the core size on the device).
+static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, int hub, const PhaseScope& ps,
                             cudaStream_t st) {
     if (!hub_pad_usable(P, W)) return TCHLL_OK;
     if (ps.active()) {
         cudaEventRecord(g_phase.hub_ev[0], st);
         g_phase.core_used = true;
     }
-    core_mark_kernel<<<sm_count() * 8, 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.segs, W.ctr + 2,
-                                                      W.max_segs, W.cbits, W.cflag, P.result);
+    core_mark_kernel<<<grid_rows(P.n_nodes, 256) < 8 * sm_count() ? grid_rows(P.n_nodes, 256) : 8 * sm_count(), 256, 0,
+                       st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, hub, P.nnz <= kMarkAllEdges,
+                             P.graph_vbase ? W.ctr + 2 : nullptr, W.cbits, W.cflag, P.result);
     TCHLL_CHECK_LAUNCH("core_mark_kernel");
     if (P.graph_vbase) {
         core_index_batch_kernel<<<(int)P.n_graphs, 1024, 0, st>>>(W.cbits, W.cflag, P.n_nodes, P.graph_vbase,
@@ -3128,7 +3136,7 @@ static int hub_threshold(const CountParams& P, const CountWs& W, const Tuning& T
 // capture: the first call of a process is never captured by this package).
 struct SideStream {
     cudaStream_t s = nullptr;
-    cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr, mid = nullptr, join = nullptr, back = nullptr;
     std::mutex mu;
 };
 static SideStream g_side[kMaxDevices];
@@ -3149,6 +3157,7 @@ class SideFork {
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming));
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.mid, cudaEventDisableTiming));
                 TCHLL_CUDA(cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming));
+                TCHLL_CUDA(cudaEventCreateWithFlags(&S.back, cudaEventDisableTiming));
             }
         }
         lock_ = std::unique_lock<std::mutex>(S.mu);
@@ -3167,6 +3176,12 @@ class SideFork {
     }
     int wait_mark() {
         TCHLL_CUDA(cudaStreamWaitEvent(caller_, side_->mid, 0));
+        return TCHLL_OK;
+    }
+    // The side stream waits for the caller's work so far (once per fork).
+    int side_waits_caller() {
+        TCHLL_CUDA(cudaEventRecord(side_->back, caller_));
+        TCHLL_CUDA(cudaStreamWaitEvent(side_->s, side_->back, 0));
         return TCHLL_OK;
     }
     // Joins: the caller's stream waits for everything enqueued on the side
@@ -3259,18 +3274,14 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 return rc;
             }
             if (pairs) {
-                // after the first pass, the hub core pass runs on the side
-                // stream beside the pair scatter; the hub kernels wait for
-                // both.  While col_idx is still being copied, the short-list
-                // pairs, which read it, come after the scatter instead.
+                // the hub core pass runs on the side stream beside the first
+                // pass and the scatter; the hub kernels wait for it.  While
+                // col_idx is still being copied, the core pass and the
+                // short-list pairs, which read it, wait for it, the latter
+                // after the scatter.
                 phase_mark(ps, 0, st);
                 P.chunk = pass_chunk(P.n_edges, T.chunk);
                 rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
-                if (rc) return rc;
-                const bool split = col_ready && hub > 0;
-                if (col_ready && !split) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
-                rc = pair_pass<false>(P, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, W.ctr, st);
-                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc) return rc;
                 SideFork fork;
                 const bool side = hub > 0 && T.overlap && hub_pad_usable(P, W);
@@ -3280,10 +3291,15 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                         const cudaError_t e = cudaStreamWaitEvent(fork.stream(), col_ready, 0);
                         if (e != cudaSuccess) rc = cuda_status(e, "cudaStreamWaitEvent(col_ready)");
                     }
-                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, ps, fork.stream());
+                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, hub, ps, fork.stream());
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
+                const bool split = col_ready && hub > 0;
+                if (col_ready && !split) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
+                rc = pair_pass<false>(P, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
+                if (rc) return rc;
                 if (hub > 0) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 if (split) {
@@ -3293,7 +3309,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 }
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, ps, st);
+                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                 }
                 phase_mark(ps, 2, st);
@@ -3319,10 +3335,9 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 // One first pass routes: it counts the short-list exact pairs
                 // (and n_fallback), lists the hub pairs' table sides and the
                 // HLL edges (estimated by hll_edges_kernel, which counts
-                // n_approx / n_clamped).  The HLL pass needs only that pass,
-                // so it forks onto the side stream there and overlaps the
-                // scatter and the hub kernels (all add integers into the same
-                // result block).
+                // n_approx / n_clamped).  The HLL pass needs only that pass
+                // and runs on the side stream beside the scatter and the hub
+                // kernels (all add integers into the same result block).
                 P.work = W.ctr;
                 P.hll_u = HW.hll_u;
                 P.hll_v = HW.hll_v;
@@ -3331,11 +3346,9 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 P.chunk = pass_chunk(P.n_edges, T.chunk);
                 rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
                 if (rc) return rc;
-                rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, W.ctr, st);
-                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
-                if (rc) return rc;
-                // side stream: the hub core pass first (the hub kernels wait
-                // for it), then the HLL pass
+                // side stream: the hub core pass (the hub kernels wait for
+                // it) and the zero masks beside the first pass, then, once
+                // that has listed the HLL edges, their pass
                 SideFork fork;
                 cudaStream_t hst = st;
                 const bool core_side = hub > 0 && T.overlap && hub_pad_usable(P, W);
@@ -3344,20 +3357,25 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     if (rc) return rc;
                     hst = fork.stream();
                     if (core_side) {
-                        rc = launch_core_pass(P, W, T, ps, hst);
+                        rc = launch_core_pass(P, W, T, hub, ps, hst);
                         if (rc == TCHLL_OK) rc = fork.mark();
                         if (rc) return rc;
                     }
                 }
+                rc = launch_zmask(P, HW, hst);
+                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                if (rc == TCHLL_OK && T.overlap) rc = fork.side_waits_caller();
+                if (rc) return rc;
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[0], hst);
                 rc = launch_hll_edges(P, HW, T, hst);
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[1], hst);
+                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc) return rc;
                 if (hub > 0) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, ps, st);
+                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                     if (rc) return rc;
                 }
@@ -3378,7 +3396,8 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                             : launch_count<MODE_HYB_EXACT>(P, T, false, st);
                 if (rc) return rc;
                 phase_mark(ps, 2, st);
-                rc = launch_hll_edges(P, HW, T, st);
+                rc = launch_zmask(P, HW, st);
+                if (rc == TCHLL_OK) rc = launch_hll_edges(P, HW, T, st);
                 phase_mark(ps, 3, st);
                 phase_used(ps, 1, 2);
                 return rc;
@@ -4000,7 +4019,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     }
     phase_mark(ps, 1, st);
     if (hubs) {
-        rc = launch_core_pass(P, B.cw, T, ps, st);
+        rc = launch_core_pass(P, B.cw, T, hub, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
     }
