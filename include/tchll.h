@@ -69,6 +69,12 @@ const char* tchll_last_error(void);
 int tchll_version(void);
 /* Number of kernels this library has launched in this process (host). */
 uint64_t tchll_launch_count(void);
+/* Reads n bytes of device memory (src) into host memory (dst) in stream order
+ * and waits for the stream: how a caller without pinned memory of its own
+ * reads a result block cheaply.  tchll_device_sync waits for the current
+ * device. */
+int tchll_fetch(void* dst /* host */, const void* src, int64_t n, void* stream);
+int tchll_device_sync(void);
 
 /* --------------------------------------------- exact / hybrid counting --- */
 /* Workspace for tchll_exact_count / tchll_hybrid_count_* on a CSR of n_nodes

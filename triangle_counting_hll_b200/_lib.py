@@ -59,6 +59,8 @@ SIGNATURES = {
     "tchll_last_error": (C.c_char_p, []),
     "tchll_version": (C.c_int, []),
     "tchll_launch_count": (_U64, []),
+    "tchll_fetch": (C.c_int, [_P, _P, _I64, _P]),
+    "tchll_device_sync": (C.c_int, []),
     "tchll_count_workspace_bytes": (C.c_int, [_I64, _I64, C.POINTER(_SZ)]),
     "tchll_hybrid_workspace_bytes": (C.c_int, [_I64, _I64, _I64, C.c_int32, C.POINTER(_SZ)]),
     "tchll_exact_count": (C.c_int, [_P, _I64, _P, _I64, _P, _P, _I64, _P, _P, _P, _SZ, _P]),
@@ -206,8 +208,45 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr() if t.numel() > 0 else None
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_handle(device=None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    idx = device.index if isinstance(device, torch.device) else None
+    return _raw_stream(torch.cuda.current_device() if idx is None else idx)
+
+
+class on_device:
+    """torch.cuda.device(dev) that costs next to nothing when dev is already
+    the current device."""
+
+    __slots__ = ("dev", "ctx")
+
+    def __init__(self, dev: torch.device):
+        self.dev = dev
+        self.ctx = None
+
+    def __enter__(self):
+        if self.dev.index is not None and self.dev.index != torch.cuda.current_device():
+            self.ctx = torch.cuda.device(self.dev)
+            self.ctx.__enter__()
+        return self
+
+    def __exit__(self, *exc):
+        if self.ctx is not None:
+            self.ctx.__exit__(*exc)
+
+
+def device_sync() -> None:
+    check(load().tchll_device_sync(), "synchronize")
+
+
+def fetch(dst, src: torch.Tensor, nbytes: int) -> None:
+    """Read nbytes of src into the ctypes object dst; waits for the current
+    stream of src's device."""
+    check(load().tchll_fetch(C.byref(dst), src.data_ptr(), nbytes, stream_handle(src.device)), "fetch")
 
 
 class Workspace:
@@ -222,7 +261,7 @@ class Workspace:
     def get(self, nbytes: int, device) -> torch.Tensor:
         dev = torch.device(device)
         idx = dev.index if dev.index is not None else torch.cuda.current_device()
-        key = (idx, torch.cuda.current_stream(idx).cuda_stream)
+        key = (idx, stream_handle(dev))
         b = self._buf.get(key)
         if b is None or b.numel() < nbytes:
             b = torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=dev)
@@ -242,8 +281,9 @@ def count_result_tensor(device) -> torch.Tensor:
 
 def read_count_result(t: torch.Tensor) -> CountResult:
     """Copy a device count result to the host (synchronises the stream)."""
-    host = t.cpu().numpy().tobytes()
-    return CountResult.from_buffer_copy(host)
+    res = CountResult()
+    fetch(res, t, RESULT_BYTES)
+    return res
 
 
 def raise_on_status(res: CountResult) -> None:

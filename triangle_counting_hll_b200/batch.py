@@ -176,8 +176,12 @@ def hybrid_from_results(res: torch.Tensor, n: int):
     r = _results(res, n)
     if (r["status"] != 0).any():
         raise ValueError(f"malformed input in {(r['status'] != 0).sum()} graph(s) of the batch")
-    totals = np.array([((int(e) << 32) + ((int(h) << 64) | int(lo))) / 4294967296
-                       for e, lo, h in zip(r["exact"], r["lo"], r["hi"])], dtype=np.float64)
+    # in units of 2^-32; sums past 64 bits one by one, in Python integers
+    fx = (r["exact"] << np.uint64(32)) + r["lo"]
+    wide = (r["hi"] != 0) | (r["exact"] >> np.uint64(31) != 0) | (r["lo"] >> np.uint64(63) != 0)
+    totals = fx.astype(np.float64) / 4294967296.0
+    for i in np.flatnonzero(wide):
+        totals[i] = ((int(r["exact"][i]) << 32) + ((int(r["hi"][i]) << 64) | int(r["lo"][i]))) / 4294967296
     stats = {k: r[k].astype(np.int64) for k in ("n_approx", "n_exact", "n_fallback", "n_clamped")}
     return totals, stats
 

@@ -75,12 +75,14 @@ def csr_from_edges(raw_u, raw_v, device=None, undirected: bool = False):
     n_raw = int(u.numel())
     nb = C.c_size_t(0)
     check(L.tchll_csr_workspace_bytes(n_raw, C.byref(nb)))
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         ws = torch.empty(max(nb.value, 256), dtype=torch.uint8, device=dev)
         sizes = torch.empty(2, dtype=torch.int64, device=dev)
         st = stream_handle(dev)
         check(L.tchll_csr_build_phase1(ptr(u), ptr(v), n_raw, ptr(sizes), ptr(ws), nb.value, st), "csr phase 1")
-        n_nodes, n_edges = (int(x) for x in sizes.cpu().tolist())
+        got = (C.c_int64 * 2)()
+        _lib.fetch(got, sizes, 16)
+        n_nodes, n_edges = got
         if n_nodes < 0:
             raise ValueError("negative vertex id in edge list")
         row_ptr = torch.empty(n_nodes + 1, dtype=torch.int32, device=dev)
@@ -400,7 +402,9 @@ def sketch_slots(row_ptr: torch.Tensor, theta: int) -> Tuple[torch.Tensor, int]:
     ns = torch.empty(1, dtype=torch.int64, device=dev)
     check(L.tchll_sketch_slots(ptr(row_ptr), n, int(theta), ptr(slot), ptr(ns), ptr(ws), ws.numel(),
                                stream_handle(dev)), "sketch slots")
-    return slot, int(ns.item())
+    got = C.c_int64(0)
+    _lib.fetch(got, ns, 8)
+    return slot, got.value
 
 
 def build_sketches_compact_tensors(row_ptr, col_idx, slot, n_rows: int, p: int,
@@ -450,14 +454,17 @@ def exact_from_result(res_t: torch.Tensor) -> int:
     return int(r.exact)
 
 
-def hybrid_from_result(res_t: torch.Tensor) -> Tuple[float, _lib.CountResult]:
-    """(total, raw result): total = exact part + HLL fixed-point part, rounded
-    once to FP64."""
-    r = _lib.read_count_result(res_t)
+def hybrid_total(r: _lib.CountResult) -> float:
+    """Exact part + HLL fixed-point part, rounded once to FP64."""
     _lib.raise_on_status(r)
     fx = (int(r.hll_fx_hi) << 64) | int(r.hll_fx_lo)
-    total = ((int(r.exact) << 32) + fx) / 4294967296
-    return float(total), r
+    return float(((int(r.exact) << 32) + fx) / 4294967296)
+
+
+def hybrid_from_result(res_t: torch.Tensor) -> Tuple[float, _lib.CountResult]:
+    """(total, raw result)."""
+    r = _lib.read_count_result(res_t)
+    return hybrid_total(r), r
 
 
 # ------------------------------------------------------------- generators

@@ -43,3 +43,46 @@ TCHLL_EXPORT const char* tchll_last_error(void) { return tchll::g_err; }
 TCHLL_EXPORT int tchll_version(void) { return 10000; }
 
 TCHLL_EXPORT uint64_t tchll_launch_count(void) { return tchll::g_launches.load(std::memory_order_relaxed); }
+
+// Small device-to-host reads.  A copy into pageable memory goes through the
+// driver's staging and costs several times a copy into pinned memory, so each
+// host thread keeps one pinned page (made on its first read, freed when the
+// thread ends); the wait for the stream is the read's own.
+namespace tchll {
+namespace {
+constexpr size_t kStageBytes = 4096;
+struct PinnedStage {
+    void* p = nullptr;
+    void* get() {
+        if (p == nullptr && cudaMallocHost(&p, kStageBytes) != cudaSuccess) {
+            cudaGetLastError();  // no pinned memory: the caller copies directly
+            p = nullptr;
+        }
+        return p;
+    }
+    ~PinnedStage() {
+        if (p) cudaFreeHost(p);
+    }
+};
+thread_local PinnedStage g_stage;
+}  // namespace
+
+int fetch_small(void* dst, const void* src, size_t n, cudaStream_t st) {
+    void* stage = n <= kStageBytes ? g_stage.get() : nullptr;
+    TCHLL_CUDA(cudaMemcpyAsync(stage ? stage : dst, src, n, cudaMemcpyDeviceToHost, st));
+    TCHLL_CUDA(cudaStreamSynchronize(st));
+    if (stage) memcpy(dst, stage, n);
+    return TCHLL_OK;
+}
+}  // namespace tchll
+
+TCHLL_EXPORT int tchll_fetch(void* dst, const void* src, int64_t n, void* stream) {
+    TCHLL_ARG(n >= 0 && (n == 0 || (dst && src)), "bad arguments");
+    if (n == 0) return TCHLL_OK;
+    return tchll::fetch_small(dst, src, (size_t)n, (cudaStream_t)stream);
+}
+
+TCHLL_EXPORT int tchll_device_sync(void) {
+    TCHLL_CUDA(cudaDeviceSynchronize());
+    return TCHLL_OK;
+}

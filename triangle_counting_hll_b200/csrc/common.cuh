@@ -44,6 +44,10 @@ void count_launch(int n = 1);
 
 int sm_count();
 
+// Copies n bytes of device memory to the host and waits for the stream
+// (through a pinned page when they fit one).
+int fetch_small(void* dst, const void* src, size_t n, cudaStream_t st);
+
 // Current device ordinal, or -1 if it cannot be read or is >= kMaxDevices
 // (per-device host caches are indexed by it).
 constexpr int kMaxDevices = 64;

@@ -677,8 +677,8 @@ TCHLL_EXPORT int tchll_csr_build_phase1(const int32_t* raw_u, const int32_t* raw
     max_id_kernel<<<grid_n(n_raw), 256, 0, st>>>(raw_u, raw_v, n_raw, W.cnt);
     TCHLL_CHECK_LAUNCH("max_id_kernel");
     int64_t hc[2] = {0, 0};
-    TCHLL_CUDA(cudaMemcpyAsync(hc, W.cnt + 2, sizeof(hc), cudaMemcpyDeviceToHost, st));
-    TCHLL_CUDA(cudaStreamSynchronize(st));
+    const int rf = fetch_small(hc, W.cnt + 2, sizeof(hc), st);
+    if (rf) return rf;
     if (hc[0]) {  // a negative id: sizes -1, nothing else
         sizes_kernel<<<1, 1, 0, st>>>(W.k0, W.e0, W.cnt, 1, 0, sizes);
         TCHLL_CHECK_LAUNCH("sizes_kernel");

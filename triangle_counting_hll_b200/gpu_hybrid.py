@@ -94,15 +94,15 @@ def gpu_exact_triangle_count(row_ptr_d, col_idx_d, edge_u_d, edge_v_d):
             count = core.exact_from_result(res)
         return count, elapsed
     rp, ci, eu, ev = _inputs(row_ptr_d, col_idx_d, edge_u_d, edge_v_d)
-    with torch.cuda.device(rp.device):
+    with _lib.on_device(rp.device):
         res = _lib.count_result_tensor(rp.device)
-        torch.cuda.synchronize()
+        _lib.device_sync()
         t0 = time.perf_counter()
         core.exact_count_tensors(rp, ci, eu, ev, result=res)
-        torch.cuda.synchronize()
+        r = _lib.read_count_result(res)  # waits for the count
         elapsed = time.perf_counter() - t0
-        count = core.exact_from_result(res)
-    return count, elapsed
+        _lib.raise_on_status(r)
+    return int(r.exact), elapsed
 
 
 def gpu_hybrid_triangle_count(row_ptr_d, col_idx_d, edge_u_d, edge_v_d, degrees_d, sketch_regs_d, has_sketch_d,
@@ -118,15 +118,15 @@ def gpu_hybrid_triangle_count(row_ptr_d, col_idx_d, edge_u_d, edge_v_d, degrees_
     regs = as_device_tensor(sketch_regs_d, torch.uint8, "sketch_regs", dev)
     has = as_device_tensor(has_sketch_d, torch.uint8, "has_sketch", dev)
     n_edges = int(eu.numel())
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         res = _lib.count_result_tensor(dev)
-        torch.cuda.synchronize()
+        _lib.device_sync()
         t0 = time.perf_counter()
         core.hybrid_count_dense_tensors(rp, ci, eu, ev, deg, regs, has, int(gamma), int(p),
                                         split_kernels=bool(split_kernels), result=res)
-        torch.cuda.synchronize()
+        r = _lib.read_count_result(res)  # waits for the count
         elapsed = time.perf_counter() - t0
-        estimate, r = core.hybrid_from_result(res)
+        estimate = core.hybrid_total(r)
     n_approx, n_exact, n_clamped = int(r.n_approx), int(r.n_exact), int(r.n_clamped)
     stats = {
         "n_approx": n_approx,
