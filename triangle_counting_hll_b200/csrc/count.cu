@@ -2168,26 +2168,30 @@ struct HllParams {
     const int64_t* slot;  // null: dense rows (row v at v * 2^p)
     const uint32_t* zm;   // zero masks, zst words per row (null: count zeros from the registers)
     int zst;
+    const double* lc;      // with zm: linear-counting estimate by zero count
     const int32_t* vbase;  // batched: per-edge results go to result[graph of u]
     int64_t n_graphs;
     int p;
     int variant;
     uint32_t lc_min;
-    int zsh;  // contiguous runs: u's mask kept in shared memory (one slot per group) when registers cannot hold it
     tchll_count_result* result;
 };
 
 // Zero-register masks: bit j of word w of row r is set iff register 32w + j
 // of the row is 0.  Rows are zst >= 4 words (16-byte aligned); bits past 2^p
 // stay clear.  One warp per row; dense layouts skip rows without a sketch
-// (no HLL edge reads them).
+// (no HLL edge reads them).  lc[z] is the linear-counting estimate of z zero
+// registers: the HLL pass looks it up instead of taking an FP64 logarithm per
+// edge.
 __global__ void __launch_bounds__(256) zmask_kernel(const uint8_t* __restrict__ regs, int64_t n_rows,
                                                     const uint8_t* __restrict__ has, int p, int zst,
-                                                    uint32_t* __restrict__ zm) {
+                                                    uint32_t* __restrict__ zm, double* __restrict__ lc) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int m = 1 << p;
+    for (int64_t z = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; z <= m; z += (int64_t)gridDim.x * blockDim.x)
+        lc[z] = z > 0 ? (double)m * log((double)m / (double)z) : 0.0;
     for (int64_t r = warp; r < n_rows; r += nwarps) {
         if (has && !__ldg(has + r)) continue;
         const uint4* row = reinterpret_cast<const uint4*>(regs + r * (int64_t)m);
@@ -2314,9 +2318,19 @@ __device__ __forceinline__ double hll_estimate_from(U128 zsum, double extra, uin
 // 16-byte words per lane) and, with CROW (rows of at most 8 16-byte words
 // per lane), u's register row too: an edge then reads only v's mask and
 // row.  Otherwise the groups stride over the list.
-template <int L, bool ZM, bool CACHE, bool CROW>
-__global__ void __launch_bounds__(256, CROW ? 2 : (CACHE ? 3 : 4)) hll_edges_kernel(const HllParams H) {
-    extern __shared__ __align__(16) uint4 zsm[];  // with H.zsh: 256 / L slots of one zero mask each
+// ZS (p >= 11, masks too long for four words per lane): u's mask stays in a
+// shared-memory slot per group.  Slots are kZsPad 16-byte words apart beyond
+// their length, so that the groups that one load instruction serves in one
+// phase (8 lanes) read different banks.  A variant of its own keeps the
+// register form's 16 words out of it (64 registers, four CTAs per SM): with
+// the padding and the table of linear-counting estimates, R-MAT 20, theta =
+// 128, alone: p = 12 609 -> 339 us, p = 14 1478 -> 1078.
+template <int L>
+constexpr int kZsPad = L < 8 ? L : 0;
+
+template <int L, bool ZM, bool CACHE, bool CROW, bool ZS>
+__global__ void __launch_bounds__(256, CROW ? 2 : (ZS ? 4 : (CACHE ? 3 : 4))) hll_edges_kernel(const HllParams H) {
+    extern __shared__ __align__(16) uint4 zsm[];  // ZS: 256 / L slots of one zero mask each
     const int lane = threadIdx.x & 31;
     const int sub = lane & (L - 1);
     const unsigned gmask = (L == 32) ? FULL : (((1u << L) - 1u) << (lane & ~(L - 1)));
@@ -2334,8 +2348,8 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (CACHE ? 3 : 4)) hll_edges_ker
     const int64_t e_step = CACHE ? 1 : ngroups;
     const int64_t w_first = gid - (lane / L);  // the warp's first group
     const int nq = H.zst >> 2;
-    constexpr int KA = CROW ? 1 : 4;  // mask words cached per lane (p <= 10 with a cached row: one)
-    const bool cache_a = CACHE && ZM && nq <= KA * L;
+    constexpr int KA = CROW || ZS ? 1 : 4;  // mask words cached per lane (p <= 10 with a cached row: one)
+    const bool cache_a = CACHE && ZM && !ZS && nq <= KA * L;
     int64_t cached = -1, cached_row = -1;
     uint4 ca[KA];
     uint4 ra[CROW ? 8 : 1];
@@ -2373,10 +2387,10 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (CACHE ? 3 : 4)) hll_edges_ker
                                      __popc(ca[kk].w & b.w);
                         }
                     }
-                } else if (CACHE && H.zsh) {
+                } else if (ZS) {
                     // u's mask in the group's shared-memory slot while
                     // consecutive edges share u: each edge reads v's only
-                    uint4* zs = zsm + (size_t)(threadIdx.x / L) * nq;
+                    uint4* zs = zsm + (size_t)(threadIdx.x / L) * (nq + kZsPad<L>);
                     if (su != cached) {  // group-uniform
                         __syncwarp(gmask);  // the group is done with the previous row
                         for (int i = sub; i < nq; i += L) zs[i] = __ldg(za + i);
@@ -2409,7 +2423,7 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (CACHE ? 3 : 4)) hll_edges_ker
         zeros = group_sum_u32<L>(zeros, gmask);
         const bool need = act && zeros < H.lc_min;  // group-uniform
         double E = 0.0;
-        if (act && !need) E = (double)m * log((double)m / (double)zeros);
+        if (act && !need) E = ZM ? __ldg(H.lc + zeros) : (double)m * log((double)m / (double)zeros);
         // rows of fewer than 32 16-byte words (p <= 8) would leave most of
         // the warp idle in a warp-wide pass 2: there each group forms Z
         if (CROW || nvec < 32) {
@@ -2754,6 +2768,7 @@ struct HybridWs {
     unsigned long long* hll_n;
     uint32_t* zm;  // null when the workspace was sized without masks
     int zst;
+    double* lc;    // with zm: 2^p + 1 linear-counting estimates
 };
 
 static int zmask_words(int p) {
@@ -2772,9 +2787,11 @@ static bool carve_count_hybrid(void* ws, size_t bytes, int64_t n_nodes, int64_t 
     H.hll_v = cv.take<int32_t>(E);
     H.zm = nullptr;
     H.zst = 0;
+    H.lc = nullptr;
     if (zm_rows > 0) {
         H.zst = zmask_words(p);
         H.zm = cv.take<uint32_t>((size_t)zm_rows * (size_t)H.zst);
+        H.lc = cv.take<double>(((size_t)1 << p) + 1);
     }
     if (need) *need = cv.off;
     if (!cv.ok()) return false;
@@ -2796,26 +2813,24 @@ static uint32_t lc_min_for(int p) {
 template <int L>
 static int launch_hll_edges_L(HllParams H, bool crow, cudaStream_t st) {
     const int grid = sm_count() * 8;
-    H.zsh = 0;
-    if (H.zm && crow && L * 8 >= ((1 << H.p) >> 4)) hll_edges_kernel<L, true, true, true><<<grid, 256, 0, st>>>(H);
+    if (H.zm && crow && L * 8 >= ((1 << H.p) >> 4)) hll_edges_kernel<L, true, true, true, false><<<grid, 256, 0, st>>>(H);
     else if (H.zm && H.p >= 11) {
         // masks too large for the 4 register words per lane go to shared
         // memory, one slot per group, while that fits 96 KB per CTA
         const int nq = H.zst >> 2;
-        const size_t smem = nq > 4 * L ? (size_t)(256 / L) * nq * sizeof(uint4) : 0;
-        size_t bytes = 0;
-        if (smem > 0 && smem <= (96u << 10)) {
+        const size_t smem = nq > 4 * L ? (size_t)(256 / L) * (nq + kZsPad<L>) * sizeof(uint4) : 0;
+        if (smem > 0 && smem <= (104u << 10)) {
             static size_t set[kMaxDevices] = {0};
-            const int rc = ensure_smem((const void*)hll_edges_kernel<L, true, true, false>, smem, set,
-                                       "cudaFuncSetAttribute(hll_edges_kernel)");
+            auto kern = hll_edges_kernel<L, true, true, false, true>;
+            const int rc = ensure_smem((const void*)kern, smem, set, "cudaFuncSetAttribute(hll_edges_kernel)");
             if (rc) return rc;
-            H.zsh = 1;
-            bytes = smem;
+            kern<<<grid, 256, smem, st>>>(H);
+        } else {
+            hll_edges_kernel<L, true, true, false, false><<<grid, 256, 0, st>>>(H);
         }
-        hll_edges_kernel<L, true, true, false><<<grid, 256, bytes, st>>>(H);
     }
-    else if (H.zm) hll_edges_kernel<L, true, false, false><<<grid, 256, 0, st>>>(H);
-    else hll_edges_kernel<L, false, false, false><<<grid, 256, 0, st>>>(H);
+    else if (H.zm) hll_edges_kernel<L, true, false, false, false><<<grid, 256, 0, st>>>(H);
+    else hll_edges_kernel<L, false, false, false, false><<<grid, 256, 0, st>>>(H);
     TCHLL_CHECK_LAUNCH("hll_edges_kernel");
     return TCHLL_OK;
 }
@@ -2826,7 +2841,7 @@ static int launch_zmask(const CountParams& P, const HybridWs& HW, cudaStream_t s
     const int64_t rows = P.slot ? P.n_rows : P.n_nodes;
     const int64_t wgrid = (rows + 7) / 8;
     const int grid = (int)(wgrid < 1 ? 1 : (wgrid > (int64_t)sm_count() * 16 ? (int64_t)sm_count() * 16 : wgrid));
-    zmask_kernel<<<grid, 256, 0, st>>>(P.regs, rows, P.slot ? nullptr : P.has, P.p, HW.zst, HW.zm);
+    zmask_kernel<<<grid, 256, 0, st>>>(P.regs, rows, P.slot ? nullptr : P.has, P.p, HW.zst, HW.zm, HW.lc);
     TCHLL_CHECK_LAUNCH("zmask_kernel");
     return TCHLL_OK;
 }
@@ -2847,21 +2862,23 @@ static int launch_hll_edges(const CountParams& P, const HybridWs& HW, const Tuni
     H.result = P.result;
     H.zm = HW.zm;
     H.zst = HW.zst;
+    H.lc = HW.lc;
     // p <= row_cache_p (with zero masks): contiguous runs per group with u's
     // register row kept in registers, m / 128 lanes per edge (8 16-byte
     // words of the row per lane; off by default: at 128 registers per
     // thread too few warps hide the loads).  With zero masks the pass is
-    // bound by the latency of its dependent loads, so narrow groups (more
-    // edges in flight per warp) win: one lane per edge for p <= 10, 4 for
-    // p = 11, 12, 8 above (R-MAT scale 22, theta = 256, beside the exact
-    // pairs: p = 10 14.2 ms per hybrid step with 1 lane against 15.5 with 8;
-    // p = 12 10.7 with 4 against 11.1 with 8; p = 14 14.0 with 8 against
-    // 17.8 with 32).  Without masks one 16-byte register load per lane per
-    // row.  T.hll_lanes > 0 overrides the width.
+    // bound by the latency of its dependent loads and by the instructions of
+    // a step, which all edges of a warp share, so narrow groups (more edges in
+    // flight per warp) win until their masks no longer coalesce (R-MAT 20,
+    // theta = 64 or 128, alone, us with 1 / 2 / 4 / 8 lanes: p = 10 363 / 328 /
+    // 514 / 840, p = 11 459 / 259 / 293 / 518, p = 12 859 / 537 / 338 / 529,
+    // p = 13 1954 / 2060 / 658 / 607, p = 14 5645 / 6165 / 3740 / 1077).
+    // Without masks one 16-byte register load per lane per row.  T.hll_lanes >
+    // 0 overrides the width.
     const bool crow = H.zm != nullptr && P.p <= T.hll_row_cache_p;
     int width = (1 << P.p) >> 4;
     if (crow) width = (1 << P.p) >> 7;
-    else if (H.zm) width = P.p <= 10 ? 1 : (P.p <= 12 ? 4 : 8);
+    else if (H.zm) width = P.p <= 9 ? 1 : P.p <= 11 ? 2 : P.p == 12 ? 4 : 8;
     if (T.hll_lanes > 0) width = T.hll_lanes;
     switch (width >= 32 ? 32 : (width < 1 ? 1 : width)) {
         case 1: return launch_hll_edges_L<1>(H, crow, st);
@@ -3923,6 +3940,7 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     B.hw.hll_v = cv.take<int32_t>(E);
     B.hw.zm = nullptr;
     B.hw.zst = 0;
+    B.hw.lc = nullptr;
     if (need) *need = cv.off;
     if (!cv.ok() || cv.dry) return cv.ok();
     carve_count(cbase, cneed, n_nodes, n_edges, B.cw, nullptr);
