@@ -110,8 +110,8 @@ int tchll_exact_count(const int32_t* row_ptr, int64_t n_nodes, const int32_t* co
 /* tchll_exact_count (no per-edge output) for a col_idx still being copied:
  * the kernels that read col_idx first wait for col_ready_event (a
  * cudaEvent_t recorded after the copy that fills col_idx; NULL: ready), so
- * the pair regrouping, which reads only row_ptr and the edges, overlaps that
- * copy.  row_ptr, edge_u and edge_v must be ready in stream order.  Same
+ * the regrouping of the hub pairs, which reads only row_ptr and the edges,
+ * overlaps that copy.  row_ptr, edge_u and edge_v must be ready in stream order.  Same
  * result as tchll_exact_count. */
 int tchll_exact_count_staged(const int32_t* row_ptr, int64_t n_nodes, const int32_t* col_idx, int64_t nnz,
                              const int32_t* edge_u, const int32_t* edge_v, int64_t n_edges,
@@ -235,12 +235,14 @@ int tchll_exact_count_noalloc(const int32_t* row_ptr, int64_t n_nodes, const int
 /* Phase timing for measurement (process-wide host state, off by default).
  * When enabled, the counting entry points record CUDA events on the
  * caller's stream around their phases; tchll_phase_times then waits for the
- * last call's events and writes milliseconds: ms3[0] pair regrouping,
- * ms3[1] exact-count kernels (pair kernel and hub kernels), ms3[2] HLL pass
+ * last call's events and writes milliseconds: ms3[0] first pass over the
+ * edges (which counts the short-list pairs) and scatter of the hub pairs,
+ * ms3[1] the hub kernels with the wait for their core pass, or the one
+ * counting launch of a graph counted as given, ms3[2] HLL pass
  * (-1 for a phase the call did not run; with the overlap on, the HLL pass
- * runs beside ms3[1] on the second stream).  tchll_phase_hub_ms writes the
- * hub pairs' share of ms3[1]: ms2[0] the hub kernels, ms2[1] the core pass
- * before them (-1 when they did not run).  While timing is on, counting
+ * runs beside ms3[1] on the second stream).  tchll_phase_hub_ms writes
+ * ms2[0] the hub kernels' time and ms2[1] the core pass's, which with the
+ * overlap on runs beside ms3[0] (-1 when they did not run).  While timing is on, counting
  * calls serialize their enqueues. */
 int tchll_set_phase_timing(int32_t enable);
 int tchll_phase_times(float* ms3 /* host */);

@@ -484,6 +484,7 @@ __global__ void prepare_kernel(const Prepare Q) {
 // in turn (null), or, batched, from the chunk list (a chunk is one graph's,
 // and so are its totals).
 enum : int { PASS_HIST = 1, PASS_SHORT = 2 };
+constexpr int kHugeList = 1 << 25;  // 32 shorter lists of this length still add up below 2^31
 // The n HLL edges of a warp's buffer go to the list.
 constexpr int kHllBuf = 160;
 __device__ __forceinline__ void flush_hll(const CountParams& P, const int2* buf, int n, int lane) {
@@ -605,7 +606,16 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             if (!(what & PASS_SHORT)) continue;
             const bool mine = ok && !to_hub;
             n_exact += __popc(__ballot_sync(FULL, mine));
-            const int np = mine ? S.yl : 0;
+            int np = mine ? S.yl : 0;
+            // lists whose lengths could overflow the stream's positions: one
+            // by one (only without a hub threshold)
+            for (unsigned huge = __ballot_sync(FULL, np > kHugeList); huge; huge &= huge - 1) {
+                const int l = __ffs(huge) - 1;
+                const int32_t xs = __shfl_sync(FULL, S.xs, l), xl = __shfl_sync(FULL, S.xl, l);
+                const int32_t ys = __shfl_sync(FULL, S.ys, l), yl = __shfl_sync(FULL, S.yl, l);
+                acc += warp_sum_u64(warp_bsearch_count(col + xs, xl, col + ys, yl, lane));
+                if (lane == l) np = 0;
+            }
             int incl = np;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -2753,7 +2763,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     W.pcol = pad ? cv.take<int32_t>((size_t)W.pcap) : nullptr;
     W.cflag = pad ? cv.take<int32_t>(N) : nullptr;
     W.pl = pad ? cv.take<int4>(N) : nullptr;
-    W.pool_cap = pad ? (int64_t)(E / 16) + 1024 : 0;
+    W.pool_cap = pad ? (int64_t)(E / 16) + 64 : 0;
     W.pool = pad ? cv.take<uint4>((size_t)W.pool_cap) : nullptr;
     if (need) *need = cv.off;
     return cv.ok();
@@ -3221,8 +3231,8 @@ class SideFork {
 };
 
 // col_ready (exact counts only; null = ready): an event the kernels that
-// read col_idx wait for, so the pair regrouping (row_ptr and the edges only)
-// overlaps a copy of col_idx still in flight.
+// read col_idx wait for, so the regrouping of the hub pairs (row_ptr and the
+// edges only) overlaps a copy of col_idx still in flight.
 static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_bytes, cudaStream_t st,
                      cudaEvent_t col_ready = nullptr) {
     const Tuning T = tuning_snapshot();
