@@ -212,7 +212,7 @@ def phase_report(pair_ms, count_ms, hub_ms, core_ms, tuning: dict) -> dict:
     """Phase times of one exact count.  pair_regroup is the first pass over the
     edges (which also counts the short-list pairs) and the scatter of the hub
     pairs.  With the overlap on, the hub core pass runs on the second stream
-    beside the scatter, so it is reported apart from the serial phases."""
+    beside both, so it is reported apart from the serial phases."""
     out = {"pair_regroup": pair_ms, "count": count_ms, "hub_kernels": hub_ms}
     if not hub_ms:
         out["pair_kernel"] = count_ms
@@ -556,14 +556,13 @@ def run_hybrid_line(args, g, dev, rank, world, barrier, max_over_ranks):
     del host
 
     peaks = load_peaks()
-    # the dominant kernel of the three: HLL pass (on the side stream, beside
-    # the others), hub pairs, other exact pairs
+    # the dominant one of the three: HLL pass (on the side stream, beside the
+    # others), hub pairs, first pass (routing, short-list pairs) and scatter
     hub_ms = avg.get("hub") or 0.0
-    core_ms = avg.get("hub_core") or 0.0
     tuning = core.get_count_tuning()
     hname = hub_kernel_name(tuning, hub_work(g, tuning["hub"])["core_vertices"])
     cands = [("hll_edges_kernel", avg["hll"], hll_bytes), (hname, hub_ms, hub_bytes),
-             ("count_kernel", avg["count"] - hub_ms - core_ms, exact_bytes - hub_bytes)]
+             ("pair_pass_kernel + pair_scatter_kernel", avg.get("pairs") or 0.0, exact_bytes - hub_bytes)]
     kname, kms, kbytes = max(cands, key=lambda c: c[1])
     traffic = load_traffic(f"rmat{args.scale}_ef16_hybrid_p{p}_theta{theta}:{kname}")
     roof = {"bound": "hbm", "kernel": kname, "peak": peaks["hbm_gbs"], "peak_source": peaks["source"],

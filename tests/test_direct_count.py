@@ -120,3 +120,21 @@ def test_batch_mixes_graphs_with_and_without_long_lists(tchll, oracle):
     want, wstats = batch.plain_hybrid_counts(csrs, batch.plain_sketches(csrs, 64, 10), 64, 10)
     assert np.array_equal(totals, want)
     assert all(np.array_equal(stats[k], wstats[k]) for k in stats)
+
+
+@pytest.mark.parametrize("length", [1 << 25, (1 << 25) + 1])
+def test_lists_longer_than_a_warp_adds_up(tchll, length):
+    """Vertex 0 is joined to all others, vertex 1 to all after it: the pair
+    (0, 1) closes one triangle for every member of the shorter list."""
+    import torch
+    from triangle_counting_hll_b200 import core
+    n = length + 2
+    row_ptr = torch.full((n + 1,), 2 * length + 1, dtype=torch.int32, device="cuda")
+    row_ptr[0] = 0
+    row_ptr[1] = length + 1
+    col = torch.cat([torch.arange(1, n, dtype=torch.int32, device="cuda"),
+                     torch.arange(2, n, dtype=torch.int32, device="cuda")])
+    u = torch.tensor([0, 0, 0], dtype=torch.int32, device="cuda")
+    v = torch.tensor([1, 2, 1], dtype=torch.int32, device="cuda")
+    res, _ = core.exact_count_tensors(row_ptr, col, u, v)
+    assert core.exact_from_result(res) == 2 * length

@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             n_exact += __popc(__ballot_sync(FULL, mine));
             int np = mine ? S.yl : 0;
             // lists whose lengths could overflow the stream's positions: one
-            // by one (only without a hub threshold)
+            // by one (only where no hub threshold applies)
             for (unsigned huge = __ballot_sync(FULL, np > kHugeList); huge; huge &= huge - 1) {
                 const int l = __ffs(huge) - 1;
                 const int32_t xs = __shfl_sync(FULL, S.xs, l), xl = __shfl_sync(FULL, S.xl, l);
@@ -1936,9 +1936,9 @@ __global__ void __launch_bounds__(256, 6) hub_bitmap_kernel(const HubParams H) {
 // conflict-free), then the key units (eight random 4-byte shared loads; a
 // unit's plane, the bitmap's half, follows from its position in the list).
 // A lane finds its unit's list as in hub_bitmap_kernel; the lists' bases sit
-// in a shared-memory slot per warp.  Bound by the L1 data pipe (81% busy on
-// R-MAT 21, issue 65%): R-MAT 18 / 20 / 22 249 / 1189 / 7291 us with key lists
-// alone, 140 / 720 / 5270 us here.
+// in a shared-memory slot per warp.  Bound by the L1 data pipe (86% busy on
+// R-MAT 21, issue 64%): R-MAT 18 / 20 / 22 249 / 1189 / 7291 us with key lists
+// alone, 140 / 707 / 5094 us here.
 constexpr int kHub16Threads = 128;
 template <int UNR>
 __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitmap16_kernel(const HubParams H) {
@@ -2334,7 +2334,8 @@ __device__ __forceinline__ double hll_estimate_from(U128 zsum, double extra, uin
 // phase (8 lanes) read different banks.  A variant of its own keeps the
 // register form's 16 words out of it (64 registers, four CTAs per SM): with
 // the padding and the table of linear-counting estimates, R-MAT 20, theta =
-// 128, alone: p = 12 609 -> 339 us, p = 14 1478 -> 1078.
+// 128, alone: p = 12 609 -> 339 us (L1 data pipe 67 -> 85% busy, which bounds
+// it now), p = 14 1478 -> 1078.
 template <int L>
 constexpr int kZsPad = L < 8 ? L : 0;
 
