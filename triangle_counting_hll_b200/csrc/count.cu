@@ -227,12 +227,16 @@ __device__ __forceinline__ void validate_rows(const int32_t* __restrict__ row_pt
         if (a < 0 || b < a || (int64_t)b > nnz) status |= ST_BAD_ROW;
     }
     const int64_t lo = __ldg(row_ptr), hi = __ldg(row_ptr + n_nodes);
-    if (lo < 0 || hi > nnz) return;
-    const int64_t l4 = min((lo + 3) & ~(int64_t)3, hi), h4 = max(hi & ~(int64_t)3, l4);
+    if (lo < 0 || hi < lo || hi > nnz) return;
+    // 16-byte loads between the first and the last 16-byte boundary: col may
+    // start on any word
+    const int64_t head = lo + (int64_t)((4 - (((uintptr_t)(col + lo) >> 2) & 3)) & 3);
+    const int64_t l4 = min(head, hi), n4 = (hi - l4) >> 2, h4 = l4 + 4 * n4;
     const uint32_t n = (uint32_t)n_nodes;
+    const uint4* __restrict__ quads = reinterpret_cast<const uint4*>(col + l4);
     bool bad = false;
-    for (int64_t q = (l4 >> 2) + t0; q < h4 >> 2; q += step) {  // col is 16-byte aligned
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(col) + q);
+    for (int64_t q = t0; q < n4; q += step) {
+        const uint4 v = __ldg(quads + q);
         bad |= v.x >= n || v.y >= n || v.z >= n || v.w >= n;
     }
     if (lo + t0 < l4) bad |= (uint32_t)__ldg(col + lo + t0) >= n;
