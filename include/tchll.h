@@ -325,6 +325,8 @@ int tchll_hash64(const int64_t* values, int64_t n, uint64_t* out, void* stream);
  * positions [row_ptr[vbase[g]], row_ptr[vbase[g+1]])).  results[n_graphs]
  * receives one tchll_count_result per graph, bit-identical to counting that
  * graph alone (an edge outside its graph's range sets status on that graph).
+ * A graph whose vertex range or edge range is malformed is not counted, nor
+ * are the graphs behind it: each gets TCHLL_STATUS_BAD_ROW.
  * Work is a device-built list of chunks that never cross a graph, claimed by
  * one persistent launch.
  */

@@ -95,6 +95,7 @@ struct CountParams {
     const int64_t* n_chunks_dev;
     const int32_t* graph_vbase;  // vertex range of graph g: [vbase[g], vbase[g+1])
     int64_t n_graphs;            // batched calls: graphs in graph_vbase (else 0)
+    unsigned long long* graph_bad;  // batched calls: of them, those from the first malformed one on
     int32_t* graph_hub;          // batched calls: 1 for a graph with hub pairs (first pass)
     int32_t* live_flag;          // batched calls: 1 for 64 rows that touch such a graph
     int32_t* live_list;          // and those blocks of 64 rows, listed
@@ -289,9 +290,11 @@ __device__ __forceinline__ PairSides sides_of(int32_t u, int32_t v, int32_t us, 
 // Hub pairs: a long table side and something to probe it with.
 __device__ __forceinline__ bool is_hub_pair(const PairSides& S, int hub) { return hub > 0 && S.xl > hub && S.yl > 0; }
 
-// Batched calls: the graph of vertex v, the last g with vbase[g] <= v.
-__device__ __forceinline__ int64_t graph_of(const int32_t* vbase, int64_t n_graphs, int32_t v) {
-    int64_t lo = 0, hi = n_graphs - 1;
+// Batched calls: the graph of vertex v, the last g with vbase[g] <= v among
+// the graphs before the first malformed one (the only ones with edges).
+__device__ __forceinline__ int64_t graph_of(const int32_t* vbase, int64_t n_graphs, const unsigned long long* bad,
+                                            int32_t v) {
+    int64_t lo = 0, hi = n_graphs - 1 - (int64_t)__ldg(bad);
     while (lo < hi) {
         const int64_t mid = (lo + hi + 1) >> 1;
         if (__ldg(vbase + mid) <= v) lo = mid; else hi = mid - 1;
@@ -2106,7 +2109,8 @@ __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitma
 __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restrict__ cnth, int64_t n_nodes, int seg,
                                                         int32_t* __restrict__ offh, unsigned long long* n_pairs,
                                                         HubSeg* segs, unsigned long long* n_segs, int64_t max_segs,
-                                                        const int32_t* __restrict__ vbase, int64_t n_graphs) {
+                                                        const int32_t* __restrict__ vbase, int64_t n_graphs,
+                                                        const unsigned long long* __restrict__ graph_bad) {
     __shared__ unsigned long long warp_sum[8], base[2];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t x0 = blockIdx.x * 1024ll + tid;
@@ -2147,7 +2151,7 @@ __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restric
     for (int i = 0; i < 4; ++i) {
         if (c[i] <= 0) continue;
         const int64_t x = x0 + 256 * i;
-        const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, (int32_t)x) : 0;
+        const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, graph_bad, (int32_t)x) : 0;
         offh[x] = at;
         for (int32_t j = 0; j < c[i]; j += seg, ++sg) {
             if (sg >= max_segs) break;  // cannot happen: sized for the worst case
@@ -2185,6 +2189,7 @@ struct HllParams {
     const double* lc;      // with zm: linear-counting estimate by zero count
     const int32_t* vbase;  // batched: per-edge results go to result[graph of u]
     int64_t n_graphs;
+    const unsigned long long* graph_bad;
     int p;
     int variant;
     uint32_t lc_min;
@@ -2536,7 +2541,7 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (ZS ? 4 : (CACHE ? 3 : 4))) hl
             const bool clamped = s_hat < 0.0 || s_hat > upper;
             const uint64_t fx = (uint64_t)__double2ull_rn(s_cl * 4294967296.0);
             if (H.vbase) {  // batched: straight into this edge's graph
-                tchll_count_result* R = H.result + graph_of(H.vbase, H.n_graphs, u);
+                tchll_count_result* R = H.result + graph_of(H.vbase, H.n_graphs, H.graph_bad, u);
                 U128 one;
                 one.lo = fx;
                 atomic_add_u128((unsigned long long*)&R->hll_fx_lo, one);
@@ -2707,8 +2712,8 @@ static int given_chunk(int64_t n_edges, int chunk) {
 
 struct CountWs {
     // counters: [0] [1] chunks, [2] hub segments made, [3] hub segments
-    // claimed, [4] HLL edges, [5] hub pairs; with ncore and cbits one run of
-    // zero_words words
+    // claimed, [4] HLL edges, [5] hub pairs, [6] batches: the graphs from the
+    // first malformed one on; with ncore and cbits one run of zero_words words
     unsigned long long* ctr;
     int64_t zero_words;
     int32_t* cnth;            // n_nodes + 1 (histogram of hub pairs)
@@ -2743,7 +2748,7 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
 // sizes and cursors (256 each), last the number of live row blocks.  Cleared
 // together.
 constexpr int kCoreWords = 4 + 2 * 256 + 1;
-constexpr int kCounters = 6;
+constexpr int kCounters = 8;
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
@@ -2865,6 +2870,7 @@ static int launch_hll_edges(const CountParams& P, const HybridWs& HW, const Tuni
     HllParams H;
     H.vbase = P.graph_vbase;
     H.n_graphs = P.n_graphs;
+    H.graph_bad = P.graph_bad;
     H.hu = HW.hll_u;
     H.hv = HW.hll_v;
     H.n_dev = HW.hll_n;
@@ -2978,13 +2984,12 @@ static int pair_pass(CountParams P, const CountWs& W, int what, int hub, unsigne
 
 // After PASS_HIST: room for the hub pairs, and the hub segments (smaller ones
 // in small graphs, so that every CTA gets a few).
-static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaStream_t st,
-                     const int32_t* vbase = nullptr, int64_t n_graphs = 0) {
+static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaStream_t st) {
     while (hub_seg > HUB_SEG_MIN && P.n_edges < (int64_t)hub_seg * 24 * sm_count()) hub_seg >>= 1;
     if (hub_seg < HUB_SEG_MIN) hub_seg = HUB_SEG_MIN;
     const int grid = (int)(P.n_nodes > 0 ? (P.n_nodes + 1023) / 1024 : 1);
     hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, P.n_nodes, hub_seg, W.offh, W.ctr + 5, W.segs, W.ctr + 2,
-                                           W.max_segs, vbase, n_graphs);
+                                           W.max_segs, P.graph_vbase, P.n_graphs, P.graph_bad);
     TCHLL_CHECK_LAUNCH("hub_alloc_kernel");
     return TCHLL_OK;
 }
@@ -3854,40 +3859,46 @@ TCHLL_EXPORT int tchll_exact_count_noalloc(const int32_t* row_ptr, int64_t n_nod
 // graph; each chunk adds its integer totals to results[g], so per-graph
 // results are bit-identical to one graph at a time.
 
-// A graph whose vertex range is malformed gets no chunks (and a status flag
-// from check_vbase_kernel); no vbase entry is used as an index unchecked.
-__device__ __forceinline__ bool graph_range(const int32_t* base, const int32_t* vbase, int64_t g, int64_t n_nodes,
-                                            int64_t& s0, int64_t& s1) {
+// Edge range of graph g; false when its vertex range or its edge range is
+// malformed (no vbase entry is used as an index unchecked, and no edge outside
+// [0, n_edges) is ever in a range).
+__device__ __forceinline__ bool graph_range(const int32_t* row_ptr, const int32_t* vbase, int64_t g, int64_t n_nodes,
+                                            int64_t n_edges, int64_t& s0, int64_t& s1) {
     const int32_t a = vbase[g], b = vbase[g + 1];
     if (a < 0 || b < a || (int64_t)b > n_nodes) return false;
-    s0 = base[a];
-    s1 = base[b];
-    return s1 >= s0;
+    s0 = row_ptr[a];
+    s1 = row_ptr[b];
+    return s0 >= 0 && s1 >= s0 && s1 <= n_edges;
 }
 
-__global__ void chunk_count_kernel(const int32_t* __restrict__ base, const int32_t* __restrict__ vbase,
-                                   int64_t n_graphs, int64_t n_nodes, int chunk, int64_t* cnt) {
+// The chunks of the graphs before the first malformed one (*bad of
+// check_vbase_kernel).  Neighbouring graphs share a bound, so these ranges
+// do not overlap and their chunks fit the list; behind a malformed graph
+// neither is sure, so the graphs there are refused as well.
+__global__ void chunk_count_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ vbase,
+                                   int64_t n_graphs, int64_t n_nodes, int64_t n_edges, int chunk,
+                                   const unsigned long long* __restrict__ bad, int64_t* cnt,
+                                   tchll_count_result* results) {
+    const int64_t good = n_graphs - (int64_t)*bad;
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g <= n_graphs;
          g += (int64_t)gridDim.x * blockDim.x) {
-        if (g == n_graphs) {
-            cnt[g] = 0;
-            continue;
-        }
-        int64_t s0, s1;
-        cnt[g] = graph_range(base, vbase, g, n_nodes, s0, s1) ? (s1 - s0 + chunk - 1) / chunk : 0;
+        int64_t s0 = 0, s1 = 0;
+        if (g < good) graph_range(row_ptr, vbase, g, n_nodes, n_edges, s0, s1);
+        else if (g < n_graphs) results[g].status |= ST_BAD_ROW;
+        cnt[g] = (s1 - s0 + chunk - 1) / chunk;
     }
 }
 
-__global__ void chunk_fill_kernel(const int32_t* __restrict__ base, const int32_t* __restrict__ vbase,
-                                  int64_t n_graphs, int64_t n_nodes, int chunk, const int64_t* __restrict__ coff,
-                                  int64_t* cstart, int32_t* clen, int32_t* cgraph) {
+__global__ void chunk_fill_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ vbase,
+                                  int64_t n_graphs, int64_t n_nodes, int64_t n_edges, int chunk,
+                                  const int64_t* __restrict__ coff, int64_t* cstart, int32_t* clen, int32_t* cgraph) {
     // one warp per graph
     const int lane = threadIdx.x & 31;
     for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; g < n_graphs;
          g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        int64_t s0 = 0, s1 = 0;
-        if (!graph_range(base, vbase, g, n_nodes, s0, s1)) continue;
         const int64_t n = coff[g + 1] - coff[g];
+        int64_t s0 = 0, s1 = 0;
+        if (n == 0 || !graph_range(row_ptr, vbase, g, n_nodes, n_edges, s0, s1)) continue;
         for (int64_t k = lane; k < n; k += 32) {
             const int64_t st = s0 + k * chunk;
             cstart[coff[g] + k] = st;
@@ -3897,12 +3908,24 @@ __global__ void chunk_fill_kernel(const int32_t* __restrict__ base, const int32_
     }
 }
 
-__global__ void check_vbase_kernel(const int32_t* __restrict__ vbase, int64_t n_graphs, int64_t n_nodes,
+// *bad (zeroed before) = n_graphs less the first malformed graph, 0 when there
+// is none; without edges (row_ptr null) only the vertex ranges count.
+__global__ void check_vbase_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ vbase,
+                                   int64_t n_graphs, int64_t n_nodes, int64_t n_edges, unsigned long long* bad,
                                    tchll_count_result* results) {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n_graphs;
          g += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t a = vbase[g], b = vbase[g + 1];
-        if (a < 0 || b < a || (int64_t)b > n_nodes) results[g].status |= ST_BAD_ROW;
+        int64_t s0, s1;
+        bool ok;
+        if (row_ptr) {
+            ok = graph_range(row_ptr, vbase, g, n_nodes, n_edges, s0, s1);
+        } else {
+            const int32_t a = vbase[g], b = vbase[g + 1];
+            ok = a >= 0 && b >= a && (int64_t)b <= n_nodes;
+        }
+        if (ok) continue;
+        results[g].status |= ST_BAD_ROW;
+        if (bad) atomicMax(bad, (unsigned long long)(n_graphs - g));
     }
 }
 
@@ -3964,12 +3987,14 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     return true;
 }
 
-// Chunk list over per-graph ranges [base[vbase[g]], base[vbase[g+1]]).
-static int build_chunks(const int32_t* base, const int32_t* vbase, int64_t n_graphs, int64_t n_nodes,
-                        const BatchWs& B, int chunk, cudaStream_t st) {
+// Chunk list over the graphs' edge ranges [row_ptr[vbase[g]],
+// row_ptr[vbase[g+1]]), after check_vbase.
+static int build_chunks(const CountParams& P, const int32_t* vbase, int64_t n_graphs, const BatchWs& B, int chunk,
+                        cudaStream_t st) {
     int64_t g = (n_graphs + 256) / 256;
     if (g > (int64_t)sm_count() * 8) g = (int64_t)sm_count() * 8;
-    chunk_count_kernel<<<(int)g, 256, 0, st>>>(base, vbase, n_graphs, n_nodes, chunk, B.cnt);
+    chunk_count_kernel<<<(int)g, 256, 0, st>>>(P.row_ptr, vbase, n_graphs, P.n_nodes, P.n_edges, chunk, P.graph_bad,
+                                               B.cnt, P.result);
     TCHLL_CHECK_LAUNCH("chunk_count_kernel");
     size_t tb = B.tmp_bytes;
     TCHLL_CUDA(cub::DeviceScan::ExclusiveSum(B.tmp, tb, B.cnt, B.coff, (int)(n_graphs + 1), st));
@@ -3977,17 +4002,17 @@ static int build_chunks(const int32_t* base, const int32_t* vbase, int64_t n_gra
     int64_t gw = (n_graphs * 32 + 255) / 256;
     if (gw > (int64_t)sm_count() * 8) gw = (int64_t)sm_count() * 8;
     if (gw < 1) gw = 1;
-    chunk_fill_kernel<<<(int)gw, 256, 0, st>>>(base, vbase, n_graphs, n_nodes, chunk, B.coff, B.cstart, B.clen,
-                                               B.cgraph);
+    chunk_fill_kernel<<<(int)gw, 256, 0, st>>>(P.row_ptr, vbase, n_graphs, P.n_nodes, P.n_edges, chunk, B.coff,
+                                               B.cstart, B.clen, B.cgraph);
     TCHLL_CHECK_LAUNCH("chunk_fill_kernel");
     return TCHLL_OK;
 }
 
-static int check_vbase(const int32_t* vbase, int64_t n_graphs, int64_t n_nodes, tchll_count_result* results,
-                       cudaStream_t st) {
+static int check_vbase(const CountParams& P, const int32_t* vbase, int64_t n_graphs, cudaStream_t st) {
     int64_t g = (n_graphs + 255) / 256;
     if (g > 1024) g = 1024;
-    check_vbase_kernel<<<(int)g, 256, 0, st>>>(vbase, n_graphs, n_nodes, results);
+    check_vbase_kernel<<<(int)g, 256, 0, st>>>(P.n_edges > 0 ? P.row_ptr : nullptr, vbase, n_graphs, P.n_nodes,
+                                               P.n_edges, P.graph_bad, P.result);
     TCHLL_CHECK_LAUNCH("check_vbase_kernel");
     return TCHLL_OK;
 }
@@ -4009,6 +4034,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     P.sparse = T.sparse;
     P.graph_vbase = vbase;
     P.n_graphs = n_graphs;
+    P.graph_bad = P.n_edges > 0 ? B.cw.ctr + 6 : nullptr;
     P.n_chunks_dev = B.coff + n_graphs;
     P.chunk_start = B.cstart;
     P.chunk_len = B.clen;
@@ -4017,7 +4043,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     P.live_flag = B.rflag;
     P.live_list = B.rlist;
     int rc;
-    if (P.n_edges == 0) return check_vbase(vbase, n_graphs, P.n_nodes, P.result, st);
+    if (P.n_edges == 0) return check_vbase(P, vbase, n_graphs, st);
     PhaseScope ps;
     phase_reset(ps);
     // Hybrid: the routing pass also appends the HLL-routed edges to a list
@@ -4032,8 +4058,8 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     // go to the hub kernels, which publish per segment into the graph of x
     const int hub = hub_threshold(P, B.cw, T);
     rc = pass_prepare(P, B.cw, hub, n_graphs, reinterpret_cast<uint32_t*>(B.ghub), (int64_t)(B.flag_bytes / 4), st);
-    if (rc == TCHLL_OK) rc = check_vbase(vbase, n_graphs, P.n_nodes, P.result, st);
-    if (rc == TCHLL_OK) rc = build_chunks(P.row_ptr, vbase, n_graphs, P.n_nodes, B, T.chunk, st);
+    if (rc == TCHLL_OK) rc = check_vbase(P, vbase, n_graphs, st);
+    if (rc == TCHLL_OK) rc = build_chunks(P, vbase, n_graphs, B, T.chunk, st);
     if (rc) return rc;
     if (hll_list || !hybrid) {
         if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, hub, B.cw.ctr, st);
@@ -4046,7 +4072,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     }
     const bool hubs = hub > 0 && (hll_list || !hybrid);
     if (hubs) {
-        rc = hub_alloc(P, B.cw, T.hub_seg, st, vbase, n_graphs);
+        rc = hub_alloc(P, B.cw, T.hub_seg, st);
         if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
         if (rc) return rc;
     }
