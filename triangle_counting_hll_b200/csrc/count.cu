@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
     const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     while (true) {
-        int32_t e0, e1;  // below 2^31
+        uint32_t e0, e1;  // below 2^31; the loop steps up to 31 past e1
         int32_t g = -1;
         uint32_t lo_v = 0, in_v = (uint32_t)P.n_nodes;
         unsigned long long chunk;
@@ -553,22 +553,22 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             chunk = c;
             if (P.chunk_start) {
                 if ((int64_t)c >= *P.n_chunks_dev) break;
-                e0 = (int32_t)__ldg(P.chunk_start + c);
-                e1 = e0 + __ldg(P.chunk_len + c);
+                e0 = (uint32_t)__ldg(P.chunk_start + c);
+                e1 = e0 + (uint32_t)__ldg(P.chunk_len + c);
                 g = __ldg(P.chunk_graph + c);
                 lo_v = (uint32_t)__ldg(P.graph_vbase + g);
                 in_v = (uint32_t)__ldg(P.graph_vbase + g + 1) - lo_v;
             } else {
                 if ((int64_t)c * P.chunk >= P.n_edges) break;
-                e0 = (int32_t)c * P.chunk;
-                e1 = (int32_t)min((int64_t)e0 + P.chunk, P.n_edges);
+                e0 = (uint32_t)c * (uint32_t)P.chunk;
+                e1 = (uint32_t)min((int64_t)e0 + P.chunk, P.n_edges);
             }
         }
         bool any_hub = false;
         // the chunk's codes: no two chunks of a batch share one
         const int64_t code0 = (e0 >> 5) + (g >= 0 ? (int64_t)chunk : 0);
-        for (int32_t eb = e0; eb < e1; eb += 32) {
-            const int32_t e = eb + lane;
+        for (uint32_t eb = e0; eb < e1; eb += 32) {
+            const uint32_t e = eb + lane;
             int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
             bool ok = e < e1, wants = false, both = false;
             if (P.rows) {
@@ -2120,7 +2120,7 @@ __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restric
     for (int i = 0; i < 4; ++i) {
         const int64_t x = x0 + 256 * i;
         c[i] = x < n_nodes ? __ldg(cnth + x) : 0;
-        mine += ((unsigned long long)c[i] << 32) + (unsigned)((c[i] + seg - 1) / seg);
+        mine += ((unsigned long long)c[i] << 32) + ((unsigned)c[i] + (unsigned)seg - 1u) / (unsigned)seg;
     }
     unsigned long long incl = mine;
 #pragma unroll
@@ -2153,12 +2153,12 @@ __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restric
         const int64_t x = x0 + 256 * i;
         const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, graph_bad, (int32_t)x) : 0;
         offh[x] = at;
-        for (int32_t j = 0; j < c[i]; j += seg, ++sg) {
+        for (int64_t j = 0; j < c[i]; j += seg, ++sg) {
             if (sg >= max_segs) break;  // cannot happen: sized for the worst case
             HubSeg s;
-            s.start = at + j;
+            s.start = at + (int32_t)j;
             s.x = (int32_t)x;
-            s.len = min(seg, c[i] - j);
+            s.len = min(seg, c[i] - (int32_t)j);
             s.graph = g;
             segs[sg] = s;
         }
@@ -3007,10 +3007,11 @@ static int grid_rows(int64_t n, int per_cta) {  // one unit of work per 256 / pe
 }
 
 // The hub core pass and kernels use the padded lists when the workspace
-// holds them and 16-byte unit indices fit int.
+// holds them and 16-byte unit indices, and steps of 128 members past the end
+// of a row, fit int.
 static bool hub_pad_usable(const CountParams& P, const CountWs& W) {
     const int64_t need_pad = pad_capacity(P.n_nodes, P.nnz);
-    return W.pcol != nullptr && need_pad <= W.pcap && need_pad <= (int64_t)INT32_MAX;
+    return W.pcol != nullptr && need_pad <= W.pcap && need_pad <= (int64_t)INT32_MAX - 128;
 }
 
 // The hub core pass (needs only the CSR and cleared counters, so it may run on
