@@ -245,8 +245,10 @@ def device_sync() -> None:
 
 def fetch(dst, src: torch.Tensor, nbytes: int) -> None:
     """Read nbytes of src into the ctypes object dst; waits for the current
-    stream of src's device."""
-    check(load().tchll_fetch(C.byref(dst), src.data_ptr(), nbytes, stream_handle(src.device)), "fetch")
+    stream of src's device, which is made current meanwhile: the default
+    stream's handle is 0 on every device and names the current device's."""
+    with on_device(src.device):
+        check(load().tchll_fetch(C.byref(dst), src.data_ptr(), nbytes, stream_handle(src.device)), "fetch")
 
 
 class Workspace:
