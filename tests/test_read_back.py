@@ -55,6 +55,15 @@ def test_current_device_is_left_alone(monkeypatch):
     assert cuda.log == [("fetch", 1, 4096, 8, 0)]
 
 
+def test_block_on_the_host(monkeypatch):
+    monkeypatch.setattr(_lib, "load", lambda: pytest.fail("no library call for a block on the host"))
+    r = _lib.CountResult()
+    r.exact, r.n_exact = 12345678901, 77
+    t = torch.frombuffer(bytearray(bytes(r)), dtype=torch.uint8)
+    assert core.exact_from_result(t) == 12345678901
+    assert _lib.read_count_result(t).n_exact == 77
+
+
 def test_device_is_put_back_after_an_error(monkeypatch):
     cuda = FakeCuda(monkeypatch, current=0)
     monkeypatch.setattr(cuda, "tchll_fetch", lambda *a: 999, raising=False)

@@ -282,7 +282,10 @@ def count_result_tensor(device) -> torch.Tensor:
 
 
 def read_count_result(t: torch.Tensor) -> CountResult:
-    """Copy a device count result to the host (synchronises the stream)."""
+    """Copy a device count result to the host (synchronises the stream); a
+    block that is on the host already is read where it is."""
+    if t.device.type != "cuda":
+        return CountResult.from_buffer_copy(t.contiguous().numpy().tobytes())
     res = CountResult()
     fetch(res, t, RESULT_BYTES)
     return res
