@@ -71,3 +71,11 @@ def test_device_is_put_back_after_an_error(monkeypatch):
     with pytest.raises(_lib.TchllError):
         _lib.read_count_result(_block(1))
     assert cuda.current == 0
+
+
+@pytest.mark.parametrize("device,index", [(None, 0), (1, 1), (torch.device("cuda"), 0), (torch.device("cuda", 1), 1),
+                                          ("cuda:1", 1), ("cuda", 0)])
+def test_stream_of_a_device_however_named(monkeypatch, device, index):
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(_lib, "_raw_stream", lambda idx: 1000 + idx)
+    assert _lib.stream_handle(device) == 1000 + index

@@ -214,7 +214,9 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 def stream_handle(device=None) -> int:
     if _raw_stream is None:
         return torch.cuda.current_stream(device).cuda_stream
-    idx = device.index if isinstance(device, torch.device) else None
+    idx = device
+    if device is not None and not isinstance(device, int):
+        idx = torch.device(device).index
     return _raw_stream(torch.cuda.current_device() if idx is None else idx)
 
 
