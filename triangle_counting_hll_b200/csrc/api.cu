@@ -3,6 +3,7 @@
 #include <stdarg.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -44,34 +45,89 @@ TCHLL_EXPORT int tchll_version(void) { return 10000; }
 
 TCHLL_EXPORT uint64_t tchll_launch_count(void) { return tchll::g_launches.load(std::memory_order_relaxed); }
 
-// Small device-to-host reads.  A copy into pageable memory goes through the
-// driver's staging and costs several times a copy into pinned memory, so each
-// host thread keeps one pinned page (made on its first read, freed when the
-// thread ends); the wait for the stream is the read's own.
 namespace tchll {
+typedef int (*CtxGetCurrentFn)(void** ctx);
+typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
+
+bool current_ctx_id(unsigned long long* id) {
+    static CtxGetCurrentFn get_cur = nullptr;
+    static CtxGetIdFn get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_cur = (CtxGetCurrentFn)f;
+        f = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = (CtxGetIdFn)f;
+    });
+    if (get_cur == nullptr || get_id == nullptr) return false;
+    void* ctx = nullptr;
+    if (get_cur(&ctx) != 0 || ctx == nullptr) return false;
+    return get_id(ctx, id) == 0;
+}
+
+// Small device-to-host reads.  A copy into pageable memory goes through the
+// driver's staging and costs several times a copy into pinned memory, so a
+// read takes a pinned page, and gives it back for later reads; the wait for
+// the stream is the read's own.  A page belongs to the context that it was
+// made in and is gone with it (cudaDeviceReset), so it is only ever used, or
+// freed, while that context is current; at most kStagePages are kept.
 namespace {
 constexpr size_t kStageBytes = 4096;
-struct PinnedStage {
-    void* p = nullptr;
-    void* get() {
-        if (p == nullptr && cudaMallocHost(&p, kStageBytes) != cudaSuccess) {
-            cudaGetLastError();  // no pinned memory: the caller copies directly
-            p = nullptr;
-        }
-        return p;
-    }
-    ~PinnedStage() {
-        if (p) cudaFreeHost(p);
-    }
+constexpr int kStagePages = 64;
+struct StagePage {
+    unsigned long long ctx_id;
+    void* p;
 };
-thread_local PinnedStage g_stage;
+std::mutex g_stage_mu;
+StagePage g_stage[kStagePages];
+int g_stage_n = 0;
+
+// A page of the current context, or p = null: the caller copies directly.
+StagePage take_stage() {
+    StagePage s{0, nullptr};
+    if (!current_ctx_id(&s.ctx_id)) return s;
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mu);
+        for (int i = 0; i < g_stage_n; ++i)
+            if (g_stage[i].ctx_id == s.ctx_id) {
+                s.p = g_stage[i].p;
+                g_stage[i] = g_stage[--g_stage_n];
+                return s;
+            }
+    }
+    if (cudaMallocHost(&s.p, kStageBytes) != cudaSuccess) {
+        cudaGetLastError();  // no pinned memory
+        s.p = nullptr;
+    }
+    return s;
+}
+
+void give_stage(StagePage s) {
+    if (s.p == nullptr) return;
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mu);
+        if (g_stage_n < kStagePages) {
+            g_stage[g_stage_n++] = s;
+            return;
+        }
+    }
+    cudaFreeHost(s.p);
+}
 }  // namespace
 
 int fetch_small(void* dst, const void* src, size_t n, cudaStream_t st) {
-    void* stage = n <= kStageBytes ? g_stage.get() : nullptr;
-    TCHLL_CUDA(cudaMemcpyAsync(stage ? stage : dst, src, n, cudaMemcpyDeviceToHost, st));
-    TCHLL_CUDA(cudaStreamSynchronize(st));
-    if (stage) memcpy(dst, stage, n);
+    StagePage s{0, nullptr};
+    if (n <= kStageBytes) s = take_stage();
+    cudaError_t e = cudaMemcpyAsync(s.p ? s.p : dst, src, n, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && s.p) memcpy(dst, s.p, n);
+    if (e != cudaSuccess) return cuda_status(e, "fetch");  // the page may still be written to: it is not used again
+    give_stage(s);
     return TCHLL_OK;
 }
 }  // namespace tchll

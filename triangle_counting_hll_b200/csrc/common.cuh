@@ -44,6 +44,11 @@ void count_launch(int n = 1);
 
 int sm_count();
 
+// Id of the calling thread's current context (cuCtxGetId: unique in the
+// process, never used again), reached through the runtime's driver entry-point
+// query, so the library needs no driver link; false when unavailable.
+bool current_ctx_id(unsigned long long* id);
+
 // Copies n bytes of device memory to the host and waits for the stream
 // (through a pinned page when they fit one).
 int fetch_small(void* dst, const void* src, size_t n, cudaStream_t st);

@@ -3770,31 +3770,6 @@ struct NoallocEntry {
 static NoallocEntry g_noalloc_cache[64];
 static int g_noalloc_used = 0;
 
-typedef int (*CtxGetCurrentFn)(void** ctx);
-typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
-
-// Id of the calling thread's current context; false when unavailable.
-static bool current_ctx_id(unsigned long long* id) {
-    static CtxGetCurrentFn get_cur = nullptr;
-    static CtxGetIdFn get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_cur = (CtxGetCurrentFn)f;
-        f = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = (CtxGetIdFn)f;
-    });
-    if (get_cur == nullptr || get_id == nullptr) return false;
-    void* ctx = nullptr;
-    if (get_cur(&ctx) != 0 || ctx == nullptr) return false;
-    return get_id(ctx, id) == 0;
-}
-
 static int noalloc_scratch_ptr(void** out) {
     int dev = -1;
     TCHLL_CUDA(cudaGetDevice(&dev));  // also makes the runtime's context current
