@@ -156,8 +156,8 @@ int tchll_hybrid_count_compact(const int32_t* row_ptr, int64_t n_nodes, const in
  * counts, which count edges as given with tables); blocks_per_sm: 0 = occupancy maximum; warps_per_cta: 1-8;
  * pairs: 1 = probe the shorter list into a table of the longer one (edges
  * with a long list regrouped by a device counting sort) when the graph has
- * more than 2^19 edges and 3 per vertex, or 128 per vertex, 2 = whatever its
- * size, 0 = edges as given; sparse: 1 = hash
+ * more than 2^17 neighbour entries or 2^19 edges are asked for, 2 = whatever
+ * its size, 0 = edges as given; sparse: 1 = hash
  * tables at load <= 1/4 where they fit (else <= 1/2).  out8 receives chunk,
  * slots_log2, tiny, blocks_per_sm, warps_per_cta, pairs, sparse and a
  * reserved 0.  Results are identical for every setting. */

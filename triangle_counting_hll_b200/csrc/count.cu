@@ -1112,7 +1112,7 @@ __global__ void core_mark_kernel(const int32_t* __restrict__ row_ptr, int64_t n_
                                  const int32_t* __restrict__ col, int hub, int count_all,
                                  const unsigned long long* __restrict__ n_segs, uint32_t* bits, int32_t* cnt,
                                  tchll_count_result* result) {
-    if (n_segs && *n_segs == 0) return;  // grid-uniform: batched, and no hub pairs
+    if (n_segs && *n_segs == 0) return;  // grid-uniform: after the first pass, which found no hub pairs
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1184,8 +1184,10 @@ __device__ __forceinline__ int pop_bucket(const uint32_t* __restrict__ bits, con
 
 __global__ void __launch_bounds__(256) core_bucket_kernel(const uint32_t* __restrict__ bits,
                                                           const int32_t* __restrict__ cnt, int64_t n_nodes,
+                                                          const unsigned long long* __restrict__ n_segs,
                                                           int32_t* hist) {
     __shared__ int h[256];
+    if (n_segs && *n_segs == 0) return;  // grid-uniform, as core_mark_kernel
     h[threadIdx.x] = 0;
     __syncthreads();
     for (int64_t w = blockIdx.x * 256ll + threadIdx.x; w < n_nodes; w += gridDim.x * 256ll) {
@@ -1202,8 +1204,10 @@ __global__ void __launch_bounds__(256) core_bucket_kernel(const uint32_t* __rest
 __global__ void __launch_bounds__(256) core_index_kernel(const uint32_t* __restrict__ bits, int32_t* cnt_cidx,
                                                          int64_t n_nodes,
                                                          const int32_t* __restrict__ hist, int32_t* cursor,
+                                                         const unsigned long long* __restrict__ n_segs,
                                                          int32_t* n_core) {
     __shared__ int h[256], part[8];
+    if (n_segs && *n_segs == 0) return;
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t per = (n_nodes + gridDim.x - 1) / gridDim.x;
     const int64_t lo = blockIdx.x * per, hi = min(n_nodes, lo + per);
@@ -1437,7 +1441,7 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
                                                          int32_t* pool_used, unsigned long long* row_ctr,
                                                          const unsigned long long* __restrict__ n_segs,
                                                          const int32_t* __restrict__ live,
-                                                         const int32_t* __restrict__ n_live,
+                                                         const int32_t* __restrict__ n_live, int checked,
                                                          tchll_count_result* result) {
     __shared__ int32_t s_stage[8][kStage];
     __shared__ __align__(16) uint32_t s_bits[8][4 * kBmMax];
@@ -1446,8 +1450,8 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
     const int sub = lane & 7, grp = lane >> 3;
     uint32_t status = 0;
     // grid-uniform; else no hub pair will read a list
-    const bool lists = live ? *n_segs > 0 : n_core[0] > 0;
-    if (!lists) validate_rows(row_ptr, n_nodes, nnz, col, status);
+    const bool lists = n_segs ? *n_segs > 0 : n_core[0] > 0;
+    if (!lists && !checked) validate_rows(row_ptr, n_nodes, nnz, col, status);
     // batched: only the listed blocks of 64 rows, those near a graph with hub
     // pairs, are ever read as lists; the other rows are only checked
     if (lists && live) validate_rows(row_ptr, n_nodes, nnz, col, status);
@@ -1524,14 +1528,14 @@ __global__ void __launch_bounds__(256, 6) core_lists_kernel(const int32_t* __res
 __global__ void core_pad_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int64_t nnz,
                                 const int32_t* __restrict__ col, const int32_t* __restrict__ cidx,
                                 const int32_t* __restrict__ n_core, int packed, int32_t* __restrict__ pcol,
-                                tchll_count_result* result) {
+                                int checked, tchll_count_result* result) {
     const int32_t C = n_core[0];
     if (packed && C <= kCore16Max) return;  // grid-uniform: core_lists_kernel writes the lists
     const int sub = threadIdx.x & 7;
     const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
     const int64_t ng = ((int64_t)gridDim.x * blockDim.x) >> 3;
     uint32_t status = 0;
-    if (C == 0) validate_rows(row_ptr, n_nodes, nnz, col, status);  // no hub pair will read a list
+    if (C == 0 && !checked) validate_rows(row_ptr, n_nodes, nnz, col, status);  // no hub pair will read a list
     for (int64_t y = C ? g : n_nodes; y < n_nodes; y += ng) {
         const int32_t rs = __ldg(row_ptr + y), re = __ldg(row_ptr + y + 1);
         if (rs < 0 || re < rs || (int64_t)re > nnz) {
@@ -2580,22 +2584,33 @@ struct Tuning {
     int hll_row_cache_p = 0;   // HLL pass: keep u's register row in registers for p <= this (0: never)
     int hll_lanes = 0;      // HLL pass: lanes per edge (0: chosen by p)
 };
-// Up to this many edges the regrouping's dozen launches cost more than it
-// saves, and the edges are counted as given, with one launch (R-MAT edge
-// factor 16 to 32, device time as given / regrouped: 85 K edges 33 / 89 us,
-// 388 K 101 / 123 us, 441 K 119 / 123 us).  Dense graphs are
-// regrouped all the same: lists beyond a warp's table (512 members) are
-// searched one by one (cliques of 600 and 1000 vertices: 260 / 139, 1734 / 208
-// us).
+// Routes are chosen by the graph (nnz members in n_nodes lists), not by the
+// edges asked for, which may be a part of it: each rank of a sharded count
+// brings the whole graph.  Up to kDirectNnz members, and kDirectEdges edges,
+// the regrouping's dozen launches cost more than it saves, and the edges are
+// counted as given, with one launch.  The line is where every list still fits a
+// warp's table of 512 members: a list oriented by degree has at most
+// sqrt(2 nnz).  Longer lists are searched one by one there (a 1,000-clique
+// with 3,000 pendant vertices, 502 K edges: 1,768 us as given, 220 regrouped);
+// up to it, as given / regrouped: R-MAT 12 (48 K edges) 59 / 103 us, a
+// 510-clique with 1,000 pendant vertices (131 K) 101 / 148 us; behind it, R-MAT 14
+// (200 K) 107 / 114, R-MAT 15 (388 K) 146 / 134.
+constexpr int64_t kDirectNnz = 1 << 17;
 constexpr int64_t kDirectEdges = 1 << 19;
-constexpr int64_t kDirectDegree = 128;  // mean forward degree
 // Of those, graphs of at most this mean forward degree are counted by
 // binary search, the others with a hash table per u: ER 100 K edges 12 / 16 us,
 // R-MAT 14 (edge factor 32, mean 28) 224 / 103 us.
 constexpr int64_t kSparseDegree = 8;
-// Up to this mean forward degree graphs of any size are counted as given:
-// road networks have no long lists at all (a million-vertex lattice, mean
-// 2.2: 120 us of device time regrouped, 45 as given).
+// Up to this mean forward degree a graph may well have no long list at all
+// (road networks), though it may have a dense core too.  The hub core pass then
+// follows the first pass on the caller's stream, where its kernels and the
+// hub kernels return at once when there is no hub pair, instead of scanning
+// the vertices beside it, and the first pass deals its chunks to the warps in
+// turn, which lists as short as these allow, instead of having them claimed.
+// A million-vertex lattice (mean 2.2) takes 145 us without both, 131 so.  (In
+// one launch, as given, it takes 85, but a 1,200-clique inside a lattice of 2 M
+// vertices then 3.6 ms against 0.45, a 4,000-clique with 10 M pendant vertices
+// 95 against 2.8.)
 constexpr int64_t kRoadDegree = 3;
 constexpr int HUB_MIN = 64;       // smallest hub threshold (bounds the segment count)
 constexpr int HUB_SEG_MIN = 256;  // smallest segment
@@ -2707,7 +2722,7 @@ static int launch_count(const CountParams& P, const Tuning& T, bool details, cud
 static int given_chunk(int64_t n_edges, int chunk) {
     int c = 8;
     while (c < 32 && n_edges >= 6144 * (int64_t)(2 * c)) c *= 2;
-    return n_edges <= kDirectEdges && c < chunk ? c : chunk;
+    return c < chunk ? c : chunk;
 }
 
 struct CountWs {
@@ -3017,17 +3032,20 @@ static bool hub_pad_usable(const CountParams& P, const CountWs& W) {
 // The hub core pass (needs only the CSR and cleared counters, so it may run on
 // a second stream from the start, beside the first pass and the scatter): core
 // members, their numbering, then the lists, packed when the core allows it,
-// else 32-bit (each list kernel checks the core size on the device).
-static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, int hub, const PhaseScope& ps,
-                            cudaStream_t st) {
+// else 32-bit (each list kernel checks the core size on the device).  Where
+// hub pairs are rare (batches, road networks) it follows the first pass and
+// the scatter instead (`after`), and its kernels return at once without any.
+static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, int hub, bool after,
+                            const PhaseScope& ps, cudaStream_t st) {
     if (!hub_pad_usable(P, W)) return TCHLL_OK;
+    const unsigned long long* n_segs = after ? W.ctr + 2 : nullptr;
     if (ps.active()) {
         cudaEventRecord(g_phase.hub_ev[0], st);
         g_phase.core_used = true;
     }
     core_mark_kernel<<<grid_rows(P.n_nodes, 256) < 8 * sm_count() ? grid_rows(P.n_nodes, 256) : 8 * sm_count(), 256, 0,
                        st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, hub, P.nnz <= kMarkAllEdges,
-                             P.graph_vbase ? W.ctr + 2 : nullptr, W.cbits, W.cflag, P.result);
+                             n_segs, W.cbits, W.cflag, P.result);
     TCHLL_CHECK_LAUNCH("core_mark_kernel");
     if (P.graph_vbase) {
         core_index_batch_kernel<<<(int)P.n_graphs, 1024, 0, st>>>(W.cbits, W.cflag, P.n_nodes, P.graph_vbase,
@@ -3037,9 +3055,10 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
     } else {
         int64_t gv = (P.n_nodes + 1023) / 1024;
         gv = gv < 1 ? 1 : (gv > 4 * (int64_t)sm_count() ? 4 * (int64_t)sm_count() : gv);
-        core_bucket_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4);
+        core_bucket_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, n_segs, W.ncore + 4);
         TCHLL_CHECK_LAUNCH("core_bucket_kernel");
-        core_index_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4, W.ncore + 4 + 256, W.ncore);
+        core_index_kernel<<<(int)gv, 256, 0, st>>>(W.cbits, W.cflag, P.n_nodes, W.ncore + 4, W.ncore + 4 + 256, n_segs,
+                                                   W.ncore);
         TCHLL_CHECK_LAUNCH("core_index_kernel");
     }
     int64_t gl = (P.n_nodes + 63) / 64;
@@ -3047,11 +3066,12 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
     core_lists_kernel<<<(int)gl, 256, 0, st>>>(
         P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag, W.ncore, T.packed, reinterpret_cast<uint16_t*>(W.pcol), W.pl,
         W.pool, (int32_t)(W.pool_cap < INT32_MAX / 2 ? W.pool_cap : INT32_MAX / 2), W.ncore + 1,
-        reinterpret_cast<unsigned long long*>(W.ncore + 2), W.ctr + 2, P.live_list, W.ncore + kCoreWords - 1, P.result);
+        reinterpret_cast<unsigned long long*>(W.ncore + 2), n_segs, P.live_list, W.ncore + kCoreWords - 1, P.check_ids,
+        P.result);
     TCHLL_CHECK_LAUNCH("core_lists_kernel");
     if (!T.packed || P.n_nodes > kCore16Max) {  // else the packed lists always apply
         core_pad_kernel<<<grid_rows(P.n_nodes, 32), 256, 0, st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, W.cflag,
-                                                                  W.ncore, T.packed, W.pcol, P.result);
+                                                                  W.ncore, T.packed, W.pcol, P.check_ids, P.result);
         TCHLL_CHECK_LAUNCH("core_pad_kernel");
     }
     if (ps.active()) cudaEventRecord(g_phase.hub_ev[1], st);
@@ -3267,10 +3287,10 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
         set_error("workspace too small: need %zu bytes, have %zu", need, ws_bytes);
         return TCHLL_EWORKSPACE;
     }
-    const bool direct = T.pairs != 2 && (P.n_edges <= kDirectEdges ? P.n_edges <= kDirectDegree * P.n_nodes
-                                                                   : P.n_edges <= kRoadDegree * P.n_nodes);
+    const bool direct = T.pairs != 2 && P.nnz <= kDirectNnz && P.n_edges <= kDirectEdges;
     const bool direct_pass = direct && T.pairs && !details;
-    const bool sparse = P.n_edges <= kSparseDegree * P.n_nodes;
+    const bool sparse = P.nnz <= kSparseDegree * P.n_nodes;
+    const bool road = P.nnz <= kRoadDegree * P.n_nodes;
     const bool pairs = T.pairs && !details && !direct;
     const bool prepared = pairs && P.n_edges > 0 &&
                           (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));  // by pass_prepare
@@ -3289,10 +3309,11 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
     P.hll_v = nullptr;
     P.hll_n = nullptr;
     if (P.n_edges == 0) return TCHLL_OK;
-    // small graphs refuse what the hub core's passes refuse in large ones
-    P.check_ids = direct_pass && T.hub > 0 && (uintptr_t)P.col_idx % 16 == 0 && hub_pad_usable(P, W) &&
+    // small graphs, and road networks without a long list, refuse what the hub
+    // core's passes refuse in others
+    P.check_ids = (direct_pass ? (uintptr_t)P.col_idx % 16 == 0 : pairs && road) && T.hub > 0 && hub_pad_usable(P, W) &&
                   (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));
-    if (direct_pass) P.chunk = P.n_edges <= kDirectEdges ? given_chunk(P.n_edges, T.chunk) : pass_chunk(P.n_edges, T.chunk);
+    if (T.pairs && !details && !prepared && P.n_edges <= kDirectEdges) P.chunk = given_chunk(P.n_edges, T.chunk);
     if (col_ready && !(mode == MODE_EXACT && pairs)) {
         TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
         col_ready = nullptr;
@@ -3322,20 +3343,22 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
                 if (rc) return rc;
                 SideFork fork;
-                const bool side = hub > 0 && T.overlap && hub_pad_usable(P, W);
+                const bool side = hub > 0 && T.overlap && hub_pad_usable(P, W) && !road;
                 if (side) {
                     rc = fork.begin(st);
                     if (rc == TCHLL_OK && col_ready) {
                         const cudaError_t e = cudaStreamWaitEvent(fork.stream(), col_ready, 0);
                         if (e != cudaSuccess) rc = cuda_status(e, "cudaStreamWaitEvent(col_ready)");
                     }
-                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, hub, ps, fork.stream());
+                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, hub, false, ps, fork.stream());
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
                 const bool split = col_ready && hub > 0;
                 if (col_ready && !split) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
-                rc = pair_pass<false>(P, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                CountParams H = P;
+                if (split) H.check_ids = 0;  // col_idx is not there yet
+                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr, st);
                 if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc) return rc;
                 if (hub > 0) rc = pairs_scatter(P, W, st);
@@ -3347,7 +3370,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 }
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, ps, st);
+                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, road, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                 }
                 phase_mark(ps, 2, st);
@@ -3389,19 +3412,19 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 // that has listed the HLL edges, their pass
                 SideFork fork;
                 cudaStream_t hst = st;
-                const bool core_side = hub > 0 && T.overlap && hub_pad_usable(P, W);
+                const bool core_side = hub > 0 && T.overlap && hub_pad_usable(P, W) && !road;
                 if (T.overlap) {
                     rc = fork.begin(st);
                     if (rc) return rc;
                     hst = fork.stream();
                     if (core_side) {
-                        rc = launch_core_pass(P, W, T, hub, ps, hst);
+                        rc = launch_core_pass(P, W, T, hub, false, ps, hst);
                         if (rc == TCHLL_OK) rc = fork.mark();
                         if (rc) return rc;
                     }
                 }
                 rc = launch_zmask(P, HW, hst);
-                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, W.ctr, st);
+                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr, st);
                 if (rc == TCHLL_OK && T.overlap) rc = fork.side_waits_caller();
                 if (rc) return rc;
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[0], hst);
@@ -3413,7 +3436,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, ps, st);
+                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, road, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                     if (rc) return rc;
                 }
@@ -4054,7 +4077,7 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     }
     phase_mark(ps, 1, st);
     if (hubs) {
-        rc = launch_core_pass(P, B.cw, T, hub, ps, st);
+        rc = launch_core_pass(P, B.cw, T, hub, true, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
     }
