@@ -171,7 +171,8 @@ int tchll_get_count_tuning(int32_t* out8 /* host */);
  * hash table of N+(x) (hash: load <= 1/16 where 2^table_log2 slots of shared
  * memory allow), at most seg_pairs of x's pairs per work unit, unroll 16-byte
  * probe loads in flight per lane; all other pairs are counted by binary search
- * of the longer list in the first pass over the edges.  threshold 128, the
+ * of the longer list in the first pass over the edges or, in graphs of evenly
+ * long lists, with a warp's hash table of it.  threshold 128, the
  * default, is taken as 64 where that is faster (up to 28 M edges; batches: a
  * mean forward degree of at least 12).  threshold 0 turns it off; otherwise
  * threshold >= 64, seg_pairs in [256, 2^20], table_log2 in [10, 15], unroll 2

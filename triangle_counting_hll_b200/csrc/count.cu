@@ -16,10 +16,11 @@
 //     members of the shorter list are looked up in the longer one, which drops
 //     the look-ups from sum d+(v) to sum min(d+u, d+v) (43.4 G list elements ->
 //     11.8 G on R-MAT scale 22).
-//   * A first pass over the edges (pair_pass_kernel) counts every pair of
-//     short lists on the spot by binary search and counts the others, the hub
-//     pairs (d+(x) > hub threshold; 98% of the look-ups on R-MAT scale 22),
-//     per table side; a counting sort then groups those by x.
+//   * A first pass over the edges (pair_pass_kernel) counts pairs of short
+//     lists on the spot by binary search and counts the others per table
+//     side; a counting sort then groups those by x.  They are the hub pairs
+//     (d+(x) > hub threshold; 98% of the look-ups on R-MAT scale 22) and, in
+//     graphs of evenly long lists, the table pairs (is_table_pair).
 //   * Hub pairs are counted by a CTA per group of x's pairs, all its warps
 //     sharing one bitmap of N+(x) in shared memory (hub_bitmap16_kernel), in
 //     the coordinates of the core, the vertices of the hub lists.
@@ -55,6 +56,14 @@ enum : uint32_t {
     ST_BAD_ROW = 2u,   // row_ptr extent outside [0, nnz] or decreasing
     ST_BAD_SLOT = 4u,  // sketch slot outside [0, n_rows)
     ST_BAD_KEY = 8u,   // neighbour id (col_idx value) outside [0, n_nodes)
+};
+
+// Pairs of one table side x, next to each other in the list of probe sides.
+struct PairSeg {
+    int32_t start;  // the first pair (the list holds < 2^31 entries)
+    int32_t x;
+    int32_t len;
+    int32_t graph;  // batched counts: the graph of x (its result block); else 0
 };
 
 struct CountParams {
@@ -96,9 +105,14 @@ struct CountParams {
     const int32_t* graph_vbase;  // vertex range of graph g: [vbase[g], vbase[g+1])
     int64_t n_graphs;            // batched calls: graphs in graph_vbase (else 0)
     unsigned long long* graph_bad;  // batched calls: of them, those from the first malformed one on
-    int32_t* graph_hub;          // batched calls: 1 for a graph with hub pairs (first pass)
+    int32_t* graph_hub;          // batched calls: what the first pass left for later, GRAPH_*
     int32_t* live_flag;          // batched calls: 1 for 64 rows that touch such a graph
     int32_t* live_list;          // and those blocks of 64 rows, listed
+    // Table pairs (count_kernel with SEGS): their segments, the first one right
+    // before segs_end, the second before that; edge_v holds the probe sides
+    const PairSeg* segs_end;
+    const unsigned long long* n_segs;
+    const unsigned long long* list_weights;  // see is_table_pair (null: no table pairs)
     // Hybrid with pairs: the routing pass appends HLL edges here
     int32_t* hll_u;
     int32_t* hll_v;
@@ -289,6 +303,23 @@ __device__ __forceinline__ PairSides sides_of(int32_t u, int32_t v, int32_t us, 
 }
 // Hub pairs: a long table side and something to probe it with.
 __device__ __forceinline__ bool is_hub_pair(const PairSides& S, int hub) { return hub > 0 && S.xl > hub && S.yl > 0; }
+// Table pairs, of the others: a table side and a probe side of some length.
+// They are grouped by table side like hub pairs and counted with a warp's
+// hash table of it (count_kernel with SEGS), where a look-up is one shared
+// load instead of a search of 4 and more steps.  That takes several pairs to a
+// table side, which skewed graphs do not have (R-MAT 20: 272 us in tables, 25 in
+// searches), so it is done where lists of such a length hold at least a
+// quarter of the graph's look-ups, measured by squared length (list_weights,
+// summed by prepare_kernel: {their lists, all}): 0 to 0.1 on R-MAT 16 and up,
+// above 0.3 where lists are evenly long.  Whole calls, us, all pairs in
+// tables / all in searches / so: a million vertices joined to 20 near ones
+// 1,493 / 1,009 / 1,024, to 30 2,088 / 2,164 / 1,886, to 40 2,755 / 3,673 / 2,651, to
+// 60 4,475 / 8,420 / 4,407; Erdos-Renyi, 40 M edges 3,808 / 4,768 / 3,480.
+constexpr int kTableList = 32;
+constexpr int kTableProbes = 16;
+__device__ __forceinline__ bool is_table_pair(const PairSides& S, int list) {
+    return list > 0 && S.xl > list && S.yl > kTableProbes;
+}
 
 // Batched calls: the graph of vertex v, the last g with vbase[g] <= v among
 // the graphs before the first malformed one (the only ones with edges).
@@ -358,7 +389,7 @@ __global__ void pair_scatter_kernel(const CountParams P, int32_t* cursor, const 
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    if (P.chunk_start) {  // batched: the chunks of the graphs with hub pairs
+    if (P.chunk_start) {  // batched: the chunks of the graphs with grouped pairs
         const int64_t n = *P.n_chunks_dev;
         for (int64_t c = warp; c < n; c += warps) {
             if (!P.graph_hub[__ldg(P.chunk_graph + c)]) continue;
@@ -445,17 +476,26 @@ struct Prepare {
     const uint8_t* has;
     int64_t n_rows;
     int2* rows;
+    int hub;
+    unsigned long long* list_weights;  // zeroed before
     int32_t* zero_n[2];   // n_nodes + 1 words each (or null)
     uint32_t* zero[3];    // words[i] words
     int64_t words[3];
 };
 __global__ void prepare_kernel(const Prepare Q) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    unsigned long long weight = 0, table_weight = 0;
     for (int64_t v = t0; v <= Q.n_nodes; v += step) {
         if (v < Q.n_nodes) {
             const int32_t a = __ldg(Q.row_ptr + v), b = __ldg(Q.row_ptr + v + 1);
             int2 r = make_int2(a, b);
-            if (a < 0 || b < a || (int64_t)b > Q.nnz) {
+            const bool bad = a < 0 || b < a || (int64_t)b > Q.nnz;
+            if (!bad) {
+                const unsigned long long w = (unsigned long long)(b - a) * (unsigned long long)(b - a);
+                weight += w;
+                if (b - a > kTableList && (Q.hub == 0 || b - a <= Q.hub)) table_weight += w;
+            }
+            if (bad) {
                 r = make_int2(kRowBad, 0);
             } else if (Q.degrees) {
                 const int64_t s = Q.slot ? __ldg(Q.slot + v) : (__ldg(Q.has + v) == 1 ? v : -1);
@@ -472,6 +512,20 @@ __global__ void prepare_kernel(const Prepare Q) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
         for (int64_t w = t0; w < Q.words[i]; w += step) Q.zero[i][w] = 0;
+    // one atomic each per CTA
+    __shared__ unsigned long long sums[2][8];
+    weight = warp_sum_u64(weight);
+    table_weight = warp_sum_u64(table_weight);
+    if ((threadIdx.x & 31) == 0) {
+        sums[0][threadIdx.x >> 5] = table_weight;
+        sums[1][threadIdx.x >> 5] = weight;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long t = 0;
+        for (int i = 0; i < 8; ++i) t += sums[threadIdx.x][i];
+        if (t) atomicAdd(Q.list_weights + threadIdx.x, t);
+    }
 }
 
 // The first pass over the edges.  Pairs with a long table side (hub pairs)
@@ -491,6 +545,7 @@ __global__ void prepare_kernel(const Prepare Q) {
 // in turn (null), or, batched, from the chunk list (a chunk is one graph's,
 // and so are its totals).
 enum : int { PASS_HIST = 1, PASS_SHORT = 2 };
+enum : int { GRAPH_HUB = 1, GRAPH_GROUPED = 2 };  // hub pairs; any pairs to group
 constexpr int kHugeList = 1 << 25;  // 32 shorter lists of this length still add up below 2^31
 // The n HLL edges of a warp's buffer go to the list.
 constexpr int kHllBuf = 160;
@@ -536,6 +591,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
     uint32_t status = 0;
     if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col, status);
     const int32_t full_quads = (int32_t)(P.nnz >> 2);
+    const int table = P.list_weights && __ldg(P.list_weights) >= __ldg(P.list_weights + 1) / 4 ? kTableList : 0;
     const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     while (true) {
@@ -564,7 +620,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
                 e1 = (uint32_t)min((int64_t)e0 + P.chunk, P.n_edges);
             }
         }
-        bool any_hub = false;
+        int left = 0;  // GRAPH_*
         // the chunk's codes: no two chunks of a batch share one
         const int64_t code0 = (e0 >> 5) + (g >= 0 ? (int64_t)chunk : 0);
         for (uint32_t eb = e0; eb < e1; eb += 32) {
@@ -599,19 +655,20 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             }
             const PairSides S = sides_of(u, v, us, ue, vs, ve);
             const bool to_hub = ok && is_hub_pair(S, hub);
-            if (hub > 0 && (what & PASS_HIST)) {
-                const unsigned m = __ballot_sync(FULL, to_hub), mu = __ballot_sync(FULL, S.x == u);
+            const bool grouped = to_hub || (ok && is_table_pair(S, table));
+            if (what & PASS_HIST) {
+                const unsigned m = __ballot_sync(FULL, grouped), mu = __ballot_sync(FULL, S.x == u);
                 if (lane == 0) P.codes[code0 + ((eb - e0) >> 5)] = make_uint2(m, mu);
                 if (m) {
                     // a run of lanes with the same table side adds with one atomic
                     int head, run;
-                    lane_runs(to_hub ? S.x : -1 - lane, lane, head, run);
-                    if (to_hub && lane == head) atomicAdd(cnth + S.x, run);
-                    any_hub = true;
+                    lane_runs(grouped ? S.x : -1 - lane, lane, head, run);
+                    if (grouped && lane == head) atomicAdd(cnth + S.x, run);
+                    left |= GRAPH_GROUPED | (g >= 0 && __any_sync(FULL, to_hub) ? GRAPH_HUB : 0);
                 }
             }
             if (!(what & PASS_SHORT)) continue;
-            const bool mine = ok && !to_hub;
+            const bool mine = ok && !grouped;
             n_exact += __popc(__ballot_sync(FULL, mine));
             int np = mine ? S.yl : 0;
             // lists whose lengths could overflow the stream's positions: one
@@ -699,7 +756,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             acc += __reduce_add_sync(FULL, hits);
         }
         if (g >= 0) {  // batched: this chunk's totals belong to its graph
-            if (any_hub && lane == 0 && __ldcg(P.graph_hub + g) == 0) P.graph_hub[g] = 1;
+            if (left && lane == 0 && (__ldcg(P.graph_hub + g) & left) != left) atomicOr(P.graph_hub + g, left);
             pass_publish(P.result + g, acc, n_exact, n_fallback, status, lane);
             acc = 0;
             n_exact = n_fallback = 0;
@@ -710,7 +767,14 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
     if (!P.chunk_start || status) pass_publish(P.result, acc, n_exact, n_fallback, status, lane);
 }
 
-template <int MODE, bool VEC, bool DETAILS>
+// SEGS: the pairs of P's segments instead of edges, claimed kSegPart at a time:
+// the first part of every segment, then the second, and so on, so that the
+// last claims are short (a whole segment takes a warp tens of microseconds:
+// R-MAT 17 388 us by parts, 596 by eight segments at a time).  Where there are
+// many segments they are claimed whole, which builds each table once.
+constexpr int kTableSeg = 256;  // pairs of a segment at most
+constexpr int kSegPart = 64;
+template <int MODE, bool VEC, bool DETAILS, bool SEGS = false>
 __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     extern __shared__ __align__(16) int32_t smem[];
     const int lane = threadIdx.x & 31;
@@ -730,14 +794,36 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     int cur_lg = 5;  // log2 slots of the current table
     const int m = 1 << P.p;
 
+    if (SEGS && *P.n_segs == 0) return;  // grid-uniform
     if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col_idx, status);
     const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + wid;
+    int32_t seg_x = 0, seg_graph = -1;
     while (true) {
         unsigned long long e0 = 0;
         int64_t e1;
         int32_t gcur = -1;
-        if (P.chunk_start) {
+        if (SEGS) {
+            const unsigned long long n = *P.n_segs;
+            const int part_len = n > 16384 ? kTableSeg : kSegPart;
+            unsigned long long part = 0;
+            if (lane == 0) part = atomicAdd(P.work, 1ull);
+            part = __shfl_sync(FULL, part, 0);
+            if (part >= n * (unsigned)(kTableSeg / part_len)) break;
+            const int4 s = __ldg(reinterpret_cast<const int4*>(P.segs_end) - 1 - (int64_t)(part % n));
+            const int32_t first = (int32_t)(part / n) * part_len;
+            if (first >= s.z) continue;
+            e0 = (unsigned long long)(s.x + first);
+            seg_x = s.y;
+            e1 = (int64_t)e0 + min(part_len, s.z - first);
+            if (P.graph_vbase && s.w != seg_graph) {  // batched: the totals so far belong to another graph
+                if (seg_graph >= 0)
+                    publish(P.result + seg_graph, acc, hacc, n_approx, n_exact, n_fallback, n_clamped, status, lane);
+                acc = 0;
+                n_exact = 0;
+                seg_graph = s.w;
+            }
+        } else if (P.chunk_start) {
             unsigned long long ci = 0;
             if (lane == 0) ci = atomicAdd(P.work, 1ull);
             ci = __shfl_sync(FULL, ci, 0);
@@ -759,7 +845,18 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
         for (int64_t eb = (int64_t)e0; eb < e1; eb += 32) {
             const int64_t e = eb + lane;
             int32_t u = 0, v = 0, us = 0, ue = 0, vs = 0, ve = 0;
-            bool valid = e < e1 && load_edge(P, e, u, v, us, ue, vs, ve, status);
+            bool valid = e < e1;
+            if (SEGS) {
+                if (valid) {  // the first pass has checked both rows
+                    u = seg_x;
+                    v = __ldcs(P.edge_v + e);
+                    const int2 ru = __ldg(P.rows + u), rv = __ldg(P.rows + v);
+                    us = ru.x & 0x7FFFFFFF, ue = ru.y & 0x7FFFFFFF;
+                    vs = rv.x & 0x7FFFFFFF, ve = rv.y & 0x7FFFFFFF;
+                }
+            } else {
+                valid = valid && load_edge(P, e, u, v, us, ue, vs, ve, status);
+            }
             if (valid && gcur >= 0) {
                 // an edge of another graph inside this graph's chunk
                 const int32_t lo_v = __ldg(P.graph_vbase + gcur), hi_v = __ldg(P.graph_vbase + gcur + 1);
@@ -1026,7 +1123,9 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
     }
 
     // ---------------------------------------------------------- publish ----
-    if (!P.chunk_start) publish(P.result, acc, hacc, n_approx, n_exact, n_fallback, n_clamped, status, lane);
+    if (!P.chunk_start)
+        publish(P.result + (SEGS && seg_graph >= 0 ? seg_graph : 0), acc, hacc, n_approx, n_exact, n_fallback, n_clamped,
+                status, lane);
 }
 
 // ------------------------------------------------------------ hub pairs ----
@@ -1037,13 +1136,6 @@ __global__ void __launch_bounds__(256, 4) count_kernel(const CountParams P) {
 // <= 1/8 (up to 2^hub_lg slots) and its warps stream the probe lists of x's
 // pairs through it (a per-warp table of 8 KB would hold N+(x) only at load
 // up to 1/2, where the overflow walks of the one-load table grow).
-struct HubSeg {
-    int32_t start;  // first pair in the hub list (pair lists hold < 2^31 entries)
-    int32_t x;
-    int32_t len;
-    int32_t graph;  // batched counts: the graph of x (its result block); else 0
-};
-
 struct HubParams {
     const int32_t* row_ptr;
     int64_t n_nodes;
@@ -1056,7 +1148,7 @@ struct HubParams {
     const int4* pl;         // packed lists per row (core_lists_kernel)
     const uint4* pool;      // their bitmap units
     int packed;             // packed 16-bit lists when C <= kCore16Max
-    const HubSeg* segs;
+    const PairSeg* segs;
     const unsigned long long* n_segs;
     int64_t max_segs;
     unsigned long long* seg_ctr;
@@ -1250,7 +1342,7 @@ __global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* 
                                                                 int32_t* live_flag, int32_t* live_list,
                                                                 int32_t* n_live, int32_t* n_core) {
     __shared__ int h[256], part[8];
-    if (graph_hub[blockIdx.x] == 0) return;  // no core
+    if ((graph_hub[blockIdx.x] & GRAPH_HUB) == 0) return;  // no core
     const int tid = threadIdx.x, lane = tid & 31;
     const int32_t lo = __ldg(vbase + blockIdx.x), hi = __ldg(vbase + blockIdx.x + 1);
     if (lo < 0 || hi < lo || (int64_t)hi > n_nodes) return;  // flagged by check_vbase_kernel
@@ -1569,7 +1661,7 @@ __global__ void core_pad_kernel(const int32_t* __restrict__ row_ptr, int64_t n_n
 template <int UNR, bool PAD>
 __global__ void __launch_bounds__(256, 5) hub_count_kernel(const HubParams H) {
     extern __shared__ __align__(16) uint32_t tbl[];
-    __shared__ HubSeg s_seg;
+    __shared__ PairSeg s_seg;
     __shared__ int s_round;
     __shared__ int s_fail;
     if (PAD && ((H.packed && *H.n_core <= kCore16Max) || (H.cap_bits > 0 && *H.n_core + 32 <= H.cap_bits)))
@@ -1593,7 +1685,7 @@ __global__ void __launch_bounds__(256, 5) hub_count_kernel(const HubParams H) {
             s_fail = 0;
         }
         __syncthreads();
-        const HubSeg sg = s_seg;
+        const PairSeg sg = s_seg;
         if (sg.x < 0) break;
         if (tid == 0) n_pairs += sg.len;
         const int32_t xs = __ldg(H.row_ptr + sg.x);
@@ -1799,7 +1891,7 @@ __global__ void __launch_bounds__(256, 5) hub_count_kernel(const HubParams H) {
 template <int UNR>
 __global__ void __launch_bounds__(256, 6) hub_bitmap_kernel(const HubParams H) {
     extern __shared__ __align__(16) uint32_t bm[];
-    __shared__ HubSeg s_seg;
+    __shared__ PairSeg s_seg;
     __shared__ int s_round;
     __shared__ int s_fail;
     const int C = *H.n_core;
@@ -1828,7 +1920,7 @@ __global__ void __launch_bounds__(256, 6) hub_bitmap_kernel(const HubParams H) {
         }
         for (int i = tid; i < nw4; i += blockDim.x) reinterpret_cast<uint4*>(bm)[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
-        const HubSeg sg = s_seg;
+        const PairSeg sg = s_seg;
         if (sg.x < 0) break;
         if (tid == 0) n_pairs += sg.len;
         const int32_t xs = __ldg(H.row_ptr + sg.x);
@@ -1954,7 +2046,7 @@ constexpr int kHub16Threads = 128;
 template <int UNR>
 __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitmap16_kernel(const HubParams H) {
     extern __shared__ __align__(16) uint32_t bm[];  // 4096 words
-    __shared__ HubSeg s_seg;
+    __shared__ PairSeg s_seg;
     __shared__ int s_round;
     __shared__ int2 s_list[kHub16Threads / 32][32];
     const int C = H.n_core[0];
@@ -1985,7 +2077,7 @@ __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitma
         }
         for (int i = tid; i < nw4; i += blockDim.x) bm4[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
-        const HubSeg sg = s_seg;
+        const PairSeg sg = s_seg;
         if (sg.x < 0) break;
         if (tid == 0) n_pairs += sg.len;
         {
@@ -2102,69 +2194,96 @@ __global__ void __launch_bounds__(kHub16Threads, 1536 / kHub16Threads) hub_bitma
     }
 }
 
-// Places of the hub pairs and the hub segments: x's cnth[x] hub pairs get the
-// range [offh[x], + cnth[x]) of the list and are cut into segments of at most
-// seg pairs, x's next to each other.  The order of the ranges does not matter,
-// so a CTA of 1024 vertices scans its own and claims room with one atomic
-// each for pairs and segments (a scan over all vertices and one atomic per x
-// took 94 us on R-MAT 22).  Batched counts (vbase != null)
-// record the graph of x, found by binary search in the ascending vertex
-// offsets vbase[0..n_graphs].
-__global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restrict__ cnth, int64_t n_nodes, int seg,
-                                                        int32_t* __restrict__ offh, unsigned long long* n_pairs,
-                                                        HubSeg* segs, unsigned long long* n_segs, int64_t max_segs,
+// Places of the grouped pairs, and their segments: x's cnth[x] pairs get the
+// range [offh[x], + cnth[x]) of the list and are cut into segments, x's next to
+// each other; those of hub pairs (x's list longer than `hub`; at most hub_seg
+// pairs each) fill segs from the front, those of table pairs (at most
+// kTableSeg) from the back.  The order of the ranges does not matter, so a CTA
+// of 1024 vertices scans its own and claims room with one atomic each for
+// pairs and segments (a scan over all vertices and one atomic per x took 94 us
+// on R-MAT 22).  Batched counts (vbase != null) record the graph of x, found
+// by binary search in the ascending vertex offsets vbase[0..n_graphs].
+struct PairRoom {
+    unsigned long long* n_pairs;
+    PairSeg* segs;
+    int64_t max_segs;
+    unsigned long long* n_hub_segs;
+    unsigned long long* n_table_segs;
+};
+__global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restrict__ cnth,
+                                                        const int2* __restrict__ rows, int64_t n_nodes, int hub,
+                                                        int hub_seg, int32_t* __restrict__ offh, const PairRoom R,
                                                         const int32_t* __restrict__ vbase, int64_t n_graphs,
                                                         const unsigned long long* __restrict__ graph_bad) {
-    __shared__ unsigned long long warp_sum[8], base[2];
+    __shared__ unsigned long long warp_sum[2][8], base[3];
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t x0 = blockIdx.x * 1024ll + tid;
     int32_t c[4];
-    unsigned long long mine = 0;  // pairs << 32 | segments
+    bool is_hub[4];
+    unsigned long long mine[2] = {0, 0};  // pairs; hub segments + table segments << 32
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int64_t x = x0 + 256 * i;
         c[i] = x < n_nodes ? __ldg(cnth + x) : 0;
-        mine += ((unsigned long long)c[i] << 32) + ((unsigned)c[i] + (unsigned)seg - 1u) / (unsigned)seg;
+        is_hub[i] = false;
+        if (c[i] > 0) {
+            const int2 r = __ldg(rows + x);
+            is_hub[i] = hub > 0 && (r.y & 0x7FFFFFFF) - (r.x & 0x7FFFFFFF) > hub;
+            const unsigned seg = is_hub[i] ? hub_seg : kTableSeg, n = ((unsigned)c[i] + seg - 1u) / seg;
+            mine[0] += (unsigned long long)c[i];
+            mine[1] += is_hub[i] ? (unsigned long long)n : (unsigned long long)n << 32;
+        }
     }
-    unsigned long long incl = mine;
+    unsigned long long incl[2] = {mine[0], mine[1]};
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += t;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const unsigned long long t = __shfl_up_sync(FULL, incl[k], o);
+            if (lane >= o) incl[k] += t;
+        }
     }
-    if (lane == 31) warp_sum[tid >> 5] = incl;
+    if (lane == 31) {
+        warp_sum[0][tid >> 5] = incl[0];
+        warp_sum[1][tid >> 5] = incl[1];
+    }
     __syncthreads();
     if (tid == 0) {
-        unsigned long long sum = 0;
-        for (int w = 0; w < 8; ++w) {
-            const unsigned long long t = warp_sum[w];
-            warp_sum[w] = sum;
-            sum += t;
-        }
-        if (sum) {
-            base[0] = atomicAdd(n_pairs, sum >> 32);
-            base[1] = atomicAdd(n_segs, sum & 0xFFFFFFFFull);
+        unsigned long long sum[2] = {0, 0};
+        for (int k = 0; k < 2; ++k)
+            for (int w = 0; w < 8; ++w) {
+                const unsigned long long t = warp_sum[k][w];
+                warp_sum[k][w] = sum[k];
+                sum[k] += t;
+            }
+        if (sum[0]) {
+            base[0] = atomicAdd(R.n_pairs, sum[0]);
+            base[1] = sum[1] & 0xFFFFFFFFull ? atomicAdd(R.n_hub_segs, sum[1] & 0xFFFFFFFFull) : 0;
+            base[2] = sum[1] >> 32 ? atomicAdd(R.n_table_segs, sum[1] >> 32) : 0;
         }
     }
     __syncthreads();
-    if (mine == 0) return;
-    const unsigned long long excl = warp_sum[tid >> 5] + incl - mine;
-    int32_t at = (int32_t)(base[0] + (excl >> 32));
-    int64_t sg = (int64_t)(base[1] + (excl & 0xFFFFFFFFull));
+    if (mine[0] == 0) return;
+    int32_t at = (int32_t)(base[0] + warp_sum[0][tid >> 5] + incl[0] - mine[0]);
+    const unsigned long long before = warp_sum[1][tid >> 5] + incl[1] - mine[1];
+    int64_t hs = (int64_t)(base[1] + (before & 0xFFFFFFFFull));
+    int64_t ts = R.max_segs - 1 - (int64_t)(base[2] + (before >> 32));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         if (c[i] <= 0) continue;
         const int64_t x = x0 + 256 * i;
         const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, graph_bad, (int32_t)x) : 0;
         offh[x] = at;
-        for (int64_t j = 0; j < c[i]; j += seg, ++sg) {
-            if (sg >= max_segs) break;  // cannot happen: sized for the worst case
-            HubSeg s;
+        const int seg = is_hub[i] ? hub_seg : kTableSeg;
+        for (int64_t j = 0; j < c[i]; j += seg) {
+            const int64_t to = is_hub[i] ? hs++ : ts--;
+            if (to < 0 || to >= R.max_segs) break;  // cannot happen: sized for the worst case
+            PairSeg s;
             s.start = at + (int32_t)j;
             s.x = (int32_t)x;
             s.len = min(seg, c[i] - (int32_t)j);
             s.graph = g;
-            segs[sg] = s;
+            R.segs[to] = s;
         }
         at += c[i];
     }
@@ -2689,9 +2808,9 @@ static void phase_reset(const PhaseScope& ps) {
     g_phase.hll_split = false;
 }
 
-template <int MODE, bool VEC, bool DETAILS>
+template <int MODE, bool VEC, bool DETAILS, bool SEGS = false>
 static int launch_mode(const CountParams& P, const Tuning& T, cudaStream_t st) {
-    auto kern = count_kernel<MODE, VEC, DETAILS>;
+    auto kern = count_kernel<MODE, VEC, DETAILS, SEGS>;
     const int threads = T.warps * 32;
     const size_t smem = (size_t)T.warps * ((size_t)1 << P.slots_log2) * sizeof(int32_t);
     static size_t smem_set[kMaxDevices] = {};
@@ -2727,8 +2846,9 @@ static int given_chunk(int64_t n_edges, int chunk) {
 
 struct CountWs {
     // counters: [0] [1] chunks, [2] hub segments made, [3] hub segments
-    // claimed, [4] HLL edges, [5] hub pairs, [6] batches: the graphs from the
-    // first malformed one on; with ncore and cbits one run of zero_words words
+    // claimed, [4] HLL edges, [5] grouped pairs, [6] batches: the graphs from
+    // the first malformed one on, [7] table segments made, [8] claimed; with
+    // ncore and cbits one run of zero_words words
     unsigned long long* ctr;
     int64_t zero_words;
     int32_t* cnth;            // n_nodes + 1 (histogram of hub pairs)
@@ -2736,7 +2856,7 @@ struct CountWs {
     int32_t* py;              // n_edges (probe sides of the hub pairs, by table side)
     int2* rows;               // n_nodes: the row table
     uint2* codes;             // n_edges / 32 + 1 (batches: their own)
-    HubSeg* segs;             // max_segs
+    PairSeg* segs;             // max_segs
     int64_t max_segs;
     int32_t* pcol;            // padded lists in core coordinates for the hub kernels, pcap entries (null: not carved)
     int64_t pcap;
@@ -2763,7 +2883,8 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
 // sizes and cursors (256 each), last the number of live row blocks.  Cleared
 // together.
 constexpr int kCoreWords = 4 + 2 * 256 + 1;
-constexpr int kCounters = 8;
+constexpr int kCounters = 10;
+constexpr int kWeights = 2;  // list_weights, in front of the counters: cleared on their own
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
@@ -2773,7 +2894,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     // [counters][ncore][cbits]
     const size_t cb = pad ? N / 32 + 1 : 0, nc = pad ? kCoreWords : 0;
     W.zero_words = (int64_t)(2 * kCounters + nc + cb);
-    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words));
+    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words + 2 * kWeights)) + kWeights;
     W.ncore = pad ? reinterpret_cast<int32_t*>(W.ctr + kCounters) : nullptr;
     W.cbits = pad ? reinterpret_cast<uint32_t*>(W.ncore + kCoreWords) : nullptr;
     W.cnth = cv.take<int32_t>(N);
@@ -2783,7 +2904,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     W.codes = cv.take<uint2>(E / 32 + 1);
     // every hub x with pairs opens one segment, every HUB_SEG_MIN pairs at most one more
     W.max_segs = (int64_t)(N < E ? N : E) + (int64_t)(E / HUB_SEG_MIN) + 1;
-    W.segs = cv.take<HubSeg>((size_t)W.max_segs);
+    W.segs = cv.take<PairSeg>((size_t)W.max_segs);
     W.pcap = pad ? pad_capacity(n_nodes, (int64_t)E) : 0;
     W.pcol = pad ? cv.take<int32_t>((size_t)W.pcap) : nullptr;
     W.cflag = pad ? cv.take<int32_t>(N) : nullptr;
@@ -2947,7 +3068,7 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     Q.slot = P.slot;
     Q.has = P.has;
     Q.n_rows = P.n_rows;
-    Q.zero_n[0] = hub > 0 ? W.cnth : nullptr;
+    Q.zero_n[0] = W.cnth;
     Q.zero_n[1] = hub > 0 ? W.cflag : nullptr;
     Q.zero[0] = reinterpret_cast<uint32_t*>(W.ctr);
     Q.words[0] = W.zero_words;
@@ -2955,8 +3076,12 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     Q.words[1] = n_results * (int64_t)(sizeof(tchll_count_result) / 4);
     Q.zero[2] = more;
     Q.words[2] = more_words;
+    Q.hub = hub;
+    Q.list_weights = W.ctr - kWeights;
+    TCHLL_CUDA(cudaMemsetAsync(Q.list_weights, 0, kWeights * sizeof(unsigned long long), st));
     prepare_kernel<<<grid_edges(P.n_nodes + 1), 256, 0, st>>>(Q);
     TCHLL_CHECK_LAUNCH("prepare_kernel");
+    P.list_weights = Q.list_weights;
     P.rows = W.rows;
     P.codes = W.codes;
     return TCHLL_OK;
@@ -2997,14 +3122,15 @@ static int pair_pass(CountParams P, const CountWs& W, int what, int hub, unsigne
     return TCHLL_OK;
 }
 
-// After PASS_HIST: room for the hub pairs, and the hub segments (smaller ones
-// in small graphs, so that every CTA gets a few).
-static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaStream_t st) {
+// After PASS_HIST: room for the grouped pairs, and their segments (smaller
+// hub segments in small graphs, so that every CTA gets a few).
+static int hub_alloc(const CountParams& P, const CountWs& W, int hub, int hub_seg, cudaStream_t st) {
     while (hub_seg > HUB_SEG_MIN && P.n_edges < (int64_t)hub_seg * 24 * sm_count()) hub_seg >>= 1;
     if (hub_seg < HUB_SEG_MIN) hub_seg = HUB_SEG_MIN;
     const int grid = (int)(P.n_nodes > 0 ? (P.n_nodes + 1023) / 1024 : 1);
-    hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, P.n_nodes, hub_seg, W.offh, W.ctr + 5, W.segs, W.ctr + 2,
-                                           W.max_segs, P.graph_vbase, P.n_graphs, P.graph_bad);
+    const PairRoom R{W.ctr + 5, W.segs, W.max_segs, W.ctr + 2, W.ctr + 7};
+    hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, W.rows, P.n_nodes, hub, hub_seg, W.offh, R, P.graph_vbase,
+                                           P.n_graphs, P.graph_bad);
     TCHLL_CHECK_LAUNCH("hub_alloc_kernel");
     return TCHLL_OK;
 }
@@ -3013,6 +3139,19 @@ static int pairs_scatter(const CountParams& P, const CountWs& W, cudaStream_t st
     pair_scatter_kernel<<<grid_edges(P.n_edges), 256, 0, st>>>(P, W.offh, W.ctr + 5, W.py);
     TCHLL_CHECK_LAUNCH("pair_scatter_kernel");
     return TCHLL_OK;
+}
+
+// The table pairs, once scattered.
+static int launch_table_pairs(const CountParams& P, const CountWs& W, const Tuning& T, cudaStream_t st) {
+    CountParams Q = P;
+    Q.edge_v = W.py;
+    Q.segs_end = W.segs + W.max_segs;
+    Q.n_segs = W.ctr + 7;
+    Q.work = W.ctr + 8;
+    Q.check_ids = 0;
+    Q.chunk_start = nullptr;
+    return (uintptr_t)P.col_idx % 16 == 0 ? launch_mode<MODE_EXACT, true, false, true>(Q, T, st)
+                                          : launch_mode<MODE_EXACT, false, false, true>(Q, T, st);
 }
 
 static int grid_rows(int64_t n, int per_cta) {  // one unit of work per 256 / per_cta threads
@@ -3354,20 +3493,21 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
-                const bool split = col_ready && hub > 0;
-                if (col_ready && !split) TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
+                const bool split = col_ready != nullptr;
                 CountParams H = P;
                 if (split) H.check_ids = 0;  // col_idx is not there yet
-                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr, st);
-                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
-                if (rc) return rc;
-                if (hub > 0) rc = pairs_scatter(P, W, st);
+                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr,
+                                      st);
+                if (rc == TCHLL_OK) rc = hub_alloc(P, W, hub, T.hub_seg, st);
+                if (rc == TCHLL_OK) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 if (split) {
                     TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
                     rc = pair_pass<false>(P, W, PASS_SHORT, hub, W.ctr + 1, st);
                     if (rc) return rc;
                 }
+                rc = launch_table_pairs(P, W, T, st);
+                if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
                     rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, road, ps, st);
@@ -3430,9 +3570,9 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[0], hst);
                 rc = launch_hll_edges(P, HW, T, hst);
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[1], hst);
-                if (rc == TCHLL_OK && hub > 0) rc = hub_alloc(P, W, T.hub_seg, st);
-                if (rc) return rc;
-                if (hub > 0) rc = pairs_scatter(P, W, st);
+                if (rc == TCHLL_OK) rc = hub_alloc(P, W, hub, T.hub_seg, st);
+                if (rc == TCHLL_OK) rc = pairs_scatter(P, W, st);
+                if (rc == TCHLL_OK) rc = launch_table_pairs(P, W, T, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
@@ -4069,14 +4209,15 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
         rc = launch_count<MODE_HYB_EXACT>(P, T, false, st);
         if (rc) return rc;
     }
-    const bool hubs = hub > 0 && (hll_list || !hybrid);
-    if (hubs) {
-        rc = hub_alloc(P, B.cw, T.hub_seg, st);
+    const bool grouped = hll_list || !hybrid;
+    if (grouped) {
+        rc = hub_alloc(P, B.cw, hub, T.hub_seg, st);
         if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
+        if (rc == TCHLL_OK) rc = launch_table_pairs(P, B.cw, T, st);
         if (rc) return rc;
     }
     phase_mark(ps, 1, st);
-    if (hubs) {
+    if (hub > 0 && grouped) {
         rc = launch_core_pass(P, B.cw, T, hub, true, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
