@@ -112,7 +112,7 @@ struct CountParams {
     // before segs_end, the second before that; edge_v holds the probe sides
     const PairSeg* segs_end;
     const unsigned long long* n_segs;
-    const unsigned long long* list_weights;  // see is_table_pair (null: no table pairs)
+    const unsigned long long* table_est;  // {sampled table pairs, lists of their length} (null: no table pairs)
     // Hybrid with pairs: the routing pass appends HLL edges here
     int32_t* hll_u;
     int32_t* hll_v;
@@ -306,17 +306,23 @@ __device__ __forceinline__ bool is_hub_pair(const PairSides& S, int hub) { retur
 // Table pairs, of the others: a table side and a probe side of some length.
 // They are grouped by table side like hub pairs and counted with a warp's
 // hash table of it (count_kernel with SEGS), where a look-up is one shared
-// load instead of a search of 4 and more steps.  That takes several pairs to a
-// table side, which skewed graphs do not have (R-MAT 20: 272 us in tables, 25 in
-// searches), so it is done where lists of such a length hold at least a
-// quarter of the graph's look-ups, measured by squared length (list_weights,
-// summed by prepare_kernel: {their lists, all}): 0 to 0.1 on R-MAT 16 and up,
-// above 0.3 where lists are evenly long.  Whole calls, us, all pairs in
-// tables / all in searches / so: a million vertices joined to 20 near ones
-// 1,493 / 1,009 / 1,024, to 30 2,088 / 2,164 / 1,886, to 40 2,755 / 3,673 / 2,651, to
-// 60 4,475 / 8,420 / 4,407; Erdos-Renyi, 40 M edges 3,808 / 4,768 / 3,480.
+// load instead of a search of 4 and more steps.  That takes many pairs to a
+// table side, which skewed graphs do not have (R-MAT 20, 4 to a side: 272 us in
+// tables, 25 in searches), so prepare_kernel estimates them, from a sample of
+// the edges and the number of lists of such a length, and below kTableMin to a
+// side the pairs are searched: R-MAT 16 to 22 have 4 to 17, graphs of evenly
+// long lists 25 and more.  So are they where they are less than one in
+// kTableShare of all pairs, which does not pay for the launch's tail (50 K
+// vertices joined to 80 near ones, one in ten: 423 us in tables, 362 in
+// searches).  Whole calls, us, all pairs in tables / all in searches / so: a
+// million vertices joined to 20 near ones 1,493 / 1,009 / 1,024, to 30 2,088 / 2,164
+// / 1,886, to 40 2,755 / 3,673 / 2,651, to 60 4,475 / 8,420 / 4,407; Erdos-Renyi, 40 M
+// edges 3,808 / 4,768 / 3,480.
 constexpr int kTableList = 32;
 constexpr int kTableProbes = 16;
+constexpr int kTableMin = 20;
+constexpr int kTableShare = 5;
+constexpr int kEdgeSample = 8192;
 __device__ __forceinline__ bool is_table_pair(const PairSides& S, int list) {
     return list > 0 && S.xl > list && S.yl > kTableProbes;
 }
@@ -477,24 +483,23 @@ struct Prepare {
     int64_t n_rows;
     int2* rows;
     int hub;
-    unsigned long long* list_weights;  // zeroed before
+    const int32_t* edge_u;
+    const int32_t* edge_v;
+    int64_t n_edges;
+    unsigned long long* table_est;  // zeroed before
     int32_t* zero_n[2];   // n_nodes + 1 words each (or null)
     uint32_t* zero[3];    // words[i] words
     int64_t words[3];
 };
 __global__ void prepare_kernel(const Prepare Q) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
-    unsigned long long weight = 0, table_weight = 0;
+    uint32_t lists = 0, pairs = 0;  // of the length of table pairs; sampled table pairs
     for (int64_t v = t0; v <= Q.n_nodes; v += step) {
         if (v < Q.n_nodes) {
             const int32_t a = __ldg(Q.row_ptr + v), b = __ldg(Q.row_ptr + v + 1);
             int2 r = make_int2(a, b);
             const bool bad = a < 0 || b < a || (int64_t)b > Q.nnz;
-            if (!bad) {
-                const unsigned long long w = (unsigned long long)(b - a) * (unsigned long long)(b - a);
-                weight += w;
-                if (b - a > kTableList && (Q.hub == 0 || b - a <= Q.hub)) table_weight += w;
-            }
+            if (!bad && b - a > kTableList && (Q.hub == 0 || b - a <= Q.hub)) ++lists;
             if (bad) {
                 r = make_int2(kRowBad, 0);
             } else if (Q.degrees) {
@@ -512,20 +517,39 @@ __global__ void prepare_kernel(const Prepare Q) {
 #pragma unroll
     for (int i = 0; i < 3; ++i)
         for (int64_t w = t0; w < Q.words[i]; w += step) Q.zero[i][w] = 0;
+    if (t0 < kEdgeSample && t0 < Q.n_edges) {
+        const int64_t e = Q.n_edges <= kEdgeSample ? t0 : t0 * Q.n_edges / kEdgeSample;
+        const int32_t u = __ldg(Q.edge_u + e), v = __ldg(Q.edge_v + e);
+        if ((uint32_t)u < (uint32_t)Q.n_nodes && (uint32_t)v < (uint32_t)Q.n_nodes) {
+            const PairSides S = sides_of(u, v, __ldg(Q.row_ptr + u), __ldg(Q.row_ptr + u + 1), __ldg(Q.row_ptr + v),
+                                         __ldg(Q.row_ptr + v + 1));
+            pairs = !is_hub_pair(S, Q.hub) && is_table_pair(S, kTableList);
+            if (Q.degrees && pairs) pairs = min(__ldg(Q.degrees + u), __ldg(Q.degrees + v)) < Q.gamma;  // else HLL
+        }
+    }
     // one atomic each per CTA
-    __shared__ unsigned long long sums[2][8];
-    weight = warp_sum_u64(weight);
-    table_weight = warp_sum_u64(table_weight);
+    __shared__ uint32_t sums[2][8];
+    pairs = __reduce_add_sync(FULL, pairs);
+    lists = __reduce_add_sync(FULL, lists);
     if ((threadIdx.x & 31) == 0) {
-        sums[0][threadIdx.x >> 5] = table_weight;
-        sums[1][threadIdx.x >> 5] = weight;
+        sums[0][threadIdx.x >> 5] = pairs;
+        sums[1][threadIdx.x >> 5] = lists;
     }
     __syncthreads();
     if (threadIdx.x < 2) {
         unsigned long long t = 0;
         for (int i = 0; i < 8; ++i) t += sums[threadIdx.x][i];
-        if (t) atomicAdd(Q.list_weights + threadIdx.x, t);
+        if (t) atomicAdd(Q.table_est + threadIdx.x, t);
     }
+}
+
+// kTableList when table pairs are worth their grouping, else 0.
+__device__ __forceinline__ int table_list(const CountParams& P) {
+    if (P.table_est == nullptr) return 0;
+    const unsigned long long pairs = __ldg(P.table_est), lists = __ldg(P.table_est + 1);
+    const unsigned long long n = (unsigned long long)P.n_edges;
+    const unsigned long long of = n < kEdgeSample ? n : kEdgeSample;
+    return pairs * kTableShare >= of && pairs * n >= kTableMin * lists * of ? kTableList : 0;
 }
 
 // The first pass over the edges.  Pairs with a long table side (hub pairs)
@@ -591,7 +615,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
     uint32_t status = 0;
     if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col, status);
     const int32_t full_quads = (int32_t)(P.nnz >> 2);
-    const int table = P.list_weights && __ldg(P.list_weights) >= __ldg(P.list_weights + 1) / 4 ? kTableList : 0;
+    const int table = table_list(P);
     const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     while (true) {
@@ -2884,7 +2908,7 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
 // together.
 constexpr int kCoreWords = 4 + 2 * 256 + 1;
 constexpr int kCounters = 10;
-constexpr int kWeights = 2;  // list_weights, in front of the counters: cleared on their own
+constexpr int kEstimates = 2;  // table_est, in front of the counters: cleared on their own
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
@@ -2894,7 +2918,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     // [counters][ncore][cbits]
     const size_t cb = pad ? N / 32 + 1 : 0, nc = pad ? kCoreWords : 0;
     W.zero_words = (int64_t)(2 * kCounters + nc + cb);
-    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words + 2 * kWeights)) + kWeights;
+    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words + 2 * kEstimates)) + kEstimates;
     W.ncore = pad ? reinterpret_cast<int32_t*>(W.ctr + kCounters) : nullptr;
     W.cbits = pad ? reinterpret_cast<uint32_t*>(W.ncore + kCoreWords) : nullptr;
     W.cnth = cv.take<int32_t>(N);
@@ -3077,11 +3101,15 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     Q.zero[2] = more;
     Q.words[2] = more_words;
     Q.hub = hub;
-    Q.list_weights = W.ctr - kWeights;
-    TCHLL_CUDA(cudaMemsetAsync(Q.list_weights, 0, kWeights * sizeof(unsigned long long), st));
-    prepare_kernel<<<grid_edges(P.n_nodes + 1), 256, 0, st>>>(Q);
+    Q.edge_u = P.edge_u;
+    Q.edge_v = P.edge_v;
+    Q.n_edges = P.n_edges;
+    Q.table_est = W.ctr - kEstimates;
+    TCHLL_CUDA(cudaMemsetAsync(Q.table_est, 0, kEstimates * sizeof(unsigned long long), st));
+    const int64_t sample = P.n_edges < kEdgeSample ? P.n_edges : kEdgeSample;
+    prepare_kernel<<<grid_edges(P.n_nodes + 1 > sample ? P.n_nodes + 1 : sample), 256, 0, st>>>(Q);
     TCHLL_CHECK_LAUNCH("prepare_kernel");
-    P.list_weights = Q.list_weights;
+    P.table_est = Q.table_est;
     P.rows = W.rows;
     P.codes = W.codes;
     return TCHLL_OK;
