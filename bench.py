@@ -293,7 +293,7 @@ def run_ours(args):
     algo_bytes = 16 * g.n_edges + 4 * int((du + dv).sum().item())
     del du, dv
     tuning = core.get_count_tuning()
-    hw = hub_work(g, tuning["hub"])
+    hw = hub_work(g, core.hub_threshold(g.row_ptr, g.col_idx, g.edge_u, g.edge_v))
     res = _lib.count_result_tensor(dev)
     if args.mode == "hybrid":
         return run_hybrid_line(args, g, dev, rank, world, barrier, max_over_ranks)
@@ -494,7 +494,7 @@ def run_hybrid_line(args, g, dev, rank, world, barrier, max_over_ranks):
     hll = torch.minimum(du, dv) >= theta
     n_hll = int(hll.sum().item())
     exact_bytes = 16 * (g.n_edges - n_hll) + 4 * int(torch.where(hll, 0, du + dv).sum().item())
-    hub_thr = core.get_count_tuning()["hub"]
+    hub_thr = core.hub_threshold(g.row_ptr, g.col_idx, g.edge_u, g.edge_v)
     hub = (~hll) & (torch.maximum(du, dv) > hub_thr) if hub_thr > 0 else torch.zeros_like(hll)
     hub_bytes = 16 * int(hub.sum().item()) + 4 * int(torch.where(hub, du + dv, 0).sum().item())
     hll_bytes = n_hll * (16 + 2 * (1 << p))
@@ -560,7 +560,7 @@ def run_hybrid_line(args, g, dev, rank, world, barrier, max_over_ranks):
     # others), hub pairs, first pass (routing, short-list pairs) and scatter
     hub_ms = avg.get("hub") or 0.0
     tuning = core.get_count_tuning()
-    hname = hub_kernel_name(tuning, hub_work(g, tuning["hub"])["core_vertices"])
+    hname = hub_kernel_name(tuning, hub_work(g, hub_thr)["core_vertices"])
     cands = [("hll_edges_kernel", avg["hll"], hll_bytes), (hname, hub_ms, hub_bytes),
              ("pair_pass_kernel + pair_scatter_kernel", avg.get("pairs") or 0.0, exact_bytes - hub_bytes)]
     kname, kms, kbytes = max(cands, key=lambda c: c[1])

@@ -172,14 +172,21 @@ int tchll_get_count_tuning(int32_t* out8 /* host */);
  * memory allow), at most seg_pairs of x's pairs per work unit, unroll 16-byte
  * probe loads in flight per lane; all other pairs are counted by binary search
  * of the longer list in the first pass over the edges or, in graphs of evenly
- * long lists, with a warp's hash table of it.  threshold 128, the
- * default, is taken as 64 where that is faster (up to 28 M edges; batches: a
- * mean forward degree of at least 12).  threshold 0 turns it off; otherwise
+ * long lists, with a warp's hash table of it.  threshold -1, the
+ * default, is automatic: 128, or 64 where the packed lists (tchll_set_count_core)
+ * are held and their core fits, which depends on the graph
+ * (tchll_count_hub_threshold).  threshold 0 turns it off; otherwise
  * threshold >= 64, seg_pairs in [256, 2^20], table_log2 in [10, 15], unroll 2
  * or 4.  out4 receives the four values.  Results are identical for every
  * setting. */
 int tchll_set_count_hub(int32_t threshold, int32_t seg_pairs, int32_t table_log2, int32_t unroll);
 int tchll_get_count_hub(int32_t* out4 /* host */);
+/* The hub threshold that tchll_exact_count would count this graph with when it
+ * regroups its pairs, 0 for none (workspace as for the count; waits for the
+ * stream). */
+int tchll_count_hub_threshold(const int32_t* row_ptr, int64_t n_nodes, const int32_t* col_idx, int64_t nnz,
+                              const int32_t* edge_u, const int32_t* edge_v, int64_t n_edges, void* workspace,
+                              size_t workspace_bytes, int32_t* out /* host */, void* stream);
 
 /* Hub core (pairs layout, with the padded lists in the workspace): the hub
  * kernels work in the coordinates of the core, the vertices that appear in

@@ -25,12 +25,14 @@ from . import _lib, core
 from ._lib import check, load, ptr, stream_handle
 
 CANDIDATES: List[Dict] = [
+    {"chunk": 256, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": -1},
+    {"chunk": 128, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": -1},
+    {"chunk": 512, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": -1},
+    {"chunk": 256, "slots_log2": 11, "tiny": 48, "sparse": 1, "hub": -1},
+    {"chunk": 256, "slots_log2": 10, "tiny": 24, "sparse": 0, "hub": -1},
+    {"chunk": 64, "slots_log2": 9, "tiny": 32, "sparse": 0, "hub": -1},
+    {"chunk": 256, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 64},
     {"chunk": 256, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 128},
-    {"chunk": 128, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 128},
-    {"chunk": 512, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 128},
-    {"chunk": 256, "slots_log2": 11, "tiny": 48, "sparse": 1, "hub": 128},
-    {"chunk": 256, "slots_log2": 10, "tiny": 24, "sparse": 0, "hub": 128},
-    {"chunk": 64, "slots_log2": 9, "tiny": 32, "sparse": 0, "hub": 128},
     {"chunk": 256, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 256},
     {"chunk": 256, "slots_log2": 10, "tiny": 24, "sparse": 0, "hub": 256},
     {"chunk": 256, "slots_log2": 11, "tiny": 16, "sparse": 0, "hub": 0},

@@ -306,7 +306,8 @@ def set_count_tuning(chunk: int = 256, slots_log2: int = 10, tiny: int = 16, blo
     pairs: 0 edges as given, 1 regrouped by the longer list when the graph is
     large enough for it to pay, 2 regrouped whatever its size.
     hub / hub_seg / hub_lg / hub_unroll: threshold on d+(x) above which a pair
-    goes to the CTA-shared table kernels (0: off), pairs per work unit, log2
+    goes to the CTA-shared table kernels (0: off, -1: 64 or 128 by the graph,
+    see hub_threshold), pairs per work unit, log2
     hash-table slots, probe loads in flight per lane.  bitmap_lg: log2 bytes
     of the 32-bit hub bitmap buffer (0: off); overlap: 0 one stream, 1 the
     hub core pass (and a hybrid's HLL pass) on a second stream beside the
@@ -349,6 +350,20 @@ def get_count_tuning() -> dict:
             "hub_unroll": hub[3], "bitmap_lg": co[0], "overlap": co[1], "packed": co[2], "bank_sort": co[3],
             "hll_row_cache_p": hp[0],
             "hll_lanes": hp[1]}
+
+
+def hub_threshold(row_ptr, col_idx, edge_u, edge_v) -> int:
+    """The hub threshold that exact_count_tensors counts this graph with when it
+    regroups its pairs (0: none); waits for the current stream."""
+    dev = row_ptr.device
+    n_nodes, n_edges = int(row_ptr.numel()) - 1, int(edge_u.numel())
+    ws = _count_ws(n_nodes, n_edges, dev)
+    out = C.c_int32(0)
+    with _lib.on_device(dev):
+        check(load().tchll_count_hub_threshold(ptr(row_ptr), n_nodes, ptr(col_idx), int(col_idx.numel()), ptr(edge_u),
+                                               ptr(edge_v), n_edges, ptr(ws), ws.numel(), C.addressof(out),
+                                               stream_handle(dev)), "hub threshold")
+    return out.value
 
 
 def set_phase_timing(enable: bool) -> None:

@@ -112,7 +112,9 @@ struct CountParams {
     // before segs_end, the second before that; edge_v holds the probe sides
     const PairSeg* segs_end;
     const unsigned long long* n_segs;
-    const unsigned long long* table_est;  // {sampled table pairs, lists of their length} (null: no table pairs)
+    unsigned long long* est;  // see Choice (null: neither hub nor table pairs)
+    int hub;
+    int hub_alt;
     // Hybrid with pairs: the routing pass appends HLL edges here
     int32_t* hll_u;
     int32_t* hll_v;
@@ -319,12 +321,45 @@ __device__ __forceinline__ bool is_hub_pair(const PairSides& S, int hub) { retur
 // / 1,886, to 40 2,755 / 3,673 / 2,651, to 60 4,475 / 8,420 / 4,407; Erdos-Renyi, 40 M
 // edges 3,808 / 4,768 / 3,480.
 constexpr int kTableList = 32;
-constexpr int kTableProbes = 16;
+constexpr int kTableProbes = 8;
 constexpr int kTableMin = 20;
 constexpr int kTableShare = 5;
 constexpr int kEdgeSample = 8192;
 __device__ __forceinline__ bool is_table_pair(const PairSides& S, int list) {
     return list > 0 && S.xl > list && S.yl > kTableProbes;
+}
+
+// Largest core that the packed lists hold (core_lists_kernel).
+constexpr int32_t kCore16Max = 131070;
+
+// The hub threshold of a call and whether it has table pairs.  The host gives
+// the threshold, and with hub_alt leaves it to the device to double it; what
+// the device goes by is est: {sampled pairs with a list in (kTableList, hub]
+// and more than kTableProbes probes, lists of that length, the same two for
+// (hub, 2 hub], vertices of a batch's largest graph}.  It is doubled where half
+// of all pairs have lists in (kTableList, 2 hub], because evenly long lists bring
+// all vertices into the core (a batch's largest graph permitting; batches of
+// more than kHub64Edges edges always, when that graph's core may not fit).
+// Whole calls, us, at 64 / at 128: Erdos-Renyi with 300 K vertices and 24 M edges
+// 3,277 / 2,930, 300 K vertices joined to 50 near ones 1,487 / 1,129; R-MAT 20, one
+// pair in ten, 1,590 / 1,800, R-MAT 22 with edge factor 2 895 / 1,013.
+constexpr int kEst = 5;
+constexpr int64_t kHub64Edges = 28000000;
+struct Choice {
+    int hub, table;
+};
+__host__ __device__ __forceinline__ Choice choose(const unsigned long long* est, int64_t n_edges, int hub, int hub_alt,
+                                                  bool batched) {
+    const unsigned long long n = (unsigned long long)n_edges, of = n < kEdgeSample ? n : kEdgeSample;
+    unsigned long long pairs = est[0], lists = est[1];
+    const bool even = 2 * (pairs + est[2]) >= of;
+    if (hub_alt && (batched ? est[4] > (unsigned long long)kCore16Max && (even || n_edges > kHub64Edges) : even)) {
+        hub *= 2;
+        pairs += est[2];
+        lists += est[3];
+    }
+    const bool table = pairs * kTableShare >= of && pairs * n >= kTableMin * lists * of;
+    return Choice{hub, table ? kTableList : 0};
 }
 
 // Batched calls: the graph of vertex v, the last g with vbase[g] <= v among
@@ -486,20 +521,23 @@ struct Prepare {
     const int32_t* edge_u;
     const int32_t* edge_v;
     int64_t n_edges;
-    unsigned long long* table_est;  // zeroed before
+    unsigned long long* est;  // zeroed before
     int32_t* zero_n[2];   // n_nodes + 1 words each (or null)
     uint32_t* zero[3];    // words[i] words
     int64_t words[3];
 };
 __global__ void prepare_kernel(const Prepare Q) {
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
-    uint32_t lists = 0, pairs = 0;  // of the length of table pairs; sampled table pairs
+    uint32_t est[4] = {0, 0, 0, 0};
     for (int64_t v = t0; v <= Q.n_nodes; v += step) {
         if (v < Q.n_nodes) {
             const int32_t a = __ldg(Q.row_ptr + v), b = __ldg(Q.row_ptr + v + 1);
             int2 r = make_int2(a, b);
             const bool bad = a < 0 || b < a || (int64_t)b > Q.nnz;
-            if (!bad && b - a > kTableList && (Q.hub == 0 || b - a <= Q.hub)) ++lists;
+            if (!bad && b - a > kTableList) {
+                if (Q.hub == 0 || b - a <= Q.hub) ++est[1];
+                else if (b - a <= 2 * (int64_t)Q.hub) ++est[3];
+            }
             if (bad) {
                 r = make_int2(kRowBad, 0);
             } else if (Q.degrees) {
@@ -523,33 +561,26 @@ __global__ void prepare_kernel(const Prepare Q) {
         if ((uint32_t)u < (uint32_t)Q.n_nodes && (uint32_t)v < (uint32_t)Q.n_nodes) {
             const PairSides S = sides_of(u, v, __ldg(Q.row_ptr + u), __ldg(Q.row_ptr + u + 1), __ldg(Q.row_ptr + v),
                                          __ldg(Q.row_ptr + v + 1));
-            pairs = !is_hub_pair(S, Q.hub) && is_table_pair(S, kTableList);
-            if (Q.degrees && pairs) pairs = min(__ldg(Q.degrees + u), __ldg(Q.degrees + v)) < Q.gamma;  // else HLL
+            const bool exact = !Q.degrees || min(__ldg(Q.degrees + u), __ldg(Q.degrees + v)) < Q.gamma;  // else HLL
+            if (exact && is_table_pair(S, kTableList)) {
+                est[0] = Q.hub == 0 || S.xl <= Q.hub;
+                est[2] = Q.hub > 0 && S.xl > Q.hub && S.xl <= 2 * (int64_t)Q.hub;
+            }
         }
     }
     // one atomic each per CTA
-    __shared__ uint32_t sums[2][8];
-    pairs = __reduce_add_sync(FULL, pairs);
-    lists = __reduce_add_sync(FULL, lists);
-    if ((threadIdx.x & 31) == 0) {
-        sums[0][threadIdx.x >> 5] = pairs;
-        sums[1][threadIdx.x >> 5] = lists;
+    __shared__ uint32_t sums[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        est[k] = __reduce_add_sync(FULL, est[k]);
+        if ((threadIdx.x & 31) == 0) sums[k][threadIdx.x >> 5] = est[k];
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
+    if (threadIdx.x < 4) {
         unsigned long long t = 0;
         for (int i = 0; i < 8; ++i) t += sums[threadIdx.x][i];
-        if (t) atomicAdd(Q.table_est + threadIdx.x, t);
+        if (t) atomicAdd(Q.est + threadIdx.x, t);
     }
-}
-
-// kTableList when table pairs are worth their grouping, else 0.
-__device__ __forceinline__ int table_list(const CountParams& P) {
-    if (P.table_est == nullptr) return 0;
-    const unsigned long long pairs = __ldg(P.table_est), lists = __ldg(P.table_est + 1);
-    const unsigned long long n = (unsigned long long)P.n_edges;
-    const unsigned long long of = n < kEdgeSample ? n : kEdgeSample;
-    return pairs * kTableShare >= of && pairs * n >= kTableMin * lists * of ? kTableList : 0;
 }
 
 // The first pass over the edges.  Pairs with a long table side (hub pairs)
@@ -598,7 +629,7 @@ __device__ __forceinline__ void pass_publish(tchll_count_result* R, uint64_t acc
 }
 
 template <bool HYB, bool VEC, int UNR = 2>
-__global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, int what, int hub,
+__global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, int what,
                                                            int32_t* __restrict__ cnth) {
     __shared__ int4 s_list[8][32];
     __shared__ int32_t s_len[8][32];
@@ -615,7 +646,7 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
     uint32_t status = 0;
     if (P.check_ids) validate_rows(P.row_ptr, P.n_nodes, P.nnz, col, status);
     const int32_t full_quads = (int32_t)(P.nnz >> 2);
-    const int table = table_list(P);
+    const Choice ch = P.est ? choose(P.est, P.n_edges, P.hub, P.hub_alt, P.graph_vbase != nullptr) : Choice{0, 0};
     const unsigned long long n_warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     unsigned long long turn = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     while (true) {
@@ -678,8 +709,8 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
                 ok = ok && !hll;
             }
             const PairSides S = sides_of(u, v, us, ue, vs, ve);
-            const bool to_hub = ok && is_hub_pair(S, hub);
-            const bool grouped = to_hub || (ok && is_table_pair(S, table));
+            const bool to_hub = ok && is_hub_pair(S, ch.hub);
+            const bool grouped = to_hub || (ok && is_table_pair(S, ch.table));
             if (what & PASS_HIST) {
                 const unsigned m = __ballot_sync(FULL, grouped), mu = __ballot_sync(FULL, S.x == u);
                 if (lane == 0) P.codes[code0 + ((eb - e0) >> 5)] = make_uint2(m, mu);
@@ -1225,10 +1256,11 @@ __device__ __forceinline__ int64_t pad_start(int32_t rs, int32_t y) {
 constexpr int64_t kMarkAllEdges = 8000000;
 constexpr int kMarkStep = 8;
 __global__ void core_mark_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, int64_t nnz,
-                                 const int32_t* __restrict__ col, int hub, int count_all,
+                                 const int32_t* __restrict__ col, const CountParams P, int count_all,
                                  const unsigned long long* __restrict__ n_segs, uint32_t* bits, int32_t* cnt,
                                  tchll_count_result* result) {
     if (n_segs && *n_segs == 0) return;  // grid-uniform: after the first pass, which found no hub pairs
+    const int hub = choose(P.est, P.n_edges, P.hub, P.hub_alt, P.graph_vbase != nullptr).hub;
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1430,7 +1462,6 @@ __global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* 
 // list loads weigh in: hub kernel on R-MAT 22 with 8, 11, 14, 18, 24, 30 to 34:
 // 6.57, 6.31, 5.65, 5.36, 5.46, 5.47 ms (keys only: 7.29 ms).
 constexpr int32_t kPlane = 65535;
-constexpr int32_t kCore16Max = 131070;
 constexpr int kBmSteps = 8;
 constexpr int kBmMax = 32;  // units of the longest bitmap
 __device__ __forceinline__ constexpr int bm_units(int k) {  // the B a row chooses from (and 0)
@@ -2235,11 +2266,13 @@ struct PairRoom {
     unsigned long long* n_table_segs;
 };
 __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restrict__ cnth,
-                                                        const int2* __restrict__ rows, int64_t n_nodes, int hub,
-                                                        int hub_seg, int32_t* __restrict__ offh, const PairRoom R,
-                                                        const int32_t* __restrict__ vbase, int64_t n_graphs,
-                                                        const unsigned long long* __restrict__ graph_bad) {
+                                                        const CountParams P, int hub_seg, int32_t* __restrict__ offh,
+                                                        const PairRoom R) {
     __shared__ unsigned long long warp_sum[2][8], base[3];
+    const int2* __restrict__ rows = P.rows;
+    const int64_t n_nodes = P.n_nodes;
+    const int32_t* __restrict__ vbase = P.graph_vbase;
+    const int hub = choose(P.est, P.n_edges, P.hub, P.hub_alt, vbase != nullptr).hub;
     const int tid = threadIdx.x, lane = tid & 31;
     const int64_t x0 = blockIdx.x * 1024ll + tid;
     int32_t c[4];
@@ -2296,7 +2329,7 @@ __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restric
     for (int i = 0; i < 4; ++i) {
         if (c[i] <= 0) continue;
         const int64_t x = x0 + 256 * i;
-        const int32_t g = vbase ? (int32_t)graph_of(vbase, n_graphs, graph_bad, (int32_t)x) : 0;
+        const int32_t g = vbase ? (int32_t)graph_of(vbase, P.n_graphs, P.graph_bad, (int32_t)x) : 0;
         offh[x] = at;
         const int seg = is_hub[i] ? hub_seg : kTableSeg;
         for (int64_t j = 0; j < c[i]; j += seg) {
@@ -2705,8 +2738,8 @@ __global__ void __launch_bounds__(256, CROW ? 2 : (ZS ? 4 : (CACHE ? 3 : 4))) hl
 }
 
 // ---------------------------------------------------------------- host ------
-constexpr int kHubDefault = 128;
-constexpr int64_t kHub64Edges = 28000000;
+constexpr int kHubAuto = -1;
+constexpr int kHubWide = 128;
 constexpr int64_t kHub64Degree = 12;
 struct Tuning {
     int chunk = 256;
@@ -2716,7 +2749,7 @@ struct Tuning {
     int warps = 8;          // warps per CTA
     int pairs = 1;          // table-side / probe-side reorientation (2: for small graphs too)
     int sparse = 0;         // table load <= 1/4 where it fits
-    int hub = kHubDefault;  // pairs with d+(x) > hub go to the CTA-table kernels (0: off)
+    int hub = kHubAuto;     // pairs with d+(x) > hub go to the CTA-table kernels (0: off; kHubAuto: set_hub)
     int hub_seg = 2048;     // hub pairs per CTA work unit
     int hub_lg = 13;        // largest CTA hash table: 2^13 slots = 32 KB
     int hub_unroll = 2;     // quads per lane in flight (2 or 4)
@@ -2908,7 +2941,8 @@ static int64_t pad_capacity(int64_t n_nodes, int64_t nnz) {
 // together.
 constexpr int kCoreWords = 4 + 2 * 256 + 1;
 constexpr int kCounters = 10;
-constexpr int kEstimates = 2;  // table_est, in front of the counters: cleared on their own
+constexpr int kEstWords = 6;  // est (an even number), in front of the counters: cleared on its own
+static_assert(kEstWords >= kEst);
 
 static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges, CountWs& W, size_t* need,
                         bool pad = true) {
@@ -2918,7 +2952,7 @@ static bool carve_count(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     // [counters][ncore][cbits]
     const size_t cb = pad ? N / 32 + 1 : 0, nc = pad ? kCoreWords : 0;
     W.zero_words = (int64_t)(2 * kCounters + nc + cb);
-    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words + 2 * kEstimates)) + kEstimates;
+    W.ctr = reinterpret_cast<unsigned long long*>(cv.take<uint32_t>((size_t)W.zero_words + 2 * kEstWords)) + kEstWords;
     W.ncore = pad ? reinterpret_cast<int32_t*>(W.ctr + kCounters) : nullptr;
     W.cbits = pad ? reinterpret_cast<uint32_t*>(W.ncore + kCoreWords) : nullptr;
     W.cnth = cv.take<int32_t>(N);
@@ -3080,8 +3114,8 @@ static int grid_edges(int64_t n) {
 
 // Before the first pass: the row table, and all counters, flags and results
 // cleared (more: words of the caller's own).
-static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_results, uint32_t* more,
-                        int64_t more_words, cudaStream_t st) {
+static int pass_prepare(CountParams& P, const CountWs& W, int64_t n_results, uint32_t* more, int64_t more_words,
+                        cudaStream_t st) {
     Prepare Q{};
     Q.row_ptr = P.row_ptr;
     Q.n_nodes = P.n_nodes;
@@ -3093,23 +3127,23 @@ static int pass_prepare(CountParams& P, const CountWs& W, int hub, int64_t n_res
     Q.has = P.has;
     Q.n_rows = P.n_rows;
     Q.zero_n[0] = W.cnth;
-    Q.zero_n[1] = hub > 0 ? W.cflag : nullptr;
+    Q.zero_n[1] = P.hub > 0 ? W.cflag : nullptr;
     Q.zero[0] = reinterpret_cast<uint32_t*>(W.ctr);
     Q.words[0] = W.zero_words;
     Q.zero[1] = reinterpret_cast<uint32_t*>(P.result);
     Q.words[1] = n_results * (int64_t)(sizeof(tchll_count_result) / 4);
     Q.zero[2] = more;
     Q.words[2] = more_words;
-    Q.hub = hub;
+    Q.hub = P.hub;
     Q.edge_u = P.edge_u;
     Q.edge_v = P.edge_v;
     Q.n_edges = P.n_edges;
-    Q.table_est = W.ctr - kEstimates;
-    TCHLL_CUDA(cudaMemsetAsync(Q.table_est, 0, kEstimates * sizeof(unsigned long long), st));
+    Q.est = W.ctr - kEstWords;
+    TCHLL_CUDA(cudaMemsetAsync(Q.est, 0, kEstWords * sizeof(unsigned long long), st));
     const int64_t sample = P.n_edges < kEdgeSample ? P.n_edges : kEdgeSample;
     prepare_kernel<<<grid_edges(P.n_nodes + 1 > sample ? P.n_nodes + 1 : sample), 256, 0, st>>>(Q);
     TCHLL_CHECK_LAUNCH("prepare_kernel");
-    P.table_est = Q.table_est;
+    P.est = Q.est;
     P.rows = W.rows;
     P.codes = W.codes;
     return TCHLL_OK;
@@ -3125,7 +3159,7 @@ static int pass_chunk(int64_t n_edges, int chunk) {
 // The first pass: `what` of PASS_HIST (hub pairs counted per table side) and
 // PASS_SHORT (all others counted for good).
 template <bool HYB>
-static int pair_pass(CountParams P, const CountWs& W, int what, int hub, unsigned long long* work, cudaStream_t st) {
+static int pair_pass(CountParams P, const CountWs& W, int what, unsigned long long* work, cudaStream_t st) {
     const bool vec = (uintptr_t)P.col_idx % 16 == 0;
     auto kern = vec ? pair_pass_kernel<HYB, true> : pair_pass_kernel<HYB, false>;
     static int bps[kMaxDevices] = {};
@@ -3145,20 +3179,19 @@ static int pair_pass(CountParams P, const CountWs& W, int what, int hub, unsigne
         const int64_t most = need > ids ? need : ids;
         if (grid > most) grid = most;
     }
-    kern<<<(int)grid, 256, 0, st>>>(P, what, hub, W.cnth);
+    kern<<<(int)grid, 256, 0, st>>>(P, what, W.cnth);
     TCHLL_CHECK_LAUNCH("pair_pass_kernel");
     return TCHLL_OK;
 }
 
 // After PASS_HIST: room for the grouped pairs, and their segments (smaller
 // hub segments in small graphs, so that every CTA gets a few).
-static int hub_alloc(const CountParams& P, const CountWs& W, int hub, int hub_seg, cudaStream_t st) {
+static int hub_alloc(const CountParams& P, const CountWs& W, int hub_seg, cudaStream_t st) {
     while (hub_seg > HUB_SEG_MIN && P.n_edges < (int64_t)hub_seg * 24 * sm_count()) hub_seg >>= 1;
     if (hub_seg < HUB_SEG_MIN) hub_seg = HUB_SEG_MIN;
     const int grid = (int)(P.n_nodes > 0 ? (P.n_nodes + 1023) / 1024 : 1);
     const PairRoom R{W.ctr + 5, W.segs, W.max_segs, W.ctr + 2, W.ctr + 7};
-    hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, W.rows, P.n_nodes, hub, hub_seg, W.offh, R, P.graph_vbase,
-                                           P.n_graphs, P.graph_bad);
+    hub_alloc_kernel<<<grid, 256, 0, st>>>(W.cnth, P, hub_seg, W.offh, R);
     TCHLL_CHECK_LAUNCH("hub_alloc_kernel");
     return TCHLL_OK;
 }
@@ -3202,8 +3235,8 @@ static bool hub_pad_usable(const CountParams& P, const CountWs& W) {
 // else 32-bit (each list kernel checks the core size on the device).  Where
 // hub pairs are rare (batches, road networks) it follows the first pass and
 // the scatter instead (`after`), and its kernels return at once without any.
-static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, int hub, bool after,
-                            const PhaseScope& ps, cudaStream_t st) {
+static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning& T, bool after, const PhaseScope& ps,
+                            cudaStream_t st) {
     if (!hub_pad_usable(P, W)) return TCHLL_OK;
     const unsigned long long* n_segs = after ? W.ctr + 2 : nullptr;
     if (ps.active()) {
@@ -3211,7 +3244,7 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
         g_phase.core_used = true;
     }
     core_mark_kernel<<<grid_rows(P.n_nodes, 256) < 8 * sm_count() ? grid_rows(P.n_nodes, 256) : 8 * sm_count(), 256, 0,
-                       st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, hub, P.nnz <= kMarkAllEdges,
+                       st>>>(P.row_ptr, P.n_nodes, P.nnz, P.col_idx, P, P.nnz <= kMarkAllEdges,
                              n_segs, W.cbits, W.cflag, P.result);
     TCHLL_CHECK_LAUNCH("core_mark_kernel");
     if (P.graph_vbase) {
@@ -3332,22 +3365,36 @@ static int launch_hub(const CountParams& P, const CountWs& W, const Tuning& T, c
     return TCHLL_OK;
 }
 
-// Hub path in use: with the packed or padded lists, or (quad loads of the
-// raw ones) a 16-byte aligned col_idx.
-// The default threshold, 128, is taken as 64 up to kHub64Edges edges: bitmap
-// lists are the faster way for pairs of 64 to 128 members too, as long as the
-// core that they bring in fits the packed lists (R-MAT 17 / 18 / 20, edge
-// factor 16 to 21: 630 / 789 / 2006 us at 128, 480 / 569 / 1719 at 64; R-MAT 22
-// with edge factor 2: 1325, 897; R-MAT 22 has a core of 108 K vertices at 128,
-// 262 K at 64).  Batches number each graph's core on its own, so the size does
-// not matter there, but they need many such pairs to a table side for the
-// core pass, which nothing overlaps, to pay: a mean forward degree of 12 (256
-// R-MAT 12, mean 19: 2.56 ms at 128, 1.85 at 64; 40 R-MAT 13, mean 10.5: 367,
-// 443 us).
-static int hub_threshold(const CountParams& P, const CountWs& W, const Tuning& T) {
-    if (T.hub <= 0 || (!hub_pad_usable(P, W) && (uintptr_t)P.col_idx % 16 != 0)) return 0;
-    const bool half = P.graph_vbase ? P.n_edges >= kHub64Degree * P.n_nodes : P.n_edges <= kHub64Edges;
-    return T.hub == kHubDefault && half ? kHubDefault / 2 : T.hub;
+// Sets P's hub threshold: 0 without the hub path, which takes the packed or
+// padded lists or, for the quad loads of the raw ones, a 16-byte aligned
+// col_idx.
+// The automatic threshold is 64 where the lists are held and their core fits
+// the packed form, else 128: bitmap lists are the faster way for pairs of 64 to
+// 128 members too, but beyond kCore16Max core vertices the 32-bit kernels
+// count (R-MAT 17, us, at 64 / 128: 318 / 367; R-MAT 22 has a core of 108 K vertices
+// at 128, 262 K at 64).  It surely fits in graphs of so few vertices and,
+// oriented by degree, of so few edges: a member of a list of over 64 has at
+// least that degree.  Up to kHub64Edges edges skewed graphs' cores fit too, and
+// the device chooses (choose).  Batches number each graph's core on its own,
+// but need many such pairs to a table side for the core pass, which nothing
+// overlaps, to pay: a mean forward degree of 12 (256 R-MAT 12, mean 23: 1,970 /
+// 2,640 us; 40 R-MAT 13, mean 13: 511 / 462); the device looks at the largest
+// graph.
+static void set_hub(CountParams& P, const CountWs& W, const Tuning& T) {
+    const bool held = hub_pad_usable(P, W);
+    P.hub_alt = 0;
+    P.hub = T.hub == kHubAuto ? kHubWide : T.hub;
+    if (!held && (uintptr_t)P.col_idx % 16 != 0) P.hub = 0;
+    if (T.hub != kHubAuto || !held) return;
+    if (P.graph_vbase) {
+        P.hub_alt = P.n_edges >= kHub64Degree * P.n_nodes;
+        if (P.hub_alt) P.hub = kHubWide / 2;
+    } else if (P.n_nodes <= kCore16Max || 2 * P.nnz < (kHubWide / 2 + 1) * (int64_t)(kCore16Max + 1)) {
+        P.hub = kHubWide / 2;
+    } else if (P.nnz <= kHub64Edges) {
+        P.hub = kHubWide / 2;
+        P.hub_alt = 1;
+    }
 }
 
 // A second stream per device for work that overlaps the caller's stream: the
@@ -3478,7 +3525,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
     if (P.n_edges == 0) return TCHLL_OK;
     // small graphs, and road networks without a long list, refuse what the hub
     // core's passes refuse in others
-    P.check_ids = (direct_pass ? (uintptr_t)P.col_idx % 16 == 0 : pairs && road) && T.hub > 0 && hub_pad_usable(P, W) &&
+    P.check_ids = (direct_pass ? (uintptr_t)P.col_idx % 16 == 0 : pairs && road) && T.hub != 0 && hub_pad_usable(P, W) &&
                   (mode == MODE_EXACT || (mode == 2 && (uintptr_t)P.regs % 16 == 0));
     if (T.pairs && !details && !prepared && P.n_edges <= kDirectEdges) P.chunk = given_chunk(P.n_edges, T.chunk);
     if (col_ready && !(mode == MODE_EXACT && pairs)) {
@@ -3486,7 +3533,8 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
         col_ready = nullptr;
     }
     int rc;
-    const int hub = hub_threshold(P, W, T);
+    set_hub(P, W, T);
+    const int hub = P.hub;
     PhaseScope ps;
     phase_reset(ps);
     switch (mode) {
@@ -3494,7 +3542,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
             if (direct_pass) {
                 P.work = nullptr;
                 phase_mark(ps, 1, st);
-                rc = sparse ? pair_pass<false>(P, W, PASS_SHORT, 0, nullptr, st) : launch_count<MODE_EXACT>(P, T, false, st);
+                rc = sparse ? pair_pass<false>(P, W, PASS_SHORT, nullptr, st) : launch_count<MODE_EXACT>(P, T, false, st);
                 phase_mark(ps, 2, st);
                 phase_used(ps, 1);
                 return rc;
@@ -3507,7 +3555,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 // after the scatter.
                 phase_mark(ps, 0, st);
                 P.chunk = pass_chunk(P.n_edges, T.chunk);
-                rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
+                rc = pass_prepare(P, W, 1, nullptr, 0, st);
                 if (rc) return rc;
                 SideFork fork;
                 const bool side = hub > 0 && T.overlap && hub_pad_usable(P, W) && !road;
@@ -3517,28 +3565,28 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                         const cudaError_t e = cudaStreamWaitEvent(fork.stream(), col_ready, 0);
                         if (e != cudaSuccess) rc = cuda_status(e, "cudaStreamWaitEvent(col_ready)");
                     }
-                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, hub, false, ps, fork.stream());
+                    if (rc == TCHLL_OK) rc = launch_core_pass(P, W, T, false, ps, fork.stream());
                     if (rc == TCHLL_OK) rc = fork.mark();
                     if (rc) return rc;
                 }
                 const bool split = col_ready != nullptr;
                 CountParams H = P;
                 if (split) H.check_ids = 0;  // col_idx is not there yet
-                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr,
+                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr,
                                       st);
-                if (rc == TCHLL_OK) rc = hub_alloc(P, W, hub, T.hub_seg, st);
+                if (rc == TCHLL_OK) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc == TCHLL_OK) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 if (split) {
                     TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
-                    rc = pair_pass<false>(P, W, PASS_SHORT, hub, W.ctr + 1, st);
+                    rc = pair_pass<false>(P, W, PASS_SHORT, W.ctr + 1, st);
                     if (rc) return rc;
                 }
                 rc = launch_table_pairs(P, W, T, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, road, ps, st);
+                    rc = side ? fork.wait_mark() : launch_core_pass(P, W, T, road, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                 }
                 phase_mark(ps, 2, st);
@@ -3573,7 +3621,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 P.hll_n = HW.hll_n;
                 phase_mark(ps, 0, st);
                 P.chunk = pass_chunk(P.n_edges, T.chunk);
-                rc = pass_prepare(P, W, hub, 1, nullptr, 0, st);
+                rc = pass_prepare(P, W, 1, nullptr, 0, st);
                 if (rc) return rc;
                 // side stream: the hub core pass (the hub kernels wait for
                 // it) and the zero masks beside the first pass, then, once
@@ -3586,25 +3634,25 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     if (rc) return rc;
                     hst = fork.stream();
                     if (core_side) {
-                        rc = launch_core_pass(P, W, T, hub, false, ps, hst);
+                        rc = launch_core_pass(P, W, T, false, ps, hst);
                         if (rc == TCHLL_OK) rc = fork.mark();
                         if (rc) return rc;
                     }
                 }
                 rc = launch_zmask(P, HW, hst);
-                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, hub, road ? nullptr : W.ctr, st);
+                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr, st);
                 if (rc == TCHLL_OK && T.overlap) rc = fork.side_waits_caller();
                 if (rc) return rc;
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[0], hst);
                 rc = launch_hll_edges(P, HW, T, hst);
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[1], hst);
-                if (rc == TCHLL_OK) rc = hub_alloc(P, W, hub, T.hub_seg, st);
+                if (rc == TCHLL_OK) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc == TCHLL_OK) rc = pairs_scatter(P, W, st);
                 if (rc == TCHLL_OK) rc = launch_table_pairs(P, W, T, st);
                 if (rc) return rc;
                 phase_mark(ps, 1, st);
                 if (hub > 0) {
-                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, hub, road, ps, st);
+                    rc = core_side ? fork.wait_mark() : launch_core_pass(P, W, T, road, ps, st);
                     if (rc == TCHLL_OK) rc = launch_hub(P, W, T, ps, st);
                     if (rc) return rc;
                 }
@@ -3621,7 +3669,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 P.hll_n = HW.hll_n;
                 phase_mark(ps, 1, st);
                 P.work = nullptr;
-                rc = sparse ? pair_pass<true>(P, W, PASS_SHORT, 0, nullptr, st)
+                rc = sparse ? pair_pass<true>(P, W, PASS_SHORT, nullptr, st)
                             : launch_count<MODE_HYB_EXACT>(P, T, false, st);
                 if (rc) return rc;
                 phase_mark(ps, 2, st);
@@ -3720,6 +3768,40 @@ TCHLL_EXPORT int tchll_exact_count_staged(const int32_t* row_ptr, int64_t n_node
                      (cudaEvent_t)col_ready_event);
 }
 
+TCHLL_EXPORT int tchll_count_hub_threshold(const int32_t* row_ptr, int64_t n_nodes, const int32_t* col_idx, int64_t nnz,
+                                           const int32_t* edge_u, const int32_t* edge_v, int64_t n_edges,
+                                           void* workspace, size_t workspace_bytes, int32_t* out, void* stream) {
+    tchll_count_result unused;
+    const int rc = check_common(row_ptr, n_nodes, col_idx, nnz, edge_u, edge_v, n_edges, &unused);
+    if (rc) return rc;
+    TCHLL_ARG(out != nullptr, "null output");
+    CountParams P{};
+    P.row_ptr = row_ptr;
+    P.n_nodes = n_nodes;
+    P.col_idx = col_idx;
+    P.nnz = nnz;
+    P.edge_u = edge_u;
+    P.edge_v = edge_v;
+    P.n_edges = n_edges;
+    const Tuning T = tuning_snapshot();
+    CountWs W;
+    size_t need = 0;
+    bool ok = carve_count(workspace, workspace_bytes, n_nodes, n_edges, W, &need, true);
+    if (!ok) ok = carve_count(workspace, workspace_bytes, n_nodes, n_edges, W, &need, false);
+    if (!ok || workspace == nullptr) {
+        set_error("workspace too small: need %zu bytes, have %zu", need, workspace_bytes);
+        return TCHLL_EWORKSPACE;
+    }
+    set_hub(P, W, T);
+    *out = P.hub;
+    if (!P.hub_alt || n_edges == 0) return TCHLL_OK;
+    unsigned long long est[kEst];
+    int r = pass_prepare(P, W, 0, nullptr, 0, (cudaStream_t)stream);
+    if (r == TCHLL_OK) r = fetch_small(est, P.est, sizeof(est), (cudaStream_t)stream);
+    if (r == TCHLL_OK) *out = choose(est, n_edges, P.hub, P.hub_alt, false).hub;
+    return r;
+}
+
 static int hybrid_common(const int32_t* row_ptr, int64_t n_nodes, const int32_t* col_idx, int64_t nnz,
                          const int32_t* edge_u, const int32_t* edge_v, int64_t n_edges, const int32_t* degrees,
                          const uint8_t* regs, int64_t n_rows, const int64_t* slot, const uint8_t* has, int32_t p,
@@ -3814,7 +3896,8 @@ TCHLL_EXPORT int tchll_set_count_table(int32_t sparse) {
 
 TCHLL_EXPORT int tchll_set_count_hub(int32_t threshold, int32_t seg_pairs, int32_t table_log2, int32_t unroll) {
     std::lock_guard<std::mutex> lock(g_tuning_mu);
-    TCHLL_ARG(threshold == 0 || threshold >= HUB_MIN, "hub threshold must be 0 (off) or >= %d", HUB_MIN);
+    TCHLL_ARG(threshold == kHubAuto || threshold == 0 || threshold >= HUB_MIN,
+              "hub threshold must be -1 (automatic), 0 (off) or >= %d", HUB_MIN);
     TCHLL_ARG(seg_pairs >= HUB_SEG_MIN && seg_pairs <= (1 << 20), "seg_pairs must be in [%d, 2^20]", HUB_SEG_MIN);
     TCHLL_ARG(table_log2 >= 10 && table_log2 <= 15, "table_log2 must be in [10, 15]");
     TCHLL_ARG(unroll == 2 || unroll == 4, "unroll must be 2 or 4");
@@ -4076,10 +4159,11 @@ __global__ void chunk_fill_kernel(const int32_t* __restrict__ row_ptr, const int
 }
 
 // *bad (zeroed before) = n_graphs less the first malformed graph, 0 when there
-// is none; without edges (row_ptr null) only the vertex ranges count.
+// is none; *largest the vertices of the largest graph, if more than the packed
+// lists' core.  Without edges (row_ptr null) only the vertex ranges count.
 __global__ void check_vbase_kernel(const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ vbase,
                                    int64_t n_graphs, int64_t n_nodes, int64_t n_edges, unsigned long long* bad,
-                                   tchll_count_result* results) {
+                                   unsigned long long* largest, tchll_count_result* results) {
     for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n_graphs;
          g += (int64_t)gridDim.x * blockDim.x) {
         int64_t s0, s1;
@@ -4090,7 +4174,11 @@ __global__ void check_vbase_kernel(const int32_t* __restrict__ row_ptr, const in
             const int32_t a = vbase[g], b = vbase[g + 1];
             ok = a >= 0 && b >= a && (int64_t)b <= n_nodes;
         }
-        if (ok) continue;
+        if (ok) {
+            const int32_t n = vbase[g + 1] - vbase[g];
+            if (largest && n > kCore16Max) atomicMax(largest, (unsigned long long)n);
+            continue;
+        }
         results[g].status |= ST_BAD_ROW;
         if (bad) atomicMax(bad, (unsigned long long)(n_graphs - g));
     }
@@ -4179,7 +4267,7 @@ static int check_vbase(const CountParams& P, const int32_t* vbase, int64_t n_gra
     int64_t g = (n_graphs + 255) / 256;
     if (g > 1024) g = 1024;
     check_vbase_kernel<<<(int)g, 256, 0, st>>>(P.n_edges > 0 ? P.row_ptr : nullptr, vbase, n_graphs, P.n_nodes,
-                                               P.n_edges, P.graph_bad, P.result);
+                                               P.n_edges, P.graph_bad, P.est ? P.est + 4 : nullptr, P.result);
     TCHLL_CHECK_LAUNCH("check_vbase_kernel");
     return TCHLL_OK;
 }
@@ -4223,14 +4311,15 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     phase_mark(ps, 0, st);
     // one pass over each graph's edges as given; pairs with a long table side
     // go to the hub kernels, which publish per segment into the graph of x
-    const int hub = hub_threshold(P, B.cw, T);
-    rc = pass_prepare(P, B.cw, hub, n_graphs, reinterpret_cast<uint32_t*>(B.ghub), (int64_t)(B.flag_bytes / 4), st);
+    set_hub(P, B.cw, T);
+    const int hub = P.hub;
+    rc = pass_prepare(P, B.cw, n_graphs, reinterpret_cast<uint32_t*>(B.ghub), (int64_t)(B.flag_bytes / 4), st);
     if (rc == TCHLL_OK) rc = check_vbase(P, vbase, n_graphs, st);
     if (rc == TCHLL_OK) rc = build_chunks(P, vbase, n_graphs, B, T.chunk, st);
     if (rc) return rc;
     if (hll_list || !hybrid) {
-        if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, hub, B.cw.ctr, st);
-        else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, hub, B.cw.ctr, st);
+        if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
+        else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
         if (rc) return rc;
     } else {
         P.work = B.cw.ctr;
@@ -4239,14 +4328,14 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     }
     const bool grouped = hll_list || !hybrid;
     if (grouped) {
-        rc = hub_alloc(P, B.cw, hub, T.hub_seg, st);
+        rc = hub_alloc(P, B.cw, T.hub_seg, st);
         if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
         if (rc == TCHLL_OK) rc = launch_table_pairs(P, B.cw, T, st);
         if (rc) return rc;
     }
     phase_mark(ps, 1, st);
     if (hub > 0 && grouped) {
-        rc = launch_core_pass(P, B.cw, T, hub, true, ps, st);
+        rc = launch_core_pass(P, B.cw, T, true, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
     }
