@@ -108,6 +108,8 @@ struct CountParams {
     int32_t* graph_hub;          // batched calls: what the first pass left for later, GRAPH_*
     int32_t* live_flag;          // batched calls: 1 for 64 rows that touch such a graph
     int32_t* live_list;          // and those blocks of 64 rows, listed
+    int32_t* n_live;             // how many
+    int32_t* big_hist;           // batched calls: 512 words per slot of a big graph (core_bucket_big_kernel)
     // Table pairs (count_kernel with SEGS): their segments, the first one right
     // before segs_end, the second before that; edge_v holds the probe sides
     const PairSeg* segs_end;
@@ -336,14 +338,15 @@ constexpr int32_t kCore16Max = 131070;
 // the threshold, and with hub_alt leaves it to the device to double it; what
 // the device goes by is est: {sampled pairs with a list in (kTableList, hub]
 // and more than kTableProbes probes, lists of that length, the same two for
-// (hub, 2 hub], vertices of a batch's largest graph}.  It is doubled where half
+// (hub, 2 hub], vertices of a batch's largest graph, whether a batch has a big
+// graph (kBigGraph)}.  It is doubled where half
 // of all pairs have lists in (kTableList, 2 hub], because evenly long lists bring
 // all vertices into the core (a batch's largest graph permitting; batches of
 // more than kHub64Edges edges always, when that graph's core may not fit).
 // Whole calls, us, at 64 / at 128: Erdos-Renyi with 300 K vertices and 24 M edges
 // 3,277 / 2,930, 300 K vertices joined to 50 near ones 1,487 / 1,129; R-MAT 20, one
 // pair in ten, 1,590 / 1,800, R-MAT 22 with edge factor 2 895 / 1,013.
-constexpr int kEst = 5;
+constexpr int kEst = 6;
 constexpr int64_t kHub64Edges = 28000000;
 struct Choice {
     int hub, table;
@@ -1391,7 +1394,12 @@ __global__ void __launch_bounds__(256) core_index_kernel(const uint32_t* __restr
 
 // Batched counts: a CTA per graph numbers that graph's core on its own (two
 // lists of a pair are the same graph's), so a batch's many small cores fit
-// the packed lists whatever their sum; C is the largest graph's.
+// the packed lists whatever their sum; C is the largest graph's.  A CTA takes
+// about 2 us per 1024 vertices, so graphs from kBigGraph on are numbered by many
+// (R-MAT 22 as a batch of one: 12.6 ms by one CTA, 8.7 so).
+constexpr int32_t kBigShift = 15;
+constexpr int32_t kBigGraph = 1 << kBigShift;
+constexpr int32_t kBigTile = 4096;
 __global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* __restrict__ bits, int32_t* cnt_cidx,
                                                                 int64_t n_nodes, const int32_t* __restrict__ vbase,
                                                                 const int32_t* __restrict__ graph_hub,
@@ -1402,6 +1410,7 @@ __global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* 
     const int tid = threadIdx.x, lane = tid & 31;
     const int32_t lo = __ldg(vbase + blockIdx.x), hi = __ldg(vbase + blockIdx.x + 1);
     if (lo < 0 || hi < lo || (int64_t)hi > n_nodes) return;  // flagged by check_vbase_kernel
+    if (hi - lo >= kBigGraph) return;                        // core_index_big_kernel
     if (tid < 256) h[tid] = 0;
     __syncthreads();
     for (int32_t w = lo + tid; w < hi; w += 1024) {
@@ -1432,6 +1441,86 @@ __global__ void __launch_bounds__(1024) core_index_batch_kernel(const uint32_t* 
         const int b = pop_bucket(bits, cnt_cidx, w);
         cnt_cidx[w] = b >= 0 ? atomicAdd(h + b, 1) : -1;
     }
+}
+
+// The big graphs of a batch: a CTA per kBigTile vertices.  The graphs there
+// that are big are those of the tile's first and last vertex at most.  A big
+// graph's bucket sizes and cursors are in big_hist, at the slot that its first
+// vertex gives it (no two big graphs begin within kBigGraph vertices).
+template <class F>
+__device__ __forceinline__ void for_big_graphs(const CountParams& P, F f) {
+    const int64_t lo = blockIdx.x * (int64_t)kBigTile, hi = min(P.n_nodes, lo + kBigTile);
+    const int32_t* __restrict__ vbase = P.graph_vbase;
+    const int64_t good = P.n_graphs - (int64_t)*P.graph_bad;
+    int64_t last = -1;
+    for (int k = 0; k < 2; ++k) {  // CTA-uniform
+        const int64_t g = graph_of(vbase, P.n_graphs, P.graph_bad, (int32_t)(k == 0 ? lo : hi - 1));
+        if (g == last || g >= good) continue;
+        last = g;
+        const int64_t a = __ldg(vbase + g), b = __ldg(vbase + g + 1);
+        if (b - a < kBigGraph || (P.graph_hub[g] & GRAPH_HUB) == 0) continue;
+        f(max(a, lo), min(b, hi), a, P.big_hist + 512 * (a >> kBigShift));
+    }
+}
+
+__global__ void __launch_bounds__(256) core_bucket_big_kernel(const uint32_t* __restrict__ bits,
+                                                              const int32_t* __restrict__ cnt, const CountParams P,
+                                                              const unsigned long long* __restrict__ n_segs) {
+    __shared__ int h[256];
+    if (*n_segs == 0 || P.est[5] == 0) return;  // grid-uniform: no big graph
+    const int tid = threadIdx.x;
+    for_big_graphs(P, [&](int64_t a, int64_t b, int64_t first, int32_t* hist) {
+        h[tid] = 0;
+        __syncthreads();
+        for (int64_t w = a + tid; w < b; w += 256) {
+            const int k = pop_bucket(bits, cnt, w);
+            if (k >= 0) atomicAdd(h + k, 1);
+            if (((w & 63) == 0 || w == first) && atomicExch(P.live_flag + (w >> 6), 1) == 0)
+                P.live_list[atomicAdd(P.n_live, 1)] = (int32_t)(w >> 6);
+        }
+        __syncthreads();
+        if (h[tid]) atomicAdd(hist + tid, h[tid]);
+        __syncthreads();
+    });
+}
+
+__global__ void __launch_bounds__(256) core_index_big_kernel(const uint32_t* __restrict__ bits, int32_t* cnt_cidx,
+                                                             const CountParams P,
+                                                             const unsigned long long* __restrict__ n_segs,
+                                                             int32_t* n_core) {
+    __shared__ int h[256], part[8];
+    if (*n_segs == 0 || P.est[5] == 0) return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    for_big_graphs(P, [&](int64_t a, int64_t b, int64_t first, int32_t* hist) {
+        h[tid] = 0;
+        __syncthreads();
+        for (int64_t w = a + tid; w < b; w += 256) {
+            const int k = pop_bucket(bits, cnt_cidx, w);
+            if (k >= 0) atomicAdd(h + k, 1);
+        }
+        const int mine = __ldg(hist + tid);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) part[tid >> 5] = incl;
+        __syncthreads();
+        int before = 0;
+        for (int i = 0; i < (tid >> 5); ++i) before += part[i];
+        const int n_here = h[tid];
+        const int base = before + incl - mine + (n_here ? atomicAdd(hist + 256 + tid, n_here) : 0);
+        if (a == first && tid == 255) atomicMax(n_core, before + incl);
+        __syncthreads();
+        h[tid] = base;
+        __syncthreads();
+        for (int64_t w = a + tid; w < b; w += 256) {
+            const int k = pop_bucket(bits, cnt_cidx, w);
+            cnt_cidx[w] = k >= 0 ? atomicAdd(h + k, 1) : -1;
+        }
+        __syncthreads();
+    });
 }
 
 // Packed probe lists (used when C <= kCore16Max; core_pad_kernel writes the
@@ -3252,6 +3341,13 @@ static int launch_core_pass(const CountParams& P, const CountWs& W, const Tuning
                                                                  P.graph_hub, P.live_flag, P.live_list,
                                                                  W.ncore + kCoreWords - 1, W.ncore);
         TCHLL_CHECK_LAUNCH("core_index_batch_kernel");
+        if (P.n_nodes >= kBigGraph) {
+            const int tiles = (int)((P.n_nodes + kBigTile - 1) / kBigTile);
+            core_bucket_big_kernel<<<tiles, 256, 0, st>>>(W.cbits, W.cflag, P, n_segs);
+            TCHLL_CHECK_LAUNCH("core_bucket_big_kernel");
+            core_index_big_kernel<<<tiles, 256, 0, st>>>(W.cbits, W.cflag, P, n_segs, W.ncore);
+            TCHLL_CHECK_LAUNCH("core_index_big_kernel");
+        }
     } else {
         int64_t gv = (P.n_nodes + 1023) / 1024;
         gv = gv < 1 ? 1 : (gv > 4 * (int64_t)sm_count() ? 4 * (int64_t)sm_count() : gv);
@@ -4177,6 +4273,7 @@ __global__ void check_vbase_kernel(const int32_t* __restrict__ row_ptr, const in
         if (ok) {
             const int32_t n = vbase[g + 1] - vbase[g];
             if (largest && n > kCore16Max) atomicMax(largest, (unsigned long long)n);
+            if (largest && n >= kBigGraph) largest[1] = 1;
             continue;
         }
         results[g].status |= ST_BAD_ROW;
@@ -4196,7 +4293,8 @@ struct BatchWs {
     int32_t* ghub;    // n_graphs: the graph has hub pairs
     int32_t* rflag;   // n_nodes / 64 + 1: 64 rows touch such a graph
     int32_t* rlist;   // those blocks
-    size_t flag_bytes;  // of ghub and rflag, which are next to each other
+    int32_t* big;     // 512 words per kBigGraph vertices
+    size_t flag_bytes;  // of ghub, rflag and big, which are next to each other
     void* tmp;
     size_t tmp_bytes;
 };
@@ -4222,10 +4320,12 @@ static bool carve_batch(void* ws, size_t bytes, int64_t n_nodes, int64_t n_edges
     B.cgraph = cv.take<int32_t>(MC);
     B.codes = cv.take<uint2>((size_t)(n_edges > 0 ? n_edges : 1) / 32 + MC + 1);
     const size_t RL = (size_t)(n_nodes > 0 ? n_nodes : 0) / 64 + 1;
-    B.flag_bytes = (G + RL) * sizeof(int32_t);
-    B.ghub = cv.take<int32_t>(G + 2 * RL);
+    const size_t BG = 512 * ((size_t)(n_nodes > 0 ? n_nodes : 0) / kBigGraph + 1);
+    B.flag_bytes = (G + RL + BG) * sizeof(int32_t);
+    B.ghub = cv.take<int32_t>(G + 2 * RL + BG);
     B.rflag = B.ghub + G;
-    B.rlist = B.rflag + RL;
+    B.big = B.rflag + RL;
+    B.rlist = B.big + BG;
     B.tmp_bytes = tb;
     B.tmp = cv.take<char>(tb);
     const size_t E = (size_t)(n_edges > 0 ? n_edges : 1);
@@ -4297,6 +4397,8 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     P.graph_hub = B.ghub;
     P.live_flag = B.rflag;
     P.live_list = B.rlist;
+    P.n_live = B.cw.ncore + kCoreWords - 1;
+    P.big_hist = B.big;
     int rc;
     if (P.n_edges == 0) return check_vbase(P, vbase, n_graphs, st);
     PhaseScope ps;
