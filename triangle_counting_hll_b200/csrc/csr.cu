@@ -528,63 +528,97 @@ __global__ void small_scatter_kernel(const unsigned long long* __restrict__ tabl
 }
 
 // Sorts the rows in[row_ptr[r] .. row_ptr[r + 1]) (distinct values) into
-// col_idx and edge_v and writes edge_u; a warp per row.  Up to 64 members: each
-// lane counts, for its two, the members below them; longer rows: a bitonic
-// sort in the warp's shared memory.
-__global__ void __launch_bounds__(128) small_sort_kernel(const int32_t* __restrict__ row_ptr, int64_t n,
+// col_idx and edge_v and writes edge_u; a warp takes `per` (1 or 32) rows at a
+// time.  Up to 4 members: a lane sorts its row in registers; up to 64: each lane
+// counts, for its two, the members below them; longer rows: a bitonic sort in
+// the warp's shared memory.  (4 M rows of at most a few members: 962 us with a
+// warp per row, 60 so; few and long rows want a warp each.)
+__device__ __forceinline__ void order(int32_t& a, int32_t& b) {
+    const int32_t lo = min(a, b);
+    b = max(a, b);
+    a = lo;
+}
+__global__ void __launch_bounds__(128) small_sort_kernel(const int32_t* __restrict__ row_ptr, int64_t n, int per,
                                                          const int32_t* __restrict__ in, int32_t* col_idx,
                                                          int32_t* edge_u, int32_t* edge_v) {
     __shared__ int32_t buf[4][kSmallRow];
     const int lane = threadIdx.x & 31;
     int32_t* b = buf[threadIdx.x >> 5];
+    const int32_t none = 0x7FFFFFFF;  // above every rank
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
-        const int32_t s = __ldg(row_ptr + r), d = __ldg(row_ptr + r + 1) - s;
-        if (d <= 64) {
-            const int32_t none = 0x7FFFFFFF;  // above every rank
-            const int32_t x0 = lane < d ? __ldg(in + s + lane) : none;
-            const int32_t x1 = 32 + lane < d ? __ldg(in + s + 32 + lane) : none;
-            int r0 = 0, r1 = 0;
-            for (int i = 0; i < d; ++i) {
-                const int32_t y = i < 32 ? __shfl_sync(0xFFFFFFFFu, x0, i) : __shfl_sync(0xFFFFFFFFu, x1, i - 32);
-                r0 += y < x0;
-                r1 += y < x1;
-            }
-            if (lane < d) {
-                col_idx[s + r0] = x0;
-                edge_v[s + r0] = x0;
-                edge_u[s + lane] = (int32_t)r;
-            }
-            if (32 + lane < d) {
-                col_idx[s + r1] = x1;
-                edge_v[s + r1] = x1;
-                edge_u[s + 32 + lane] = (int32_t)r;
-            }
-            continue;
+    for (int64_t r0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * per; r0 < n; r0 += warps * per) {
+        int32_t my_s = 0, my_d = 0;
+        if (lane < per && r0 + lane < n) {
+            my_s = __ldg(row_ptr + r0 + lane);
+            my_d = __ldg(row_ptr + r0 + lane + 1) - my_s;
         }
-        int m = 128;  // the next power of two
-        while (m < d) m <<= 1;
-        __syncwarp();
-        for (int i = lane; i < m; i += 32) b[i] = i < d ? __ldg(in + s + i) : 0x7FFFFFFF;
-        __syncwarp();
-        for (int k = 2; k <= m; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int t = lane; t < m / 2; t += 32) {
-                    const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
-                    const int32_t x = b[lo], y = b[hi];
-                    if ((x > y) == ((lo & k) == 0)) {
-                        b[lo] = y;
-                        b[hi] = x;
-                    }
+        if (my_d > 0 && my_d <= 4) {
+            int32_t x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = i < my_d ? __ldg(in + my_s + i) : none;
+            order(x[0], x[1]);
+            order(x[2], x[3]);
+            order(x[0], x[2]);
+            order(x[1], x[3]);
+            order(x[1], x[2]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (i < my_d) {
+                    col_idx[my_s + i] = x[i];
+                    edge_v[my_s + i] = x[i];
+                    edge_u[my_s + i] = (int32_t)(r0 + lane);
                 }
-                __syncwarp();
             }
         }
-        for (int i = lane; i < d; i += 32) {
-            const int32_t x = b[i];
-            col_idx[s + i] = x;
-            edge_v[s + i] = x;
-            edge_u[s + i] = (int32_t)r;
+        for (unsigned todo = __ballot_sync(0xFFFFFFFFu, my_d > 4); todo; todo &= todo - 1) {
+            const int k = __ffs(todo) - 1;
+            const int32_t s = __shfl_sync(0xFFFFFFFFu, my_s, k), d = __shfl_sync(0xFFFFFFFFu, my_d, k);
+            const int64_t r = r0 + k;
+            if (d <= 64) {
+                const int32_t x0 = lane < d ? __ldg(in + s + lane) : none;
+                const int32_t x1 = 32 + lane < d ? __ldg(in + s + 32 + lane) : none;
+                int c0 = 0, c1 = 0;
+                for (int i = 0; i < d; ++i) {
+                    const int32_t y = i < 32 ? __shfl_sync(0xFFFFFFFFu, x0, i) : __shfl_sync(0xFFFFFFFFu, x1, i - 32);
+                    c0 += y < x0;
+                    c1 += y < x1;
+                }
+                if (lane < d) {
+                    col_idx[s + c0] = x0;
+                    edge_v[s + c0] = x0;
+                    edge_u[s + lane] = (int32_t)r;
+                }
+                if (32 + lane < d) {
+                    col_idx[s + c1] = x1;
+                    edge_v[s + c1] = x1;
+                    edge_u[s + 32 + lane] = (int32_t)r;
+                }
+                continue;
+            }
+            int m = 128;  // the next power of two
+            while (m < d) m <<= 1;
+            __syncwarp();
+            for (int i = lane; i < m; i += 32) b[i] = i < d ? __ldg(in + s + i) : none;
+            __syncwarp();
+            for (int k2 = 2; k2 <= m; k2 <<= 1) {
+                for (int j = k2 >> 1; j > 0; j >>= 1) {
+                    for (int t = lane; t < m / 2; t += 32) {
+                        const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
+                        const int32_t x = b[lo], y = b[hi];
+                        if ((x > y) == ((lo & k2) == 0)) {
+                            b[lo] = y;
+                            b[hi] = x;
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            for (int i = lane; i < d; i += 32) {
+                const int32_t x = b[i];
+                col_idx[s + i] = x;
+                edge_v[s + i] = x;
+                edge_u[s + i] = (int32_t)r;
+            }
         }
     }
 }
@@ -782,9 +816,10 @@ TCHLL_EXPORT int tchll_csr_build_phase2(int64_t n_raw, int64_t n_nodes, int64_t 
         TCHLL_CHECK_LAUNCH("small_rows_kernel");
         small_scatter_kernel<<<grid_n(slots), 256, 0, st>>>(table, slots, W.deg, rank, W.fdeg, W.cb);
         TCHLL_CHECK_LAUNCH("small_scatter_kernel");
-        int64_t g = (n_nodes + 3) / 4;
-        if (g > (int64_t)sm_count() * 7) g = (int64_t)sm_count() * 7;
-        small_sort_kernel<<<(int)g, 128, 0, st>>>(row_ptr, n_nodes, W.cb, col_idx, edge_u, edge_v);
+        const int64_t warps = 4 * (int64_t)sm_count() * 7;
+        const int per = n_nodes >= 32 * warps ? 32 : 1;
+        const int64_t g = per == 32 ? warps / 4 : (n_nodes + 3) / 4 < warps / 4 ? (n_nodes + 3) / 4 : warps / 4;
+        small_sort_kernel<<<(int)g, 128, 0, st>>>(row_ptr, n_nodes, per, W.cb, col_idx, edge_u, edge_v);
         TCHLL_CHECK_LAUNCH("small_sort_kernel");
         return TCHLL_OK;
     }
