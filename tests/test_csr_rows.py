@@ -25,3 +25,18 @@ def test_many_short_rows_and_some_long(tchll, oracle, n, spread):
     order = rng.permutation(len(u))
     assert len(u) < 1 << 21
     _check(oracle, u[order], v[order])
+
+
+# one id in every edge, first or last or all over; one pair; few pairs, often
+@pytest.mark.parametrize("kind", ["star", "star of the last", "star among others", "one pair", "few pairs"])
+@pytest.mark.parametrize("n_raw", [33, 5000, 300_000])
+def test_popular_ids_and_repeated_edges(tchll, oracle, kind, n_raw):
+    rng = np.random.default_rng(n_raw)
+    at = np.arange(n_raw)
+    u, v = {"star": (0 * at, at + 1), "star of the last": (at, 0 * at + n_raw + 7),
+            "star among others": (np.where(at % 2, 3, rng.integers(0, n_raw, n_raw)), rng.integers(0, n_raw, n_raw)),
+            "one pair": (0 * at + 4, 0 * at + 2), "few pairs": (at % 5, at % 3)}[kind]
+    order = rng.permutation(n_raw)
+    for o in (at, order):
+        _check(oracle, u[o], v[o])
+        _check(oracle, v[o] * 5000 % (2**31 - 1), u[o] * 5000 % (2**31 - 1))

@@ -363,37 +363,68 @@ __global__ void small_ends_kernel(const int32_t* __restrict__ ru, const int32_t*
     }
 }
 
+// Whether several neighbouring lanes hold the same x (called by whole warps).
+// Comparing all lanes at every step would cost R-MAT 17 several percent.
+template <class T>
+__device__ __forceinline__ bool lanes_repeat(T x, bool in) {
+    const T other = __shfl_xor_sync(0xFFFFFFFFu, x, 1);  // every lane takes part
+    return __popc(__ballot_sync(0xFFFFFFFFu, in && x == other)) >= 4;
+}
+
+// Adds 1 to deg[id] of every lane with id >= 0, lanes of one id with one atomic
+// where they repeat: a popular id would queue up.
+__device__ __forceinline__ void add_same(int32_t* deg, int32_t id, int lane) {
+    if (!lanes_repeat(id, id >= 0)) {
+        if (id >= 0) atomicAdd(deg + id, 1);
+        return;
+    }
+    const unsigned same = __match_any_sync(0xFFFFFFFFu, id);
+    if (id >= 0 && lane == __ffs(same) - 1) atomicAdd(deg + id, __popc(same));
+}
+
 // cnt[0] += unique pairs; deg[id]: undirected degrees.  With nodes (sorted,
-// cnt[1] of them) an id stands for its place there.
+// cnt[1] of them) an id stands for its place there.  Of a warp's lanes with
+// the same pair one goes to the table (a list of few pairs repeated often
+// would queue up on their slots; reading a slot before claiming it costs every
+// other list a second trip: R-MAT 17 433 -> 502 us).
 __global__ void small_insert_kernel(const int32_t* __restrict__ ru, const int32_t* __restrict__ rv, int64_t n,
                                     const uint32_t* __restrict__ nodes, unsigned long long* table, uint32_t slots,
                                     int32_t* deg, int64_t* cnt) {
     uint32_t fresh = 0;
+    const int lane = threadIdx.x & 31;
     const int64_t nn = nodes ? n_real_nodes(nodes, cnt) : 0;
-    GRID_STRIDE(i, n) {
-        int32_t u = ru[i], v = rv[i];
-        if (u == v) continue;  // negative ids never get here
-        if (nodes) {
+    WARP_GRID_STRIDE(i, n) {
+        int32_t u = -1, v = -1;
+        if (i < n) {
+            u = ru[i];  // negative ids never get here
+            v = rv[i];
+        }
+        bool mine = u != v;
+        if (mine && nodes) {
             u = (int32_t)lower_bound_u32(nodes, nn, (uint32_t)u);
             v = (int32_t)lower_bound_u32(nodes, nn, (uint32_t)v);
         }
-        const uint64_t key = ((uint64_t)(uint32_t)min(u, v) << 32) | (uint32_t)max(u, v);
-        uint32_t s = pair_slot(key, slots);
-        bool mine = false;
-        for (uint32_t k = 0; k < slots; ++k) {  // at most half the slots ever fill
-            const unsigned long long old = atomicCAS(table + s, kEmptySlot, key);
-            mine = old == kEmptySlot;
-            if (mine || old == key) break;
-            s = s + 1 < slots ? s + 1 : 0;
+        const unsigned long long key =
+            mine ? ((unsigned long long)(uint32_t)min(u, v) << 32) | (uint32_t)max(u, v) : kEmptySlot;
+        if (lanes_repeat(key, mine)) {  // warp-uniform
+            const unsigned same = __match_any_sync(0xFFFFFFFFu, key);
+            if (lane != __ffs(same) - 1) mine = false;
         }
         if (mine) {
-            ++fresh;
-            atomicAdd(deg + u, 1);
-            atomicAdd(deg + v, 1);
+            uint32_t s = pair_slot(key, slots);
+            for (uint32_t k = 0; k < slots; ++k) {  // at most half the slots ever fill
+                const unsigned long long old = atomicCAS(table + s, kEmptySlot, key);
+                mine = old == kEmptySlot;
+                if (mine || old == key) break;
+                s = s + 1 < slots ? s + 1 : 0;
+            }
         }
+        fresh += mine;
+        add_same(deg, mine ? u : -1, lane);
+        add_same(deg, mine ? v : -1, lane);
     }
     fresh = __reduce_add_sync(0xFFFFFFFFu, fresh);
-    if ((threadIdx.x & 31) == 0 && fresh) atomicAdd((unsigned long long*)cnt, (unsigned long long)fresh);
+    if (lane == 0 && fresh) atomicAdd((unsigned long long*)cnt, (unsigned long long)fresh);
 }
 
 // Tiles of 1024 entries, 256 threads: how many entries count (FLAG: 1 per
