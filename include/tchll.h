@@ -381,7 +381,10 @@ int tchll_degree_stats(const int32_t* degrees, const int32_t* row_ptr, int64_t n
  * Negative ids are TCHLL_EINVAL via sizes[0] = -1.  Phase 1 waits for the
  * stream once, early, to read the largest id (16 bytes): it sets the width of
  * the sort keys and, when ids 0 .. max fit twice n_raw entries, lets a direct
- * rank table replace the sort of all endpoints.
+ * rank table replace the sort of all endpoints.  Lists of up to 2^21 edges are
+ * built with a hash table instead, unless they have more than 2^17 edges and
+ * 256 to an id; phase 2 reads the largest id once more where it takes that to
+ * tell (more than 2^17 edges, 256 to a vertex).
  */
 int tchll_csr_workspace_bytes(int64_t n_raw, size_t* bytes);
 int tchll_csr_build_phase1(const int32_t* raw_u, const int32_t* raw_v, int64_t n_raw, int64_t* sizes,

@@ -40,3 +40,13 @@ def test_popular_ids_and_repeated_edges(tchll, oracle, kind, n_raw):
     for o in (at, order):
         _check(oracle, u[o], v[o])
         _check(oracle, v[o] * 5000 % (2**31 - 1), u[o] * 5000 % (2**31 - 1))
+
+
+# few ids in many edges, on both sides of the line, with and without unused ids
+@pytest.mark.parametrize("n_raw", [(1 << 17), (1 << 17) + 1, 200_000])
+@pytest.mark.parametrize("ids", [512, 513, 700, 900])
+@pytest.mark.parametrize("step", [1, 7, 100_000])
+def test_dense_lists(tchll, oracle, n_raw, ids, step):
+    rng = np.random.default_rng(ids + n_raw)
+    u, v = rng.integers(0, ids, n_raw) * step, rng.integers(0, ids, n_raw) * step
+    _check(oracle, u, v)

@@ -345,7 +345,16 @@ static int bits_for(int64_t maxv) {
 // Whole builds, sorted / so: R-MAT 10, 13, 15, 16, 17 (16 K, 90 K, 524 K, 1 M, 2 M
 // raw edges) 197 / 119, 236 / 138, 281 / 208, 343 / 289, 507 / 437 us; bound by
 // launches and the two read-backs, then by the atomics on the popular ids.
+// Lists of more than kDenseRaw edges with kDenseEnds and more to an id go by
+// sorting all the same: their few counters are contended whatever the order,
+// and their rows are long (clique of 1,000 / 1,400 / 2,000 vertices, by sorting / by
+// table: 270 / 311, 315 / 470, 402 / 627 us; of 300: 209 / 155).
 constexpr int64_t kSmallRaw = 1 << 21;
+constexpr int64_t kDenseRaw = 1 << 17;
+constexpr int64_t kDenseEnds = 256;
+__host__ __device__ __forceinline__ bool small_route(int64_t n_raw, int64_t max_id) {
+    return n_raw <= kSmallRaw && (n_raw <= kDenseRaw || n_raw < kDenseEnds * (max_id + 1));
+}
 constexpr int kSmallRow = 2048;
 constexpr uint64_t kEmptySlot = ~0ull;
 
@@ -750,7 +759,7 @@ TCHLL_EXPORT int tchll_csr_build_phase1(const int32_t* raw_u, const int32_t* raw
         return TCHLL_OK;
     }
     const int64_t max_id = hc[1];
-    if (n_raw <= kSmallRaw) {
+    if (small_route(n_raw, max_id)) {
         // deg in W.deg (cleared above), rank in W.e1, nodes in W.e0, tile sums
         // in W.fdeg
         const bool places = max_id + 1 > 2 * (int64_t)R;
@@ -832,7 +841,15 @@ TCHLL_EXPORT int tchll_csr_build_phase2(int64_t n_raw, int64_t n_nodes, int64_t 
         return TCHLL_EWORKSPACE;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (n_edges > 0 && n_raw <= kSmallRaw) {
+    bool small = n_raw <= kSmallRaw;
+    if (small && n_edges > 0 && n_raw > kDenseRaw && n_raw >= kDenseEnds * n_nodes) {
+        // phase 1 may have sorted (it goes by the largest id, which is at least n_nodes - 1)
+        int64_t max_id = 0;
+        const int rf = fetch_small(&max_id, W.cnt + 3, sizeof(max_id), st);
+        if (rf) return rf;
+        small = small_route(n_raw, max_id);
+    }
+    if (n_edges > 0 && small) {
         TCHLL_ARG(n_nodes > 1, "sizes out of range");
         const int64_t slots = 2 * n_raw, tiles = (n_nodes + 1023) / 1024;
         const unsigned long long* table = reinterpret_cast<const unsigned long long*>(W.k0);
