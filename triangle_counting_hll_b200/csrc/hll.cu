@@ -51,6 +51,57 @@ __device__ __forceinline__ void sketch_list(uint32_t* words, const int32_t* __re
     }
 }
 
+// The lists of over kCtaList members, where a warp takes a vertex: a CTA each
+// (one list of 1.5 M members, p = 10: 8.8 ms by a warp, 1.2 so).  A launch of its own, 8
+// us on R-MAT 22, because the same within sketch_kernel costs it registers and
+// every build 5%.  Lists oriented by degree are that long from 2^27 edges on.
+constexpr int kCtaList = 16384;
+template <bool DENSE>
+__global__ void __launch_bounds__(kSketchThreads)
+    sketch_long_kernel(const int32_t* __restrict__ row_ptr, int64_t n_nodes, const int32_t* __restrict__ col_idx,
+                       const int64_t* __restrict__ keys, int64_t nnz, int64_t theta, int p,
+                       const int64_t* __restrict__ slot, int64_t n_rows, uint8_t* rows) {
+    extern __shared__ __align__(16) uint32_t words[];
+    __shared__ int64_t list[4 * kSketchThreads];
+    __shared__ int n_list;
+    uint4* w4 = reinterpret_cast<uint4*>(words);
+    const int m16 = 1 << (p - 4);
+    constexpr int64_t kTile = 4 * kSketchThreads;
+    for (int64_t base = blockIdx.x * kTile; base < n_nodes; base += gridDim.x * kTile) {
+        bool mine[4];
+        bool any = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t u = base + i * kSketchThreads + threadIdx.x;
+            mine[i] = false;
+            if (u < n_nodes) {
+                const int32_t rs = __ldg(row_ptr + u), re = __ldg(row_ptr + u + 1);
+                mine[i] = rs >= 0 && re >= rs && (int64_t)re <= nnz && re - rs > kCtaList &&
+                          (DENSE ? (int64_t)(re - rs) >= theta : slot[u] >= 0 && slot[u] < n_rows);
+            }
+            any |= mine[i];
+        }
+        if (!__syncthreads_or(any)) continue;
+        if (threadIdx.x == 0) n_list = 0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (mine[i]) list[atomicAdd(&n_list, 1)] = base + i * kSketchThreads + threadIdx.x;
+        __syncthreads();
+        for (int t = 0; t < n_list; ++t) {
+            const int64_t u = list[t];
+            uint4* row4 = reinterpret_cast<uint4*>(rows + ((DENSE ? u : slot[u]) << p));
+            for (int i = threadIdx.x; i < m16; i += kSketchThreads) w4[i] = DENSE ? row4[i] : make_uint4(0u, 0u, 0u, 0u);
+            __syncthreads();
+            sketch_list<DENSE>(words, col_idx, keys, n_nodes, __ldg(row_ptr + u), __ldg(row_ptr + u + 1), p, threadIdx.x,
+                               kSketchThreads);
+            __syncthreads();
+            for (int i = threadIdx.x; i < m16; i += kSketchThreads) row4[i] = w4[i];
+            __syncthreads();
+        }
+    }
+}
+
 // A CTA's tile is 32 groups of 8 consecutive vertices, the groups spread
 // evenly over the vertex range: sketched vertices cluster (at low ids in
 // R-MAT graphs), and 256 consecutive ones could all be sketched while most
@@ -89,7 +140,7 @@ __global__ void __launch_bounds__(kSketchThreads)
                 const int64_t s = slot[u];
                 flag = s >= 0 && s < n_rows;
             }
-            flag = flag && rs >= 0 && re >= rs && (int64_t)re <= nnz;
+            flag = flag && rs >= 0 && re >= rs && (int64_t)re <= nnz && (!WARP || re - rs <= kCtaList);
         }
         const unsigned bal = __ballot_sync(FULL, flag);
         if (lane == 0) warp_cnt[wid] = __popc(bal);
@@ -239,6 +290,12 @@ static int launch_sketch(const int32_t* row_ptr, int64_t n, const int32_t* col_i
     if (g > tiles) g = tiles;
     kern<<<(int)g, kSketchThreads, smem, st>>>(row_ptr, n, col_idx, keys, nnz, theta, p, has, slot, n_rows, rows);
     TCHLL_CHECK_LAUNCH("sketch_kernel");
+    if (warp && nnz > kCtaList) {
+        const int64_t gl = (n + 4 * kSketchThreads - 1) / (4 * kSketchThreads), most = (int64_t)sm_count() * 8;
+        sketch_long_kernel<DENSE><<<(int)(gl < most ? gl : most), kSketchThreads, (size_t)1 << p, st>>>(
+            row_ptr, n, col_idx, keys, nnz, theta, p, slot, n_rows, rows);
+        TCHLL_CHECK_LAUNCH("sketch_long_kernel");
+    }
     return TCHLL_OK;
 }
 
