@@ -51,3 +51,28 @@ def test_skewed_graphs(tchll):
     b = batch.GraphBatch.from_edge_lists(graphs)
     csrs = [core.csr_from_edges(u, v) for u, v, _ in graphs]
     assert np.array_equal(b.exact_counts(), batch.plain_exact_counts(csrs))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 8])
+def test_register_rows_at_any_byte(tchll, shift):
+    """Register rows that do not start on 16 bytes: the same result blocks, and
+    the pairs of long lists still go by the hub kernels."""
+    import torch
+    from triangle_counting_hll_b200 import _lib, batch, core
+    graphs = [(*core.gen_rmat(s, 16, seed=s), 1 << s) for s in (9, 13, 14)]
+    b = batch.GraphBatch.from_edge_lists(graphs)
+    rows, slot = b.sketches(100, 8)
+    buf = torch.empty(rows.numel() + shift, dtype=torch.uint8, device="cuda")
+    buf[shift:] = rows
+    blocks = []
+    core.set_phase_timing(True)
+    try:
+        for r in (rows, buf[shift:]):
+            res = torch.zeros(3 * _lib.RESULT_BYTES, dtype=torch.uint8, device="cuda")
+            b.hybrid_launch(res, r, slot, 8, 100)
+            assert core.phase_times()["hub"] is not None
+            blocks.append(res.cpu())
+    finally:
+        core.set_phase_timing(False)
+    assert torch.equal(blocks[0], blocks[1])
+    assert batch.hybrid_from_results(blocks[0], 3)[1]["n_approx"].sum() > 0

@@ -699,15 +699,17 @@ __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, 
             }
             if (HYB) {
                 const bool hll = ok && wants && both;
-                n_fallback += __popc(__ballot_sync(FULL, ok && wants && !both));
-                // HLL edges wait in the warp's buffer: one atomic on the shared
-                // counter per 128 or so
-                const unsigned m = __ballot_sync(FULL, hll);
-                if (hll) hbuf[n_hll + __popc(m & (lane_le >> 1))] = make_int2(u, v);
-                n_hll += __popc(m);
-                if (n_hll > kHllBuf - 32) {
-                    flush_hll(P, hbuf, n_hll, lane);
-                    n_hll = 0;
+                if (P.hll_u) {  // uniform; else another launch looks for the HLL edges, and counts n_fallback
+                    n_fallback += __popc(__ballot_sync(FULL, ok && wants && !both));
+                    // HLL edges wait in the warp's buffer: one atomic on the shared
+                    // counter per 128 or so
+                    const unsigned m = __ballot_sync(FULL, hll);
+                    if (hll) hbuf[n_hll + __popc(m & (lane_le >> 1))] = make_int2(u, v);
+                    n_hll += __popc(m);
+                    if (n_hll > kHllBuf - 32) {
+                        flush_hll(P, hbuf, n_hll, lane);
+                        n_hll = 0;
+                    }
                 }
                 ok = ok && !hll;
             }
@@ -4419,24 +4421,14 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     if (rc == TCHLL_OK) rc = check_vbase(P, vbase, n_graphs, st);
     if (rc == TCHLL_OK) rc = build_chunks(P, vbase, n_graphs, B, T.chunk, st);
     if (rc) return rc;
-    if (hll_list || !hybrid) {
-        if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
-        else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
-        if (rc) return rc;
-    } else {
-        P.work = B.cw.ctr;
-        rc = launch_count<MODE_HYB_EXACT>(P, T, false, st);
-        if (rc) return rc;
-    }
-    const bool grouped = hll_list || !hybrid;
-    if (grouped) {
-        rc = hub_alloc(P, B.cw, T.hub_seg, st);
-        if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
-        if (rc == TCHLL_OK) rc = launch_table_pairs(P, B.cw, T, st);
-        if (rc) return rc;
-    }
+    if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
+    else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
+    if (rc == TCHLL_OK) rc = hub_alloc(P, B.cw, T.hub_seg, st);
+    if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
+    if (rc == TCHLL_OK) rc = launch_table_pairs(P, B.cw, T, st);
+    if (rc) return rc;
     phase_mark(ps, 1, st);
-    if (hub > 0 && grouped) {
+    if (hub > 0) {
         rc = launch_core_pass(P, B.cw, T, true, ps, st);
         if (rc == TCHLL_OK) rc = launch_hub(P, B.cw, T, ps, st, true);
         if (rc) return rc;
