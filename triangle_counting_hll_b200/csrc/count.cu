@@ -3250,20 +3250,22 @@ static int pass_chunk(int64_t n_edges, int chunk) {
 // The first pass: `what` of PASS_HIST (hub pairs counted per table side) and
 // PASS_SHORT (all others counted for good).
 template <bool HYB>
-static int pair_pass(CountParams P, const CountWs& W, int what, unsigned long long* work, cudaStream_t st) {
+static int pair_pass(CountParams P, const CountWs& W, const Tuning& T, int what, unsigned long long* work,
+                     cudaStream_t st) {
     const bool vec = (uintptr_t)P.col_idx % 16 == 0;
     auto kern = vec ? pair_pass_kernel<HYB, true> : pair_pass_kernel<HYB, false>;
-    static int bps[kMaxDevices] = {};
+    static std::atomic<int> fit[2][kMaxDevices] = {};  // per kernel
     const int dev = current_device();
     if (dev < 0) return cuda_status(cudaErrorInvalidDevice, "cudaGetDevice");
-    if (bps[dev] == 0) {
-        int b = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 256, 0);
+    int bps = T.blocks_per_sm > 0 ? T.blocks_per_sm : fit[vec][dev].load();
+    if (bps == 0) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kern, 256, 0);
         if (e != cudaSuccess) return cuda_status(e, "occupancy(pair_pass_kernel)");
-        bps[dev] = b < 1 ? 1 : b;
+        if (bps < 1) bps = 1;
+        fit[vec][dev].store(bps);
     }
     P.work = work;
-    int64_t grid = (int64_t)sm_count() * bps[dev];
+    int64_t grid = (int64_t)sm_count() * bps;
     if (!P.chunk_start) {  // no more warps than chunks
         const int64_t need = (P.n_edges + 8 * (int64_t)P.chunk - 1) / (8 * (int64_t)P.chunk);
         const int64_t ids = P.check_ids ? (P.n_nodes > P.nnz / 4 ? P.n_nodes : P.nnz / 4) / 1024 + 1 : 1;
@@ -3640,7 +3642,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
             if (direct_pass) {
                 P.work = nullptr;
                 phase_mark(ps, 1, st);
-                rc = sparse ? pair_pass<false>(P, W, PASS_SHORT, nullptr, st) : launch_count<MODE_EXACT>(P, T, false, st);
+                rc = sparse ? pair_pass<false>(P, W, T, PASS_SHORT, nullptr, st) : launch_count<MODE_EXACT>(P, T, false, st);
                 phase_mark(ps, 2, st);
                 phase_used(ps, 1);
                 return rc;
@@ -3670,14 +3672,14 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 const bool split = col_ready != nullptr;
                 CountParams H = P;
                 if (split) H.check_ids = 0;  // col_idx is not there yet
-                rc = pair_pass<false>(H, W, split ? PASS_HIST : PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr,
+                rc = pair_pass<false>(H, W, T, split ? PASS_HIST : PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr,
                                       st);
                 if (rc == TCHLL_OK) rc = hub_alloc(P, W, T.hub_seg, st);
                 if (rc == TCHLL_OK) rc = pairs_scatter(P, W, st);
                 if (rc) return rc;
                 if (split) {
                     TCHLL_CUDA(cudaStreamWaitEvent(st, col_ready, 0));
-                    rc = pair_pass<false>(P, W, PASS_SHORT, W.ctr + 1, st);
+                    rc = pair_pass<false>(P, W, T, PASS_SHORT, W.ctr + 1, st);
                     if (rc) return rc;
                 }
                 rc = launch_table_pairs(P, W, T, st);
@@ -3738,7 +3740,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                     }
                 }
                 rc = launch_zmask(P, HW, hst);
-                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr, st);
+                if (rc == TCHLL_OK) rc = pair_pass<true>(P, W, T, PASS_HIST | PASS_SHORT, road ? nullptr : W.ctr, st);
                 if (rc == TCHLL_OK && T.overlap) rc = fork.side_waits_caller();
                 if (rc) return rc;
                 if (ps.active()) cudaEventRecord(g_phase.hll_ev[0], hst);
@@ -3767,7 +3769,7 @@ static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_
                 P.hll_n = HW.hll_n;
                 phase_mark(ps, 1, st);
                 P.work = nullptr;
-                rc = sparse ? pair_pass<true>(P, W, PASS_SHORT, nullptr, st)
+                rc = sparse ? pair_pass<true>(P, W, T, PASS_SHORT, nullptr, st)
                             : launch_count<MODE_HYB_EXACT>(P, T, false, st);
                 if (rc) return rc;
                 phase_mark(ps, 2, st);
@@ -4421,8 +4423,8 @@ static int run_batch(CountParams P, bool hybrid, const int32_t* vbase, int64_t n
     if (rc == TCHLL_OK) rc = check_vbase(P, vbase, n_graphs, st);
     if (rc == TCHLL_OK) rc = build_chunks(P, vbase, n_graphs, B, T.chunk, st);
     if (rc) return rc;
-    if (hybrid) rc = pair_pass<true>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
-    else rc = pair_pass<false>(P, B.cw, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
+    if (hybrid) rc = pair_pass<true>(P, B.cw, T, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
+    else rc = pair_pass<false>(P, B.cw, T, PASS_HIST | PASS_SHORT, B.cw.ctr, st);
     if (rc == TCHLL_OK) rc = hub_alloc(P, B.cw, T.hub_seg, st);
     if (rc == TCHLL_OK) rc = pairs_scatter(P, B.cw, st);
     if (rc == TCHLL_OK) rc = launch_table_pairs(P, B.cw, T, st);
