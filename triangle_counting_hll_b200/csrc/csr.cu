@@ -61,29 +61,38 @@ struct CsrWs {
     size_t tmp_bytes;
 };
 
-// (the same call asks three times per build: the last answer of the thread is kept)
+// (a build asks three times: the thread's last answer is kept, with the device
+// it is for, as the sizes may depend on it, and only if all queries succeeded)
 static size_t csr_cub_tmp(int64_t n_raw) {
     static thread_local int64_t last_n = -1;
+    static thread_local int last_dev = -1;
     static thread_local size_t last_bytes = 0;
-    if (n_raw == last_n) return last_bytes;
+    const int dev = current_device();
+    if (n_raw == last_n && dev == last_dev && dev >= 0) return last_bytes;
     const int R = (int)(n_raw > 0 ? n_raw : 1);
     size_t a = 0, b = 0, c = 0, d = 0, e = 0, f = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, a, (uint64_t*)nullptr, (uint64_t*)nullptr, R, 0, 63);
-    cub::DeviceSelect::Unique(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t*)nullptr, R);
-    cub::DeviceRadixSort::SortKeys(nullptr, c, (uint32_t*)nullptr, (uint32_t*)nullptr, 2 * R, 0, 32);
-    cub::DeviceSelect::Unique(nullptr, d, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t*)nullptr, 2 * R);
-    cub::DeviceScan::ExclusiveSum(nullptr, e, thrust::make_transform_iterator((int32_t*)nullptr, Occurs()),
-                                  (int32_t*)nullptr, 2 * R + 1);
-    cub::DeviceRadixSort::SortPairs(nullptr, f, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
-                                    (uint32_t*)nullptr, R, 0, 32);
+    const cudaError_t rc[6] = {
+        cub::DeviceRadixSort::SortKeys(nullptr, a, (uint64_t*)nullptr, (uint64_t*)nullptr, R, 0, 63),
+        cub::DeviceSelect::Unique(nullptr, b, (uint64_t*)nullptr, (uint64_t*)nullptr, (int64_t*)nullptr, R),
+        cub::DeviceRadixSort::SortKeys(nullptr, c, (uint32_t*)nullptr, (uint32_t*)nullptr, 2 * R, 0, 32),
+        cub::DeviceSelect::Unique(nullptr, d, (uint32_t*)nullptr, (uint32_t*)nullptr, (int64_t*)nullptr, 2 * R),
+        cub::DeviceScan::ExclusiveSum(nullptr, e, thrust::make_transform_iterator((int32_t*)nullptr, Occurs()),
+                                      (int32_t*)nullptr, 2 * R + 1),
+        cub::DeviceRadixSort::SortPairs(nullptr, f, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
+                                        (uint32_t*)nullptr, R, 0, 32)};
+    bool ok = true;
+    for (const cudaError_t r : rc) ok &= r == cudaSuccess;
     size_t m = a;
     if (b > m) m = b;
     if (c > m) m = c;
     if (d > m) m = d;
     if (e > m) m = e;
     if (f > m) m = f;
-    last_n = n_raw;
-    last_bytes = m;
+    if (ok) {
+        last_n = n_raw;
+        last_dev = dev;
+        last_bytes = m;
+    }
     return m;
 }
 
