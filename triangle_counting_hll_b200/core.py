@@ -380,7 +380,7 @@ def phase_times() -> dict:
     hub = (C.c_float * 2)()
     check(load().tchll_phase_hub_ms(C.cast(hub, C.c_void_p)))
     res["hub"] = float(hub[0]) if hub[0] >= 0 else None        # hub kernels, part of "count"
-    res["hub_core"] = float(hub[1]) if hub[1] >= 0 else None   # core pass before them, part of "count"
+    res["hub_core"] = float(hub[1]) if hub[1] >= 0 else None   # core pass, beside "pairs" on the second stream (overlap)
     return res
 
 

@@ -69,7 +69,7 @@ struct PairSeg {
 struct CountParams {
     const int32_t* row_ptr;
     const int2* rows;  // the row table, or null
-    uint2* codes;      // per 32 edges of the first pass: {hub pairs, of them those with x = u} (with rows)
+    uint2* codes;      // per 32 edges of the first pass: {grouped pairs, those with x = u} (with rows)
     int64_t n_nodes;
     const int32_t* col_idx;
     int64_t nnz;
@@ -405,8 +405,8 @@ __device__ __forceinline__ void append_hll(const CountParams& P, bool hll, int32
     }
 }
 
-// Hub pairs' probe sides, grouped by table side: py[cursor[x] ...).  Which
-// edges are hub pairs and which end is x comes from the first pass, two bits
+// The grouped pairs' probe sides, by table side: py[cursor[x] ...).  Which
+// edges they are and which end is x comes from the first pass, two bits
 // per edge, so no row is looked up again (R-MAT 22: 1.12 ms with the rows looked up again, 0.81 so).
 __device__ __forceinline__ void scatter_step(const CountParams& P, int64_t e, uint2 code, int32_t* cursor, int32_t* py,
                                              int lane) {
@@ -587,9 +587,9 @@ __global__ void prepare_kernel(const Prepare Q) {
 }
 
 // The first pass over the edges.  Pairs with a long table side (hub pairs)
-// are counted per table side in cnth, for the hub kernels; every other pair
-// is counted here and now, by looking each member of its shorter list up in
-// the longer one by binary search.  A warp takes 32 edges at a time and deals
+// are counted per table side in cnth, for the hub kernels, and so are table
+// pairs (is_table_pair); every other pair is counted here and now, by looking
+// each member of its shorter list up in the longer one by binary search.  A warp takes 32 edges at a time and deals
 // their probe members to its lanes as one stream (two windows of 32 in
 // flight), so lists of any length keep the lanes busy; a search touches the
 // few lines of one short list, mostly in L1.  No table has to be built, so
@@ -631,13 +631,14 @@ __device__ __forceinline__ void pass_publish(tchll_count_result* R, uint64_t acc
     }
 }
 
-template <bool HYB, bool VEC, int UNR = 2>
+template <bool HYB, bool VEC>
 __global__ void __launch_bounds__(256, 6) pair_pass_kernel(const CountParams P, int what,
                                                            int32_t* __restrict__ cnth) {
     __shared__ int4 s_list[8][32];
     __shared__ int32_t s_len[8][32];
     __shared__ int2 s_hll[HYB ? 8 : 1][HYB ? kHllBuf : 1];
     const int lane = threadIdx.x & 31;
+    constexpr int UNR = 2;  // windows of 32 look-ups in flight
     int4* lst = s_list[threadIdx.x >> 5];
     int32_t* len = s_len[threadIdx.x >> 5];
     int2* hbuf = s_hll[HYB ? threadIdx.x >> 5 : 0];
@@ -2602,14 +2603,16 @@ __device__ __forceinline__ double hll_estimate_from(U128 zsum, double extra, uin
 // (coalesced loads, no lane idling while one group reads two whole rows),
 // so narrow groups cost nothing when a few of their edges need the
 // registers; smaller rows are read by the edge's own group.
-// CACHE: each group takes a contiguous run of the edge list.  The routing
-// pass appends edges in CSR order, so consecutive HLL edges mostly share u,
-// and the group keeps u's zero mask in registers across them (up to four
-// 16-byte words per lane) and, with CROW (rows of at most 8 16-byte words
-// per lane), u's register row too: an edge then reads only v's mask and
-// row.  Otherwise the groups stride over the list.
-// ZS (p >= 11, masks too long for four words per lane): u's mask stays in a
-// shared-memory slot per group.  Slots are kZsPad 16-byte words apart beyond
+// CACHE (p >= 11, or CROW): each group takes a contiguous run of the edge
+// list.  The routing pass appends edges in CSR order, so consecutive HLL edges
+// mostly share u, and the group keeps u's zero mask across them: in a
+// shared-memory slot (ZS: p = 11 to 14 at the default widths), in registers
+// where it is at most four 16-byte words per lane (wider groups, by tuning);
+// at p = 15 and 16, too long for either, it is read per edge.  With CROW (rows
+// of at most 8 16-byte words per lane) u's register row stays in registers too:
+// an edge then reads only v's mask and row.  Otherwise the groups stride over
+// the list.
+// ZS:  Slots are kZsPad 16-byte words apart beyond
 // their length, so that the groups that one load instruction serves in one
 // phase (8 lanes) read different banks.  A variant of its own keeps the
 // register form's 16 words out of it (64 registers, four CTAs per SM): with
@@ -2999,9 +3002,9 @@ struct CountWs {
     // ncore and cbits one run of zero_words words
     unsigned long long* ctr;
     int64_t zero_words;
-    int32_t* cnth;            // n_nodes + 1 (histogram of hub pairs)
+    int32_t* cnth;            // n_nodes + 1 (histogram of grouped pairs)
     int32_t* offh;            // n_nodes + 1 (scan, then scatter cursor)
-    int32_t* py;              // n_edges (probe sides of the hub pairs, by table side)
+    int32_t* py;              // n_edges (probe sides of the grouped pairs, by table side)
     int2* rows;               // n_nodes: the row table
     uint2* codes;             // n_edges / 32 + 1 (batches: their own)
     PairSeg* segs;             // max_segs
@@ -3121,7 +3124,7 @@ static int launch_hll_edges_L(HllParams H, bool crow, cudaStream_t st) {
     if (H.zm && crow && L * 8 >= ((1 << H.p) >> 4)) hll_edges_kernel<L, true, true, true, false><<<grid, 256, 0, st>>>(H);
     else if (H.zm && H.p >= 11) {
         // masks too large for the 4 register words per lane go to shared
-        // memory, one slot per group, while that fits 96 KB per CTA
+        // memory, one slot per group, while that fits 104 KB per CTA
         const int nq = H.zst >> 2;
         const size_t smem = nq > 4 * L ? (size_t)(256 / L) * (nq + kZsPad<L>) * sizeof(uint4) : 0;
         if (smem > 0 && smem <= (104u << 10)) {
@@ -3247,7 +3250,7 @@ static int pass_chunk(int64_t n_edges, int chunk) {
     return chunk < 32 ? 32 : chunk & ~31;
 }
 
-// The first pass: `what` of PASS_HIST (hub pairs counted per table side) and
+// The first pass: `what` of PASS_HIST (grouped pairs counted per table side) and
 // PASS_SHORT (all others counted for good).
 template <bool HYB>
 static int pair_pass(CountParams P, const CountWs& W, const Tuning& T, int what, unsigned long long* work,
@@ -3576,7 +3579,7 @@ class SideFork {
 };
 
 // col_ready (exact counts only; null = ready): an event the kernels that
-// read col_idx wait for, so the regrouping of the hub pairs (row_ptr and the
+// read col_idx wait for, so the grouping of hub and table pairs (row_ptr and the
 // edges only) overlaps a copy of col_idx still in flight.
 static int run_count(CountParams P, int mode, bool details, void* ws, size_t ws_bytes, cudaStream_t st,
                      cudaEvent_t col_ready = nullptr) {
@@ -4294,7 +4297,7 @@ struct BatchWs {
     int32_t* clen;
     int32_t* cgraph;
     uint2* codes;     // n_edges / 32 + max chunks + 1
-    int32_t* ghub;    // n_graphs: the graph has hub pairs
+    int32_t* ghub;    // n_graphs: GRAPH_*
     int32_t* rflag;   // n_nodes / 64 + 1: 64 rows touch such a graph
     int32_t* rlist;   // those blocks
     int32_t* big;     // 512 words per kBigGraph vertices
