@@ -2383,6 +2383,7 @@ __global__ void __launch_bounds__(256) hub_alloc_kernel(const int32_t* __restric
             mine[1] += is_hub[i] ? (unsigned long long)n : (unsigned long long)n << 32;
         }
     }
+    if (!__syncthreads_or(mine[0] != 0)) return;  // nothing grouped here, as in most of a batch or a road network
     unsigned long long incl[2] = {mine[0], mine[1]};
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
