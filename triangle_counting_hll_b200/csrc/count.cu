@@ -1547,8 +1547,8 @@ __global__ void __launch_bounds__(256) core_index_big_kernel(const uint32_t* __r
 // Why bitmaps: a key costs a random 4-byte shared load (3.8 wavefronts per
 // 32), a bitmap unit one conflict-free 16-byte one for 128 columns; ordered
 // by popularity, the low columns are dense enough for that on every skewed
-// graph (R-MAT 22: 58 M hub pairs probe 11.5 G keys = 1.47 G key units;
-// with bitmaps about 0.4 G bitmap + 0.7 G key units).  B is one of a few
+// graph (R-MAT 22: 58 M hub pairs probe 11.5 G keys = 1.49 G key units;
+// with bitmaps 0.29 G bitmap + 0.81 G key units).  B is one of a few
 // sizes up to 32, chosen per row by kUnitCost per bitmap unit against kKeyCost per
 // unit of 8 keys.  The L1 pipe alone would put the ratio at 0.35, but the
 // list loads weigh in: hub kernel on R-MAT 22 with 8, 11, 14, 18, 24, 30 to 34:
